@@ -1,0 +1,122 @@
+"""The row kernels that work in pieces of eight elements against the same operators an element at a time: one operand
+moved off its 16-byte boundary takes the general form.  Both compute in f32; they differ in the order of sums over at most
+8192 values (relative error below 1e-6 of a statistic), so f32 results agree to 2e-6 and bf16 ones to a rounding."""
+
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BF16, F32, I32, I64 = torch.bfloat16, torch.float32, torch.int32, torch.int64
+TYPES = [F32, BF16]
+
+
+@pytest.fixture(scope="module")
+def ops():
+    import tilert_b200 as tb
+    from tilert_b200 import gqa_ops
+
+    tb.load_backend("ralasun")
+    tb.tilert_init(0, "ralasun")
+    yield gqa_ops
+    assert tb.device_status(0, "ralasun") == 0
+
+
+def rnd(seed, *shape, std=1.0, mean=0.0, dtype=F32):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * std + mean).to(dtype).cuda()
+
+
+def moved(t):
+    """The same values one element off a 16-byte boundary, with the same strides."""
+    buf = torch.zeros(t.numel() + 8, dtype=t.dtype, device=t.device)
+    v = buf[1: 1 + t.numel()].view(t.shape)
+    v.copy_(t)
+    return v
+
+
+def same(name, a, b):
+    a, b = a.double(), b.double()
+    # bf16: half a unit in the last place apart at most where f32 values differ by an ulp, 2^-8 of the value
+    lim = 2e-6 if name.endswith("f32") else 2.0 ** -8
+    assert float((a - b).abs().max()) <= lim * float(b.abs().max()), name
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("dim", [8, 256, 2048, 2056, 4096, 4104, 8192])
+def test_residual_and_embedding(ops, dtype, dim):
+    rows, top, t = 5, 3, "f32" if dtype == F32 else "bf16"
+    y, add, x0 = rnd(0, rows, dim, mean=3.0), rnd(1, dim), rnd(2, rows, dim)
+    n1, n2 = (ops.Norm(rnd(s, dim), rnd(s + 1, dim), centered=True) for s in (3, 5))
+    gain = rnd(7, dim)
+    ye, ysh = rnd(8, rows * top, dim, dtype=dtype), rnd(9, rows, dim, dtype=dtype)
+    slot = torch.randperm(rows * top, generator=torch.Generator().manual_seed(1)).to(I32).view(rows, top).cuda()
+    w = rnd(10, rows, top)
+    forms = [dict(norm=n1, y=y, add=add, norm2=n2), dict(norm=n1, y=y), dict(norm=None, add=add, norm2=n2),
+             dict(norm=gain, experts=ye, slot_row=slot, slot_w=w, shared=ysh), dict(norm=gain, experts=ye, slot_row=slot, slot_w=w)]
+    for i, f in enumerate(forms):
+        out = []
+        for general in (False, True):
+            x, xh = x0.clone(), torch.zeros(rows, dim, dtype=dtype, device="cuda")
+            if general:
+                x = moved(x)
+            ops.residual_norm(x, None if i == 1 and dtype == F32 else xh, eps=1e-5, dim=dim, rows=rows, **f)
+            out.append((x.clone(), xh))
+        same(f"x of form {i}, f32", out[0][0], out[1][0])
+        same(f"xh of form {i}, {t}", out[0][1], out[1][1])
+    table, toks = rnd(11, 9, dim, dtype=BF16), torch.tensor([8, 0, 3], device="cuda")
+    for g in (gain, None):
+        out = []
+        for general in (False, True):
+            x, xh = torch.zeros(3, dim, device="cuda"), torch.zeros(3, dim, dtype=dtype, device="cuda")
+            ops.embed_norm(toks, table, g, 1e-5, dim, moved(x) if general else x, xh)
+            out.append(xh)
+            if not general:
+                assert torch.equal(x.to(dtype), xh)
+        same(f"embedding, {t}", *out)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(3, 1, 8, 24), (8, 2, 96, 64), (16, 16, 128, 128), (64, 8, 128, 256)])
+def test_queries_keys_values(ops, dtype, heads, kv_heads, dim, vdim):
+    rows, ring, pos, t = 7, 16, 12, "f32" if dtype == F32 else "bf16"
+    mix = types.SimpleNamespace(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim)
+    qkv, qg, kg = rnd(0, rows, heads * dim + kv_heads * (dim + vdim)), rnd(1, heads * dim), rnd(2, kv_heads * dim)
+    lam, first, cur = torch.tensor([0.3], device="cuda"), rnd(3, rows, kv_heads * vdim), torch.tensor([pos], dtype=I32, device="cuda")
+    for mode in (ops.VMIX_NONE, ops.VMIX_FIRST, ops.VMIX_BLEND):
+        out = []
+        for general in (False, True):
+            vf = torch.zeros_like(first) if mode == ops.VMIX_FIRST else first
+            cache = types.SimpleNamespace(k=torch.zeros(kv_heads, ring, ops.pad(dim, 16), dtype=dtype, device="cuda"),
+                                          v=torch.zeros(kv_heads, ring, ops.pad(vdim, 16), dtype=dtype, device="cuda"), ring=ring)
+            q = torch.zeros(rows, heads, ops.pad(dim, 16), dtype=dtype, device="cuda")
+            ops.qkv_rows(qkv, moved(qg) if general else qg, kg, 1e-5, mode, lam, vf, rows, mix, cache, cur, q)
+            out.append((q, cache.k, cache.v, vf.to(dtype)))
+        for name, a, b in zip(("q", "k", "v", "first"), *out):
+            same(f"{name}, mode {mode}, {t}", a, b)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("heads,dim,rot,rank,q_rank", [(1, 8, 16, 8, 8), (5, 96, 32, 72, 304), (16, 128, 64, 512, 1536), (3, 40, 128, 1024, 24)])
+def test_latents_and_queries(ops, dtype, interleaved, heads, dim, rot, rank, q_rank):
+    rows, ring, pos, t = 6, 9, 40, "f32" if dtype == F32 else "bf16"
+    mix = types.SimpleNamespace(heads=heads, dim=dim, rot_dim=rot, vdim=64, kv_rank=rank)
+    rope = ops.Rotation(ops.rotation_table(1e4, rot, 64, "cuda"), interleaved)
+    cur, ldh = torch.tensor([pos], dtype=I32, device="cuda"), dim + rot
+    z, qg, cg = rnd(0, rows, q_rank + rank + rot), rnd(1, q_rank), rnd(2, rank)
+    q = rnd(3, rows, heads * ldh)
+    out = []
+    for general in (False, True):
+        cache = types.SimpleNamespace(rows=torch.zeros(ring, ops.latent_row_len(rank, rot), dtype=dtype, device="cuda"), ring=ring)
+        cq = torch.zeros(rows, q_rank, dtype=dtype, device="cuda")
+        ops.latent_tokens(z, q_rank, q_rank + rank, q_rank, moved(qg) if general else qg, cg, 1e-5, rows, mix, rope, cache, cur, cq)
+        src = moved(q) if general else q
+        wide = torch.zeros(rows, heads, ops.pad(dim, 16) + ops.pad(rot, 16), dtype=dtype, device="cuda")
+        ops.latent_queries(src, rows, mix, rope, cur, wide)
+        qn, lat = torch.zeros(heads, rows, dim, dtype=dtype, device="cuda"), torch.zeros(heads, rows, ops.latent_row_len(rank, rot), device="cuda")
+        ops.latent_queries(src, rows, mix, rope, cur, qn, lat)
+        out.append((cache.rows, cq, wide, qn, lat))
+    for name, a, b in zip(("cache", "cq", "expanded", "absorbed", "rotated"), *out):
+        same(f"{name}, {'f32' if name == 'rotated' else t}", a, b)

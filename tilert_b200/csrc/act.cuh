@@ -31,6 +31,15 @@ __device__ __forceinline__ void act_ld8(const float* p, float (&f)[8]) {
   f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
+// and back
+__device__ __forceinline__ void act_st8(__nv_bfloat16* p, const float (&f)[8]) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+__device__ __forceinline__ void act_st8(float* p, const float (&f)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+
 // Sum over the CTA (up to 32 warps); `red` holds 32 floats, every thread gets the sum.
 __device__ __forceinline__ float cta_sum(float v, float* red) {
   const int lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;

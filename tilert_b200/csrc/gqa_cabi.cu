@@ -6,6 +6,7 @@
 #include <cuda.h>
 
 #include <cmath>
+#include <initializer_list>
 #include <mutex>
 
 #include "host_util.h"
@@ -165,6 +166,25 @@ extern "C" int tilert_gqa_residual_norm_op(TgContext* ctx, const float* y, long 
   TB_REQUIRE((gain2 == nullptr || xh != nullptr) && (bias2 == nullptr || gain2 != nullptr));
   TB_REQUIRE(y != nullptr ? ldy >= dim
                           : (ye == nullptr || (slot_row != nullptr && slot_w != nullptr && top >= 1 && stride_ok(lde, dim) && aligned16(ye) &&
+namespace {
+
+// Whether rows of `dim` elements can be held as pieces of eight: whole pieces, as many as the threads have room for,
+// every operand (null where there is none) 16-byte aligned with strides of whole pieces.
+bool row_pieces(int dim, std::initializer_list<const void*> operands, std::initializer_list<long long> strides) {
+  bool ok = dim % 8 == 0 && dim <= kRowThreads * 8 * kRowPieces;
+  for (const void* o : operands) ok = ok && aligned16(o);
+  for (long long ld : strides) ok = ok && ld % 8 == 0;
+  return ok;
+}
+// The instance with just enough threads and pieces: 2048, 4096 or 8192 elements.
+template <class P>
+int by_pieces(int dim, int rows, void* stream, const P& p, void (*narrow)(P), void (*one)(P), void (*two)(P)) {
+  const int half = kRowThreads / 2;
+  return go(dim <= half * 8 ? narrow : (dim <= kRowThreads * 8 ? one : two), dim3(rows), dim3(dim <= half * 8 ? half : kRowThreads), 0, stream, p);
+}
+
+}  // namespace
+
                                                (ysh == nullptr || (stride_ok(ldsh, dim) && aligned16(ysh))))));
   const ResidualNormParams p{y,    ldy, ye,    lde,   slot_row, slot_w, top, ysh, ldsh, gain, bias,
                              add,  gain2, bias2, centered, eps, dim,    x,   ldx, xh,   ldh};
@@ -172,6 +192,12 @@ extern "C" int tilert_gqa_residual_norm_op(TgContext* ctx, const float* y, long 
   if (f32) return go(residual_norm_kernel<float>, dim3(rows), dim3(kNormThreads), smem, stream, p);
   return go(residual_norm_kernel<__nv_bfloat16>, dim3(rows), dim3(kNormThreads), smem, stream, p);
 }
+  if (row_pieces(dim, {table, gain, x, xh}, {ld_table, ldx, ldh})) {
+    return f32 ? by_pieces(dim, rows, stream, p, embed_norm_pieces_kernel<float, 256, 1>, embed_norm_pieces_kernel<float, 512, 1>,
+                           embed_norm_pieces_kernel<float, 512, 2>)
+               : by_pieces(dim, rows, stream, p, embed_norm_pieces_kernel<__nv_bfloat16, 256, 1>, embed_norm_pieces_kernel<__nv_bfloat16, 512, 1>,
+                           embed_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
+  }
 
 extern "C" int tilert_gqa_gather_norm_op(TgContext* ctx, const float* x, long long ldx, const int* rows, int n, const float* gain,
                                          const float* bias, int centered, float eps, int dim, void* out, long long ldo, int f32, void* stream) {
@@ -189,6 +215,12 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
   TB_REQUIRE(ctx != nullptr && x != nullptr && w != nullptr && out != nullptr);
   TB_REQUIRE(rows >= 1 && n >= 1 && k >= 1 && n_groups >= 0 && n_groups <= kMaxGroups);
   TB_REQUIRE(stride_ok(ldx, k) && stride_ok(ldw, k) && ldo >= n && aligned16(x) && aligned16(w));
+  if (row_pieces(dim, {y, ye, ysh, gain, bias, add, gain2, bias2, x, xh}, {ldy, lde, ldsh, ldx, ldh})) {
+    return f32 ? by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<float, 256, 1>, residual_norm_pieces_kernel<float, 512, 1>,
+                           residual_norm_pieces_kernel<float, 512, 2>)
+               : by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<__nv_bfloat16, 256, 1>,
+                           residual_norm_pieces_kernel<__nv_bfloat16, 512, 1>, residual_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
+  }
   TB_REQUIRE(bias == nullptr || (n_groups == 0 && !gated));
   const int per = gated ? 2 : 1;
   TB_REQUIRE(static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n < (1ll << 31) - 256);
@@ -269,6 +301,8 @@ int run_prefill_attn(const AttnPrefillParams& p, void* stream) {
   const dim3 grid((p.rows + tpb - 1) / tpb, p.s.kv_heads * ((group + hpb - 1) / hpb));
   if (p.s.vdimp <= 64) return launch_prefill_attn<4>(p, grid, stream);
   if (p.s.vdimp <= 128) return launch_prefill_attn<8>(p, grid, stream);
+  a.eights = dim % 8 == 0 && vdim % 8 == 0 && ld % 4 == 0 && aligned16(qkv) && aligned16(q_gain) && aligned16(k_gain) && aligned16(v_first) &&
+             aligned16(q) && aligned16(k_cache) && aligned16(v_cache);
   return launch_prefill_attn<16>(p, grid, stream);
 }
 
@@ -561,6 +595,8 @@ extern "C" int tilert_gqa_latent_attn_op(TgContext* ctx, const float* q, const v
     p.n_rows = heads * tokens;
     p.tokens = tokens;
     p.ring = ring;
+  p.eights = p.rope.eights(rot) && q_rank % 8 == 0 && rank % 8 == 0 && off_c % 4 == 0 && off_r % 4 == 0 && ldz % 4 == 0 && ldq % 8 == 0 &&
+             aligned16(z) && aligned16(q_gain) && aligned16(c_gain) && aligned16(rope) && aligned16(cq) && aligned16(cache);
     p.window = window;
     p.pos = pos;
     p.q = q;
@@ -594,6 +630,7 @@ extern "C" int tilert_gqa_latent_merge_op(TgContext* ctx, const float* part, int
   const LatentRow r = latent_row(rank, rot);
   TB_REQUIRE(ctx != nullptr && part != nullptr && out != nullptr && tokens >= 1 && heads >= 1 && n_splits >= 1 && n_splits <= 1024 && ldo >= rank);
   const LatentMergeParams p{part, heads * tokens, tokens, n_splits, rank, r.rankp, sink, out, ldo};
+  p.eights = p.rope.eights(rot) && dim % 8 == 0 && ldq % 4 == 0 && aligned16(q) && aligned16(rope) && aligned16(out) && aligned16(lat);
   const size_t smem = sizeof(float) * n_splits;
   if (f32) return go(latent_merge_kernel<float>, dim3(heads * tokens), dim3(128), smem, stream, p);
   return go(latent_merge_kernel<__nv_bfloat16>, dim3(heads * tokens), dim3(128), smem, stream, p);
