@@ -1034,47 +1034,52 @@ int record_hook(TbContext* ctx, const AttnPrepParams& prep) {
   return TB_OK;
 }
 
+template <int TOK, typename X, typename W>
+int launch_gemv_long(TbContext* ctx, const GemvBf16Params& p, cudaStream_t st) {
+  const size_t smem = TOK * GemvX<X>::bytes(p.k);
+  TB_REQUIRE(smem <= 200 * 1024);
+  const int warps = kGemvBf16Threads / 32 * kGemvBf16Rows, need = (p.n + warps - 1) / warps;
+  TB_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<TOK, X, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  // few rows: still a CTA per SM, with fewer busy warps each
+  TB_CUDA(launch(gemv_bf16_kernel<TOK, X, W>, dim3(need < ctx->num_sms && p.n < ctx->num_sms * kGemvBf16Rows ? need : ctx->num_sms),
+                 dim3(kGemvBf16Threads), smem, st, p));
+  return TB_OK;
+}
+template <typename X, typename W>
+int launch_gemv_long(TbContext* ctx, const GemvBf16Params& p, cudaStream_t st) {
+  if (p.n_tokens == 1) return launch_gemv_long<1, X, W>(ctx, p, st);
+  if (p.n_tokens == 2) return launch_gemv_long<2, X, W>(ctx, p, st);
+  return launch_gemv_long<4, X, W>(ctx, p, st);
+}
+
+template <int TOK>
+int launch_gemv_short(const GemvBf16Params& p, cudaStream_t st) {
+  const size_t smem = static_cast<size_t>(TOK) * p.k * sizeof(float);
+  TB_REQUIRE(smem <= 200 * 1024);
+  TB_CUDA(cudaFuncSetAttribute(gemv_bf16_ksplit_kernel<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  TB_CUDA(launch(gemv_bf16_ksplit_kernel<TOK>, dim3((p.n + kGemvBf16SmallRows - 1) / kGemvBf16SmallRows), dim3(kGemvBf16SmallThreads), smem, st, p));
+  return TB_OK;
+}
+
 int launch_gemv_bf16(TbContext* ctx, GemvBf16Params& p, cudaStream_t st) {
   TB_REQUIRE(p.n_tokens >= 1 && p.n_tokens <= 4);
   TB_REQUIRE(p.k % 256 == 0);
   if (ctx->rec.active)
     return fail(TB_ESTATE, "a bf16 row product cannot be recorded into a chain (pack the weight with "
                            "pack_bf16_two_term and use tilert_rmsnorm_proj_rows2_op)%s");
-  const int tok_t = p.n_tokens == 1 ? 1 : (p.n_tokens == 2 ? 2 : 4);
-  const size_t smem = static_cast<size_t>(tok_t) * p.k * sizeof(float);
-  const int warps = kGemvBf16Threads / 32;
-  int grid = (p.n + warps - 1) / warps;
-  const int cap = ctx->num_sms * 2;
-  if (grid > cap) grid = cap;
-  static bool attr_set = false;
-  if (!attr_set) {
-    TB_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TB_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TB_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_set = true;
-  }
-  TB_REQUIRE(smem <= 200 * 1024);
+  int rc;
   if (p.n <= 2048 && p.k <= 8192 && p.x2 == nullptr) {
-    static bool attr2_set = false;
-    if (!attr2_set) {
-      TB_CUDA(cudaFuncSetAttribute(gemv_bf16_ksplit_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-      TB_CUDA(cudaFuncSetAttribute(gemv_bf16_ksplit_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-      TB_CUDA(cudaFuncSetAttribute(gemv_bf16_ksplit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr2_set = true;
-    }
-    const int g2 = (p.n + kGemvBf16SmallRows - 1) / kGemvBf16SmallRows;
-    if (tok_t == 1)
-      TB_CUDA(launch(gemv_bf16_ksplit_kernel<1>, dim3(g2), dim3(kGemvBf16SmallThreads), smem, st, p));
-    else if (tok_t == 2)
-      TB_CUDA(launch(gemv_bf16_ksplit_kernel<2>, dim3(g2), dim3(kGemvBf16SmallThreads), smem, st, p));
+    rc = p.n_tokens == 1 ? launch_gemv_short<1>(p, st) : (p.n_tokens == 2 ? launch_gemv_short<2>(p, st) : launch_gemv_short<4>(p, st));
+  } else {
+    auto a16 = [](const void* q, long long ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 8 == 0; };
+    p.aligned = a16(p.x, p.x_stride) && (p.x2 == nullptr || (a16(p.x2, p.x2_stride) && p.k1 % 8 == 0));
+    const bool half = p.gamma == nullptr || p.round_norm_bf16;  // the staged activations are bf16 values
+    if (p.w_is_f32)
+      rc = half ? launch_gemv_long<__nv_bfloat16, float>(ctx, p, st) : launch_gemv_long<float, float>(ctx, p, st);
     else
-      TB_CUDA(launch(gemv_bf16_ksplit_kernel<4>, dim3(g2), dim3(kGemvBf16SmallThreads), smem, st, p));
-  } else if (tok_t == 1)
-    TB_CUDA(launch(gemv_bf16_kernel<1>, dim3(grid), dim3(kGemvBf16Threads), smem, st, p));
-  else if (tok_t == 2)
-    TB_CUDA(launch(gemv_bf16_kernel<2>, dim3(grid), dim3(kGemvBf16Threads), smem, st, p));
-  else
-    TB_CUDA(launch(gemv_bf16_kernel<4>, dim3(grid), dim3(kGemvBf16Threads), smem, st, p));
+      rc = half ? launch_gemv_long<__nv_bfloat16, __nv_bfloat16>(ctx, p, st) : launch_gemv_long<float, __nv_bfloat16>(ctx, p, st);
+  }
+  if (rc != TB_OK) return rc;
   ++g_launches;
   TB_CUDA(cudaGetLastError());
   return TB_OK;
@@ -1143,7 +1148,8 @@ extern "C" int tilert_rmsnorm_head_proj_op(TbContext* ctx, const void* x, const 
 }
 
 // Multi-token-prediction input: (optionally enorm / hnorm, then) concat and eh_proj [dim, 2*dim] bf16.
-// At most two tokens fit the kernel's shared memory at 2*dim = 14336; more tokens take two launches.
+// The normalised vectors are bf16 values, so up to four tokens fit the kernel's shared memory at 2*dim = 14336; a wider
+// model takes two tokens per launch.
 namespace {
 // Rows [row_begin, row_begin + n_rows) of the product (n_rows <= 0: all of them); `out` is the full [tokens, dim] tensor.
 int launch_eh_proj(TbContext* ctx, const void* e, const void* h, const float* gamma_e, const float* gamma_h, float eps,
@@ -1155,8 +1161,9 @@ int launch_eh_proj(TbContext* ctx, const void* e, const void* h, const float* ga
     n_rows = dim;
   }
   TB_REQUIRE(row_begin >= 0 && row_begin + n_rows <= dim);
-  for (int t0 = 0; t0 < tokens; t0 += 2) {
-    const int nt = tokens - t0 < 2 ? tokens - t0 : 2;
+  const int per = 4 * GemvX<__nv_bfloat16>::bytes(2 * dim) <= 200 * 1024 ? 4 : 2;
+  for (int t0 = 0; t0 < tokens; t0 += per) {
+    const int nt = tokens - t0 < per ? tokens - t0 : per;
     GemvBf16Params p{};
     p.w = reinterpret_cast<const __nv_bfloat16*>(w) + static_cast<long long>(row_begin) * 2 * dim;
     p.n = n_rows;

@@ -1,7 +1,7 @@
 // bf16-weight GEMV with f32 accumulation for the products that are not FP8 in the checkpoint:
 // the MoE router gate, the indexer head-weight projection and the vocabulary head.
-// HBM-bound on the weight stream: each warp owns whole rows and keeps several 16-byte
-// loads per lane in flight; the (optionally RMS-normalised) activations sit in shared memory.
+// HBM-bound on the weight stream: each warp keeps several 16-byte loads per lane in flight; the (optionally
+// RMS-normalised) activations sit in shared memory.
 #pragma once
 
 #include "common.cuh"
@@ -31,116 +31,243 @@ struct GemvBf16Params {
   void* out;                     // [tokens, n] f32 (out_bf16 = 0) or bf16 (out_bf16 = 1)
   int out_bf16;
   long long out_stride;
+  int aligned;                   // x, x2 and their rows are 16-byte aligned
 };
 
 constexpr int kGemvBf16Threads = 512;
+constexpr int kGemvBf16Rows = 4;   // weight rows that a warp works on together
+constexpr int kGemvBf16Ahead = 2;  // steps of a warp (256 elements of its rows) requested beyond the current one
 
-template <int TOK>
-__global__ void __launch_bounds__(kGemvBf16Threads) gemv_bf16_kernel(const GemvBf16Params p) {
+// Eight activations (a piece) of a token as staged in shared memory: bf16 where they are bf16 values (rounded, or not
+// normalised), else f32 with the halves of a piece apart -- a warp's 16-byte reads are free of bank conflicts either way.
+template <typename X>
+struct GemvX;
+template <>
+struct GemvX<__nv_bfloat16> {
+  static __host__ __device__ size_t bytes(int k) { return static_cast<size_t>(k) * 2; }
+  static __device__ __forceinline__ void get(const uint8_t* base, int, int piece, float (&f)[8]) {
+    const uint4 u = reinterpret_cast<const uint4*>(base)[piece];
+    f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
+    f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
+    f[4] = __uint_as_float(u.z << 16); f[5] = __uint_as_float(u.z & 0xffff0000u);
+    f[6] = __uint_as_float(u.w << 16); f[7] = __uint_as_float(u.w & 0xffff0000u);
+  }
+  static __device__ __forceinline__ void put(uint8_t* base, int, int piece, const float (&f)[8]) {
+    reinterpret_cast<uint4*>(base)[piece] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+  }
+};
+template <>
+struct GemvX<float> {
+  static __host__ __device__ size_t bytes(int k) { return static_cast<size_t>(k) * 4; }
+  static __device__ __forceinline__ void get(const uint8_t* base, int k, int piece, float (&f)[8]) {
+    const float4 a = reinterpret_cast<const float4*>(base)[piece], b = reinterpret_cast<const float4*>(base)[k / 8 + piece];
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+    f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+  }
+  static __device__ __forceinline__ void put(uint8_t* base, int k, int piece, const float (&f)[8]) {
+    reinterpret_cast<float4*>(base)[piece] = make_float4(f[0], f[1], f[2], f[3]);
+    reinterpret_cast<float4*>(base)[k / 8 + piece] = make_float4(f[4], f[5], f[6], f[7]);
+  }
+};
+// Eight weights as loaded.
+template <typename W>
+struct GemvW;
+template <>
+struct GemvW<__nv_bfloat16> {
+  uint4 u;
+  __device__ __forceinline__ void load(const void* w, long long at) {
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+                 : "l"(reinterpret_cast<const __nv_bfloat16*>(w) + at));
+  }
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
+    f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
+    f[4] = __uint_as_float(u.z << 16); f[5] = __uint_as_float(u.z & 0xffff0000u);
+    f[6] = __uint_as_float(u.w << 16); f[7] = __uint_as_float(u.w & 0xffff0000u);
+  }
+};
+template <>
+struct GemvW<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const void* w, long long at) {
+    const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w) + at);
+    a = __ldg(p);
+    b = __ldg(p + 1);
+  }
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+    f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+  }
+};
+
+// Sums v[0 .. N) over the warp, N a power of two up to 32: while there are several, lanes an offset apart exchange the
+// halves they do not keep, so N sums cost about N + 4 shuffles.  Lane l ends with the sum of v[l >> (5 - log2 N)].
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+  int cnt = N;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (cnt > 1) {
+      cnt >>= 1;
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) {
+        if (i < cnt) {
+          const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + cnt], o);
+          v[i] = (up ? v[i + cnt] : v[i]) + got;
+        }
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
+// Long weights (vocabulary head, eh_proj).  A warp owns four rows at a time, so that a staged piece of the activations
+// serves four weights, and keeps the next two steps of 256 elements requested: 12 sixteen-byte loads per lane.  (With a
+// row per warp the reads of the activations were the bound for several tokens.)  Head 16160 x 7168, one / two / four
+// tokens: 47.7 / 49.9 / 54.9 us against 59.5 / 103.4 / 148.1 a row at a time; eh_proj 7168 x 14336: 46.4 / 48.2 / 54.9
+// against 61.5 / 91.7 / 182.0.
+template <int TOK, typename X, typename W>
+__global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const GemvBf16Params p) {
   pdl_launch_dependents();
-  pdl_wait();
-  extern __shared__ __align__(16) float xs[];  // [TOK][k]
-  __shared__ float red[TOK][32];
+  extern __shared__ __align__(16) uint8_t gsm[];  // [TOK] GemvX<X>
+  __shared__ float red[2][TOK][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nwarps = blockDim.x >> 5;
+  constexpr int kWarps = kGemvBf16Threads / 32;
+  const size_t x_bytes = GemvX<X>::bytes(p.k);
+  const int pieces = p.k / 8, steps = pieces / 32;
+  const int groups = (p.n + kGemvBf16Rows - 1) / kGemvBf16Rows, stride = gridDim.x * kWarps;
 
-  // stage (and normalise) the activations; with a second segment each half has its own statistics
+  GemvW<W> w[kGemvBf16Ahead + 1][kGemvBf16Rows];
+  auto request = [&](int group, int step, GemvW<W> (&dst)[kGemvBf16Rows]) {
+#pragma unroll
+    for (int r = 0; r < kGemvBf16Rows; ++r)  // rows past the end: the last one, dropped below
+      dst[r].load(p.w, static_cast<long long>(min(group * kGemvBf16Rows + r, p.n - 1)) * p.k + (step * 32 + lane) * 8);
+  };
+  int group = warp * gridDim.x + blockIdx.x;  // neighbouring CTAs read neighbouring rows
+  int pg = group, ps = 0;                     // the next step to request
+  auto advance = [&] {
+    if (++ps == steps) {
+      ps = 0;
+      pg += stride;
+    }
+  };
+  // the weights do not depend on the predecessor
+#pragma unroll
+  for (int d = 0; d < kGemvBf16Ahead; ++d) {
+    if (pg < groups) request(pg, ps, w[d]);
+    advance();
+  }
+
+  // stage (and normalise) the activations; with a second segment each one has its own statistics
+  pdl_wait();
   const int k1 = p.x2 != nullptr ? p.k1 : p.k;
   float ss[TOK], ss2[TOK];
 #pragma unroll
   for (int t = 0; t < TOK; ++t) ss[t] = ss2[t] = 0.f;
-  for (int i = threadIdx.x; i < p.k; i += blockDim.x) {
+  for (int i = threadIdx.x; i < pieces; i += kGemvBf16Threads) {
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
-      float v = 0.f;
-      if (t < p.n_tokens) v = i < k1 ? bf2f(p.x[t * p.x_stride + i]) : bf2f(p.x2[t * p.x2_stride + i - k1]);
-      xs[t * p.k + i] = v;
-      if (i < k1) ss[t] += v * v; else ss2[t] += v * v;
+      float f[8] = {};
+      if (t < p.n_tokens) {
+        const __nv_bfloat16* src = i * 8 < k1 ? p.x + t * p.x_stride + i * 8 : p.x2 + t * p.x2_stride + i * 8 - k1;
+        if (p.aligned) {
+          const uint4 u = *reinterpret_cast<const uint4*>(src);
+          const uint32_t q[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            f[2 * j] = __uint_as_float(q[j] << 16);
+            f[2 * j + 1] = __uint_as_float(q[j] & 0xffff0000u);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = bf2f(src[j]);
+        }
+      }
+      GemvX<X>::put(gsm + t * x_bytes, p.k, i, f);
+      float s = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += f[j] * f[j];
+      if (i * 8 < k1) ss[t] += s; else ss2[t] += s;
     }
   }
   if (p.gamma != nullptr) {
-    __shared__ float red2[TOK][32];
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
       const float s = warp_sum(ss[t]), s2 = warp_sum(ss2[t]);
       if (lane == 0) {
-        red[t][warp] = s;
-        red2[t][warp] = s2;
+        red[0][t][warp] = s;
+        red[1][t][warp] = s2;
       }
     }
     __syncthreads();
     float rinv[TOK], rinv2[TOK];
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
-      float tot = lane < nwarps ? red[t][lane] : 0.f, tot2 = lane < nwarps ? red2[t][lane] : 0.f;
-      tot = warp_sum(tot);
-      tot2 = warp_sum(tot2);
+      const float tot = warp_sum(lane < kWarps ? red[0][t][lane] : 0.f), tot2 = warp_sum(lane < kWarps ? red[1][t][lane] : 0.f);
       rinv[t] = rsqrtf(tot / static_cast<float>(k1) + p.eps);
       rinv2[t] = rsqrtf(tot2 / static_cast<float>(p.k - k1 > 0 ? p.k - k1 : 1) + p.eps);
     }
-    for (int i = threadIdx.x; i < p.k; i += blockDim.x) {
-      const float g = i < k1 ? p.gamma[i] : p.gamma2[i - k1];
+    for (int i = threadIdx.x; i < pieces; i += kGemvBf16Threads) {  // every thread rescales what it wrote
+      const bool first = i * 8 < k1;
+      float g[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = first ? p.gamma[i * 8 + j] : p.gamma2[i * 8 - k1 + j];
 #pragma unroll
       for (int t = 0; t < TOK; ++t) {
-        float v = xs[t * p.k + i] * (i < k1 ? rinv[t] : rinv2[t]) * g;
-        if (p.round_norm_bf16) v = bf2f(f2bf(v));
-        xs[t * p.k + i] = v;
-        if (blockIdx.x == 0 && t < p.n_tokens) {
-          if (i < k1) {
-            if (p.xnorm_out != nullptr) p.xnorm_out[t * p.xnorm_stride + i] = f2bf(v);
-          } else if (p.xnorm2_out != nullptr) {
-            p.xnorm2_out[t * p.xnorm2_stride + i - k1] = f2bf(v);
-          }
+        float f[8];
+        GemvX<X>::get(gsm + t * x_bytes, p.k, i, f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] *= (first ? rinv[t] : rinv2[t]) * g[j];
+        GemvX<X>::put(gsm + t * x_bytes, p.k, i, f);
+        __nv_bfloat16* out = first ? p.xnorm_out : p.xnorm2_out;
+        if (blockIdx.x == 0 && t < p.n_tokens && out != nullptr) {
+          out += first ? t * p.xnorm_stride + i * 8 : t * p.xnorm2_stride + i * 8 - k1;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) out[j] = f2bf(f[j]);
         }
       }
     }
   }
   __syncthreads();
 
-  const int gw = blockIdx.x * nwarps + warp, tw = gridDim.x * nwarps;
-  for (int row = gw; row < p.n; row += tw) {
-    float acc[TOK];
+  for (; group < groups; group += stride) {
+    float acc[kGemvBf16Rows * TOK];
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) acc[t] = 0.f;
-    if (p.w_is_f32) {
-      const float* wr = reinterpret_cast<const float*>(p.w) + static_cast<long long>(row) * p.k;
-      for (int k0 = lane * 4; k0 < p.k; k0 += 128) {
-        const float4 wv = __ldg(reinterpret_cast<const float4*>(wr + k0));
+    for (int i = 0; i < kGemvBf16Rows * TOK; ++i) acc[i] = 0.f;
+#pragma unroll 3
+    for (int s = 0; s < steps; ++s) {
+      if (pg < groups) request(pg, ps, w[kGemvBf16Ahead]);
+      advance();
+      float wf[kGemvBf16Rows][8];
 #pragma unroll
-        for (int t = 0; t < TOK; ++t) {
-          const float4 xv = *reinterpret_cast<const float4*>(&xs[t * p.k + k0]);
-          acc[t] += wv.x * xv.x + wv.y * xv.y + wv.z * xv.z + wv.w * xv.w;
-        }
+      for (int r = 0; r < kGemvBf16Rows; ++r) w[0][r].get(wf[r]);
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) {
+        float f[8];
+        GemvX<X>::get(gsm + t * x_bytes, p.k, s * 32 + lane, f);
+#pragma unroll
+        for (int r = 0; r < kGemvBf16Rows; ++r)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[r * TOK + t] += wf[r][j] * f[j];
       }
-    } else {
-      const __nv_bfloat16* wr = reinterpret_cast<const __nv_bfloat16*>(p.w) + static_cast<long long>(row) * p.k;
-#pragma unroll 4
-      for (int k0 = lane * 8; k0 < p.k; k0 += 256) {
-        uint4 wv;
-        asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
-                     : "l"(wr + k0));
-        const float w0 = __uint_as_float(wv.x << 16), w1 = __uint_as_float(wv.x & 0xffff0000u);
-        const float w2 = __uint_as_float(wv.y << 16), w3 = __uint_as_float(wv.y & 0xffff0000u);
-        const float w4 = __uint_as_float(wv.z << 16), w5 = __uint_as_float(wv.z & 0xffff0000u);
-        const float w6 = __uint_as_float(wv.w << 16), w7 = __uint_as_float(wv.w & 0xffff0000u);
 #pragma unroll
-        for (int t = 0; t < TOK; ++t) {
-          const float4 xa = *reinterpret_cast<const float4*>(&xs[t * p.k + k0]);
-          const float4 xb = *reinterpret_cast<const float4*>(&xs[t * p.k + k0 + 4]);
-          acc[t] += w0 * xa.x + w1 * xa.y + w2 * xa.z + w3 * xa.w + w4 * xb.x + w5 * xb.y + w6 * xb.z + w7 * xb.w;
-        }
-      }
+      for (int d = 0; d < kGemvBf16Ahead; ++d)
+#pragma unroll
+        for (int r = 0; r < kGemvBf16Rows; ++r) w[d][r] = w[d + 1][r];
     }
-#pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      const float s = warp_sum(acc[t]);
-      if (lane == 0 && t < p.n_tokens) {
-        if (p.out_bf16)
-          reinterpret_cast<__nv_bfloat16*>(p.out)[t * p.out_stride + row] = f2bf(s);
-        else
-          reinterpret_cast<float*>(p.out)[t * p.out_stride + row] = s;
-      }
+    constexpr int kSums = kGemvBf16Rows * TOK, kLanes = 32 / kSums;  // lanes that hold the same sum
+    const float sum = warp_sums<kSums>(acc);
+    const int i = lane / kLanes, row = group * kGemvBf16Rows + i / TOK, t = i % TOK;
+    if (lane % kLanes == 0 && row < p.n && t < p.n_tokens) {
+      if (p.out_bf16)
+        reinterpret_cast<__nv_bfloat16*>(p.out)[t * p.out_stride + row] = f2bf(sum);
+      else
+        reinterpret_cast<float*>(p.out)[t * p.out_stride + row] = sum;
     }
   }
 }
