@@ -1,7 +1,7 @@
 // Products of many token rows with bf16 weights (prefill):  out[t, n] = W[n, :] . x[t, :].
 //
 //   gemm_tc_kernel<BN, GATED>   bf16 rows on the tensor cores
-//   gemm_f32_kernel<GATED>      f32 rows, f32 arithmetic (the exact mode)
+//   gemm_f32_kernel<.., GATED>  f32 rows, f32 arithmetic (the exact mode)
 //
 // GATED: the weight holds gate rows, then up rows, and the result is their clamped gated unit.
 // Grouped launches have one weight per group (expert) and the token rows sorted by group; the number of rows per
@@ -47,6 +47,7 @@ struct TileWalk {
   const int* rows0;
   const int* tiles0;
   int n_groups, ft, bn;
+  int bf = 128;          // features of a tile
   int group = 0;
 
   struct Tile {
@@ -57,7 +58,7 @@ struct TileWalk {
     const int local = i - tiles0[group], r0 = rows0[group], r1 = rows0[group + 1];
     const int tt = (r1 - r0 + bn - 1) / bn;
     const int f = local / tt, t = local - f * tt;
-    return {group, f * 128, r0 + t * bn, min(r0 + (t + 1) * bn, r1)};
+    return {group, f * bf, r0 + t * bn, min(r0 + (t + 1) * bn, r1)};
   }
 };
 
@@ -365,66 +366,150 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 }
 
 // ------------------------------------------------------------------ f32
-constexpr int kF32Threads = 256, kF32Tile = 64, kF32K = 16;
+// Tiles of BF features x BT tokens, K by KB through shared memory; a thread has 4 features x RT tokens of one of KG equal
+// parts of every step of K, and the parts' sums are added in order at the end.  The next KB of both operands are in
+// registers while a step is computed, and the reads of a step are 16 bytes along K from rows an odd number of 16-byte units
+// apart (no bank conflicts).  Two shapes: 64 x 64 where such tiles fill the SMs twice, else 32 x 32 with four groups of
+// threads along K: few rows leave a walk along K bound by latency, which larger steps of more warps shorten.
+// 97 rows, 1152 features, K 1024: 19.5 us (64 x 64 tiles without a next step on its way 128); 388 x 704 x 1024: 35.5
+// (136); 200 x 2048 x 1024 on 64 x 64 tiles: 67.0 (150).
+template <int BF, int BT, int KB, int KG, bool GATED>
+struct F32Shape {
+  static constexpr int kFt = BF / 4;                     // threads along the features
+  static constexpr int kRt = BF * BT == 1024 ? 2 : 4;    // tokens of a thread
+  static constexpr int kGroup = kFt * (BT / kRt);        // threads of a part of K
+  static constexpr int kThreads = kGroup * KG;
+  static constexpr int kW = GATED ? 2 : 1;
+  static constexpr int kPitch = KB + 4;                  // (KB / 4 + 1) units of 16 bytes
+  static constexpr int kWPieces = (BF * KB / 8 + kThreads - 1) / kThreads, kXPieces = (BT * KB / 4 + kThreads - 1) / kThreads;  // loads of a thread
+  static constexpr int kFloats = (kW * BF + BT) * kPitch;
+  static_assert((KB / 4) % 2 == 0 && KB % (4 * KG) == 0 && kThreads <= 512, "odd pitch, whole parts");
+  static_assert((KG - 1) * kW * 4 * kRt * kGroup <= kFloats, "the parts' sums fit the operands' place");
+};
 
-template <bool GATED>
-__global__ void __launch_bounds__(kF32Threads) gemm_f32_kernel(const GemmRowsParams p) {
-  __shared__ float ws[GATED ? 2 : 1][kF32K][kF32Tile + 4], xs[kF32K][kF32Tile + 4];
+template <int BF, int BT, int KB, int KG, bool GATED>
+__global__ void __launch_bounds__(F32Shape<BF, BT, KB, KG, GATED>::kThreads) gemm_f32_kernel(const GemmRowsParams p) {
+  using S = F32Shape<BF, BT, KB, KG, GATED>;
+  constexpr int kW = S::kW, RT = S::kRt;
+  __shared__ __align__(16) float buf[S::kFloats];
+  float(*ws)[BF][S::kPitch] = reinterpret_cast<float(*)[BF][S::kPitch]>(buf);
+  float(*xs)[S::kPitch] = reinterpret_cast<float(*)[S::kPitch]>(buf + kW * BF * S::kPitch);
   __shared__ int s_rows[kMaxGroups + 1], s_tiles[kMaxGroups + 1];
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int kW = GATED ? 2 : 1;
-  // tiles of 128 features are walked as two halves of 64
-  const int ft = (p.n + 127) / 128;
-  tile_prefix(p, kF32Tile, ft, s_rows, s_tiles);
+  const int ft = (p.n + BF - 1) / BF;
+  tile_prefix(p, BT, ft, s_rows, s_tiles);
   const int groups = p.n_groups > 0 ? p.n_groups : 1;
   const int n_tiles = s_tiles[groups];
-  TileWalk walk{s_rows, s_tiles, groups, ft, kF32Tile};
-  const int tn = threadIdx.x & 15, tt = threadIdx.x >> 4;  // features tn + 16 i, tokens tt + 16 i
-  for (int i2 = blockIdx.x; i2 < 2 * n_tiles; i2 += gridDim.x) {
-    const TileWalk::Tile t = walk.at(i2 >> 1);
-    const int f0 = t.feature0 + (i2 & 1) * kF32Tile;
-    if (f0 >= p.n) continue;  // uniform over the CTA
-    float acc[kW][4][4];
+  TileWalk walk{s_rows, s_tiles, groups, ft, BT, BF};
+  const int kg = threadIdx.x / S::kGroup, th = threadIdx.x - kg * S::kGroup;
+  const int tf = th % S::kFt, tt = th / S::kFt;  // features tf + kFt i, tokens tt + (BT / RT) i
+  for (int i = blockIdx.x; i < n_tiles; i += gridDim.x) {
+    const TileWalk::Tile t = walk.at(i);
+    uint4 wr[kW][S::kWPieces];
+    float4 xr[S::kXPieces];
+    auto request = [&](int k0) {
+#pragma unroll
+      for (int e = 0; e < S::kWPieces; ++e) {
+        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 8), k = k0 + c % (KB / 8) * 8;
+#pragma unroll
+        for (int h = 0; h < kW; ++h) {
+          const long long row = (static_cast<long long>(t.group) * kW + h) * p.n + t.feature0 + r;
+          wr[h][e] = c < BF * KB / 8 && k < p.k && t.feature0 + r < p.n ? __ldg(reinterpret_cast<const uint4*>(p.w + row * p.ldw + k)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < S::kXPieces; ++e) {
+        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 4), k = k0 + c % (KB / 4) * 4;
+        xr[e] = c < BT * KB / 4 && k < p.k && t.row0 + r < t.row1 ? *reinterpret_cast<const float4*>(p.x + static_cast<long long>(t.row0 + r) * p.ldx + k)
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    auto deposit = [&](int k0) {  // what lies between k and the end of its piece is no operand
+#pragma unroll
+      for (int e = 0; e < S::kWPieces; ++e) {
+        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 8), k = c % (KB / 8) * 8;
+        if (c >= BF * KB / 8) break;
+#pragma unroll
+        for (int h = 0; h < kW; ++h) {
+          float f[8];
+          bf16x8_to_f32(wr[h][e], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (k0 + k + j >= p.k) f[j] = 0.f;
+          *reinterpret_cast<float4*>(&ws[h][r][k]) = make_float4(f[0], f[1], f[2], f[3]);
+          *reinterpret_cast<float4*>(&ws[h][r][k + 4]) = make_float4(f[4], f[5], f[6], f[7]);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < S::kXPieces; ++e) {
+        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 4), k = c % (KB / 4) * 4;
+        if (c >= BT * KB / 4) break;
+        float4 v = xr[e];
+        if (k0 + k + 1 >= p.k) v.y = 0.f;
+        if (k0 + k + 2 >= p.k) v.z = 0.f;
+        if (k0 + k + 3 >= p.k) v.w = 0.f;
+        *reinterpret_cast<float4*>(&xs[r][k]) = v;
+      }
+    };
+    float acc[kW][4][RT];
 #pragma unroll
     for (int h = 0; h < kW; ++h)
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[h][a][b] = 0.f;
-    for (int k0 = 0; k0 < p.k; k0 += kF32K) {
-      for (int e = threadIdx.x; e < kF32Tile * kF32K; e += kF32Threads) {
-        const int r = e / kF32K, c = e % kF32K;
-        const bool kin = k0 + c < p.k;
-#pragma unroll
-        for (int h = 0; h < kW; ++h) {
-          const long long row = (static_cast<long long>(t.group) * kW + h) * p.n + f0 + r;
-          ws[h][c][r] = kin && f0 + r < p.n ? bf2f(p.w[row * p.ldw + k0 + c]) : 0.f;
-        }
-        xs[c][r] = kin && t.row0 + r < t.row1 ? p.x[static_cast<long long>(t.row0 + r) * p.ldx + k0 + c] : 0.f;
-      }
+        for (int b = 0; b < RT; ++b) acc[h][a][b] = 0.f;
+    request(0);
+    for (int k0 = 0; k0 < p.k; k0 += KB) {
+      __syncthreads();  // the step before has been read
+      deposit(k0);
       __syncthreads();
+      if (k0 + KB < p.k) request(k0 + KB);
+#pragma unroll 4
+      for (int c = kg * (KB / KG); c < (kg + 1) * (KB / KG); c += 4) {
+        float4 xv[RT];
 #pragma unroll
-      for (int c = 0; c < kF32K; ++c) {
-        float xv[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) xv[b] = xs[c][tt + 16 * b];
+        for (int b = 0; b < RT; ++b) xv[b] = *reinterpret_cast<const float4*>(&xs[tt + BT / RT * b][c]);
 #pragma unroll
         for (int h = 0; h < kW; ++h)
 #pragma unroll
           for (int a = 0; a < 4; ++a) {
-            const float wv = ws[h][c][tn + 16 * a];
+            const float4 wv = *reinterpret_cast<const float4*>(&ws[h][tf + S::kFt * a][c]);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[h][a][b] += wv * xv[b];
+            for (int b = 0; b < RT; ++b) {
+              acc[h][a][b] += wv.x * xv[b].x;
+              acc[h][a][b] += wv.y * xv[b].y;
+              acc[h][a][b] += wv.z * xv[b].z;
+              acc[h][a][b] += wv.w * xv[b].w;
+            }
           }
       }
+    }
+    if (KG > 1) {
+      __syncthreads();  // the last step has been read
+#pragma unroll
+      for (int h = 0; h < kW; ++h)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < RT; ++b)
+            if (kg > 0) buf[(((kg - 1) * kW + h) * 4 * RT + a * RT + b) * S::kGroup + th] = acc[h][a][b];
       __syncthreads();
+      if (kg > 0) continue;  // (the next tile's first step waits for the threads that read)
+#pragma unroll
+      for (int g = 0; g < KG - 1; ++g)
+#pragma unroll
+        for (int h = 0; h < kW; ++h)
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < RT; ++b) acc[h][a][b] += buf[((g * kW + h) * 4 * RT + a * RT + b) * S::kGroup + th];
     }
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int f = f0 + tn + 16 * a, r = t.row0 + tt + 16 * b;
+      for (int b = 0; b < RT; ++b) {
+        const int f = t.feature0 + tf + S::kFt * a, r = t.row0 + tt + BT / RT * b;
         if (f < p.n && r < t.row1) {
           const float v = GATED ? clamped_gate(acc[0][a][b], acc[kW - 1][a][b], p.limit, p.alpha)
                                 : acc[0][a][b] + (p.bias != nullptr ? p.bias[f] : 0.f);

@@ -87,6 +87,11 @@ int launch_tc(TgContext* ctx, const GemmRowsParams& p, long long w_rows, void* s
   return go(gemm_tc_kernel<BN, GATED>, dim3(ctx->num_sms), dim3(kTcThreads), TcShape<BN, GATED>::kSmemBytes, stream, wmap, xmap, p);
 }
 
+template <int BF, int BT, int KB, int KG, bool GATED>
+int launch_f32(TgContext* ctx, const GemmRowsParams& p, void* stream) {
+  return go(gemm_f32_kernel<BF, BT, KB, KG, GATED>, dim3(ctx->num_sms * 4), dim3(F32Shape<BF, BT, KB, KG, GATED>::kThreads), 0, stream, p);
+}
+
 QkvShape qkv_shape(int heads, int kv_heads, int dim, int vdim, int ring, int window) {
   return {heads, kv_heads, dim, vdim, pad_to(dim, 16), pad_to(vdim, 16), ring, window};
 }
@@ -145,27 +150,6 @@ extern "C" int tilert_gqa_set_wait_budget(TgContext* ctx, long long cycles) {
 }
 
 // ------------------------------------------------------------------------------- norms
-extern "C" int tilert_gqa_embed_norm_op(TgContext* ctx, const long long* tokens, const void* table, long long ld_table, int vocab,
-                                        const float* gain, float eps, int rows, int dim, float* x, long long ldx, void* xh,
-                                        long long ldh, int f32, void* stream) {
-  TB_REQUIRE(ctx != nullptr && tokens != nullptr && table != nullptr && x != nullptr);
-  TB_REQUIRE(rows >= 1 && dim >= 1 && vocab >= 1 && ld_table >= dim && ldx >= dim && (xh == nullptr || ldh >= dim));
-  const EmbedNormParams p{tokens, reinterpret_cast<const __nv_bfloat16*>(table), ld_table, vocab, gain, eps, dim, x, ldx, xh, ldh,
-                          ctx->status};
-  if (f32) return go(embed_norm_kernel<float>, dim3(rows), dim3(kNormThreads), 0, stream, p);
-  return go(embed_norm_kernel<__nv_bfloat16>, dim3(rows), dim3(kNormThreads), 0, stream, p);
-}
-
-extern "C" int tilert_gqa_residual_norm_op(TgContext* ctx, const float* y, long long ldy, const void* ye, long long lde,
-                                           const int* slot_row, const float* slot_w, int top, const void* ysh, long long ldsh,
-                                           const float* gain, const float* bias, const float* add, const float* gain2,
-                                           const float* bias2, int centered, float eps, int rows, int dim, float* x, long long ldx,
-                                           void* xh, long long ldh, int f32, void* stream) {
-  TB_REQUIRE(ctx != nullptr && x != nullptr && rows >= 1 && dim >= 1 && ldx >= dim && (xh == nullptr || ldh >= dim));
-  TB_REQUIRE((gain != nullptr) == (y != nullptr || ye != nullptr) && (bias == nullptr || gain != nullptr));
-  TB_REQUIRE((gain2 == nullptr || xh != nullptr) && (bias2 == nullptr || gain2 != nullptr));
-  TB_REQUIRE(y != nullptr ? ldy >= dim
-                          : (ye == nullptr || (slot_row != nullptr && slot_w != nullptr && top >= 1 && stride_ok(lde, dim) && aligned16(ye) &&
 namespace {
 
 // Whether rows of `dim` elements can be held as pieces of eight: whole pieces, as many as the threads have room for,
@@ -185,19 +169,46 @@ int by_pieces(int dim, int rows, void* stream, const P& p, void (*narrow)(P), vo
 
 }  // namespace
 
-                                               (ysh == nullptr || (stride_ok(ldsh, dim) && aligned16(ysh))))));
-  const ResidualNormParams p{y,    ldy, ye,    lde,   slot_row, slot_w, top, ysh, ldsh, gain, bias,
-                             add,  gain2, bias2, centered, eps, dim,    x,   ldx, xh,   ldh};
-  const size_t smem = static_cast<size_t>(dim) * sizeof(float);
-  if (f32) return go(residual_norm_kernel<float>, dim3(rows), dim3(kNormThreads), smem, stream, p);
-  return go(residual_norm_kernel<__nv_bfloat16>, dim3(rows), dim3(kNormThreads), smem, stream, p);
-}
+extern "C" int tilert_gqa_embed_norm_op(TgContext* ctx, const long long* tokens, const void* table, long long ld_table, int vocab,
+                                        const float* gain, float eps, int rows, int dim, float* x, long long ldx, void* xh,
+                                        long long ldh, int f32, void* stream) {
+  TB_REQUIRE(ctx != nullptr && tokens != nullptr && table != nullptr && x != nullptr);
+  TB_REQUIRE(rows >= 1 && dim >= 1 && vocab >= 1 && ld_table >= dim && ldx >= dim && (xh == nullptr || ldh >= dim));
+  const EmbedNormParams p{tokens, reinterpret_cast<const __nv_bfloat16*>(table), ld_table, vocab, gain, eps, dim, x, ldx, xh, ldh,
+                          ctx->status};
   if (row_pieces(dim, {table, gain, x, xh}, {ld_table, ldx, ldh})) {
     return f32 ? by_pieces(dim, rows, stream, p, embed_norm_pieces_kernel<float, 256, 1>, embed_norm_pieces_kernel<float, 512, 1>,
                            embed_norm_pieces_kernel<float, 512, 2>)
                : by_pieces(dim, rows, stream, p, embed_norm_pieces_kernel<__nv_bfloat16, 256, 1>, embed_norm_pieces_kernel<__nv_bfloat16, 512, 1>,
                            embed_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
   }
+  if (f32) return go(embed_norm_kernel<float>, dim3(rows), dim3(kNormThreads), 0, stream, p);
+  return go(embed_norm_kernel<__nv_bfloat16>, dim3(rows), dim3(kNormThreads), 0, stream, p);
+}
+
+extern "C" int tilert_gqa_residual_norm_op(TgContext* ctx, const float* y, long long ldy, const void* ye, long long lde,
+                                           const int* slot_row, const float* slot_w, int top, const void* ysh, long long ldsh,
+                                           const float* gain, const float* bias, const float* add, const float* gain2,
+                                           const float* bias2, int centered, float eps, int rows, int dim, float* x, long long ldx,
+                                           void* xh, long long ldh, int f32, void* stream) {
+  TB_REQUIRE(ctx != nullptr && x != nullptr && rows >= 1 && dim >= 1 && ldx >= dim && (xh == nullptr || ldh >= dim));
+  TB_REQUIRE((gain != nullptr) == (y != nullptr || ye != nullptr) && (bias == nullptr || gain != nullptr));
+  TB_REQUIRE((gain2 == nullptr || xh != nullptr) && (bias2 == nullptr || gain2 != nullptr));
+  TB_REQUIRE(y != nullptr ? ldy >= dim
+                          : (ye == nullptr || (slot_row != nullptr && slot_w != nullptr && top >= 1 && stride_ok(lde, dim) && aligned16(ye) &&
+                                               (ysh == nullptr || (stride_ok(ldsh, dim) && aligned16(ysh))))));
+  const ResidualNormParams p{y,    ldy, ye,    lde,   slot_row, slot_w, top, ysh, ldsh, gain, bias,
+                             add,  gain2, bias2, centered, eps, dim,    x,   ldx, xh,   ldh};
+  if (row_pieces(dim, {y, ye, ysh, gain, bias, add, gain2, bias2, x, xh}, {ldy, lde, ldsh, ldx, ldh})) {
+    return f32 ? by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<float, 256, 1>, residual_norm_pieces_kernel<float, 512, 1>,
+                           residual_norm_pieces_kernel<float, 512, 2>)
+               : by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<__nv_bfloat16, 256, 1>,
+                           residual_norm_pieces_kernel<__nv_bfloat16, 512, 1>, residual_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
+  }
+  const size_t smem = static_cast<size_t>(dim) * sizeof(float);
+  if (f32) return go(residual_norm_kernel<float>, dim3(rows), dim3(kNormThreads), smem, stream, p);
+  return go(residual_norm_kernel<__nv_bfloat16>, dim3(rows), dim3(kNormThreads), smem, stream, p);
+}
 
 extern "C" int tilert_gqa_gather_norm_op(TgContext* ctx, const float* x, long long ldx, const int* rows, int n, const float* gain,
                                          const float* bias, int centered, float eps, int dim, void* out, long long ldo, int f32, void* stream) {
@@ -215,12 +226,6 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
   TB_REQUIRE(ctx != nullptr && x != nullptr && w != nullptr && out != nullptr);
   TB_REQUIRE(rows >= 1 && n >= 1 && k >= 1 && n_groups >= 0 && n_groups <= kMaxGroups);
   TB_REQUIRE(stride_ok(ldx, k) && stride_ok(ldw, k) && ldo >= n && aligned16(x) && aligned16(w));
-  if (row_pieces(dim, {y, ye, ysh, gain, bias, add, gain2, bias2, x, xh}, {ldy, lde, ldsh, ldx, ldh})) {
-    return f32 ? by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<float, 256, 1>, residual_norm_pieces_kernel<float, 512, 1>,
-                           residual_norm_pieces_kernel<float, 512, 2>)
-               : by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<__nv_bfloat16, 256, 1>,
-                           residual_norm_pieces_kernel<__nv_bfloat16, 512, 1>, residual_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
-  }
   TB_REQUIRE(bias == nullptr || (n_groups == 0 && !gated));
   const int per = gated ? 2 : 1;
   TB_REQUIRE(static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n < (1ll << 31) - 256);
@@ -242,9 +247,11 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
   p.x = reinterpret_cast<const float*>(x);
   p.ldx = ldx;
   if (f32) {
-    const dim3 grid(ctx->num_sms * 4);
-    return gated ? go(gemm_f32_kernel<true>, grid, dim3(kF32Threads), 0, stream, p)
-                 : go(gemm_f32_kernel<false>, grid, dim3(kF32Threads), 0, stream, p);
+    // rows per group as the host knows them: an average where the counts are on the device
+    const int each = n_groups > 0 && counts != nullptr ? (rows + n_groups - 1) / n_groups : rows;
+    const long long large = static_cast<long long>(n_groups > 0 ? n_groups : 1) * ((n + 63) / 64) * ((each + 63) / 64);
+    if (large >= 2 * ctx->num_sms && each >= 48) return gated ? launch_f32<64, 64, 32, 1, true>(ctx, p, stream) : launch_f32<64, 64, 32, 1, false>(ctx, p, stream);
+    return gated ? launch_f32<32, 32, 64, 4, true>(ctx, p, stream) : launch_f32<32, 32, 128, 4, false>(ctx, p, stream);
   }
   const long long w_rows = static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n;
   const int ft = (n + 127) / 128;
@@ -278,6 +285,8 @@ extern "C" int tilert_gqa_qkv_rows_op(TgContext* ctx, const float* qkv, long lon
   a.q = q;
   a.k_cache = k_cache;
   a.v_cache = v_cache;
+  a.eights = dim % 8 == 0 && vdim % 8 == 0 && ld % 4 == 0 && aligned16(qkv) && aligned16(q_gain) && aligned16(k_gain) && aligned16(v_first) &&
+             aligned16(q) && aligned16(k_cache) && aligned16(v_cache);
   if (f32) return go(qkv_rows_kernel<float>, dim3(rows), dim3(256), 0, stream, a);
   return go(qkv_rows_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, a);
 }
@@ -301,8 +310,6 @@ int run_prefill_attn(const AttnPrefillParams& p, void* stream) {
   const dim3 grid((p.rows + tpb - 1) / tpb, p.s.kv_heads * ((group + hpb - 1) / hpb));
   if (p.s.vdimp <= 64) return launch_prefill_attn<4>(p, grid, stream);
   if (p.s.vdimp <= 128) return launch_prefill_attn<8>(p, grid, stream);
-  a.eights = dim % 8 == 0 && vdim % 8 == 0 && ld % 4 == 0 && aligned16(qkv) && aligned16(q_gain) && aligned16(k_gain) && aligned16(v_first) &&
-             aligned16(q) && aligned16(k_cache) && aligned16(v_cache);
   return launch_prefill_attn<16>(p, grid, stream);
 }
 
@@ -543,6 +550,8 @@ extern "C" int tilert_gqa_latent_tokens_op(TgContext* ctx, const float* z, long 
   p.cq = cq;
   p.ldq = ldq;
   p.cache = cache;
+  p.eights = p.rope.eights(rot) && q_rank % 8 == 0 && rank % 8 == 0 && off_c % 4 == 0 && off_r % 4 == 0 && ldz % 4 == 0 && ldq % 8 == 0 &&
+             aligned16(z) && aligned16(q_gain) && aligned16(c_gain) && aligned16(rope) && aligned16(cq) && aligned16(cache);
   if (f32) return go(latent_tokens_kernel<float>, dim3(rows), dim3(256), 0, stream, p);
   return go(latent_tokens_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, p);
 }
@@ -576,6 +585,7 @@ extern "C" int tilert_gqa_latent_queries_op(TgContext* ctx, const float* q, long
   } else {
     p.off_rot = pad_to(dim, 16);
   }
+  p.eights = p.rope.eights(rot) && dim % 8 == 0 && ldq % 4 == 0 && aligned16(q) && aligned16(rope) && aligned16(out) && aligned16(lat);
   if (f32) return go(latent_queries_kernel<float>, dim3(rows), dim3(256), 0, stream, p);
   return go(latent_queries_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, p);
 }
@@ -595,8 +605,6 @@ extern "C" int tilert_gqa_latent_attn_op(TgContext* ctx, const float* q, const v
     p.n_rows = heads * tokens;
     p.tokens = tokens;
     p.ring = ring;
-  p.eights = p.rope.eights(rot) && q_rank % 8 == 0 && rank % 8 == 0 && off_c % 4 == 0 && off_r % 4 == 0 && ldz % 4 == 0 && ldq % 8 == 0 &&
-             aligned16(z) && aligned16(q_gain) && aligned16(c_gain) && aligned16(rope) && aligned16(cq) && aligned16(cache);
     p.window = window;
     p.pos = pos;
     p.q = q;
@@ -630,7 +638,6 @@ extern "C" int tilert_gqa_latent_merge_op(TgContext* ctx, const float* part, int
   const LatentRow r = latent_row(rank, rot);
   TB_REQUIRE(ctx != nullptr && part != nullptr && out != nullptr && tokens >= 1 && heads >= 1 && n_splits >= 1 && n_splits <= 1024 && ldo >= rank);
   const LatentMergeParams p{part, heads * tokens, tokens, n_splits, rank, r.rankp, sink, out, ldo};
-  p.eights = p.rope.eights(rot) && dim % 8 == 0 && ldq % 4 == 0 && aligned16(q) && aligned16(rope) && aligned16(out) && aligned16(lat);
   const size_t smem = sizeof(float) * n_splits;
   if (f32) return go(latent_merge_kernel<float>, dim3(heads * tokens), dim3(128), smem, stream, p);
   return go(latent_merge_kernel<__nv_bfloat16>, dim3(heads * tokens), dim3(128), smem, stream, p);
