@@ -8,6 +8,8 @@
 #include <cmath>
 #include <initializer_list>
 #include <mutex>
+#include <set>
+#include <utility>
 
 #include "host_util.h"
 
@@ -34,10 +36,27 @@ constexpr size_t kMaxSmem = 227 * 1024;
 
 cudaStream_t stream_of(void* s) { return static_cast<cudaStream_t>(s); }
 
+// Lets a kernel have all the shared memory there is, once per kernel and device.
+cudaError_t allow_smem(const void* kernel) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> done;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({device, kernel})) return cudaSuccess;
+  cudaFuncAttributes at;
+  e = cudaFuncGetAttributes(&at, kernel);  // (the limit holds for the static part too)
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem - at.sharedSizeBytes));
+  if (e == cudaSuccess) done.insert({device, kernel});
+  return e;
+}
+
 template <typename... KArgs, typename... Args>
 int go(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, void* stream, Args&&... args) {
   TB_REQUIRE(smem <= kMaxSmem);
-  if (smem > 48 * 1024) TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  if (smem > 48 * 1024) TB_CUDA(allow_smem(reinterpret_cast<const void*>(kernel)));
   TB_CUDA(launch(kernel, grid, block, smem, stream_of(stream), std::forward<Args>(args)...));
   ++g_launches;
   TB_CUDA(cudaGetLastError());

@@ -49,11 +49,24 @@ def _p(t: torch.Tensor | None):
     return None if t is None else t.data_ptr()
 
 
+_fns: dict = {}   # operators of the loaded library by name
+_ctxs: dict = {}  # its contexts by device index; both live as long as the process
+
+
 def _call(name: str, ref: torch.Tensor, *args) -> None:
+    """A portion of a prompt is some twenty of these per layer, and few rows leave the GPU waiting for them: what does not
+    change between calls is looked up once, and the current stream is asked for without building a stream object."""
     if not ref.is_cuda:
         raise ValueError(f"{name}: CUDA tensors are needed (there is no CPU path)")
-    fn = getattr(_tb.lib(_TYPE), f"tilert_gqa_{name}_op")
-    _tb.check(fn(_tb.tilert_init(ref.device.index, _TYPE), *args, torch.cuda.current_stream(ref.device).cuda_stream), _TYPE)
+    dev = ref.get_device()
+    fn, ctx = _fns.get(name), _ctxs.get(dev)
+    if fn is None:
+        fn = _fns[name] = getattr(_tb.lib(_TYPE), f"tilert_gqa_{name}_op")
+    if ctx is None:
+        ctx = _ctxs[dev] = _tb.tilert_init(dev, _TYPE)
+    rc = fn(ctx, *args, torch._C._cuda_getCurrentRawStream(dev))
+    if rc != 0:
+        _tb.check(rc, _TYPE)
 
 
 def _need(name: str, t: torch.Tensor | None, dtype, optional: bool = False) -> None:
@@ -67,12 +80,16 @@ def _need(name: str, t: torch.Tensor | None, dtype, optional: bool = False) -> N
 
 def _f32(*acts: torch.Tensor | None) -> int:
     """1 for the exact mode; every activation operand of a call has the same type."""
-    kinds = {t.dtype for t in acts if t is not None}
-    if kinds == {F32}:
-        return 1
-    if kinds == {BF16}:
-        return 0
-    raise ValueError(f"activations must all be bfloat16 or all be float32, got {kinds}")
+    kind = None
+    for t in acts:
+        if t is None or t.dtype is kind:
+            continue
+        if kind is not None or t.dtype is not F32 and t.dtype is not BF16:
+            raise ValueError(f"activations must all be bfloat16 or all be float32, got {[t.dtype for t in acts if t is not None]}")
+        kind = t.dtype
+    if kind is None:
+        raise ValueError("activations must all be bfloat16 or all be float32, got none")
+    return int(kind is F32)
 
 
 def num_sms(device) -> int:

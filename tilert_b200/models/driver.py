@@ -177,6 +177,10 @@ class PortionDriver(SequenceDriver):
         in ``self.logits``.  Advances the position."""
         raise NotImplementedError
 
+    def _upload(self, values: list[int], dtype: torch.dtype) -> torch.Tensor:
+        """On the device, without waiting for what the stream still has to do (a copy from pageable memory would)."""
+        return torch.tensor(values, dtype=dtype, pin_memory=True).to(self.device, non_blocking=True)
+
     def _graph_key(self, pos: int) -> int:
         """A bound of the keys any layer attends to: a power of two, constant once every window is full."""
         n = 256

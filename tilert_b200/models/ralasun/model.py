@@ -73,7 +73,7 @@ class RalasunModel(PortionDriver):
     # -- prompts --
     def _prefill_portion(self, tokens: list[int], want: list[int], last: bool) -> torch.Tensor:
         a, sc, n = self.args, self.scratch, len(tokens)
-        ids = torch.tensor(tokens, dtype=I64).to(self.device)
+        ids = self._upload(tokens, I64)
         x, xh = sc.get("x", self.portion, pad(a.dim)), sc.get("xh", self.portion, pad(a.dim), dtype=self.dtype)
         ops.embed_norm(ids, self.embed, self.embed_norm, a.eps, a.dim, x, xh)
         for layer in self.layers:
@@ -82,7 +82,7 @@ class RalasunModel(PortionDriver):
                 self.layer_taps.append(x[:n, : a.dim].clone())
         out = torch.empty(len(want), a.vocab_size, dtype=F32, device=self.device)
         if want:
-            rows = torch.tensor(want, dtype=I32).to(self.device)
+            rows = self._upload(want, I32)
             xn = torch.zeros(len(want), pad(a.dim), dtype=self.dtype, device=self.device)
             ops.gather_norm(x, rows, self.final_norm, a.eps, a.dim, xn)
             ops.gemm(xn, self.head, out, len(want), a.vocab_size, a.dim)

@@ -87,7 +87,7 @@ class RozesunModel(PortionDriver):
     # -- prompts --
     def _prefill_portion(self, tokens: list[int], want: list[int], last: bool) -> torch.Tensor:
         a, sc, n = self.args, self.scratch, len(tokens)
-        ids = torch.tensor(tokens, dtype=I64).to(self.device)
+        ids = self._upload(tokens, I64)
         st = RowStream(sc.get("x", self.portion, pad(a.dim)), sc.get("xh", self.portion, pad(a.dim), dtype=self.dtype), n, a.dim, a.eps)
         ops.embed_norm(ids, self.embed, None, a.eps, a.dim, st.x)
         for layer, nr, add in self.runs:
@@ -98,7 +98,7 @@ class RozesunModel(PortionDriver):
         x = st.settle()
         out = torch.empty(len(want), a.vocab_size, dtype=F32, device=self.device)
         if want:
-            rows = torch.tensor(want, dtype=I32).to(self.device)
+            rows = self._upload(want, I32)
             xn = torch.zeros(len(want), pad(a.dim), dtype=self.dtype, device=self.device)
             ops.gather_norm(x, rows, self.final_norm, a.eps, a.dim, xn)
             ops.gemm(xn, self.embed, out, len(want), a.vocab_size, a.dim)
