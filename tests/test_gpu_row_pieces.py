@@ -98,6 +98,30 @@ def test_queries_keys_values(ops, dtype, heads, kv_heads, dim, vdim):
 
 
 @pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("dim", [8, 1992, 2048, 2816, 4096, 7168, 8192])
+def test_rms_forms_have_the_same_bits(ops, dtype, dim):
+    """An expert is chosen behind these norms: the form a row takes may not decide a near tie."""
+    rows, top = 19, 6
+    gain, gain2, x0, y = rnd(0, dim), rnd(1, dim), rnd(2, rows, dim), rnd(3, rows, dim)
+    ye, ysh = rnd(4, rows * top, dim, dtype=dtype), rnd(5, rows, dim, dtype=dtype)
+    slot = torch.randperm(rows * top, generator=torch.Generator().manual_seed(1)).to(I32).view(rows, top).cuda()
+    w = rnd(6, rows, top).softmax(-1)
+    for f in (dict(norm=gain, y=y), dict(norm=gain, y=y, norm2=gain2), dict(norm=gain, experts=ye, slot_row=slot, slot_w=w, shared=ysh)):
+        got = []
+        for x in (x0.clone(), moved(x0)):
+            xh = torch.zeros(rows, dim, dtype=dtype, device="cuda")
+            ops.residual_norm(x, xh, eps=1e-6, dim=dim, rows=rows, **f)
+            got.append((x, xh))
+        assert all(torch.equal(a, b) for a, b in zip(*got)), list(f)
+    table, toks = rnd(7, 50, dim, dtype=BF16), torch.arange(rows, device="cuda") * 2
+    got = []
+    for x in (torch.zeros(rows, dim, device="cuda"), moved(torch.zeros(rows, dim, device="cuda"))):
+        ops.embed_norm(toks, table, gain, 1e-6, dim, x)
+        got.append(x)
+    assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("heads,dim,rot,rank,q_rank", [(1, 8, 16, 8, 8), (5, 96, 32, 72, 304), (16, 128, 64, 512, 1536), (3, 40, 128, 1024, 24)])
 def test_latents_and_queries(ops, dtype, interleaved, heads, dim, rot, rank, q_rank):

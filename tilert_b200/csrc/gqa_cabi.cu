@@ -179,11 +179,13 @@ bool row_pieces(int dim, std::initializer_list<const void*> operands, std::initi
   for (long long ld : strides) ok = ok && ld % 8 == 0;
   return ok;
 }
-// The instance with just enough threads and pieces: 2048, 4096 or 8192 elements.
+// The instance with just enough threads and pieces: 2048, 4096 or 8192 elements.  `turned`: an RMS norm turns rows over in
+// shared memory.
 template <class P>
-int by_pieces(int dim, int rows, void* stream, const P& p, void (*narrow)(P), void (*one)(P), void (*two)(P)) {
+int by_pieces(int dim, int rows, bool turned, void* stream, const P& p, void (*narrow)(P), void (*one)(P), void (*two)(P)) {
   const int half = kRowThreads / 2;
-  return go(dim <= half * 8 ? narrow : (dim <= kRowThreads * 8 ? one : two), dim3(rows), dim3(dim <= half * 8 ? half : kRowThreads), 0, stream, p);
+  return go(dim <= half * 8 ? narrow : (dim <= kRowThreads * 8 ? one : two), dim3(rows), dim3(dim <= half * 8 ? half : kRowThreads),
+            turned ? sizeof(float) * dim : 0, stream, p);
 }
 
 }  // namespace
@@ -196,9 +198,9 @@ extern "C" int tilert_gqa_embed_norm_op(TgContext* ctx, const long long* tokens,
   const EmbedNormParams p{tokens, reinterpret_cast<const __nv_bfloat16*>(table), ld_table, vocab, gain, eps, dim, x, ldx, xh, ldh,
                           ctx->status};
   if (row_pieces(dim, {table, gain, x, xh}, {ld_table, ldx, ldh})) {
-    return f32 ? by_pieces(dim, rows, stream, p, embed_norm_pieces_kernel<float, 256, 1>, embed_norm_pieces_kernel<float, 512, 1>,
+    return f32 ? by_pieces(dim, rows, gain != nullptr, stream, p, embed_norm_pieces_kernel<float, 256, 1>, embed_norm_pieces_kernel<float, 512, 1>,
                            embed_norm_pieces_kernel<float, 512, 2>)
-               : by_pieces(dim, rows, stream, p, embed_norm_pieces_kernel<__nv_bfloat16, 256, 1>, embed_norm_pieces_kernel<__nv_bfloat16, 512, 1>,
+               : by_pieces(dim, rows, gain != nullptr, stream, p, embed_norm_pieces_kernel<__nv_bfloat16, 256, 1>, embed_norm_pieces_kernel<__nv_bfloat16, 512, 1>,
                            embed_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
   }
   if (f32) return go(embed_norm_kernel<float>, dim3(rows), dim3(kNormThreads), 0, stream, p);
@@ -219,9 +221,9 @@ extern "C" int tilert_gqa_residual_norm_op(TgContext* ctx, const float* y, long 
   const ResidualNormParams p{y,    ldy, ye,    lde,   slot_row, slot_w, top, ysh, ldsh, gain, bias,
                              add,  gain2, bias2, centered, eps, dim,    x,   ldx, xh,   ldh};
   if (row_pieces(dim, {y, ye, ysh, gain, bias, add, gain2, bias2, x, xh}, {ldy, lde, ldsh, ldx, ldh})) {
-    return f32 ? by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<float, 256, 1>, residual_norm_pieces_kernel<float, 512, 1>,
+    return f32 ? by_pieces(dim, rows, !centered, stream, p, residual_norm_pieces_kernel<float, 256, 1>, residual_norm_pieces_kernel<float, 512, 1>,
                            residual_norm_pieces_kernel<float, 512, 2>)
-               : by_pieces(dim, rows, stream, p, residual_norm_pieces_kernel<__nv_bfloat16, 256, 1>,
+               : by_pieces(dim, rows, !centered, stream, p, residual_norm_pieces_kernel<__nv_bfloat16, 256, 1>,
                            residual_norm_pieces_kernel<__nv_bfloat16, 512, 1>, residual_norm_pieces_kernel<__nv_bfloat16, 512, 2>);
   }
   const size_t smem = static_cast<size_t>(dim) * sizeof(float);

@@ -7,7 +7,8 @@
 // it) and have two forms.  Up to 8192 wide, in multiples of eight and with aligned rows, a thread owns one or two pieces
 // of eight elements and keeps them in registers from the loads to the stores: every operand is requested in 16-byte
 // pieces before the first reduction, and memory sees each element once.  Other shapes take an element at a time through
-// shared memory.
+// shared memory.  Both forms of an RMS norm sum the squares in one order, so that a row has the same bits in either: what
+// follows such a norm may be a choice of experts, where a last bit can decide a near tie.
 #pragma once
 
 #include "act.cuh"
@@ -54,19 +55,27 @@ __device__ __forceinline__ void each_piece(int dim, Each each) {
     if (e < dim) each(j, e);
   }
 }
-// Pieces beyond dim hold zeros.
+// Pieces beyond dim hold zeros.  The RMS norm turns the row over in shared memory (`vals`, [dim]) and sums as row_stat with
+// kNormThreads threads does.
 template <int TH, int NJ>
-__device__ __forceinline__ RowStat piece_stat(const float (&v)[NJ][8], int dim, float eps, int centered, float* red) {
-  float mean = 0.f;
-  if (centered) {
-    float s = 0.f;
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) s += v[j][q];
-    mean = cta_sum(s, red) / static_cast<float>(dim);
-  }
+__device__ __forceinline__ RowStat piece_stat(const float (&v)[NJ][8], int dim, float eps, int centered, float* red, float* vals) {
   float ss = 0.f;
+  if (!centered) {
+    static_assert(TH >= kNormThreads, "every partial sum has its thread");
+    each_piece<TH, NJ>(dim, [&](int j, int e) { act_st8(vals + e, v[j]); });
+    __syncthreads();
+    if (threadIdx.x < kNormThreads) {
+#pragma unroll 8
+      for (int i = threadIdx.x; i < dim; i += kNormThreads) ss += vals[i] * vals[i];
+    }
+    return {0.f, 1.f / sqrtf(cta_sum(ss, red) / static_cast<float>(dim) + eps)};
+  }
+  float s = 0.f;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += v[j][q];
+  const float mean = cta_sum(s, red) / static_cast<float>(dim);
   each_piece<TH, NJ>(dim, [&](int j, int) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) ss += (v[j][q] - mean) * (v[j][q] - mean);
@@ -122,6 +131,7 @@ template <typename T, int TH, int NJ>
 __global__ void __launch_bounds__(TH) embed_norm_pieces_kernel(const EmbedNormParams p) {
   pdl_launch_dependents();
   pdl_wait();
+  extern __shared__ __align__(16) float vals[];  // [dim], with a gain
   __shared__ float red[32];
   const int t = blockIdx.x;
   const long long tok = p.tokens[t];
@@ -133,7 +143,7 @@ __global__ void __launch_bounds__(TH) embed_norm_pieces_kernel(const EmbedNormPa
   float v[NJ][8] = {};
   each_piece<TH, NJ>(p.dim, [&](int j, int e) { act_ld8(row + e, v[j]); });
   if (p.gain != nullptr) {
-    const RowStat st = piece_stat<TH, NJ>(v, p.dim, p.eps, 0, red);
+    const RowStat st = piece_stat<TH, NJ>(v, p.dim, p.eps, 0, red, vals);
     each_piece<TH, NJ>(p.dim, [&](int j, int e) { norm_piece(v[j], st, p.gain, nullptr, e); });
   }
   each_piece<TH, NJ>(p.dim, [&](int j, int e) {
@@ -230,6 +240,7 @@ template <typename T, int TH, int NJ>
 __global__ void __launch_bounds__(TH, NJ == 1 ? 1536 / TH : 1024 / TH) residual_norm_pieces_kernel(const ResidualNormParams p) {
   pdl_launch_dependents();
   pdl_wait();
+  extern __shared__ __align__(16) float vals[];  // [dim], not centered
   __shared__ float red[32];
   const int t = blockIdx.x;
   float* x = p.x + t * p.ldx;
@@ -259,7 +270,7 @@ __global__ void __launch_bounds__(TH, NJ == 1 ? 1536 / TH : 1024 / TH) residual_
       });
   }
   if (p.gain != nullptr) {
-    const RowStat st = piece_stat<TH, NJ>(v, p.dim, p.eps, p.centered, red);
+    const RowStat st = piece_stat<TH, NJ>(v, p.dim, p.eps, p.centered, red, vals);
     each_piece<TH, NJ>(p.dim, [&](int j, int e) {
       norm_piece(v[j], st, p.gain, p.bias, e);
 #pragma unroll
@@ -277,7 +288,7 @@ __global__ void __launch_bounds__(TH, NJ == 1 ? 1536 / TH : 1024 / TH) residual_
   if (p.xh == nullptr) return;
   T* xh = reinterpret_cast<T*>(p.xh) + t * p.ldh;
   if (p.gain2 != nullptr) {
-    const RowStat st = piece_stat<TH, NJ>(r, p.dim, p.eps, p.centered, red);
+    const RowStat st = piece_stat<TH, NJ>(r, p.dim, p.eps, p.centered, red, vals);
     each_piece<TH, NJ>(p.dim, [&](int j, int e) { norm_piece(r[j], st, p.gain2, p.bias2, e); });
   }
   each_piece<TH, NJ>(p.dim, [&](int j, int e) { act_st8(xh + e, r[j]); });
