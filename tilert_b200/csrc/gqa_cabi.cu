@@ -6,6 +6,7 @@
 #include <cuda.h>
 
 #include <cmath>
+#include <exception>
 #include <initializer_list>
 #include <mutex>
 #include <set>
@@ -36,8 +37,8 @@ constexpr size_t kMaxSmem = 227 * 1024;
 
 cudaStream_t stream_of(void* s) { return static_cast<cudaStream_t>(s); }
 
-// Lets a kernel have all the shared memory there is, once per kernel and device.
-cudaError_t allow_smem(const void* kernel) {
+// Lets a kernel have all the shared memory there is, once per kernel and device.  (No exception leaves a C entry point.)
+cudaError_t allow_smem(const void* kernel) try {
   static std::mutex mu;
   static std::set<std::pair<int, const void*>> done;
   int device = 0;
@@ -51,6 +52,8 @@ cudaError_t allow_smem(const void* kernel) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem - at.sharedSizeBytes));
   if (e == cudaSuccess) done.insert({device, kernel});
   return e;
+} catch (const std::exception&) {
+  return cudaErrorMemoryAllocation;
 }
 
 template <typename... KArgs, typename... Args>
