@@ -14,6 +14,7 @@
 
 #include "host_util.h"
 
+#include "expanded_attention.cuh"
 #include "gemm_rows.cuh"
 #include "latent_attention.cuh"
 #include "latent_rows.cuh"
@@ -676,6 +677,41 @@ extern "C" int tilert_gqa_gate_heads_op(TgContext* ctx, const float* o, int ldv,
   return go(gate_heads_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, p);
 }
 
+namespace {
+
+template <int NQ>
+int launch_expanded(const ExpandedAttnParams& p, const CUtensorMap& q, const CUtensorMap& kv, const CUtensorMap& rot, void* stream) {
+  const dim3 grid(p.heads, (p.rows + NQ * kXaTile - 1) / (NQ * kXaTile));
+  return go(expanded_attn_kernel<NQ>, grid, dim3(128 + 128 * NQ), expanded_attn_smem(NQ, p.k_boxes, p.v_boxes, p.v_stages), stream, q, kv, rot, p);
+}
+
+// tcgen05 tiles: at least a tile of tokens (the key tiles of fewer could reach past the rows in use), sizes whose tiles fit.
+bool expanded_tiles_fit(int rows, int dimp, int rotp, int vdimp, float scale) {
+  const int k_boxes = (dimp + 63) / 64 + (rotp + 63) / 64, v_boxes = (vdimp + 63) / 64;
+  return rows >= kXaTile && vdimp <= 128 && scale > 0.f && expanded_attn_smem(2, k_boxes, v_boxes, 1) + 1024 <= kMaxSmem;
+}
+
+int run_expanded(TgContext* ctx, ExpandedAttnParams& p, const void* q, const void* kv, const void* cache, int row, void* stream) {
+  p.dim_boxes = (p.dimp + 63) / 64;
+  p.k_boxes = p.dim_boxes + (p.rotp + 63) / 64;
+  p.v_boxes = (p.vdimp + 63) / 64;
+  // A CTA takes about as long for two query tiles as for one (the products of one run under the softmax of the other): two,
+  // unless one each takes no more rounds over the SMs.
+  auto rounds = [&](int nq) { return (p.heads * ((p.rows + nq * kXaTile - 1) / (nq * kXaTile)) + ctx->num_sms - 1) / ctx->num_sms; };
+  const int nq = rounds(1) <= rounds(2) ? 1 : 2;
+  p.v_stages = 3;
+  while (p.v_stages > 1 && expanded_attn_smem(nq, p.k_boxes, p.v_boxes, p.v_stages) + 1024 > kMaxSmem) --p.v_stages;
+  const int wide = p.dimp + p.rotp, cols = p.heads * (p.dimp + p.vdimp);
+  CUtensorMap qm, kvm, rm;
+  int rc = make_map(&qm, q, p.rows, p.heads * wide, static_cast<long long>(p.heads) * wide, kXaTile);
+  if (rc == TB_OK) rc = make_map(&kvm, kv, p.ring, cols, cols, kXaTile);
+  if (rc == TB_OK) rc = make_map(&rm, cache, p.ring, row, row, kXaTile);
+  if (rc != TB_OK) return rc;
+  return nq == 2 ? launch_expanded<2>(p, qm, kvm, rm, stream) : launch_expanded<1>(p, qm, kvm, rm, stream);
+}
+
+}  // namespace
+
 extern "C" int tilert_gqa_expanded_attn_op(TgContext* ctx, const void* q, const void* kv, const void* cache, int rows, int heads, int dim,
                                            int rot, int vdim, int rank, const int* pos, int window, int ring, float scale,
                                            const float* sink, const float* gate, long long ldg, int per_head, void* out, long long ldo,
@@ -688,6 +724,27 @@ extern "C" int tilert_gqa_expanded_attn_op(TgContext* ctx, const void* q, const 
   TB_REQUIRE(aligned16(q) && aligned16(kv) && aligned16(cache) && dim >= 1 && vdim >= 1 && window >= 0 && window + rows - 1 <= ring);
   TB_REQUIRE(prefill_attn_fits(dimp + rotp, vdimp) && ldo >= static_cast<long long>(heads) * vdim && (vdim % 2 == 1 || ldo % 2 == 0));
   TB_REQUIRE(gate == nullptr || ldg >= (per_head ? heads : heads * vdim));
+  if (expanded_tiles_fit(rows, dimp, rotp, vdimp, scale)) {
+    ExpandedAttnParams e{};
+    e.rows = rows;
+    e.heads = heads;
+    e.dimp = dimp;
+    e.rotp = rotp;
+    e.vdim = vdim;
+    e.vdimp = vdimp;
+    e.rankp = r.rankp;
+    e.ring = ring;
+    e.window = window;
+    e.pos = pos;
+    e.scale = scale;
+    e.sink = sink;
+    e.gate = {gate, ldg, gate != nullptr ? per_head : 0};
+    e.out = reinterpret_cast<__nv_bfloat16*>(out);
+    e.ldo = ldo;
+    e.eights = vdim % 8 == 0 && ldo % 8 == 0 && aligned16(out) && (gate == nullptr || per_head || (ldg % 4 == 0 && aligned16(gate)));
+    e.status = ctx->status;
+    return run_expanded(ctx, e, q, kv, cache, r.row, stream);
+  }
   AttnPrefillParams p{};
   p.s = {heads, heads, dim + rot, vdim, dimp + rotp, vdimp, ring, window};
   p.pos = pos;
