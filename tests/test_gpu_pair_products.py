@@ -1,0 +1,70 @@
+"""Products of many rows on pairs of SMs against f64 on the same bf16 operands, at the edges of their tiles.
+
+The tensor cores add sixteen products at a time to an f32 sum and may cut off what does not fit: up to 2^-23 of the sum (of
+size 8 at most here) in each of k / 16 steps, and a few more such roundings in the bias or the gated unit.  A bf16 result adds
+2^-9 of its value."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BF16, F32, F64, I32 = torch.bfloat16, torch.float32, torch.float64, torch.int32
+
+
+@pytest.fixture(scope="module")
+def ops():
+    import tilert_b200 as tb
+    from tilert_b200 import gqa_ops
+
+    tb.load_backend("ralasun")
+    tb.tilert_init(0, "ralasun")
+    yield gqa_ops
+    assert tb.device_status(0, "ralasun") == 0
+
+
+def padded(ops, gen, rows, k, std):
+    t = torch.zeros(rows, ops.pad(k), dtype=BF16, device="cuda")
+    t[:, :k] = torch.randn(rows, k, generator=gen, device="cuda") * std
+    return t
+
+
+def check(ops, n, k, gated, out_type, counts, rows=None):
+    gen = torch.Generator(device="cuda").manual_seed(n * 31 + k)
+    total = rows or sum(counts)
+    groups = 0 if counts is None else len(counts)
+    x = padded(ops, gen, total, k, 1.0)
+    w = padded(ops, gen, max(groups, 1) * (2 if gated else 1) * n, k, 1.5 * k ** -0.5)
+    bias = None if groups or gated else torch.randn(n, generator=gen, device="cuda")
+    out = torch.full((total + 3, ops.pad(n)), 77.0, dtype=out_type, device="cuda")
+    ops.gemm(x, w, out, total, n, k, gated=(1.5, 1.702) if gated else None, n_groups=groups,
+             counts=None if counts is None else torch.tensor(counts, dtype=I32, device="cuda"), bias=bias)
+    bound = (k / 16 + 8) * 2.0 ** -23 * 8
+    ws = w.to(F64).view(max(groups, 1), 2 if gated else 1, n, -1)
+    lo = 0
+    for g, c in enumerate(counts or [total]):
+        z = torch.einsum("tk,hnk->htn", x[lo: lo + c].to(F64), ws[g])
+        if gated:
+            a, u = z[0].clamp(max=1.5), z[1].clamp(-1.5, 1.5)
+            want = a * torch.sigmoid(1.702 * a) * (u + 1)
+        else:
+            want = z[0] + (0 if bias is None else bias.to(F64))
+        off = (out[lo: lo + c, :n].to(F64) - want).abs()
+        assert float((off - (2.0 ** -8 * want.abs() if out_type == BF16 else 0)).max() if c else 0) <= bound, (g, c)
+        lo += c
+    assert bool((out[total:] == 77).all()) and bool((out[:, n:] == 77).all())  # nothing beyond the rows and features
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("out_type", [BF16, F32])
+@pytest.mark.parametrize("n,k", [(7, 8), (129, 72), (136, 64), (258, 200), (512, 136)])
+@pytest.mark.parametrize("counts", [[0, 1, 300], [64, 64, 65, 63], [257, 512, 0, 255, 1]])
+def test_groups(ops, gated, out_type, n, k, counts):
+    check(ops, n, k, gated, out_type, counts)
+
+
+@pytest.mark.parametrize("rows,n,k,gated,out_type", [
+    (2048, 700, 2000, False, F32), (2047, 1288, 1000, True, BF16), (1357, 4104, 520, False, BF16), (1025, 2049, 1032, True, BF16),
+    (700, 3000, 2000, False, F32), (37, 5632, 1024, True, BF16), (257, 20001, 72, False, F32)])
+def test_one_weight(ops, rows, n, k, gated, out_type):
+    check(ops, n, k, gated, out_type, None, rows)

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int k_bytes = p.k_boxes * kXaBox, v_bytes = p.v_boxes * kXaBox;
   uint8_t* qs = base;
   uint8_t* ks = qs + NQ * k_bytes;
@@ -159,12 +159,12 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&s_tmem);
+  const uint32_t tmem = warp_uniform(*reinterpret_cast<volatile uint32_t*>(&s_tmem));
   pdl_wait();
 
   // heads vary fastest and the tokens with the longest key ranges come first
   const int head = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * (NQ * kXaTile);
-  const int pos0 = *p.pos;
+  const int pos0 = warp_uniform(*p.pos);
   const int win = p.window > 0 ? p.window : 0x7fffffff;
   // keys that query tile i sees: [lo(i), hi(i)); tile 0 always has tokens
   auto lo_of = [&](int i) { return p.window > 0 ? max(0, pos0 + t0 + i * kXaTile - p.window + 1) : 0; };
@@ -175,23 +175,25 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
   volatile int* abort = &s_abort;
 
   if (warp == 0) {  // queries and keys
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&q_full, nq * k_bytes);
       for (int i = 0; i < nq; ++i)
         for (int c = 0; c < p.k_boxes; ++c) {
           const int x = head * (p.dimp + p.rotp) + (c < p.dim_boxes ? c * 64 : p.dimp + (c - p.dim_boxes) * 64);
           tma_load_2d(qs + i * k_bytes + c * kXaBox, &qmap, x, t0 + i * kXaTile, &q_full);
         }
-      uint32_t it = 0;
-      for (int a = lo; a < hi; ++it) {
-        const XaKeyTile t(a, hi, p.ring);
-        a = t.b;
-        const uint32_t s = it % kXaKeyStages;
-        if (!mbar_wait(&k_empty[s], ((it / kXaKeyStages) & 1u) ^ 1u, abort)) {
-          set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
-          *abort = 1;
-          break;
-        }
+    }
+    uint32_t it = 0;
+    for (int a = lo; a < hi; ++it) {
+      const XaKeyTile t(a, hi, p.ring);
+      a = t.b;
+      const uint32_t s = it % kXaKeyStages;
+      if (!mbar_wait_warp(&k_empty[s], ((it / kXaKeyStages) & 1u) ^ 1u, abort)) {
+        set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+        *abort = 1;
+        break;
+      }
+      if (elect_one()) {
         mbar_expect_tx(&k_full[s], k_bytes);
         for (int c = 0; c < p.k_boxes; ++c) {
           uint8_t* dst = ks + s * k_bytes + c * kXaBox;
@@ -201,93 +203,93 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
             tma_load_2d(dst, &rotmap, p.rankp + (c - p.dim_boxes) * 64, t.row0, &k_full[s]);
         }
       }
-      // copies still in flight must land before this CTA's shared memory goes away
-      mbar_wait(&q_full, 0);
-      for (uint32_t j = it > kXaKeyStages ? it - kXaKeyStages : 0; j < it; ++j) mbar_wait(&k_full[j % kXaKeyStages], (j / kXaKeyStages) & 1u);
     }
+    // copies still in flight must land before this CTA's shared memory goes away
+    mbar_wait(&q_full, 0);
+    for (uint32_t j = it > kXaKeyStages ? it - kXaKeyStages : 0; j < it; ++j) mbar_wait(&k_full[j % kXaKeyStages], (j / kXaKeyStages) & 1u);
   } else if (warp == 2) {  // values, on their own: they wait for other products than the keys do
-    if (lane == 0) {
-      const uint32_t stages = p.v_stages;
-      uint32_t it = 0;
-      for (int a = lo; a < hi; ++it) {
-        const XaKeyTile t(a, hi, p.ring);
-        a = t.b;
-        const uint32_t s = it % stages;
-        if (!mbar_wait(&v_empty[s], ((it / stages) & 1u) ^ 1u, abort)) {
-          set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
-          *abort = 1;
-          break;
-        }
+    const uint32_t stages = p.v_stages;
+    uint32_t it = 0;
+    for (int a = lo; a < hi; ++it) {
+      const XaKeyTile t(a, hi, p.ring);
+      a = t.b;
+      const uint32_t s = it % stages;
+      if (!mbar_wait_warp(&v_empty[s], ((it / stages) & 1u) ^ 1u, abort)) {
+        set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+        *abort = 1;
+        break;
+      }
+      if (elect_one()) {
         mbar_expect_tx(&v_full[s], v_bytes);
         for (int c = 0; c < p.v_boxes; ++c)
           tma_load_2d(vs + s * v_bytes + c * kXaBox, &kvmap, p.heads * p.dimp + head * p.vdimp + c * 64, t.row0, &v_full[s]);
       }
-      for (uint32_t j = it > stages ? it - stages : 0; j < it; ++j) mbar_wait(&v_full[j % stages], (j / stages) & 1u);
     }
+    for (uint32_t j = it > stages ? it - stages : 0; j < it; ++j) mbar_wait(&v_full[j % stages], (j / stages) & 1u);
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t s_idesc = umma_idesc_bf16(kXaTile, kXaTile), v_idesc = umma_idesc_bf16(kXaTile, p.vdimp) | (1u << 16);
-      const uint64_t qd0 = umma_desc_sw128(smem_u32(qs)), kd0 = umma_desc_sw128(smem_u32(ks)), vd0 = umma_desc_sw128_columns(smem_u32(vs));
-      auto scores = [&](int i, uint32_t stage) {
-        uint64_t qd = qd0 + static_cast<uint32_t>(i * k_bytes >> 4), kd = kd0 + (stage * k_bytes >> 4);
-        const uint32_t d = tmem + i * kXaTile;
-        for (int c = 0; c < p.k_boxes; ++c, qd += kXaBox >> 4, kd += kXaBox >> 4) {
-          const int left = c < p.dim_boxes ? p.dimp / 16 - c * 4 : p.rotp / 16 - (c - p.dim_boxes) * 4;  // steps of 16 columns, 32 bytes
-          if (left >= 4) {
+    const uint32_t s_idesc = umma_idesc_bf16(kXaTile, kXaTile), v_idesc = umma_idesc_bf16(kXaTile, p.vdimp) | (1u << 16);
+    const uint64_t qd0 = umma_desc_sw128(smem_u32(qs)), kd0 = umma_desc_sw128(smem_u32(ks)), vd0 = umma_desc_sw128_columns(smem_u32(vs));
+    auto scores = [&](int i, uint32_t stage) {
+      uint64_t qd = qd0 + static_cast<uint32_t>(i * k_bytes >> 4), kd = kd0 + (stage * k_bytes >> 4);
+      const uint32_t d = tmem + i * kXaTile;
+      for (int c = 0; c < p.k_boxes; ++c, qd += kXaBox >> 4, kd += kXaBox >> 4) {
+        const int left = c < p.dim_boxes ? p.dimp / 16 - c * 4 : p.rotp / 16 - (c - p.dim_boxes) * 4;  // steps of 16 columns, 32 bytes
+        if (left >= 4) {
+          if (elect_one()) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) umma_bf16(d, qd + 2 * q, kd + 2 * q, s_idesc, c | q);
-          } else {
-            for (int q = 0; q < left; ++q) umma_bf16(d, qd + 2 * q, kd + 2 * q, s_idesc, c | q);
           }
+        } else if (elect_one()) {
+          for (int q = 0; q < left; ++q) umma_bf16(d, qd + 2 * q, kd + 2 * q, s_idesc, c | q);
         }
-        umma_commit(&s_full[i]);
-      };
-      auto values = [&](int i, uint32_t stage, bool first) {
-        const uint64_t vd = vd0 + (stage * v_bytes >> 4);
+      }
+      if (elect_one()) umma_commit(&s_full[i]);
+    };
+    auto values = [&](int i, uint32_t stage, bool first) {
+      const uint64_t vd = vd0 + (stage * v_bytes >> 4);
+      if (elect_one()) {
 #pragma unroll
         for (int c = 0; c < kXaTile / 16; ++c)  // sixteen keys: eight columns of probabilities, sixteen rows of values
           umma_bf16_ta(tmem + (NQ + i) * kXaTile, tmem + i * kXaTile + c * 8, vd + c * (2048 >> 4), v_idesc, !first || c != 0);
-      };
-      bool ok = mbar_wait(&q_full, 0, abort);
-      uint32_t n_p[NQ] = {};  // tiles whose probabilities have been taken
-      uint32_t it = 0;
-      int prev = -1;          // beginning of the tile before
-      for (int a = lo; ok; ++it) {
-        const bool more = a < hi;
-        const XaKeyTile t(more ? a : hi - 1, hi, p.ring), u(prev < 0 ? lo : prev, hi, p.ring);
-        const uint32_t ksg = it % kXaKeyStages, vsg = (it - 1) % p.v_stages;
-        if (prev >= 0) ok = mbar_wait(&v_full[vsg], ((it - 1) / p.v_stages) & 1u, abort);
+      }
+    };
+    bool ok = mbar_wait_warp(&q_full, 0, abort);
+    uint32_t n_p[NQ] = {};  // tiles whose probabilities have been taken
+    uint32_t it = 0;
+    int prev = -1;          // beginning of the tile before
+    for (int a = lo; ok; ++it) {
+      const bool more = a < hi;
+      const XaKeyTile t(more ? a : hi - 1, hi, p.ring), u(prev < 0 ? lo : prev, hi, p.ring);
+      const uint32_t ksg = it % kXaKeyStages, vsg = (it - 1) % p.v_stages;
+      if (prev >= 0) ok = mbar_wait_warp(&v_full[vsg], ((it - 1) / p.v_stages) & 1u, abort);
 #pragma unroll
-        for (int i = 0; i < NQ; ++i) {
-          if (ok && prev >= 0 && sees(i, u)) {
-            ok = mbar_wait(&p_full[i], n_p[i] & 1u, abort);
-            if (ok) {
-              tc_fence_after();
-              values(i, vsg, n_p[i] == 0);
-              ++n_p[i];
-              if (u.b >= hi_of(i)) umma_commit(&o_full[i]);
-            }
-          }
-          if (ok && more && i == 0) ok = mbar_wait(&k_full[ksg], (it / kXaKeyStages) & 1u, abort);
-          if (ok && more && sees(i, t)) {
+      for (int i = 0; i < NQ; ++i) {
+        if (ok && prev >= 0 && sees(i, u)) {
+          ok = mbar_wait_warp(&p_full[i], n_p[i] & 1u, abort);
+          if (ok) {
             tc_fence_after();
-            scores(i, ksg);
+            values(i, vsg, n_p[i] == 0);
+            ++n_p[i];
+            if (u.b >= hi_of(i) && elect_one()) umma_commit(&o_full[i]);
           }
         }
-        if (!ok) break;
-        if (prev >= 0) umma_commit(&v_empty[vsg]);
-        if (!more) break;
-        umma_commit(&k_empty[ksg]);
-        prev = a;
-        a = t.b;
+        if (ok && more && i == 0) ok = mbar_wait_warp(&k_full[ksg], (it / kXaKeyStages) & 1u, abort);
+        if (ok && more && sees(i, t)) scores(i, ksg);
       }
-      if (!ok) {
-        set_status(p.status, ST_WAIT_FULL_TIMEOUT);
-        *abort = 1;
-      }
-      umma_commit(&drain);  // products still running read shared memory and write TMEM
-      mbar_wait(&drain, 0);
+      if (!ok) break;
+      if (prev >= 0 && elect_one()) umma_commit(&v_empty[vsg]);
+      if (!more) break;
+      if (elect_one()) umma_commit(&k_empty[ksg]);
+      prev = a;
+      a = t.b;
     }
+    if (!ok) {
+      set_status(p.status, ST_WAIT_FULL_TIMEOUT);
+      *abort = 1;
+    }
+    __syncwarp();
+    if (elect_one()) umma_commit(&drain);  // products still running read shared memory and write TMEM
+    mbar_wait(&drain, 0);
   } else if (warp >= 4 && (warp - 4) / 4 < nq) {
     const int i = (warp - 4) / 4, quad = warp & 3;
     const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;

@@ -1,6 +1,7 @@
 // Products of many token rows with bf16 weights (prefill):  out[t, n] = W[n, :] . x[t, :].
 //
-//   gemm_tc_kernel<BN, GATED>   bf16 rows on the tensor cores
+//   gemm_tc_kernel<BN, GATED>   bf16 rows on the tensor cores, an SM on a tile: few tokens, small groups
+//   gemm_pair_kernel<GATED>     the same, a pair of SMs on a tile
 //   gemm_f32_kernel<.., GATED>  f32 rows, f32 arithmetic (the exact mode)
 //
 // GATED: the weight holds gate rows, then up rows, and the result is their clamped gated unit.
@@ -53,6 +54,10 @@ struct TileWalk {
   struct Tile {
     int group, feature0, row0, row1;
   };
+  __device__ __forceinline__ Tile at_warp(int i) {  // the same by a whole warp
+    const Tile t = at(i);
+    return {warp_uniform(t.group), warp_uniform(t.feature0), warp_uniform(t.row0), warp_uniform(t.row1)};
+  }
   __device__ __forceinline__ Tile at(int i) {  // i must not decrease between calls
     while (i >= tiles0[group + 1]) ++group;
     const int local = i - tiles0[group], r0 = rows0[group], r1 = rows0[group + 1];
@@ -173,6 +178,46 @@ __device__ __forceinline__ uint4 turn_eight(const float* v, int lane) {
   return b2 ? make_uint4(g0, g1, lo[1], hi[1]) : make_uint4(lo[0], hi[0], g0, g1);
 }
 
+enum StoreForm : int { STORE_F32, STORE_EIGHTS, STORE_PAIRS, STORE_ONES };
+__device__ __forceinline__ StoreForm store_form(const GemmRowsParams& p) {
+  if (!p.out_bf16) return STORE_F32;
+  if ((p.n & 7) == 0 && (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0) return STORE_EIGHTS;
+  return (p.n & 1) == 0 && (p.ldo & 1) == 0 ? STORE_PAIRS : STORE_ONES;
+}
+// Stores v[j], feature f of row `row0 + j` (below row1); eight lanes that begin at a multiple of eight have eight features
+// in a row and the same rows.
+__device__ __forceinline__ void store_eight(const GemmRowsParams& p, StoreForm how, const float* v, int f, bool f_ok, int row0, int row1, int lane) {
+  const int left = row1 - row0;
+  const long long at = static_cast<long long>(row0) * p.ldo;
+  if (how == STORE_F32) {
+    float* o = reinterpret_cast<float*>(p.out) + at + f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (f_ok && j < left) o[j * p.ldo] = v[j];
+  } else if (how == STORE_EIGHTS) {
+    // the lanes turn their eight features of eight rows over: a lane stores eight features of one row
+    const uint4 w = turn_eight(v, lane);
+    const int j = lane & 7;
+    if (f_ok && j < left) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + at + j * p.ldo + (f & ~7)) = w;
+  } else if (how == STORE_PAIRS) {
+    // neighbouring lanes exchange one value, so that a lane stores two features of one row
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + at + (f & ~1);
+    const bool odd = lane & 1;
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+      const int jj = j + (odd ? 1 : 0);
+      const uint32_t w = odd ? pack_bf16x2(got, v[j + 1]) : pack_bf16x2(v[j], got);
+      if (f_ok && jj < left) *reinterpret_cast<uint32_t*>(o + jj * p.ldo) = w;
+    }
+  } else {
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + at + f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (f_ok && j < left) o[j * p.ldo] = f2bf(v[j]);
+  }
+}
+
 template <int BN, bool GATED>
 __global__ void __launch_bounds__(kTcThreads, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const GemmRowsParams p) {
@@ -183,7 +228,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   __shared__ int s_abort;
   __shared__ int s_rows[kMaxGroups + 1], s_tiles[kMaxGroups + 1];
   uint8_t* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
@@ -207,89 +252,89 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&s_tmem);
+  const uint32_t tmem = warp_uniform(*reinterpret_cast<volatile uint32_t*>(&s_tmem));
   pdl_wait();
   const int ft = (p.n + 127) / 128;
   tile_prefix(p, BN, ft, s_rows, s_tiles);
   const int groups = p.n_groups > 0 ? p.n_groups : 1;
-  const int n_tiles = s_tiles[groups];
+  const int n_tiles = warp_uniform(s_tiles[groups]);
   const int n_kb = (p.k + kTcK - 1) / kTcK;
   volatile int* abort = &s_abort;
   TileWalk walk{s_rows, s_tiles, groups, ft, BN};
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x) {
-        const TileWalk::Tile t = walk.at(i);
-        const int wrow = t.group * (GATED ? 2 : 1) * p.n + t.feature0;
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const uint32_t s = it % S::kStages, ph = (it / S::kStages) & 1u;
-          if (!mbar_wait(&empty[s], ph ^ 1u, abort)) {
-            set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
-            ok = false;
-            break;
-          }
-          uint8_t* st = ring + s * S::kStageBytes;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x) {
+      const TileWalk::Tile t = walk.at_warp(i);
+      const int wrow = t.group * (GATED ? 2 : 1) * p.n + t.feature0;
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        const uint32_t s = it % S::kStages, ph = (it / S::kStages) & 1u;
+        if (!mbar_wait_warp(&empty[s], ph ^ 1u, abort)) {
+          set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+          ok = false;
+          break;
+        }
+        uint8_t* st = ring + s * S::kStageBytes;
+        if (elect_one()) {
           mbar_expect_tx(&full[s], S::kStageBytes);
           tma_load_2d(st, &wmap, kb * kTcK, wrow, &full[s]);
           if (GATED) tma_load_2d(st + S::kWBytes, &wmap, kb * kTcK, wrow + p.n, &full[s]);
           tma_load_2d(st + (GATED ? 2 : 1) * S::kWBytes, &xmap, kb * kTcK, t.row0, &full[s]);
         }
       }
-      if (!ok) *abort = 1;
-      // copies still in flight must land before this CTA's shared memory goes away
-      for (uint32_t j = it > S::kStages ? it - S::kStages : 0; j < it; ++j) mbar_wait(&full[j % S::kStages], (j / S::kStages) & 1u);
     }
+    if (!ok) *abort = 1;
+    // copies still in flight must land before this CTA's shared memory goes away
+    for (uint32_t j = it > S::kStages ? it - S::kStages : 0; j < it; ++j) mbar_wait(&full[j % S::kStages], (j / S::kStages) & 1u);
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, BN);
-      uint32_t it = 0, n_done = 0;
-      bool ok = true;
-      for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x, ++n_done) {
-        const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
-        if (!mbar_wait(&acc_empty[buf], aph ^ 1u, abort)) {
-          set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+    constexpr uint32_t idesc = umma_idesc_bf16(128, BN);
+    uint32_t it = 0, n_done = 0;
+    bool ok = true, seen = false;
+    for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x, ++n_done) {
+      const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
+      if (!mbar_wait_warp(&acc_empty[buf], aph ^ 1u, abort)) {
+        set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t d = tmem + buf * S::kAccCols;
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        const uint32_t s = it % S::kStages, ph = (it / S::kStages) & 1u;
+        if (!mbar_wait_warp(&full[s], ph, abort, seen)) {
+          set_status(p.status, ST_WAIT_FULL_TIMEOUT);
           ok = false;
           break;
         }
-        tc_fence_after();
-        const uint32_t d = tmem + buf * S::kAccCols;
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const uint32_t s = it % S::kStages, ph = (it / S::kStages) & 1u;
-          if (!mbar_wait(&full[s], ph, abort)) {
-            set_status(p.status, ST_WAIT_FULL_TIMEOUT);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t base = smem_u32(ring + s * S::kStageBytes);
-          const uint64_t wd = umma_desc_sw128(base), ud = umma_desc_sw128(base + S::kWBytes);
-          const uint64_t xd = umma_desc_sw128(base + (GATED ? 2 : 1) * S::kWBytes);
+        seen = mbar_test(&full[(it + 1) % S::kStages], ((it + 1) / S::kStages) & 1u);  // (known by the time it is asked for)
+        const uint32_t base = smem_u32(ring + s * S::kStageBytes);
+        const uint64_t wd = umma_desc_sw128(base), ud = umma_desc_sw128(base + S::kWBytes);
+        const uint64_t xd = umma_desc_sw128(base + (GATED ? 2 : 1) * S::kWBytes);
+        if (elect_one()) {
 #pragma unroll
           for (int q = 0; q < kTcK / 16; ++q) {  // 32 bytes along K per instruction
             umma_bf16(d, wd + 2 * q, xd + 2 * q, idesc, (kb | q) != 0);
             if (GATED) umma_bf16(d + BN, ud + 2 * q, xd + 2 * q, idesc, (kb | q) != 0);
           }
           umma_commit(&empty[s]);
+          if (kb == n_kb - 1) umma_commit(&acc_full[buf]);
         }
-        if (ok) umma_commit(&acc_full[buf]);
       }
-      if (!ok) *abort = 1;
-      umma_commit(&drain);  // products still running read shared memory and write TMEM
-      mbar_wait(&drain, 0);
     }
+    if (!ok) *abort = 1;
+    __syncwarp();
+    if (elect_one()) umma_commit(&drain);  // products still running read shared memory and write TMEM
+    mbar_wait(&drain, 0);
   } else {
     const int quad = warp & 3;  // TMEM lanes this warp may read
     constexpr int kCols = BN / (kTcEpiWarps / 4);
     const int c0 = (warp - 2) / 4 * kCols;  // its columns
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const bool pairs = p.out_bf16 && (p.n & 1) == 0 && (p.ldo & 1) == 0;
-    const bool eights = p.out_bf16 && (p.n & 7) == 0 && (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+    const StoreForm how = store_form(p);
     uint32_t n_done = 0;
     for (int i = blockIdx.x; i < n_tiles; i += gridDim.x, ++n_done) {
-      const TileWalk::Tile t = walk.at(i);
+      const TileWalk::Tile t = walk.at_warp(i);
       const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
       const bool ok = mbar_wait(&acc_full[buf], aph, abort);
       if (__any_sync(0xffffffffu, !ok)) {  // warp-uniform: tcgen05.ld needs every lane
@@ -318,38 +363,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias;
         }
-        const int left = t.row1 - (t.row0 + c);
-        if (!p.out_bf16) {
-          float* o = reinterpret_cast<float*>(p.out) + static_cast<long long>(t.row0 + c) * p.ldo + f;
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (f_ok && j < left) o[j * p.ldo] = v[j];
-        } else if (eights) {
-          // eight lanes turn their eight features of eight tokens over: a lane stores eight features of one token
-          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(t.row0 + c) * p.ldo + (f & ~7);
-#pragma unroll
-          for (int j = 0; j < 16; j += 8) {
-            const uint4 w = turn_eight(v + j, lane);
-            const int jj = j + (lane & 7);
-            if (f_ok && jj < left) *reinterpret_cast<uint4*>(o + jj * p.ldo) = w;
-          }
-        } else if (pairs) {
-          // neighbouring lanes exchange one value, so that a lane stores two features of one token
-          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(t.row0 + c) * p.ldo + (f & ~1);
-          const bool odd = lane & 1;
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
-            const int jj = j + (odd ? 1 : 0);
-            const uint32_t w = odd ? pack_bf16x2(got, v[j + 1]) : pack_bf16x2(v[j], got);
-            if (f_ok && jj < left) *reinterpret_cast<uint32_t*>(o + jj * p.ldo) = w;
-          }
-        } else {
-          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(t.row0 + c) * p.ldo + f;
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (f_ok && j < left) o[j * p.ldo] = f2bf(v[j]);
-        }
+        store_eight(p, how, v, f, f_ok, t.row0 + c, t.row1, lane);
+        store_eight(p, how, v + 8, f, f_ok, t.row0 + c + 8, t.row1, lane);
       }
       tc_fence_before();
       __syncwarp();
@@ -362,6 +377,246 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (warp == 2) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::kTmemCols) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ tensor cores, a pair of SMs on one tile
+// The same roles on clusters of two CTAs: the pair's tile is 256 weight rows x up to 256 token rows, either CTA has 128 of
+// the weight rows (its TMEM lanes) and half of the token rows in its shared memory, and the products of both
+// (tcgen05.mma.cta_group::2) are issued by the first.  A step of 64 along K then moves 32 KB into an SM where a tile of
+// 128 x 256 of its own moves 48, which is what paced that kernel.  A gated tile is 128 features: a CTA's 128 weight rows
+// are 64 gate rows and their 64 up rows in turns of sixteen, so that a warp has both of sixteen features and half-warps
+// exchange halves.  Sums run along K in the same order as in the kernel above: the results have the same bits.
+//
+// 2048 rows, K 4096, gated 11264 features: 250 us (1.51 PFLOP/s), on single SMs in tiles of 128 rows 332; 4096 features, K
+// 11264: 133 us (1.41), 149 in tiles of 256; 1357 rows, gated 18432 features, K 7168: 507 (639); 7168 features, K 8192: 126
+// (152).
+constexpr int kPairMaxStages = 8;
+
+struct PairTiles {
+  int bn;                // token rows of a tile: a multiple of 32, at most 256
+  int stages, stage_bytes;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// shared::cluster address of a CTA's copy of a variable
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// loads into this CTA's shared memory that complete on a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives at the barrier at this place in both CTAs when the products issued so far are complete
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
+}
+
+template <bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
+    gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const GemmRowsParams p, const PairTiles q) {
+  constexpr int kWBytes = 128 * kTcK * 2, kFeats = GATED ? 64 : 128;  // of a CTA
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full[kPairMaxStages], empty[kPairMaxStages], acc_full[2], acc_empty[2], drain;
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_abort;
+  __shared__ int s_rows[kMaxGroups + 1], s_tiles[kMaxGroups + 1];
+  uint8_t* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank(), stages = q.stages;
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kPairMaxStages; ++i) {
+      mbar_init(&full[i], 1);   // (the first CTA's counts the bytes of both)
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 2 * kTcEpiWarps);
+    }
+    mbar_init(&drain, 1);
+    s_abort = 0;
+    mbar_fence_init();
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers are there
+  tc_fence_after();
+  const uint32_t tmem = warp_uniform(*reinterpret_cast<volatile uint32_t*>(&s_tmem));
+  pdl_wait();
+  const int ft = (p.n + 2 * kFeats - 1) / (2 * kFeats);
+  tile_prefix(p, q.bn, ft, s_rows, s_tiles);
+  const int groups = p.n_groups > 0 ? p.n_groups : 1;
+  const int n_tiles = warp_uniform(s_tiles[groups]);
+  const int n_kb = (p.k + kTcK - 1) / kTcK;
+  volatile int* abort = &s_abort;
+  TileWalk walk{s_rows, s_tiles, groups, ft, q.bn, 2 * kFeats};
+  const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
+  const int half = q.bn / 2;  // token rows of a CTA
+
+  if (warp == 0) {
+    uint32_t it = 0, s = 0, ph = 0;
+    bool ok = true;
+    for (int i = first; ok && i < n_tiles; i += stride) {
+      const TileWalk::Tile t = walk.at_warp(i);
+      const int f0 = t.feature0 + static_cast<int>(rank) * kFeats;
+      const int x0 = t.row0 + static_cast<int>(rank) * half;
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        if (!mbar_wait_warp(&empty[s], ph ^ 1u, abort)) {
+          set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+          ok = false;
+          break;
+        }
+        uint8_t* st = ring + s * q.stage_bytes;
+        if (elect_one()) {
+          const uint32_t bar = cluster_addr(&full[s], 0);
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * q.stage_bytes);
+          if (GATED) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) tma_load_3d_pair(st + g * (kWBytes / 4), &wmap, kb * kTcK, f0 + 16 * g, 2 * t.group, bar);
+          } else {
+            tma_load_2d_pair(st, &wmap, kb * kTcK, t.group * p.n + f0, bar);
+          }
+          tma_load_2d_pair(st + kWBytes, &xmap, kb * kTcK, x0, bar);
+        }
+        if (++s == stages) s = 0, ph ^= 1u;
+      }
+    }
+    if (!ok) *abort = 1;
+    // What is under way into this shared memory lands before the CTA goes: copies, and arrivals of the other CTA's products.
+    const uint32_t from = it > stages ? it - stages : 0;
+    if (rank == 0)
+      for (uint32_t j = from; j < it; ++j) mbar_wait(&full[j % stages], (j / stages) & 1u, abort);
+    for (uint32_t j = from; j < it; ++j) mbar_wait(&empty[j % stages], (j / stages) & 1u, abort);
+  } else if (warp == 1) {
+    if (rank == 0) {
+      const uint32_t idesc = umma_idesc_bf16(256, q.bn);
+      uint32_t s = 0, ph = 0, n_done = 0;
+      bool ok = true, seen = false;
+      for (int i = first; ok && i < n_tiles; i += stride, ++n_done) {
+        const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
+        if (!mbar_wait_warp(&acc_empty[buf], aph ^ 1u, abort)) {
+          set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t d = tmem + buf * 256;
+        for (int kb = 0; kb < n_kb; ++kb) {
+          if (!mbar_wait_warp(&full[s], ph, abort, seen)) {
+            set_status(p.status, ST_WAIT_FULL_TIMEOUT);
+            ok = false;
+            break;
+          }
+          const bool wrap = s + 1 == stages;
+          seen = mbar_test(&full[wrap ? 0 : s + 1], ph ^ (wrap ? 1u : 0u));  // (known by the time it is asked for)
+          const uint32_t base = smem_u32(ring + s * q.stage_bytes);
+          const uint64_t wd = umma_desc_sw128(base), xd = umma_desc_sw128(base + kWBytes);
+          if (elect_one()) {
+#pragma unroll
+            for (int c = 0; c < kTcK / 16; ++c) umma_bf16_pair(d, wd + 2 * c, xd + 2 * c, idesc, (kb | c) != 0);
+            umma_commit_pair(&empty[s]);
+            if (kb == n_kb - 1) umma_commit_pair(&acc_full[buf]);
+          }
+          if (++s == stages) s = 0, ph ^= 1u;
+        }
+      }
+      if (!ok) *abort = 1;
+      __syncwarp();
+      // products still running read shared memory and write TMEM
+      if (elect_one()) asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&drain)) : "memory");
+      mbar_wait(&drain, 0);
+    }
+  } else {
+    const int quad = warp & 3;  // TMEM lanes this warp may read
+    const int part = (warp - 2) / 4;
+    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
+    const StoreForm how = store_form(p);
+    uint32_t n_done = 0;
+    for (int i = first; i < n_tiles; i += stride, ++n_done) {
+      const TileWalk::Tile t = walk.at_warp(i);
+      const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
+      const bool ok = mbar_wait(&acc_full[buf], aph, abort);
+      if (__any_sync(0xffffffffu, !ok)) {  // warp-uniform: tcgen05.ld needs every lane
+        if (!ok) set_status(p.status, ST_WAIT_FULL_TIMEOUT);
+        *abort = 1;
+        break;
+      }
+      tc_fence_after();
+      const int f = t.feature0 + static_cast<int>(rank) * kFeats + (GATED ? quad * 16 + (lane & 15) : quad * 32 + lane);
+      const bool f_ok = f < p.n;
+      const float bias = p.bias != nullptr && f_ok ? p.bias[f] : 0.f;
+      const uint32_t acc = tmem + buf * 256 + lane_off;
+      const int c0 = part * half;  // (columns in multiples of sixteen)
+      for (int c = c0; c < c0 + half && t.row0 + c < t.row1; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(acc + c, r);
+        tmem_ld16_wait(r);
+        float v[16];
+        if (GATED) {
+          // lanes 0-15 have gates, 16-31 the ups of the same features: the first half-warp takes rows 0-7, the other 8-15
+          const bool up = lane & 16;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float got = __uint_as_float(__shfl_xor_sync(0xffffffffu, up ? r[j] : r[8 + j], 16));
+            v[j] = clamped_gate(up ? got : __uint_as_float(r[j]), up ? __uint_as_float(r[8 + j]) : got, p.limit, p.alpha);
+          }
+          store_eight(p, how, v, f, f_ok, t.row0 + c + (up ? 8 : 0), t.row1, lane);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias;
+          store_eight(p, how, v, f, f_ok, t.row0 + c, t.row1, lane);
+          store_eight(p, how, v + 8, f, f_ok, t.row0 + c + 8, t.row1, lane);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // neither CTA's memory goes while the other may signal it or compute from it
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
 }
 

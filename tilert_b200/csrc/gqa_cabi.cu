@@ -100,6 +100,32 @@ int make_map(CUtensorMap* map, const void* base, long long rows, int k, long lon
   return TB_OK;
 }
 
+// The halves of a gated weight [n_groups][2][n, ld]: boxes of 64 columns x 16 rows of both halves
+int make_gated_map(CUtensorMap* map, const void* base, int groups, int n, int k, long long ld) {
+  if (encode_tiled() == nullptr) return fail(TB_ESTATE, "cuTensorMapEncodeTiled is not available%s");
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(n), static_cast<cuuint64_t>(groups) * 2};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(ld) * 2 * n};
+  const cuuint32_t box[3] = {kTcK, 16, 2};
+  const cuuint32_t steps[3] = {1, 1, 1};
+  const CUresult r = encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, steps,
+                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(TB_ECUDA, "cuTensorMapEncodeTiled failed%s");
+  return TB_OK;
+}
+
+template <bool GATED>
+int launch_pair(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int bn, void* stream) {
+  PairTiles q{bn, 0, 128 * kTcK * 2 + bn / 2 * kTcK * 2};
+  q.stages = 196608 / q.stage_bytes < kPairMaxStages ? 196608 / q.stage_bytes : kPairMaxStages;
+  CUtensorMap wmap, xmap;
+  int rc = GATED ? make_gated_map(&wmap, p.w, p.n_groups > 0 ? p.n_groups : 1, p.n, p.k, p.ldw) : make_map(&wmap, p.w, w_rows, p.k, p.ldw, 128);
+  const long long x_rows = p.n_groups > 0 && p.counts == nullptr ? static_cast<long long>(p.n_groups) * p.rows : p.rows;
+  if (rc == TB_OK) rc = make_map(&xmap, p.x, x_rows, p.k, p.ldx, bn / 2);
+  if (rc != TB_OK) return rc;
+  return go(gemm_pair_kernel<GATED>, dim3(ctx->num_sms / 2 * 2), dim3(kTcThreads), static_cast<size_t>(q.stages) * q.stage_bytes + 1024, stream, wmap, xmap, p, q);
+}
+
 template <int BN, bool GATED>
 int launch_tc(TgContext* ctx, const GemmRowsParams& p, long long w_rows, void* stream) {
   CUtensorMap wmap, xmap;
@@ -279,18 +305,30 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     return gated ? launch_f32<32, 32, 64, 4, true>(ctx, p, stream) : launch_f32<32, 32, 128, 4, false>(ctx, p, stream);
   }
   const long long w_rows = static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n;
-  const int ft = (n + 127) / 128;
-  // Token tile.  One weight: waves of tiles over the SMs times the relative cost of a tile (a narrow tile moves more
-  // bytes per product through the L2).  Groups: the widest tile that an average group nearly fills.
-  auto cost = [&](int bn, double tile) {
-    if (n_groups > 0) return bn == 64 || (counts != nullptr ? rows / n_groups : rows) >= bn * 3 / 4 ? 1.0 / bn : 1.0;
-    return std::ceil(static_cast<double>(ft) * ((rows + bn - 1) / bn) / ctx->num_sms) * tile;
-  };
-  if (gated) return cost(128, 1.0) <= cost(64, 0.6) ? launch_tc<128, true>(ctx, p, w_rows, stream) : launch_tc<64, true>(ctx, p, w_rows, stream);
-  const double c256 = cost(256, 1.0), c128 = cost(128, 0.75), c64 = cost(64, 0.55);
-  if (c256 <= c128 && c256 <= c64) return launch_tc<256, false>(ctx, p, w_rows, stream);
-  if (c128 <= c64) return launch_tc<128, false>(ctx, p, w_rows, stream);
-  return launch_tc<64, false>(ctx, p, w_rows, stream);
+  // One SM (64 token rows a tile) or a pair on a tile, and its token rows: what takes the fewest rounds over the SMs, a round
+  // being one step along K of each of its tiles.  The microseconds of a step are measured ones (2048 x 6208 x 4096,
+  // 2048 x 4096 x 11264 and gated 2048 x 11264 x 4096 at every tile size), a pair costs its hand-shakes once.
+  const int n_kb = (p.k + kTcK - 1) / kTcK, wide = n_groups > 0 ? n_groups : 1;
+  auto tiles = [&](int feats, int bn) { return static_cast<long long>(wide) * ((n + feats - 1) / feats) * ((rows + bn - 1) / bn); };
+  auto round_up = [](long long tiles, int units) { return static_cast<double>((tiles + units - 1) / units); };
+  if (n_groups > 0 && counts != nullptr) {
+    // The counts are on the device: a tile that holds an average group and a fifth.  Below 64 rows a group it is the weights'
+    // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 118 and 141 us); 75 rows
+    // 120 us on single SMs, 92 in pairs, 156 rows 383 and 303, 256 rows 487 and 449 (gated, 1000 to 1536 features).
+    const int each = rows / n_groups, bn = (each * 6 / 5 + 31) / 32 * 32;
+    if (each < 64) return gated ? launch_tc<64, true>(ctx, p, w_rows, stream) : launch_tc<64, false>(ctx, p, w_rows, stream);
+    return gated ? launch_pair<true>(ctx, p, w_rows, bn < 256 ? bn : 256, stream) : launch_pair<false>(ctx, p, w_rows, bn < 256 ? bn : 256, stream);
+  }
+  const double single = round_up(tiles(128, 64), ctx->num_sms) * n_kb * (gated ? 0.32 : 0.22);
+  constexpr double kStep[] = {0.21, 0.23, 0.25, 0.29, 0.31, 0.34, 0.39};  // 64, 96, .. 256 rows
+  double pair = 1e30;
+  int bn = 0;
+  for (int i = 0; i < 7; ++i) {
+    const double c = round_up(tiles(gated ? 128 : 256, 64 + 32 * i), ctx->num_sms / 2) * n_kb * kStep[i] + 1.3;
+    if (c < pair) pair = c, bn = 64 + 32 * i;
+  }
+  if (single <= pair) return gated ? launch_tc<64, true>(ctx, p, w_rows, stream) : launch_tc<64, false>(ctx, p, w_rows, stream);
+  return gated ? launch_pair<true>(ctx, p, w_rows, bn, stream) : launch_pair<false>(ctx, p, w_rows, bn, stream);
 }
 
 // ------------------------------------------------------------------------------- attention of a portion

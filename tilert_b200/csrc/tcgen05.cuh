@@ -9,6 +9,34 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
+// The loops that issue copies and products run on whole warps and one lane issues: what the instructions take is then
+// computed in uniform registers.  Under a branch on the lane every operand of every tcgen05.mma is moved there on its own,
+// which paces the products at about 90 cycles each, whatever their size.
+// (A value that the compiler cannot see to be the same in all lanes -- the warp's number, what shared memory holds -- passes
+// through warp_uniform first: branches and loops on it count as divergent otherwise.)
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+// without blocking
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait of a whole warp; true in every lane or in none.  `seen`: the barrier has been found complete already.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const volatile int* abort, bool seen = false) {
+  if (__all_sync(0xffffffffu, seen || mbar_test(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort));
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // Issue / completion halves of the same load, so that other work can overlap its latency.  The
