@@ -60,7 +60,8 @@ cudaError_t allow_smem(const void* kernel) try {
 template <typename... KArgs, typename... Args>
 int go(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, void* stream, Args&&... args) {
   TB_REQUIRE(smem <= kMaxSmem);
-  if (smem > 48 * 1024) TB_CUDA(allow_smem(reinterpret_cast<const void*>(kernel)));
+  // (48 KB need no permission, but a kernel's static shared memory counts as well: up to 13 KB here)
+  if (smem > 32 * 1024) TB_CUDA(allow_smem(reinterpret_cast<const void*>(kernel)));
   TB_CUDA(launch(kernel, grid, block, smem, stream_of(stream), std::forward<Args>(args)...));
   ++g_launches;
   TB_CUDA(cudaGetLastError());
