@@ -1,4 +1,4 @@
-"""Products of many rows on pairs of SMs against f64 on the same bf16 operands, at the edges of their tiles.
+"""Products of many rows on pairs of SMs, and of few rows on single ones, against f64 on the same bf16 operands, at the edges of their tiles.
 
 The tensor cores add sixteen products at a time to an f32 sum and may cut off what does not fit: up to 2^-23 of the sum (of
 size 8 at most here) in each of k / 16 steps, and a few more such roundings in the bias or the gated unit.  A bf16 result adds
@@ -63,7 +63,15 @@ def test_groups(ops, gated, out_type, n, k, counts):
     check(ops, n, k, gated, out_type, counts)
 
 
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("n,k", [(7, 8), (65, 72), (136, 200), (20000, 64)])
+@pytest.mark.parametrize("counts", [[1, 0, 2, 0], [63, 64, 0, 65, 1], [40] * 7])
+def test_few_rows_a_group(ops, gated, n, k, counts):
+    check(ops, n, k, gated, BF16, counts)
+
+
 @pytest.mark.parametrize("rows,n,k,gated,out_type", [
+    (1, 64, 200, False, F32), (37, 2048, 1032, False, F32), (64, 65, 64, False, BF16), (65, 12000, 136, False, BF16), (173, 129, 72, True, BF16),
     (2048, 700, 2000, False, F32), (2047, 1288, 1000, True, BF16), (1357, 4104, 520, False, BF16), (1025, 2049, 1032, True, BF16),
     (700, 3000, 2000, False, F32), (37, 5632, 1024, True, BF16), (257, 20001, 72, False, F32)])
 def test_one_weight(ops, rows, n, k, gated, out_type):

@@ -1,6 +1,6 @@
 // Products of many token rows with bf16 weights (prefill):  out[t, n] = W[n, :] . x[t, :].
 //
-//   gemm_tc_kernel<BN, GATED>   bf16 rows on the tensor cores, an SM on a tile: few tokens, small groups
+//   gemm_tc_kernel<BM, GATED>   bf16 rows on the tensor cores, an SM on a tile: few tokens, small groups
 //   gemm_pair_kernel<GATED>     the same, a pair of SMs on a tile
 //   gemm_f32_kernel<.., GATED>  f32 rows, f32 arithmetic (the exact mode)
 //
@@ -8,8 +8,8 @@
 // Grouped launches have one weight per group (expert) and the token rows sorted by group; the number of rows per
 // group is device data, so the tiles are enumerated on the device and the grid is the SM count.
 //
-// Tensor-core kernel: persistent, warp-specialised, one CTA per SM.  The 128 weight rows of a tile are M (so a TMEM
-// lane is an output feature and a store covers consecutive features), BN token rows are N; K goes by 64.  One thread
+// Tensor-core kernel: persistent, warp-specialised, one CTA per SM.  The 128 or 64 weight rows of a tile are M (so a TMEM
+// lane is an output feature and a store covers consecutive features), 64 token rows are N; K goes by 128.  One thread
 // issues the TMA loads (128-byte swizzle) into a ring of stages, one thread issues the tcgen05.mma, eight warps read
 // the accumulators back; two accumulators alternate so that the epilogue of a tile overlaps the products of the next.
 #pragma once
@@ -106,13 +106,20 @@ constexpr int kTcEpiWarps = 8;  // two per quarter of the TMEM lanes, each with 
 constexpr int kTcThreads = 64 + 32 * kTcEpiWarps;  // and a producer warp, an MMA warp
 constexpr int kTcK = 64;
 
-template <int BN, bool GATED>
+// BM features x 64 token rows.  Few tiles leave most SMs idle and a step along K bound by one SM's loads and by the
+// hand-shakes of a stage: 64 features spread the weights over twice the SMs.  37 rows, 2048 features, K 5632: 16.0 us in tiles
+// of 64 features, 18.3 of 128, 24.0 with stages of 64 along K; 173 x 2048 x 2048 8.5, 9.1, 10.9.  A stage is two blocks of 64 along K (hand-shakes cost as much as a block's products), one
+// where two would leave two stages.
+template <int BM, bool GATED>
 struct TcShape {
-  static constexpr int kWBytes = 128 * kTcK * 2;
-  static constexpr int kXBytes = BN * kTcK * 2;
-  static constexpr int kStageBytes = (GATED ? 2 : 1) * kWBytes + kXBytes;
+  static constexpr int kBN = 64;
+  static constexpr int kBlocks = GATED && BM == 128 ? 1 : 2;
+  static constexpr int kWBytes = BM * kTcK * 2;
+  static constexpr int kXBytes = kBN * kTcK * 2;
+  static constexpr int kBlockBytes = (GATED ? 2 : 1) * kWBytes + kXBytes;
+  static constexpr int kStageBytes = kBlocks * kBlockBytes;
   static constexpr int kStages = 196608 / kStageBytes < 8 ? 196608 / kStageBytes : 8;
-  static constexpr int kAccCols = GATED ? 2 * BN : BN;
+  static constexpr int kAccCols = GATED ? 2 * kBN : kBN;
   static constexpr int kTmemCols = 2 * kAccCols;
   static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM allocation size");
   static constexpr size_t kSmemBytes = static_cast<size_t>(kStages) * kStageBytes + 1024;  // + alignment of the ring
@@ -218,10 +225,11 @@ __device__ __forceinline__ void store_eight(const GemmRowsParams& p, StoreForm h
   }
 }
 
-template <int BN, bool GATED>
+template <int BM, bool GATED>
 __global__ void __launch_bounds__(kTcThreads, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const GemmRowsParams p) {
-  using S = TcShape<BN, GATED>;
+  using S = TcShape<BM, GATED>;
+  constexpr int BN = S::kBN;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[S::kStages], empty[S::kStages], acc_full[2], acc_empty[2], drain;
   __shared__ uint32_t s_tmem;
@@ -254,13 +262,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   tc_fence_after();
   const uint32_t tmem = warp_uniform(*reinterpret_cast<volatile uint32_t*>(&s_tmem));
   pdl_wait();
-  const int ft = (p.n + 127) / 128;
+  const int ft = (p.n + BM - 1) / BM;
   tile_prefix(p, BN, ft, s_rows, s_tiles);
   const int groups = p.n_groups > 0 ? p.n_groups : 1;
   const int n_tiles = warp_uniform(s_tiles[groups]);
-  const int n_kb = (p.k + kTcK - 1) / kTcK;
+  const int n_kb = (p.k + kTcK * S::kBlocks - 1) / (kTcK * S::kBlocks);  // (what lies beyond K is zero)
   volatile int* abort = &s_abort;
-  TileWalk walk{s_rows, s_tiles, groups, ft, BN};
+  TileWalk walk{s_rows, s_tiles, groups, ft, BN, BM};
 
   if (warp == 0) {
     uint32_t it = 0;
@@ -278,9 +286,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         uint8_t* st = ring + s * S::kStageBytes;
         if (elect_one()) {
           mbar_expect_tx(&full[s], S::kStageBytes);
-          tma_load_2d(st, &wmap, kb * kTcK, wrow, &full[s]);
-          if (GATED) tma_load_2d(st + S::kWBytes, &wmap, kb * kTcK, wrow + p.n, &full[s]);
-          tma_load_2d(st + (GATED ? 2 : 1) * S::kWBytes, &xmap, kb * kTcK, t.row0, &full[s]);
+#pragma unroll
+          for (int b = 0; b < S::kBlocks; ++b, st += S::kBlockBytes) {
+            const int k0 = (kb * S::kBlocks + b) * kTcK;
+            tma_load_2d(st, &wmap, k0, wrow, &full[s]);
+            if (GATED) tma_load_2d(st + S::kWBytes, &wmap, k0, wrow + p.n, &full[s]);
+            tma_load_2d(st + (GATED ? 2 : 1) * S::kWBytes, &xmap, k0, t.row0, &full[s]);
+          }
         }
       }
     }
@@ -288,7 +300,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // copies still in flight must land before this CTA's shared memory goes away
     for (uint32_t j = it > S::kStages ? it - S::kStages : 0; j < it; ++j) mbar_wait(&full[j % S::kStages], (j / S::kStages) & 1u);
   } else if (warp == 1) {
-    constexpr uint32_t idesc = umma_idesc_bf16(128, BN);
+    constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
     uint32_t it = 0, n_done = 0;
     bool ok = true, seen = false;
     for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x, ++n_done) {
@@ -313,10 +325,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const uint64_t xd = umma_desc_sw128(base + (GATED ? 2 : 1) * S::kWBytes);
         if (elect_one()) {
 #pragma unroll
-          for (int q = 0; q < kTcK / 16; ++q) {  // 32 bytes along K per instruction
-            umma_bf16(d, wd + 2 * q, xd + 2 * q, idesc, (kb | q) != 0);
-            if (GATED) umma_bf16(d + BN, ud + 2 * q, xd + 2 * q, idesc, (kb | q) != 0);
-          }
+          for (int b = 0; b < S::kBlocks; ++b)
+#pragma unroll
+            for (int q = 0; q < kTcK / 16; ++q) {  // 32 bytes along K per instruction
+              const uint32_t off = (b * S::kBlockBytes + q * 32) >> 4;
+              umma_bf16(d, wd + off, xd + off, idesc, (kb | b | q) != 0);
+              if (GATED) umma_bf16(d + BN, ud + off, xd + off, idesc, (kb | b | q) != 0);
+            }
           umma_commit(&empty[s]);
           if (kb == n_kb - 1) umma_commit(&acc_full[buf]);
         }
@@ -343,8 +358,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         break;
       }
       tc_fence_after();
-      const int f = t.feature0 + quad * 32 + lane;
-      const bool f_ok = f < p.n;
+      // 64 features: sixteen in the first half of every quarter of the lanes
+      const int f = t.feature0 + (BM == 64 ? quad * 16 : quad * 32) + lane;
+      const bool f_ok = f < p.n && (BM == 128 || lane < 16);
       const float bias = p.bias != nullptr && f_ok ? p.bias[f] : 0.f;
       const uint32_t acc = tmem + buf * S::kAccCols + lane_off;
       for (int c = c0; c < c0 + kCols && t.row0 + c < t.row1; c += 16) {
@@ -395,6 +411,7 @@ constexpr int kPairMaxStages = 8;
 
 struct PairTiles {
   int bn;                // token rows of a tile: a multiple of 32, at most 256
+  int blocks;            // of 64 along K in a stage
   int stages, stage_bytes;
 };
 
@@ -484,7 +501,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
   tile_prefix(p, q.bn, ft, s_rows, s_tiles);
   const int groups = p.n_groups > 0 ? p.n_groups : 1;
   const int n_tiles = warp_uniform(s_tiles[groups]);
-  const int n_kb = (p.k + kTcK - 1) / kTcK;
+  const int n_kb = (p.k + kTcK * q.blocks - 1) / (kTcK * q.blocks);  // (what lies beyond K is zero)
+  const int block_bytes = kWBytes + q.bn / 2 * kTcK * 2;
   volatile int* abort = &s_abort;
   TileWalk walk{s_rows, s_tiles, groups, ft, q.bn, 2 * kFeats};
   const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
@@ -507,13 +525,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         if (elect_one()) {
           const uint32_t bar = cluster_addr(&full[s], 0);
           if (rank == 0) mbar_expect_tx(&full[s], 2 * q.stage_bytes);
-          if (GATED) {
+          for (int k0 = kb * q.blocks * kTcK, b = 0; b < q.blocks; ++b, k0 += kTcK, st += block_bytes) {
+            if (GATED) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) tma_load_3d_pair(st + g * (kWBytes / 4), &wmap, kb * kTcK, f0 + 16 * g, 2 * t.group, bar);
-          } else {
-            tma_load_2d_pair(st, &wmap, kb * kTcK, t.group * p.n + f0, bar);
+              for (int g = 0; g < 4; ++g) tma_load_3d_pair(st + g * (kWBytes / 4), &wmap, k0, f0 + 16 * g, 2 * t.group, bar);
+            } else {
+              tma_load_2d_pair(st, &wmap, k0, t.group * p.n + f0, bar);
+            }
+            tma_load_2d_pair(st + kWBytes, &xmap, k0, x0, bar);
           }
-          tma_load_2d_pair(st + kWBytes, &xmap, kb * kTcK, x0, bar);
         }
         if (++s == stages) s = 0, ph ^= 1u;
       }
@@ -547,10 +567,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
           const bool wrap = s + 1 == stages;
           seen = mbar_test(&full[wrap ? 0 : s + 1], ph ^ (wrap ? 1u : 0u));  // (known by the time it is asked for)
           const uint32_t base = smem_u32(ring + s * q.stage_bytes);
-          const uint64_t wd = umma_desc_sw128(base), xd = umma_desc_sw128(base + kWBytes);
+          uint64_t wd = umma_desc_sw128(base), xd = umma_desc_sw128(base + kWBytes);
           if (elect_one()) {
+            for (int b = 0; b < q.blocks; ++b, wd += block_bytes >> 4, xd += block_bytes >> 4) {
 #pragma unroll
-            for (int c = 0; c < kTcK / 16; ++c) umma_bf16_pair(d, wd + 2 * c, xd + 2 * c, idesc, (kb | c) != 0);
+              for (int c = 0; c < kTcK / 16; ++c) umma_bf16_pair(d, wd + 2 * c, xd + 2 * c, idesc, (kb | b | c) != 0);
+            }
             umma_commit_pair(&empty[s]);
             if (kb == n_kb - 1) umma_commit_pair(&acc_full[buf]);
           }

@@ -117,7 +117,8 @@ int make_gated_map(CUtensorMap* map, const void* base, int groups, int n, int k,
 
 template <bool GATED>
 int launch_pair(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int bn, void* stream) {
-  PairTiles q{bn, 0, 128 * kTcK * 2 + bn / 2 * kTcK * 2};
+  const int blocks = bn <= 160 ? 2 : 1;  // (wider tiles: a step's products hide its hand-shakes, and the ring wants the stages)
+  PairTiles q{bn, blocks, 0, blocks * (128 * kTcK * 2 + bn / 2 * kTcK * 2)};
   q.stages = 196608 / q.stage_bytes < kPairMaxStages ? 196608 / q.stage_bytes : kPairMaxStages;
   CUtensorMap wmap, xmap;
   int rc = GATED ? make_gated_map(&wmap, p.w, p.n_groups > 0 ? p.n_groups : 1, p.n, p.k, p.ldw) : make_map(&wmap, p.w, w_rows, p.k, p.ldw, 128);
@@ -127,19 +128,24 @@ int launch_pair(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int b
   return go(gemm_pair_kernel<GATED>, dim3(ctx->num_sms / 2 * 2), dim3(kTcThreads), static_cast<size_t>(q.stages) * q.stage_bytes + 1024, stream, wmap, xmap, p, q);
 }
 
-template <int BN, bool GATED>
+template <int BM, bool GATED>
 int launch_tc(TgContext* ctx, const GemmRowsParams& p, long long w_rows, void* stream) {
   CUtensorMap wmap, xmap;
-  int rc = make_map(&wmap, p.w, w_rows, p.k, p.ldw, 128);
+  int rc = make_map(&wmap, p.w, w_rows, p.k, p.ldw, BM);
   const long long x_rows = p.n_groups > 0 && p.counts == nullptr ? static_cast<long long>(p.n_groups) * p.rows : p.rows;
-  if (rc == TB_OK) rc = make_map(&xmap, p.x, x_rows, p.k, p.ldx, BN);
+  if (rc == TB_OK) rc = make_map(&xmap, p.x, x_rows, p.k, p.ldx, TcShape<BM, GATED>::kBN);
   if (rc != TB_OK) return rc;
-  return go(gemm_tc_kernel<BN, GATED>, dim3(ctx->num_sms), dim3(kTcThreads), TcShape<BN, GATED>::kSmemBytes, stream, wmap, xmap, p);
+  return go(gemm_tc_kernel<BM, GATED>, dim3(ctx->num_sms), dim3(kTcThreads), TcShape<BM, GATED>::kSmemBytes, stream, wmap, xmap, p);
 }
 
 template <int BF, int BT, int KB, int KG, bool GATED>
 int launch_f32(TgContext* ctx, const GemmRowsParams& p, void* stream) {
   return go(gemm_f32_kernel<BF, BT, KB, KG, GATED>, dim3(ctx->num_sms * 4), dim3(F32Shape<BF, BT, KB, KG, GATED>::kThreads), 0, stream, p);
+}
+
+template <bool GATED>
+int launch_single(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int bm, void* stream) {
+  return bm == 64 ? launch_tc<64, GATED>(ctx, p, w_rows, stream) : launch_tc<128, GATED>(ctx, p, w_rows, stream);
 }
 
 QkvShape qkv_shape(int heads, int kv_heads, int dim, int vdim, int ring, int window) {
@@ -306,30 +312,36 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     return gated ? launch_f32<32, 32, 64, 4, true>(ctx, p, stream) : launch_f32<32, 32, 128, 4, false>(ctx, p, stream);
   }
   const long long w_rows = static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n;
-  // One SM (64 token rows a tile) or a pair on a tile, and its token rows: what takes the fewest rounds over the SMs, a round
-  // being one step along K of each of its tiles.  The microseconds of a step are measured ones (2048 x 6208 x 4096,
-  // 2048 x 4096 x 11264 and gated 2048 x 11264 x 4096 at every tile size), a pair costs its hand-shakes once.
+  // One SM (128 or 64 features x 64 token rows) or a pair (256 x up to 256) on a tile: what takes the fewest rounds over the
+  // SMs, a round being the steps along K of a tile.  The microseconds of a step of 64 are measured ones (2048 x 6208 x 4096,
+  // 1357 x 7168 x 18432, gated 1357 x 18432 x 7168 and others at every tile size, 37 and 173 x 2048 x 2048 to 5632 on single
+  // SMs).
   const int n_kb = (p.k + kTcK - 1) / kTcK, wide = n_groups > 0 ? n_groups : 1;
   auto tiles = [&](int feats, int bn) { return static_cast<long long>(wide) * ((n + feats - 1) / feats) * ((rows + bn - 1) / bn); };
   auto round_up = [](long long tiles, int units) { return static_cast<double>((tiles + units - 1) / units); };
   if (n_groups > 0 && counts != nullptr) {
     // The counts are on the device: a tile that holds an average group and a fifth.  Below 64 rows a group it is the weights'
-    // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 118 and 141 us); 75 rows
-    // 120 us on single SMs, 92 in pairs, 156 rows 383 and 303, 256 rows 487 and 449 (gated, 1000 to 1536 features).
+    // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 114 us, in pairs 141; 75 rows
+    // 97 in pairs, was 120; 156 rows 303, 256 rows 440; gated, 1000 to 1536 features), in small tiles if the groups that
+    // there can be are few (16 rows over 30 experts 16.0 us, in tiles of 128 features 19.5).
     const int each = rows / n_groups, bn = (each * 6 / 5 + 31) / 32 * 32;
-    if (each < 64) return gated ? launch_tc<64, true>(ctx, p, w_rows, stream) : launch_tc<64, false>(ctx, p, w_rows, stream);
+    if (each < 64) {
+      const int bm = static_cast<long long>(rows < n_groups ? rows : n_groups) * ((n + 127) / 128) <= ctx->num_sms ? 64 : 128;
+      return gated ? launch_single<true>(ctx, p, w_rows, bm, stream) : launch_single<false>(ctx, p, w_rows, bm, stream);
+    }
     return gated ? launch_pair<true>(ctx, p, w_rows, bn < 256 ? bn : 256, stream) : launch_pair<false>(ctx, p, w_rows, bn < 256 ? bn : 256, stream);
   }
-  const double single = round_up(tiles(128, 64), ctx->num_sms) * n_kb * (gated ? 0.32 : 0.22);
-  constexpr double kStep[] = {0.21, 0.23, 0.25, 0.29, 0.31, 0.34, 0.39};  // 64, 96, .. 256 rows
+  constexpr double kStep[] = {0.17, 0.19, 0.22, 0.295, 0.30, 0.335, 0.37};  // pairs: 64, 96, .. 256 rows
   double pair = 1e30;
   int bn = 0;
   for (int i = 0; i < 7; ++i) {
-    const double c = round_up(tiles(gated ? 128 : 256, 64 + 32 * i), ctx->num_sms / 2) * n_kb * kStep[i] + 1.3;
+    const double c = round_up(tiles(gated ? 128 : 256, 64 + 32 * i), ctx->num_sms / 2) * n_kb * kStep[i] + 0.4;
     if (c < pair) pair = c, bn = 64 + 32 * i;
   }
-  if (single <= pair) return gated ? launch_tc<64, true>(ctx, p, w_rows, stream) : launch_tc<64, false>(ctx, p, w_rows, stream);
-  return gated ? launch_pair<true>(ctx, p, w_rows, bn, stream) : launch_pair<false>(ctx, p, w_rows, bn, stream);
+  if (gated) return launch_pair<true>(ctx, p, w_rows, bn, stream);
+  const double large = round_up(tiles(128, 64), ctx->num_sms) * n_kb * 0.17, small = round_up(tiles(64, 64), ctx->num_sms) * n_kb * 0.145;
+  if (large > pair && small > pair) return launch_pair<false>(ctx, p, w_rows, bn, stream);
+  return launch_single<false>(ctx, p, w_rows, small <= large ? 64 : 128, stream);
 }
 
 // ------------------------------------------------------------------------------- attention of a portion
