@@ -6,14 +6,17 @@
 // from and are the A operand of the value product straight from TMEM.  With two query tiles the products of one run under
 // the softmax of the other, and the tiles share the keys and values in shared memory.
 //
-// The reference of the exponentials is a running maximum that follows the true one only when it is passed by a factor of
-// 2^8: the sums of a row are then rescaled in TMEM, which after a row's first tiles hardly happens.
+// The reference of the exponentials is the largest score so far, so that the largest probability of a row is an exact one in
+// bf16, and a warp rescales its rows' sums in TMEM where one has grown.  (A reference that lags behind by up to 2^8 saves
+// most of that, 2 to 8 % of the time, but rounds the largest probability too: the error against 64 bits rises by up to a quarter
+// for peaked scores.)
 //
-// Bound by the pace of the products (sixteen columns of K take about as long for 128 keys as for 64) and by the loads of keys
-// and values, 80 KB a tile of 128 keys at 192 + 128 columns.  Against the mma.sync kernel of window_attention.cuh (64 rows a
-// CTA), which keeps portions of less than a tile and heads whose tiles do not fit: 32 heads of 128 + 64 / 128 columns, 2048
-// queries behind 4096 keys 325 us (660 TFLOP/s), was 1787; a window of 1024 122 (452); 64 heads, 1357 queries from the start
-// 130 (470); 16 heads, 300 queries 25 (46); 32 heads, 128 queries 21 (30).
+// Bound by the chain of a query tile's scores, softmax (a row's 128 exponentials) and value product, of which two run under
+// each other, and by the loads of keys and values, 80 KB a tile of 128 keys at 192 + 128 columns.  Against the mma.sync kernel
+// of window_attention.cuh (64 rows a CTA), which keeps portions of less than a tile and heads whose tiles do not fit: 32 heads
+// of 128 + 64 / 128 columns, 2048 queries behind 4096 keys 294 us (730 TFLOP/s), was 1787; a window of 1024 114 (452); 64
+// heads, 1357 queries from the start 123 (470); 16 heads, 300 queries 24 (46); 32 heads, 128 queries 20 (30).  The error
+// against 64 bits is that kernel's to half a per cent, 0.0016 to 0.0023 over sizes and spreads of scores.
 //
 // Keys lie in a ring.  A tile ends at the last key, after 128 keys, or at the ring's end, so that its rows are consecutive;
 // a tile of fewer keys loads the 128 rows that end with its last one (from the ring's beginning if there are fewer before
@@ -29,7 +32,6 @@ namespace tb {
 constexpr int kXaTile = 128;                       // queries, and keys, of a tile
 constexpr int kXaBox = kXaTile * 64 * 2;           // bytes of 128 rows x 64 columns, 128-byte swizzle
 constexpr int kXaKeyStages = 2;
-constexpr float kXaSlack = 8.f;                    // log2 of what a sum may grow by before it is rescaled
 
 struct ExpandedAttnParams {
   int rows, heads;
@@ -332,26 +334,11 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
 #pragma unroll
       for (int j = 0; j < 32; ++j)
         mx = fmaxf(mx, fmaxf(fmaxf(__uint_as_float(r[0][j]), __uint_as_float(r[1][j])), fmaxf(__uint_as_float(r[2][j]), __uint_as_float(r[3][j]))));
-      if (n == 0) {
-        m = mx;
-      } else {
-        const bool far = (mx - m) * c > kXaSlack || (m == -INFINITY && mx > m);
-        if (__any_sync(0xffffffffu, far)) {
-          // (the product that wrote the sums is complete: the scores of this tile were issued behind it)
-          const float corr = far ? exp2_approx((m - mx) * c) : 1.f;
+      mx = fmaxf(mx, m);
+      const float corr = mx == m ? 1.f : exp2_approx((m - mx) * c);
+      m = mx;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) l[q] *= corr;
-          if (far) m = mx;
-          for (int v = 0; v < p.vdimp; v += 16) {
-            uint32_t o[16];
-            tmem_ld16(so + v, o);
-            tmem_ld16_wait(o);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
-            tmem_st16(so + v, o);
-          }
-        }
-      }
+      for (int q = 0; q < 4; ++q) l[q] *= corr;
       const float mc = m == -INFINITY ? 0.f : m * c;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -367,6 +354,27 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
             w[q * 16 + j / 2] = pack_bf16x2(e0, e1);
           }
         tmem_st32(sc + h * 32, w);
+      }
+      // (the product that wrote the sums is complete: the scores of this tile were issued behind it)
+      if (n > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
+        int v = 0;
+        for (; v + 32 <= p.vdimp; v += 32) {
+          uint32_t o[32];
+          tmem_ld32_issue(so + v, o);
+          tmem_wait_ld();
+          tmem_use32(o);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+          tmem_st32(so + v, o);
+        }
+        if (v < p.vdimp) {
+          uint32_t o[16];
+          tmem_ld16(so + v, o);
+          tmem_ld16_wait(o);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+          tmem_st16(so + v, o);
+        }
       }
       tmem_wait_st();
       tc_fence_before();
