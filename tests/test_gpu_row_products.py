@@ -124,3 +124,32 @@ def test_two_segments(ops, tokens, dim):
 
     # (the two normalised vectors are bf16 values: 2^-9 each, as the result)
     close("eh_proj", torch.cat([norm(e, ge), norm(h, gh)], -1) @ w.to(F64).T, o, 2.0 ** -8)
+
+
+def in_order(x, w, piece):
+    """The sums of a long product as the kernel takes them, in f32: a lane's pieces of `piece` elements a warp's width apart, each
+    summed on its own and added to the lane's sum, then halves of the warp."""
+    x, w = x.to(F64), w.to(F64)
+    z = lambda v: v.reshape(*v.shape[:-1], -1, 32, piece)
+    x, w = z(x)[:, None], z(w)[None]
+    acc = torch.zeros(x.shape[0], w.shape[1], 32, device="cuda")
+    for s in range(w.shape[2]):
+        part = (x[:, :, s, :, 1] * w[:, :, s, :, 1]).to(F32)
+        for j in (0, *range(2, piece)):
+            part = (x[:, :, s, :, j] * w[:, :, s, :, j] + part.to(F64)).to(F32)  # an fma: the product is exact in f64
+        acc += part
+    while acc.shape[-1] > 1:
+        acc = acc[..., : acc.shape[-1] // 2] + acc[..., acc.shape[-1] // 2:]
+    return acc[..., 0]
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 3, 4])
+@pytest.mark.parametrize("n,k,dtype", [(2050, 256, BF16), (2053, 1280, BF16), (2050, 1280, F32), (33, 8448, F32)])
+def test_order_of_long_sums(tokens, n, k, dtype):
+    """However many rows a warp works on, a sum has the bits of a row at a time: a choice between near ties may hang on them."""
+    from tilert_b200.models.deepseek_v3_2 import ops as dsa
+
+    x, w = rnd(0, 1, tokens, k, dtype=BF16), rnd(1, n, k, dtype=dtype, std=k ** -0.5)
+    o = torch.zeros(1, tokens, n, device="cuda")
+    dsa.rmsnorm_expert_proj(x, None, w, o, None, eps=1e-6)
+    assert torch.equal(o[0], in_order(x[0], w, 8 if dtype == BF16 else 4))

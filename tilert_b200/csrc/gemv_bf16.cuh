@@ -52,6 +52,10 @@ struct GemvX<__nv_bfloat16> {
     f[4] = __uint_as_float(u.z << 16); f[5] = __uint_as_float(u.z & 0xffff0000u);
     f[6] = __uint_as_float(u.w << 16); f[7] = __uint_as_float(u.w & 0xffff0000u);
   }
+  static __device__ __forceinline__ float4 four(const uint8_t* base, int, int i) {
+    const uint2 u = *reinterpret_cast<const uint2*>(base + i * 2);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+  }
   static __device__ __forceinline__ void put(uint8_t* base, int, int piece, const float (&f)[8]) {
     reinterpret_cast<uint4*>(base)[piece] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
   }
@@ -64,21 +68,32 @@ struct GemvX<float> {
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
     f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
   }
+  static __device__ __forceinline__ float4 four(const uint8_t* base, int k, int i) {
+    return reinterpret_cast<const float4*>(base)[(i & 4 ? k / 8 : 0) + (i >> 3)];
+  }
   static __device__ __forceinline__ void put(uint8_t* base, int k, int piece, const float (&f)[8]) {
     reinterpret_cast<float4*>(base)[piece] = make_float4(f[0], f[1], f[2], f[3]);
     reinterpret_cast<float4*>(base)[k / 8 + piece] = make_float4(f[4], f[5], f[6], f[7]);
   }
 };
-// Eight weights as loaded.
+// A lane's eight weights, as loaded, and activations of a step of 256 elements: a piece of eight bf16 weights, or two pieces of
+// four f32 ones 128 elements apart.  A piece's products are summed first, then added to the lane's sum.
 template <typename W>
 struct GemvW;
 template <>
 struct GemvW<__nv_bfloat16> {
   uint4 u;
-  __device__ __forceinline__ void load(const void* w, long long at) {
+  __device__ __forceinline__ void load(const void* w, long long step_at, int lane) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
-                 : "l"(reinterpret_cast<const __nv_bfloat16*>(w) + at));
+                 : "l"(reinterpret_cast<const __nv_bfloat16*>(w) + step_at + lane * 8));
+  }
+  template <typename X>
+  static __device__ __forceinline__ void operand(const uint8_t* base, int k, int step, int lane, float (&f)[8]) {
+    GemvX<X>::get(base, k, step * 32 + lane, f);
+  }
+  static __device__ __forceinline__ void add(float& acc, const float (&w)[8], const float (&f)[8]) {
+    acc += w[0] * f[0] + w[1] * f[1] + w[2] * f[2] + w[3] * f[3] + w[4] * f[4] + w[5] * f[5] + w[6] * f[6] + w[7] * f[7];
   }
   __device__ __forceinline__ void get(float (&f)[8]) const {
     f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
@@ -90,10 +105,20 @@ struct GemvW<__nv_bfloat16> {
 template <>
 struct GemvW<float> {
   float4 a, b;
-  __device__ __forceinline__ void load(const void* w, long long at) {
-    const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w) + at);
+  __device__ __forceinline__ void load(const void* w, long long step_at, int lane) {
+    const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w) + step_at) + lane;
     a = __ldg(p);
-    b = __ldg(p + 1);
+    b = __ldg(p + 32);
+  }
+  template <typename X>
+  static __device__ __forceinline__ void operand(const uint8_t* base, int k, int step, int lane, float (&f)[8]) {
+    const float4 x = GemvX<X>::four(base, k, step * 256 + lane * 4), y = GemvX<X>::four(base, k, step * 256 + 128 + lane * 4);
+    f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w;
+    f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
+  }
+  static __device__ __forceinline__ void add(float& acc, const float (&w)[8], const float (&f)[8]) {
+    acc += w[0] * f[0] + w[1] * f[1] + w[2] * f[2] + w[3] * f[3];
+    acc += w[4] * f[4] + w[5] * f[5] + w[6] * f[6] + w[7] * f[7];
   }
   __device__ __forceinline__ void get(float (&f)[8]) const {
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
@@ -128,14 +153,15 @@ __device__ __forceinline__ float warp_sums(float (&v)[N]) {
 
 // Long weights (vocabulary head, eh_proj).  A warp owns four rows at a time, so that a staged piece of the activations
 // serves four weights, and keeps the next two steps of 256 elements requested: 12 sixteen-byte loads per lane.  (With a
-// row per warp the reads of the activations were the bound for several tokens.)  Head 16160 x 7168, one / two / four
-// tokens: 47.7 / 49.9 / 54.9 us against 59.5 / 103.4 / 148.1 a row at a time; eh_proj 7168 x 14336: 46.4 / 48.2 / 54.9
-// against 61.5 / 91.7 / 182.0.
+// row per warp the reads of the activations were the bound for several tokens.)  Statistics and products are summed in the
+// order of a row per warp and an element per thread, so that the results have the bits of that form.  Back to back, head
+// 16160 x 7168, one / two / four tokens: 46.4 / 48.6 / 53.5 us against 64.9 / 114.9 / 147.5 a row at a time; eh_proj
+// 7168 x 14336: 45.0 / 46.8 / 54.2 against 69.1 / 93.8 / 187.1.
 template <int TOK, typename X, typename W>
 __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const GemvBf16Params p) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t gsm[];  // [TOK] GemvX<X>
-  __shared__ float red[2][TOK][32];
+  __shared__ float red[2][TOK][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kWarps = kGemvBf16Threads / 32;
   const size_t x_bytes = GemvX<X>::bytes(p.k);
@@ -146,7 +172,7 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
   auto request = [&](int group, int step, GemvW<W> (&dst)[kGemvBf16Rows]) {
 #pragma unroll
     for (int r = 0; r < kGemvBf16Rows; ++r)  // rows past the end: the last one, dropped below
-      dst[r].load(p.w, static_cast<long long>(min(group * kGemvBf16Rows + r, p.n - 1)) * p.k + (step * 32 + lane) * 8);
+      dst[r].load(p.w, static_cast<long long>(min(group * kGemvBf16Rows + r, p.n - 1)) * p.k + step * 256, lane);
   };
   int group = warp * gridDim.x + blockIdx.x;  // neighbouring CTAs read neighbouring rows
   int pg = group, ps = 0;                     // the next step to request
@@ -166,9 +192,6 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
   // stage (and normalise) the activations; with a second segment each one has its own statistics
   pdl_wait();
   const int k1 = p.x2 != nullptr ? p.k1 : p.k;
-  float ss[TOK], ss2[TOK];
-#pragma unroll
-  for (int t = 0; t < TOK; ++t) ss[t] = ss2[t] = 0.f;
   for (int i = threadIdx.x; i < pieces; i += kGemvBf16Threads) {
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
@@ -189,26 +212,42 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
         }
       }
       GemvX<X>::put(gsm + t * x_bytes, p.k, i, f);
-      float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += f[j] * f[j];
-      if (i * 8 < k1) ss[t] += s; else ss2[t] += s;
     }
   }
   if (p.gamma != nullptr) {
+    // Four warps per token.  A thread sums the squares of four neighbouring elements of every 512, each on its own, and 32 such
+    // sums are added as a warp that holds one each would add them.
+    __syncthreads();
+    if (warp / 4 < TOK) {
+      const int t = warp / 4, q = threadIdx.x & 127;
+      float ss[4] = {}, ss2[4] = {};
+#pragma unroll 7
+      for (int i = q * 4; i < p.k; i += 512) {
+        const float4 v = GemvX<X>::four(gsm + t * x_bytes, p.k, i);
+        const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      const float s = warp_sum(ss[t]), s2 = warp_sum(ss2[t]);
-      if (lane == 0) {
-        red[0][t][warp] = s;
-        red[1][t][warp] = s2;
+        for (int j = 0; j < 4; ++j) {
+          if (i < k1) ss[j] += f[j] * f[j]; else ss2[j] += f[j] * f[j];
+        }
+      }
+      auto thirty_two = [](float (&v)[4]) {
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+        return (v[0] + v[2]) + (v[1] + v[3]);
+      };
+      const float s = thirty_two(ss), s2 = thirty_two(ss2);
+      if (q % 8 == 0) {
+        red[0][t][q / 8] = s;
+        red[1][t][q / 8] = s2;
       }
     }
     __syncthreads();
     float rinv[TOK], rinv2[TOK];
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
-      const float tot = warp_sum(lane < kWarps ? red[0][t][lane] : 0.f), tot2 = warp_sum(lane < kWarps ? red[1][t][lane] : 0.f);
+      const float tot = warp_sum(lane < 16 ? red[0][t][lane] : 0.f), tot2 = warp_sum(lane < 16 ? red[1][t][lane] : 0.f);
       rinv[t] = rsqrtf(tot / static_cast<float>(k1) + p.eps);
       rinv2[t] = rsqrtf(tot2 / static_cast<float>(p.k - k1 > 0 ? p.k - k1 : 1) + p.eps);
     }
@@ -222,7 +261,7 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
         float f[8];
         GemvX<X>::get(gsm + t * x_bytes, p.k, i, f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] *= (first ? rinv[t] : rinv2[t]) * g[j];
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * (first ? rinv[t] : rinv2[t]) * g[j];
         GemvX<X>::put(gsm + t * x_bytes, p.k, i, f);
         __nv_bfloat16* out = first ? p.xnorm_out : p.xnorm2_out;
         if (blockIdx.x == 0 && t < p.n_tokens && out != nullptr) {
@@ -249,11 +288,9 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
 #pragma unroll
       for (int t = 0; t < TOK; ++t) {
         float f[8];
-        GemvX<X>::get(gsm + t * x_bytes, p.k, s * 32 + lane, f);
+        GemvW<W>::template operand<X>(gsm + t * x_bytes, p.k, s, lane, f);
 #pragma unroll
-        for (int r = 0; r < kGemvBf16Rows; ++r)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[r * TOK + t] += wf[r][j] * f[j];
+        for (int r = 0; r < kGemvBf16Rows; ++r) GemvW<W>::add(acc[r * TOK + t], wf[r], f);
       }
 #pragma unroll
       for (int d = 0; d < kGemvBf16Ahead; ++d)
