@@ -100,17 +100,6 @@ __device__ __forceinline__ void scaled_pieces(T* dst, const float* src, int n, f
     act_st8(dst + e, f);
   }
 }
-// this thread's share of the sum of squares, in pieces of four
-__device__ __forceinline__ float sum_squares4(const float* v, int n) {
-  float s = 0.f;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < n / 4; i += blockDim.x) {
-    const float4 f = reinterpret_cast<const float4*>(v)[i];
-    s += (f.x * f.x + f.y * f.y) + (f.z * f.z + f.w * f.w);
-  }
-  return s;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256) latent_tokens_kernel(const LatentTokensParams a) {
   pdl_launch_dependents();
@@ -121,13 +110,9 @@ __global__ void __launch_bounds__(256) latent_tokens_kernel(const LatentTokensPa
   const float* c = z + a.off_c;
   const float* kr = z + a.off_r;
   float sq = 0.f, sc = 0.f;
-  if (a.eights) {
-    sq = sum_squares4(z, a.q_rank);
-    sc = sum_squares4(c, a.r.rank);
-  } else {
-    for (int i = threadIdx.x; i < a.q_rank; i += 256) sq += z[i] * z[i];
-    for (int i = threadIdx.x; i < a.r.rank; i += 256) sc += c[i] * c[i];
-  }
+  // (an element at a time in both forms: the statistics have the same bits)
+  for (int i = threadIdx.x; i < a.q_rank; i += 256) sq += z[i] * z[i];
+  for (int i = threadIdx.x; i < a.r.rank; i += 256) sc += c[i] * c[i];
   const float rq = 1.f / sqrtf(cta_sum(sq, red) / static_cast<float>(a.q_rank) + a.eps);
   const float rc = 1.f / sqrtf(cta_sum(sc, red) / static_cast<float>(a.r.rank) + a.eps);
   T* cq = reinterpret_cast<T*>(a.cq) + t * a.ldq;
