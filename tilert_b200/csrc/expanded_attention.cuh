@@ -1,22 +1,24 @@
 // Attention of a portion of tokens over expanded keys and values (every head has its own) on tcgen05.
 //
 // A CTA has NQ tiles of 128 queries of one head and walks over the keys they see in tiles of 128.  Two threads issue the
-// TMA loads, one the products, and a warpgroup per query tile does the softmax with a row per thread (a TMEM lane): no
-// exchange between lanes anywhere.  Scores are f32 in TMEM; the probabilities go back, as bf16, over the scores they come
-// from and are the A operand of the value product straight from TMEM.  With two query tiles the products of one run under
-// the softmax of the other, and the tiles share the keys and values in shared memory.
+// TMA loads, one per query tile the products, and a warpgroup per query tile does the softmax with a row per thread (a TMEM
+// lane): no exchange between lanes anywhere.  Scores are f32 in TMEM; the probabilities go back, as bf16, over the scores they
+// come from and are the A operand of the value product straight from TMEM.  Either half of a tile's keys has its own scores,
+// probabilities and hand-over: the products of one half run under the softmax of the other, and of the other query tile, with
+// which the keys and values in shared memory are shared.
 //
-// The reference of the exponentials is the largest score so far, so that the largest probability of a row is an exact one in
-// bf16, and a warp rescales its rows' sums in TMEM where one has grown.  (A reference that lags behind by up to 2^8 saves
-// most of that, 2 to 8 % of the time, but rounds the largest probability too: the error against 64 bits rises by up to a quarter
-// for peaked scores.)
+// The reference of the exponentials is the largest score so far, taken anew for every 64 keys, so that the largest probability
+// of a row is an exact one in bf16; a warp rescales its rows' sums in TMEM where one has grown, once the half before has been
+// added to them.  (One reference for 128 keys: errors up to 0.8 % larger, 275 us in place of 263 for the first size below, with
+// the products of a whole tile handed over at once.  A reference that lags behind by up to 2^8 saves most of the rescaling, 2 to
+// 8 % of the time, but rounds the largest probability too: errors up to a quarter larger for peaked scores.)
 //
-// Bound by the chain of a query tile's scores, softmax (a row's 128 exponentials) and value product, of which two run under
-// each other, and by the loads of keys and values, 80 KB a tile of 128 keys at 192 + 128 columns.  Against the mma.sync kernel
-// of window_attention.cuh (64 rows a CTA), which keeps portions of less than a tile and heads whose tiles do not fit: 32 heads
-// of 128 + 64 / 128 columns, 2048 queries behind 4096 keys 294 us (730 TFLOP/s), was 1787; a window of 1024 114 (452); 64
-// heads, 1357 queries from the start 123 (470); 16 heads, 300 queries 24 (46); 32 heads, 128 queries 20 (30).  The error
-// against 64 bits is that kernel's to half a per cent, 0.0016 to 0.0023 over sizes and spreads of scores.
+// Bound by the chain of a half's scores, softmax (64 exponentials of a row) and value product, several of which run under each
+// other, and by the loads of keys and values, 80 KB a tile of 128 keys at 192 + 128 columns.  Against the mma.sync kernel of
+// window_attention.cuh (64 rows a CTA), which keeps portions of less than a tile and heads whose tiles do not fit: 32 heads of
+// 128 + 64 / 128 columns, 2048 queries behind 4096 keys 263 us (817 TFLOP/s), was 1724; a window of 1024 93 (461), was 375; 64
+// heads, 1357 queries from the start 88 (429), was 375; 16 heads, 300 queries 17 (27), was 31; 32 heads, 128 queries 14 (12),
+// was 17.  The error against 64 bits is that kernel's to 0.1 %, 0.0016 to 0.0023 over sizes and spreads of scores.
 //
 // Keys lie in a ring.  A tile ends at the last key, after 128 keys, or at the ring's end, so that its rows are consecutive;
 // a tile of fewer keys loads the 128 rows that end with its last one (from the ring's beginning if there are fewer before
@@ -31,6 +33,7 @@ namespace tb {
 
 constexpr int kXaTile = 128;                       // queries, and keys, of a tile
 constexpr int kXaBox = kXaTile * 64 * 2;           // bytes of 128 rows x 64 columns, 128-byte swizzle
+constexpr int kXaHalf = 64;                        // keys whose exponentials have a common reference
 constexpr int kXaKeyStages = 2;
 
 struct ExpandedAttnParams {
@@ -122,8 +125,8 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
                          const __grid_constant__ CUtensorMap rotmap, const ExpandedAttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int kMaxV = 3;
-  __shared__ __align__(8) uint64_t q_full, k_full[kXaKeyStages], k_empty[kXaKeyStages], v_full[kMaxV], v_empty[kMaxV], s_full[NQ], p_full[NQ],
-      o_full[NQ], drain;
+  __shared__ __align__(8) uint64_t q_full, k_full[kXaKeyStages], k_empty[kXaKeyStages], v_full[kMaxV], v_empty[kMaxV], s_full[NQ][2],
+      p_full[NQ][2], v_done[NQ][2], o_full[NQ], drain[NQ];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -134,23 +137,30 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
   uint8_t* vs = ks + kXaKeyStages * k_bytes;
   constexpr int kTmemCols = NQ * 256;  // a score tile and a sum of each query tile
 
+  // heads vary fastest and the tokens with the longest key ranges come first
+  const int head = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * (NQ * kXaTile);
+  const int nq = NQ > 1 && t0 + kXaTile < p.rows ? NQ : 1;
+
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
     for (int i = 0; i < kXaKeyStages; ++i) {
       mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
+      mbar_init(&k_empty[i], nq);
     }
     for (int i = 0; i < kMaxV; ++i) {
       mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
+      mbar_init(&v_empty[i], nq);
     }
     for (int i = 0; i < NQ; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 4);
+      for (int h = 0; h < 2; ++h) {
+        mbar_init(&s_full[i][h], 1);
+        mbar_init(&p_full[i][h], 4);
+        mbar_init(&v_done[i][h], 1);
+      }
       mbar_init(&o_full[i], 1);
+      mbar_init(&drain[i], 1);
     }
-    mbar_init(&drain, 1);
     s_abort = 0;
     mbar_fence_init();
   }
@@ -164,14 +174,11 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
   const uint32_t tmem = warp_uniform(*reinterpret_cast<volatile uint32_t*>(&s_tmem));
   pdl_wait();
 
-  // heads vary fastest and the tokens with the longest key ranges come first
-  const int head = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * (NQ * kXaTile);
   const int pos0 = warp_uniform(*p.pos);
   const int win = p.window > 0 ? p.window : 0x7fffffff;
   // keys that query tile i sees: [lo(i), hi(i)); tile 0 always has tokens
   auto lo_of = [&](int i) { return p.window > 0 ? max(0, pos0 + t0 + i * kXaTile - p.window + 1) : 0; };
   auto hi_of = [&](int i) { return pos0 + min(t0 + (i + 1) * kXaTile, p.rows); };
-  const int nq = NQ > 1 && t0 + kXaTile < p.rows ? NQ : 1;
   const int lo = lo_of(0), hi = hi_of(nq - 1);
   auto sees = [&](int i, const XaKeyTile& t) { return i < nq && t.a < hi_of(i) && t.b > lo_of(i); };
   volatile int* abort = &s_abort;
@@ -228,12 +235,15 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
       }
     }
     for (uint32_t j = it > stages ? it - stages : 0; j < it; ++j) mbar_wait(&v_full[j % stages], (j / stages) & 1u);
-  } else if (warp == 1) {
-    const uint32_t s_idesc = umma_idesc_bf16(kXaTile, kXaTile), v_idesc = umma_idesc_bf16(kXaTile, p.vdimp) | (1u << 16);
-    const uint64_t qd0 = umma_desc_sw128(smem_u32(qs)), kd0 = umma_desc_sw128(smem_u32(ks)), vd0 = umma_desc_sw128_columns(smem_u32(vs));
-    auto scores = [&](int i, uint32_t stage) {
-      uint64_t qd = qd0 + static_cast<uint32_t>(i * k_bytes >> 4), kd = kd0 + (stage * k_bytes >> 4);
-      const uint32_t d = tmem + i * kXaTile;
+  } else if (warp == 1 || (warp == 3 && nq == 2)) {  // the products of a query tile
+    const int i = warp >> 1;
+    const uint32_t s_idesc = umma_idesc_bf16(kXaTile, kXaHalf), v_idesc = umma_idesc_bf16(kXaTile, p.vdimp) | (1u << 16);
+    const uint64_t qd0 = umma_desc_sw128(smem_u32(qs + i * k_bytes)), kd0 = umma_desc_sw128(smem_u32(ks));
+    const uint64_t vd0 = umma_desc_sw128_columns(smem_u32(vs));
+    const uint32_t ts = tmem + i * kXaTile, to = tmem + (NQ + i) * kXaTile;
+    auto scores = [&](int h, uint32_t stage) {
+      uint64_t qd = qd0, kd = kd0 + ((stage * k_bytes + h * kXaHalf * 128) >> 4);
+      const uint32_t d = ts + h * kXaHalf;
       for (int c = 0; c < p.k_boxes; ++c, qd += kXaBox >> 4, kd += kXaBox >> 4) {
         const int left = c < p.dim_boxes ? p.dimp / 16 - c * 4 : p.rotp / 16 - (c - p.dim_boxes) * 4;  // steps of 16 columns, 32 bytes
         if (left >= 4) {
@@ -245,40 +255,44 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
           for (int q = 0; q < left; ++q) umma_bf16(d, qd + 2 * q, kd + 2 * q, s_idesc, c | q);
         }
       }
-      if (elect_one()) umma_commit(&s_full[i]);
+      if (elect_one()) umma_commit(&s_full[i][h]);
     };
-    auto values = [&](int i, uint32_t stage, bool first) {
-      const uint64_t vd = vd0 + (stage * v_bytes >> 4);
+    auto values = [&](int h, uint32_t stage, bool first) {
+      const uint64_t vd = vd0 + ((stage * v_bytes + h * kXaHalf * 128) >> 4);
       if (elect_one()) {
 #pragma unroll
-        for (int c = 0; c < kXaTile / 16; ++c)  // sixteen keys: eight columns of probabilities, sixteen rows of values
-          umma_bf16_ta(tmem + (NQ + i) * kXaTile, tmem + i * kXaTile + c * 8, vd + c * (2048 >> 4), v_idesc, !first || c != 0);
+        for (int c = 0; c < kXaHalf / 16; ++c)  // sixteen keys: eight columns of probabilities, sixteen rows of values
+          umma_bf16_ta(to, ts + h * kXaHalf + c * 8, vd + c * (2048 >> 4), v_idesc, !first || c != 0);
+        umma_commit(&v_done[i][h]);
       }
     };
     bool ok = mbar_wait_warp(&q_full, 0, abort);
-    uint32_t n_p[NQ] = {};  // tiles whose probabilities have been taken
+    uint32_t n_p = 0;  // tiles whose probabilities have been taken
     uint32_t it = 0;
-    int prev = -1;          // beginning of the tile before
+    int prev = -1;     // beginning of the tile before
     for (int a = lo; ok; ++it) {
       const bool more = a < hi;
       const XaKeyTile t(more ? a : hi - 1, hi, p.ring), u(prev < 0 ? lo : prev, hi, p.ring);
       const uint32_t ksg = it % kXaKeyStages, vsg = (it - 1) % p.v_stages;
+      const bool take = prev >= 0 && sees(i, u), give = more && sees(i, t);
       if (prev >= 0) ok = mbar_wait_warp(&v_full[vsg], ((it - 1) / p.v_stages) & 1u, abort);
 #pragma unroll
-      for (int i = 0; i < NQ; ++i) {
-        if (ok && prev >= 0 && sees(i, u)) {
-          ok = mbar_wait_warp(&p_full[i], n_p[i] & 1u, abort);
+      for (int h = 0; h < 2; ++h) {
+        if (ok && take) {
+          ok = mbar_wait_warp(&p_full[i][h], n_p & 1u, abort);
           if (ok) {
             tc_fence_after();
-            values(i, vsg, n_p[i] == 0);
-            ++n_p[i];
-            if (u.b >= hi_of(i) && elect_one()) umma_commit(&o_full[i]);
+            values(h, vsg, (n_p | h) == 0);
           }
         }
-        if (ok && more && i == 0) ok = mbar_wait_warp(&k_full[ksg], (it / kXaKeyStages) & 1u, abort);
-        if (ok && more && sees(i, t)) scores(i, ksg);
+        if (ok && more && h == 0) ok = mbar_wait_warp(&k_full[ksg], (it / kXaKeyStages) & 1u, abort);
+        if (ok && give) scores(h, ksg);
       }
       if (!ok) break;
+      if (take) {
+        ++n_p;
+        if (u.b >= hi_of(i) && elect_one()) umma_commit(&o_full[i]);
+      }
       if (prev >= 0 && elect_one()) umma_commit(&v_empty[vsg]);
       if (!more) break;
       if (elect_one()) umma_commit(&k_empty[ksg]);
@@ -290,8 +304,8 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
       *abort = 1;
     }
     __syncwarp();
-    if (elect_one()) umma_commit(&drain);  // products still running read shared memory and write TMEM
-    mbar_wait(&drain, 0);
+    if (elect_one()) umma_commit(&drain[i]);  // products still running read shared memory and write TMEM
+    mbar_wait(&drain[i], 0);
   } else if (warp >= 4 && (warp - 4) / 4 < nq) {
     const int i = (warp - 4) / 4, quad = warp & 3;
     const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
@@ -301,85 +315,94 @@ __global__ void __launch_bounds__(128 + 128 * NQ, 1)
     const int qpos = t < p.rows ? pos0 + t : -1;  // a row without a token sees nothing
     const float c = p.scale * 1.4426950408889634f;
     float m = -INFINITY, l[4] = {0.f, 0.f, 0.f, 0.f};
+    auto rescale = [&](float corr) {
+      int v = 0;
+      for (; v + 32 <= p.vdimp; v += 32) {
+        uint32_t o[32];
+        tmem_ld32_issue(so + v, o);
+        tmem_wait_ld();
+        tmem_use32(o);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+        tmem_st32(so + v, o);
+      }
+      if (v < p.vdimp) {
+        uint32_t o[16];
+        tmem_ld16(so + v, o);
+        tmem_ld16_wait(o);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+        tmem_st16(so + v, o);
+      }
+    };
     uint32_t n = 0;
     bool ok = true;
     for (int a = lo; a < hi;) {
       const XaKeyTile kt(a, hi, p.ring);
       a = kt.b;
       if (!sees(i, kt)) continue;
-      ok = mbar_wait(&s_full[i], n & 1u, abort);
-      if (__any_sync(0xffffffffu, !ok)) {  // warp-uniform: tcgen05.ld needs every lane
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      uint32_t r[4][32];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) tmem_ld32_issue(sc + q * 32, r[q]);
-      tmem_wait_ld();
-#pragma unroll
-      for (int q = 0; q < 4; ++q) tmem_use32(r[q]);
       // every key of an inner tile is visible to every row (rows without a token are never stored)
-      if (!(kt.key0 == kt.a && kt.b == kt.a + kXaTile && kt.b - 1 <= first_q && last_q - kt.a < win)) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int key = kt.key0 + q * 32 + j;
-            const bool hidden = key < kt.a || key >= kt.b || key > qpos || qpos - key >= win;
-            if (hidden) r[q][j] = 0xff800000u;
-          }
-      }
-      float mx = -INFINITY;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        mx = fmaxf(mx, fmaxf(fmaxf(__uint_as_float(r[0][j]), __uint_as_float(r[1][j])), fmaxf(__uint_as_float(r[2][j]), __uint_as_float(r[3][j]))));
-      mx = fmaxf(mx, m);
-      const float corr = mx == m ? 1.f : exp2_approx((m - mx) * c);
-      m = mx;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) l[q] *= corr;
-      const float mc = m == -INFINITY ? 0.f : m * c;
+      const bool inner = kt.key0 == kt.a && kt.b == kt.a + kXaTile && kt.b - 1 <= first_q && last_q - kt.a < win;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
+        ok = mbar_wait(&s_full[i][h], n & 1u, abort);
+        if (__any_sync(0xffffffffu, !ok)) {  // warp-uniform: tcgen05.ld needs every lane
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        uint32_t r[2][32];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) tmem_ld32_issue(sc + h * kXaHalf + q * 32, r[q]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) tmem_use32(r[q]);
+        if (!inner) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int key = kt.key0 + h * kXaHalf + q * 32 + j;
+              const bool hidden = key < kt.a || key >= kt.b || key > qpos || qpos - key >= win;
+              if (hidden) r[q][j] = 0xff800000u;
+            }
+        }
+        float top = m;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) top = fmaxf(top, fmaxf(__uint_as_float(r[0][j]), __uint_as_float(r[1][j])));
+        const float corr = top == m ? 1.f : exp2_approx((m - top) * c);
+        m = top;
+        const float mc = m == -INFINITY ? 0.f : m * c;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) l[q] *= corr;
         uint32_t w[32];
 #pragma unroll
         for (int q = 0; q < 2; ++q)
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float e0 = exp2_approx(fmaf(__uint_as_float(r[2 * h + q][j]), c, -mc));
-            const float e1 = exp2_approx(fmaf(__uint_as_float(r[2 * h + q][j + 1]), c, -mc));
+            const float e0 = exp2_approx(fmaf(__uint_as_float(r[q][j]), c, -mc));
+            const float e1 = exp2_approx(fmaf(__uint_as_float(r[q][j + 1]), c, -mc));
             l[2 * q] += e0;
             l[2 * q + 1] += e1;
             w[q * 16 + j / 2] = pack_bf16x2(e0, e1);
           }
-        tmem_st32(sc + h * 32, w);
-      }
-      // (the product that wrote the sums is complete: the scores of this tile were issued behind it)
-      if (n > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-        int v = 0;
-        for (; v + 32 <= p.vdimp; v += 32) {
-          uint32_t o[32];
-          tmem_ld32_issue(so + v, o);
-          tmem_wait_ld();
-          tmem_use32(o);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
-          tmem_st32(so + v, o);
+        tmem_st32(sc + h * kXaHalf, w);
+        if ((n > 0 || h > 0) && __any_sync(0xffffffffu, corr != 1.f)) {
+          // the product of the half before writes the sums too
+          ok = mbar_wait(&v_done[i][h ^ 1], (n - (h ^ 1)) & 1u, abort);
+          if (__any_sync(0xffffffffu, !ok)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          rescale(corr);
         }
-        if (v < p.vdimp) {
-          uint32_t o[16];
-          tmem_ld16(so + v, o);
-          tmem_ld16_wait(o);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
-          tmem_st16(so + v, o);
-        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[i][h]);
       }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[i]);
+      if (!ok) break;
       ++n;
     }
     if (ok) ok = mbar_wait(&o_full[i], 0, abort);
