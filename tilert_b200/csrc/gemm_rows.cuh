@@ -504,6 +504,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
   const int n_kb = (p.k + kTcK * q.blocks - 1) / (kTcK * q.blocks);  // (what lies beyond K is zero)
   const int block_bytes = kWBytes + q.bn / 2 * kTcK * 2;
   volatile int* abort = &s_abort;
+  auto give_up = [&] {  // a wait that ran out ends both CTAs' roles
+    *abort = 1;
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(&s_abort, rank ^ 1u)), "r"(1) : "memory");
+  };
   TileWalk walk{s_rows, s_tiles, groups, ft, q.bn, 2 * kFeats};
   const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
   const int half = q.bn / 2;  // token rows of a CTA
@@ -538,11 +542,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         if (++s == stages) s = 0, ph ^= 1u;
       }
     }
-    if (!ok) *abort = 1;
-    // What is under way into this shared memory lands before the CTA goes: copies, and arrivals of the other CTA's products.
+    if (!ok) give_up();
+    // What is under way into shared memory lands before the pair goes: copies, which the first CTA waits for on behalf of both
+    // and whatever has failed, and arrivals of the other CTA's products.  After a failure one CTA may have requested a stage
+    // that the other has not; no barrier tells when such a copy lands, so a wait that runs out gives it its time, once.
     const uint32_t from = it > stages ? it - stages : 0;
-    if (rank == 0)
-      for (uint32_t j = from; j < it; ++j) mbar_wait(&full[j % stages], (j / stages) & 1u, abort);
+    if (rank == 0) {
+      bool landed = true;
+      for (uint32_t j = from; landed && j < it; ++j) landed = mbar_wait(&full[j % stages], (j / stages) & 1u);
+      if (landed && !ok) mbar_wait(&full[it % stages], (it / stages) & 1u);
+    }
     for (uint32_t j = from; j < it; ++j) mbar_wait(&empty[j % stages], (j / stages) & 1u, abort);
   } else if (warp == 1) {
     if (rank == 0) {
@@ -579,7 +588,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
           if (++s == stages) s = 0, ph ^= 1u;
         }
       }
-      if (!ok) *abort = 1;
+      if (!ok) give_up();
       __syncwarp();
       // products still running read shared memory and write TMEM
       if (elect_one()) asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&drain)) : "memory");
@@ -597,7 +606,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
       const bool ok = mbar_wait(&acc_full[buf], aph, abort);
       if (__any_sync(0xffffffffu, !ok)) {  // warp-uniform: tcgen05.ld needs every lane
         if (!ok) set_status(p.status, ST_WAIT_FULL_TIMEOUT);
-        *abort = 1;
+        give_up();
         break;
       }
       tc_fence_after();
