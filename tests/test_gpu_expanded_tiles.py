@@ -132,3 +132,23 @@ def test_error_of_the_probabilities(ops, rows, pos, window, spread):
         top = new
     rounded = (num / den).to(BF16).to(F64).transpose(0, 1)
     assert float((out.view_as(want).to(F64) - want).norm()) <= 1.001 * float((rounded - want).norm())
+
+
+@pytest.mark.parametrize("rows,pos,window,ring", [(200, 1189, 30, 600), (129, 700, 1, 300), (300, 2 * 450 - 7, 70, 450), (640, 1000, 129, 801)])
+def test_rows_that_no_query_sees(ops, rows, pos, window, ring):
+    """Cache rows of positions before the window of the first query change nothing, whatever they hold; tiles that end with the
+    ring have keys of other tiles, or such rows, next to them."""
+    heads, dim, rot, vdim, rank, t = 3, 64, 32, 64, 64, pos + rows
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    mix = types.SimpleNamespace(heads=heads, dim=dim, rot_dim=rot, vdim=vdim, kv_rank=rank, scale=(dim + rot) ** -0.5)
+    q, kv = rnd(gen, rows, heads, dim + rot), rnd(gen, ring, heads * (dim + vdim))
+    cache = types.SimpleNamespace(rows=rnd(gen, ring, ops.latent_row_len(rank, rot)), ring=ring, window=window)
+    unseen = torch.ones(ring, dtype=torch.bool, device="cuda")
+    unseen[torch.arange(pos - window + 1, t, device="cuda") % ring] = False
+    outs = []
+    for other in (0.0, float("nan"), float("inf")):
+        kv[unseen], cache.rows[unseen] = other, other
+        out = torch.zeros(rows, heads * vdim, dtype=BF16, device="cuda")
+        ops.expanded_attn(q, kv, cache, rows, mix, torch.tensor([pos], dtype=I32, device="cuda"), None, None, False, out)
+        outs.append(out)
+    assert bool(outs[0].isfinite().all()) and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])

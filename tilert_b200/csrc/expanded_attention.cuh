@@ -20,9 +20,10 @@
 // heads, 1357 queries from the start 88 (429), was 375; 16 heads, 300 queries 17 (27), was 31; 32 heads, 128 queries 14 (12),
 // was 17.  The error against 64 bits is that kernel's to 0.1 %, 0.0016 to 0.0023 over sizes and spreads of scores.
 //
-// Keys lie in a ring.  A tile ends at the last key, after 128 keys, or at the ring's end, so that its rows are consecutive;
-// a tile of fewer keys loads the 128 rows that end with its last one (from the ring's beginning if there are fewer before
-// it) and hides the others.  That stays inside the rows in use because a launch has at least 128 tokens.
+// Keys lie in a ring.  A tile ends at the last key, after 128 keys, or at the ring's end, so that its rows are consecutive; 128
+// rows are loaded, from the first key at the ring's end and up to the last key elsewhere, and what is no key of the tile is
+// hidden.  Those rows are outside of the ring (and zeros), or hold tokens of this portion, which has at least 128: a hidden
+// value has a probability of zero, but is multiplied by it, and a row that no query may see can hold anything.
 #pragma once
 
 #include "act.cuh"
@@ -62,7 +63,7 @@ struct XaKeyTile {
   __device__ __forceinline__ XaKeyTile(int a_, int hi, int ring) : a(a_) {
     const int slot = a % ring;
     b = min(min(a + kXaTile, hi), a + ring - slot);
-    row0 = max(0, slot + (b - a) - kXaTile);
+    row0 = b - a == ring - slot ? slot : slot + (b - a) - kXaTile;  // rows outside of [0, ring) are loaded as zeros
     key0 = a - (slot - row0);
   }
 };
