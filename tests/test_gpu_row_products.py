@@ -144,7 +144,7 @@ def in_order(x, w, piece):
 
 
 @pytest.mark.parametrize("tokens", [1, 2, 3, 4])
-@pytest.mark.parametrize("n,k,dtype", [(2050, 256, BF16), (2053, 1280, BF16), (2050, 1280, F32), (33, 8448, F32)])
+@pytest.mark.parametrize("n,k,dtype", [(2050, 256, BF16), (2053, 1280, BF16), (2368, 1280, F32), (33, 8448, F32), (2369, 768, F32), (4099, 256, BF16)])
 def test_order_of_long_sums(tokens, n, k, dtype):
     """However many rows a warp works on, a sum has the bits of a row at a time: a choice between near ties may hang on them."""
     from tilert_b200.models.deepseek_v3_2 import ops as dsa
@@ -153,3 +153,26 @@ def test_order_of_long_sums(tokens, n, k, dtype):
     o = torch.zeros(1, tokens, n, device="cuda")
     dsa.rmsnorm_expert_proj(x, None, w, o, None, eps=1e-6)
     assert torch.equal(o[0], in_order(x[0], w, 8 if dtype == BF16 else 4))
+
+
+@pytest.mark.parametrize("tokens", [1, 4])
+def test_few_long_rows(tokens):
+    """A rank's row share of an input product, fewer rows than the GPU has warps: no walk of a warp over four rows, which takes as
+    long as four times the SMs' warps in rows do.  (Measured: two thirds of the whole product's time, was nine tenths.)"""
+    from tilert_b200.models.deepseek_v3_2 import ops as dsa
+
+    dim = 7168
+    e, h, ge, gh = rnd(0, 1, tokens, dim, dtype=BF16), rnd(1, 1, tokens, dim, dtype=BF16), rnd(2, dim), rnd(3, dim)
+    w, o = torch.zeros(dim, 2 * dim, dtype=BF16, device="cuda"), torch.zeros(1, tokens, dim, dtype=BF16, device="cuda")
+
+    def us(rows):
+        begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        for i in range(50):
+            if i == 10:
+                begin.record()
+            dsa.mtp_preprocess_rows(e, h, ge, gh, w, o, 0, rows)
+        end.record()
+        torch.cuda.synchronize()
+        return begin.elapsed_time(end)
+
+    assert min(us(512) for _ in range(3)) < 0.8 * min(us(dim) for _ in range(3))

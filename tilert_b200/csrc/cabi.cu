@@ -1034,22 +1034,24 @@ int record_hook(TbContext* ctx, const AttnPrepParams& prep) {
   return TB_OK;
 }
 
-template <int TOK, typename X, typename W>
+template <int TOK, int ROWS, typename X, typename W>
 int launch_gemv_long(TbContext* ctx, const GemvBf16Params& p, cudaStream_t st) {
   const size_t smem = TOK * GemvX<X>::bytes(p.k);
   TB_REQUIRE(smem <= 200 * 1024);
-  const int warps = kGemvBf16Threads / 32 * kGemvBf16Rows, need = (p.n + warps - 1) / warps;
-  TB_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<TOK, X, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  // few rows: still a CTA per SM, with fewer busy warps each
-  TB_CUDA(launch(gemv_bf16_kernel<TOK, X, W>, dim3(need < ctx->num_sms && p.n < ctx->num_sms * kGemvBf16Rows ? need : ctx->num_sms),
-                 dim3(kGemvBf16Threads), smem, st, p));
+  TB_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<TOK, ROWS, X, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  const int groups = (p.n + ROWS - 1) / ROWS;  // a group a CTA first, then a second: few rows are spread over all SMs
+  TB_CUDA(launch(gemv_bf16_kernel<TOK, ROWS, X, W>, dim3(groups < ctx->num_sms ? groups : ctx->num_sms), dim3(kGemvBf16Threads), smem, st, p));
   return TB_OK;
 }
 template <typename X, typename W>
 int launch_gemv_long(TbContext* ctx, const GemvBf16Params& p, cudaStream_t st) {
-  if (p.n_tokens == 1) return launch_gemv_long<1, X, W>(ctx, p, st);
-  if (p.n_tokens == 2) return launch_gemv_long<2, X, W>(ctx, p, st);
-  return launch_gemv_long<4, X, W>(ctx, p, st);
+  // A row per warp while all SMs have a warp for each, else four.  One / two / four tokens, us: 512 rows of 14336 30 / 32 / 36
+  // (four rows per warp: 40 / 42 / 46), 2368 rows 32 / 34 / 40 (41 / 42 / 46), 3072 rows 58 / 59 / 64 (42 / 43 / 48); 2368 rows
+  // of 7168 15 / 17 / 21 (19 / 21 / 25), 3000 rows 24 / 26 / 30 (21 / 23 / 27).
+  const bool one = p.n <= ctx->num_sms * (kGemvBf16Threads / 32);
+  if (p.n_tokens == 1) return one ? launch_gemv_long<1, 1, X, W>(ctx, p, st) : launch_gemv_long<1, 4, X, W>(ctx, p, st);
+  if (p.n_tokens == 2) return one ? launch_gemv_long<2, 1, X, W>(ctx, p, st) : launch_gemv_long<2, 4, X, W>(ctx, p, st);
+  return one ? launch_gemv_long<4, 1, X, W>(ctx, p, st) : launch_gemv_long<4, 4, X, W>(ctx, p, st);
 }
 
 template <int TOK>

@@ -35,8 +35,6 @@ struct GemvBf16Params {
 };
 
 constexpr int kGemvBf16Threads = 512;
-constexpr int kGemvBf16Rows = 4;   // weight rows that a warp works on together
-constexpr int kGemvBf16Ahead = 2;  // steps of a warp (256 elements of its rows) requested beyond the current one
 
 // Eight activations (a piece) of a token as staged in shared memory: bf16 where they are bf16 values (rounded, or not
 // normalised), else f32 with the halves of a piece apart -- a warp's 16-byte reads are free of bank conflicts either way.
@@ -153,26 +151,28 @@ __device__ __forceinline__ float warp_sums(float (&v)[N]) {
 
 // Long weights (vocabulary head, eh_proj).  A warp owns four rows at a time, so that a staged piece of the activations
 // serves four weights, and keeps the next two steps of 256 elements requested: 12 sixteen-byte loads per lane.  (With a
-// row per warp the reads of the activations were the bound for several tokens.)  Statistics and products are summed in the
-// order of a row per warp and an element per thread, so that the results have the bits of that form.  Back to back, head
-// 16160 x 7168, one / two / four tokens: 46.4 / 48.6 / 53.5 us against 64.9 / 114.9 / 147.5 a row at a time; eh_proj
-// 7168 x 14336: 45.0 / 46.8 / 54.2 against 69.1 / 93.8 / 187.1.
-template <int TOK, typename X, typename W>
+// row per warp the reads of the activations are the bound for several tokens.)  Rows that are no more than the warps go one
+// to a warp with seven steps requested: nothing is shared, and a walk along K is all there is to wait for.
+// Statistics and products are summed in the order of a row per warp and an element per thread in every form, so that the
+// results have the same bits.  Back to back, head 16160 x 7168, one / two / four tokens: 46.4 / 48.6 / 53.5 us (a row per
+// warp, without steps requested, 64.9 / 114.9 / 147.5); eh_proj 7168 x 14336: 45.0 / 46.8 / 54.2 (69.1 / 93.8 / 187.1).
+template <int TOK, int ROWS, typename X, typename W>
 __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const GemvBf16Params p) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t gsm[];  // [TOK] GemvX<X>
   __shared__ float red[2][TOK][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kWarps = kGemvBf16Threads / 32;
+  constexpr int kAhead = ROWS == 1 ? (sizeof(W) == 2 ? 7 : 3) : 2;  // steps (256 elements of the warp's rows) requested beyond the current one
   const size_t x_bytes = GemvX<X>::bytes(p.k);
   const int pieces = p.k / 8, steps = pieces / 32;
-  const int groups = (p.n + kGemvBf16Rows - 1) / kGemvBf16Rows, stride = gridDim.x * kWarps;
+  const int groups = (p.n + ROWS - 1) / ROWS, stride = gridDim.x * kWarps;
 
-  GemvW<W> w[kGemvBf16Ahead + 1][kGemvBf16Rows];
-  auto request = [&](int group, int step, GemvW<W> (&dst)[kGemvBf16Rows]) {
+  GemvW<W> w[kAhead + 1][ROWS];
+  auto request = [&](int group, int step, GemvW<W> (&dst)[ROWS]) {
 #pragma unroll
-    for (int r = 0; r < kGemvBf16Rows; ++r)  // rows past the end: the last one, dropped below
-      dst[r].load(p.w, static_cast<long long>(min(group * kGemvBf16Rows + r, p.n - 1)) * p.k + step * 256, lane);
+    for (int r = 0; r < ROWS; ++r)  // rows past the end: the last one, dropped below
+      dst[r].load(p.w, static_cast<long long>(min(group * ROWS + r, p.n - 1)) * p.k + step * 256, lane);
   };
   int group = warp * gridDim.x + blockIdx.x;  // neighbouring CTAs read neighbouring rows
   int pg = group, ps = 0;                     // the next step to request
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
   };
   // the weights do not depend on the predecessor
 #pragma unroll
-  for (int d = 0; d < kGemvBf16Ahead; ++d) {
+  for (int d = 0; d < kAhead; ++d) {
     if (pg < groups) request(pg, ps, w[d]);
     advance();
   }
@@ -275,31 +275,31 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
   __syncthreads();
 
   for (; group < groups; group += stride) {
-    float acc[kGemvBf16Rows * TOK];
+    float acc[ROWS * TOK];
 #pragma unroll
-    for (int i = 0; i < kGemvBf16Rows * TOK; ++i) acc[i] = 0.f;
-#pragma unroll 3
+    for (int i = 0; i < ROWS * TOK; ++i) acc[i] = 0.f;
+#pragma unroll (kAhead + 1)
     for (int s = 0; s < steps; ++s) {
-      if (pg < groups) request(pg, ps, w[kGemvBf16Ahead]);
+      if (pg < groups) request(pg, ps, w[kAhead]);
       advance();
-      float wf[kGemvBf16Rows][8];
+      float wf[ROWS][8];
 #pragma unroll
-      for (int r = 0; r < kGemvBf16Rows; ++r) w[0][r].get(wf[r]);
+      for (int r = 0; r < ROWS; ++r) w[0][r].get(wf[r]);
 #pragma unroll
       for (int t = 0; t < TOK; ++t) {
         float f[8];
         GemvW<W>::template operand<X>(gsm + t * x_bytes, p.k, s, lane, f);
 #pragma unroll
-        for (int r = 0; r < kGemvBf16Rows; ++r) GemvW<W>::add(acc[r * TOK + t], wf[r], f);
+        for (int r = 0; r < ROWS; ++r) GemvW<W>::add(acc[r * TOK + t], wf[r], f);
       }
 #pragma unroll
-      for (int d = 0; d < kGemvBf16Ahead; ++d)
+      for (int d = 0; d < kAhead; ++d)
 #pragma unroll
-        for (int r = 0; r < kGemvBf16Rows; ++r) w[d][r] = w[d + 1][r];
+        for (int r = 0; r < ROWS; ++r) w[d][r] = w[d + 1][r];
     }
-    constexpr int kSums = kGemvBf16Rows * TOK, kLanes = 32 / kSums;  // lanes that hold the same sum
+    constexpr int kSums = ROWS * TOK, kLanes = 32 / kSums;  // lanes that hold the same sum
     const float sum = warp_sums<kSums>(acc);
-    const int i = lane / kLanes, row = group * kGemvBf16Rows + i / TOK, t = i % TOK;
+    const int i = lane / kLanes, row = group * ROWS + i / TOK, t = i % TOK;
     if (lane % kLanes == 0 && row < p.n && t < p.n_tokens) {
       if (p.out_bf16)
         reinterpret_cast<__nv_bfloat16*>(p.out)[t * p.out_stride + row] = f2bf(sum);
