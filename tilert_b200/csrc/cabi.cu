@@ -1076,8 +1076,9 @@ int launch_gemv_bf16(TbContext* ctx, GemvBf16Params& p, cudaStream_t st) {
     auto a16 = [](const void* q, long long ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 8 == 0; };
     p.aligned = a16(p.x, p.x_stride) && (p.x2 == nullptr || (a16(p.x2, p.x2_stride) && p.k1 % 8 == 0));
     const bool half = p.gamma == nullptr || p.round_norm_bf16;  // the staged activations are bf16 values
+    TB_REQUIRE(half || !p.w_is_f32);                            // (f32 weights are the router's, which rounds its input)
     if (p.w_is_f32)
-      rc = half ? launch_gemv_long<__nv_bfloat16, float>(ctx, p, st) : launch_gemv_long<float, float>(ctx, p, st);
+      rc = launch_gemv_long<__nv_bfloat16, float>(ctx, p, st);
     else
       rc = half ? launch_gemv_long<__nv_bfloat16, __nv_bfloat16>(ctx, p, st) : launch_gemv_long<float, __nv_bfloat16>(ctx, p, st);
   }
