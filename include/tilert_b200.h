@@ -19,7 +19,12 @@
  *     ordered on one stream.  Whatever the context, streaming launches (every FP8 product, chained launches, the
  *     indexer's selection, `tilert_b200_matvec_fp8_static`) must not overlap on a device: each needs all of its
  *     thread blocks resident at once (they wait on one another, bounded), so two of them running side by side from
- *     different streams can each be left half resident, wait out their budget and return a status code.
+ *     different streams can each be left half resident, wait out their budget and return a status code;
+ *   - weights (products' matrices, norm gains, rotation tables) are constants to the library: a call may read them
+ *     before the launches queued ahead of it on its stream have finished (the vocabulary head and the product of
+ *     `tilert_mtp_preprocess_op` too, which once waited first).  A caller that changes a weight waits for the change,
+ *     on the host or with an event, before it queues the first call that uses it.  Activations, caches, positions and
+ *     routing are read in stream order.
  *
  * Weight operands named `*_packed` are in the library's block format (128x128 e4m3 tiles in
  * the tensor core's shared-memory operand order followed by their scales, see tilert_b200/csrc/formats.h); they are
