@@ -173,7 +173,11 @@ int tilert_gqa_latent_merge_op(TgContext* ctx, const float* part, int tokens, in
 int tilert_gqa_gate_heads_op(TgContext* ctx, const float* o, int ldv, int rows, int heads, int vdim, const float* gate,
                              long long ldg, int per_head, void* out, long long ldo, int f32, void* stream);
 /* The expanded form on bf16 tiles: kv [ring, heads * pad16(dim) | heads * pad16(vdim)] holds the keys and values of the
- * cache rows in use, the rotated key part is read from the cache.  Sink and gate as above, out [rows, heads * vdim]. */
+ * cache rows in use, the rotated key part is read from the cache.  Sink and gate as above, out [rows, heads * vdim].
+ * Queries share tiles of keys: an infinity or NaN in the value row of a token of the portion, or of one in the window of its
+ * first query, reaches all of the up to 128 queries next to one another that walk over its tile of 128 keys (64 and 64 where
+ * the portion has fewer than 128 tokens or the sizes do not fit the wide tiles), also those that do not see it.  Rows that no
+ * query of the portion sees are not read. */
 int tilert_gqa_expanded_attn_op(TgContext* ctx, const void* q, const void* kv, const void* cache, int rows, int heads, int dim,
                                 int rot, int vdim, int rank, const int* pos, int window, int ring, float scale,
                                 const float* sink, const float* gate, long long ldg, int per_head, void* out, long long ldo,
