@@ -108,8 +108,9 @@ constexpr int kTcK = 64;
 
 // BM features x 64 token rows.  Few tiles leave most SMs idle and a step along K bound by one SM's loads and by the
 // hand-shakes of a stage: 64 features spread the weights over twice the SMs.  37 rows, 2048 features, K 5632: 16.0 us in tiles
-// of 64 features, 18.3 of 128, 24.0 with stages of 64 along K; 173 x 2048 x 2048 8.5, 9.1, 10.9.  A stage is two blocks of 64 along K (hand-shakes cost as much as a block's products), one
-// where two would leave two stages.
+// of 64 features, 18.3 of 128, 24.0 with stages of 64 along K; 173 x 2048 x 2048 8.5, 9.1, 10.9.
+// A stage is two blocks of 64 along K, since its hand-shakes cost as much as a block's products; one where two would leave two
+// stages.
 template <int BM, bool GATED>
 struct TcShape {
   static constexpr int kBN = 64;

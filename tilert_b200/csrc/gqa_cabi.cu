@@ -117,7 +117,10 @@ int make_gated_map(CUtensorMap* map, const void* base, int groups, int n, int k,
 
 template <bool GATED>
 int launch_pair(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int bn, void* stream) {
-  const int blocks = bn <= 160 ? 2 : 1;  // (wider tiles: a step's products hide its hand-shakes, and the ring wants the stages)
+  // Two blocks a stage where a block's products do not hide its hand-shakes: 128 rows 322 us with two, 428 with one (1357 x 7168 x
+  // 18432), 224 rows 593 and 561 (gated 1357 x 18432 x 7168), where the ring wants the stages.  Tiles of 160 rows, of whose
+  // stages three fit with two blocks, take the same either way: 0.94 to 1.08 over nine products, 1.00 in the mean.
+  const int blocks = bn <= 160 ? 2 : 1;
   PairTiles q{bn, blocks, 0, blocks * (128 * kTcK * 2 + bn / 2 * kTcK * 2)};
   q.stages = 196608 / q.stage_bytes < kPairMaxStages ? 196608 / q.stage_bytes : kPairMaxStages;
   CUtensorMap wmap, xmap;
@@ -320,7 +323,8 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
   auto tiles = [&](int feats, int bn) { return static_cast<long long>(wide) * ((n + feats - 1) / feats) * ((rows + bn - 1) / bn); };
   auto round_up = [](long long tiles, int units) { return static_cast<double>((tiles + units - 1) / units); };
   if (n_groups > 0 && counts != nullptr) {
-    // The counts are on the device: a tile that holds an average group and a fifth.  Below 64 rows a group it is the weights'
+    // The counts are on the device: a tile that holds an average group and a fifth, or, above 213 rows a group, the largest, of
+    // which a group may need a second that it does not fill.  Below 64 rows a group it is the weights'
     // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 114 us, in pairs 141; 75 rows
     // 97 in pairs, was 120; 156 rows 303, 256 rows 440; gated, 1000 to 1536 features), in small tiles if the groups that
     // there can be are few (16 rows over 30 experts 16.0 us, in tiles of 128 features 19.5).

@@ -9,11 +9,11 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-// The loops that issue copies and products run on whole warps and one lane issues: what the instructions take is then
-// computed in uniform registers.  Under a branch on the lane every operand of every tcgen05.mma is moved there on its own,
-// which paces the products at about 90 cycles each, whatever their size.
-// (A value that the compiler cannot see to be the same in all lanes -- the warp's number, what shared memory holds -- passes
-// through warp_uniform first: branches and loops on it count as divergent otherwise.)
+// The loops that issue copies and products run on whole warps and one elected lane issues.  Measured: in a loop under a branch
+// on the lane the products were paced at about 90 cycles each, whatever their size; with an elected lane, and with what steers
+// the loop passed through warp_uniform, at what their size takes.  The likely reason is that their operands can then be kept
+// in registers that a warp shares, which needs values that the compiler can see to be the same in all lanes: the warp's number
+// and what shared memory holds are not, unless they come out of a shuffle.
 __device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t e;

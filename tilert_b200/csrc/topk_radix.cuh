@@ -34,7 +34,7 @@ __device__ __forceinline__ void topk_radix_row(const float* row, int n, int k, i
   __shared__ int s_base_sel, s_base_eq;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-  // every element in any order, four at a time where the row's address allows it and sixteen loads of a thread together
+  // every element in any order, four at a time where the row's address allows it: four loads, sixteen elements, of a thread together
   auto each = [&](auto visit) {
     int done = 0;
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
