@@ -76,3 +76,27 @@ def test_few_rows_a_group(ops, gated, n, k, counts):
     (700, 3000, 2000, False, F32), (37, 5632, 1024, True, BF16), (257, 20001, 72, False, F32)])
 def test_one_weight(ops, rows, n, k, gated, out_type):
     check(ops, n, k, gated, out_type, None, rows)
+
+
+@pytest.mark.parametrize("out_type", [BF16, F32])
+@pytest.mark.parametrize("gated", [False, True])
+def test_forms_have_the_same_bits(ops, gated, out_type):
+    """A row's result does not depend on the tile it is in (64 or 128 features on one SM, 256 on a pair with 64 to 256 rows, one or
+    two blocks of K a stage): a choice of experts behind a product may hang on a last bit.  The sizes make the rule choose each on
+    148 SMs; without groups gated products are always a pair's."""
+    n, k = (1500, 520) if gated else (2048, 1032)
+    sizes = [1, 400, 600, 800, 1000, 1200, 1400, 1440] if gated else [1, 37, 300, 600, 900, 1200, 1500, 1800, 2048]
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x, w = padded(ops, gen, sizes[-1], k, 1.0), padded(ops, gen, (1 + gated) * n, k, 1.5 * k ** -0.5)
+
+    def product(rows, groups=0, counts=None):
+        out = torch.zeros(rows, ops.pad(n), dtype=out_type, device="cuda")
+        ops.gemm(x, w if not groups else w.repeat(groups, 1), out, rows, n, k, gated=(1.5, 1.702) if gated else None, n_groups=groups,
+                 counts=None if counts is None else torch.tensor(counts, dtype=I32, device="cuda"))
+        return out
+
+    whole = product(sizes[-1])
+    for rows in sizes[:-1]:
+        assert torch.equal(product(rows), whole[:rows]), rows
+    for counts in ([37, 0, 60], [40] * 13, [64] * 4, [100, 200, 130], [300, 256, 1]):  # 64 features, 128, pairs of 96, 192, 224 rows
+        assert torch.equal(product(sum(counts), len(counts), counts), whole[: sum(counts)]), counts
