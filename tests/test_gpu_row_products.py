@@ -1,7 +1,7 @@
-"""Products with bf16 weight rows in the forms that the number of rows chooses: clusters that split K (few rows, one weight or
-groups of equal size), the exact mode's two tile shapes, long weights of the FP8 models' head and input product.  References
-are f64 on the same operands.  f32 sums of up to 18432 products in any order: relative rms error below 1e-5 (the sums of the
-exact mode, with f32 inputs, below 2e-6); bf16 results a rounding more, 2^-8."""
+"""Products with bf16 weight rows in the forms that the number of rows chooses: tiles of 64 and of 128 features on single SMs, a
+pair of SMs on a tile, groups of equal size; the exact mode's two tile shapes; long weights of the FP8 models' head and input
+product, a row or four rows a warp.  References are f64 on the same operands.  f32 sums of up to 18432 products in any order:
+relative rms error below 1e-5 (the sums of the exact mode, with f32 inputs, below 2e-6); bf16 results a rounding more, 2^-8."""
 
 import pytest
 import torch
