@@ -1,6 +1,7 @@
 """The row kernels that work in pieces of eight elements against the same operators an element at a time: one operand
-moved off its 16-byte boundary takes the general form.  Both compute in f32; they differ in the order of sums over at most
-8192 values (relative error below 1e-6 of a statistic), so f32 results agree to 2e-6 and bf16 ones to a rounding."""
+moved off its 16-byte boundary takes the general form.  Both compute in f32 and, but for layer norms, in the same order: equal
+bits.  A layer norm's sums over at most 8192 values are taken in another order (relative error below 1e-6 of a statistic): f32
+results agree to 4e-6 of their value and of their row's rms, bf16 ones to a unit in the last place more."""
 
 import types
 
@@ -37,16 +38,16 @@ def moved(t):
 
 
 def same(name, a, b):
+    lim = 2.0 ** -7 if a.dtype == BF16 else 4e-6
     a, b = a.double(), b.double()
-    # bf16: half a unit in the last place apart at most where f32 values differ by an ulp, 2^-8 of the value
-    lim = 2e-6 if name.endswith("f32") else 2.0 ** -8
-    assert float((a - b).abs().max()) <= lim * float(b.abs().max()), name
+    off = (a - b).abs() - lim * b.abs() - 4e-6 * b.square().mean(-1, keepdim=True).sqrt()
+    assert float(off.max()) <= 0, name
 
 
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("dim", [8, 256, 2048, 2056, 4096, 4104, 8192])
 def test_residual_and_embedding(ops, dtype, dim):
-    rows, top, t = 5, 3, "f32" if dtype == F32 else "bf16"
+    rows, top = 5, 3
     y, add, x0 = rnd(0, rows, dim, mean=3.0), rnd(1, dim), rnd(2, rows, dim)
     n1, n2 = (ops.Norm(rnd(s, dim), rnd(s + 1, dim), centered=True) for s in (3, 5))
     gain = rnd(7, dim)
@@ -63,8 +64,11 @@ def test_residual_and_embedding(ops, dtype, dim):
                 x = moved(x)
             ops.residual_norm(x, None if i == 1 and dtype == F32 else xh, eps=1e-5, dim=dim, rows=rows, **f)
             out.append((x.clone(), xh))
-        same(f"x of form {i}, f32", out[0][0], out[1][0])
-        same(f"xh of form {i}, {t}", out[0][1], out[1][1])
+        if "norm2" in f or i == 1:  # layer norms
+            same(f"x of form {i}", out[0][0], out[1][0])
+            same(f"xh of form {i}", out[0][1], out[1][1])
+        else:
+            assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), i
     table, toks = rnd(11, 9, dim, dtype=BF16), torch.tensor([8, 0, 3], device="cuda")
     for g in (gain, None):
         out = []
@@ -74,13 +78,13 @@ def test_residual_and_embedding(ops, dtype, dim):
             out.append(xh)
             if not general:
                 assert torch.equal(x.to(dtype), xh)
-        same(f"embedding, {t}", *out)
+        assert torch.equal(*out)
 
 
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(3, 1, 8, 24), (8, 2, 96, 64), (16, 16, 128, 128), (64, 8, 128, 256)])
 def test_queries_keys_values(ops, dtype, heads, kv_heads, dim, vdim):
-    rows, ring, pos, t = 7, 16, 12, "f32" if dtype == F32 else "bf16"
+    rows, ring, pos = 7, 16, 12
     mix = types.SimpleNamespace(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim)
     qkv, qg, kg = rnd(0, rows, heads * dim + kv_heads * (dim + vdim)), rnd(1, heads * dim), rnd(2, kv_heads * dim)
     lam, first, cur = torch.tensor([0.3], device="cuda"), rnd(3, rows, kv_heads * vdim), torch.tensor([pos], dtype=I32, device="cuda")
@@ -94,7 +98,7 @@ def test_queries_keys_values(ops, dtype, heads, kv_heads, dim, vdim):
             ops.qkv_rows(qkv, moved(qg) if general else qg, kg, 1e-5, mode, lam, vf, rows, mix, cache, cur, q)
             out.append((q, cache.k, cache.v, vf.to(dtype)))
         for name, a, b in zip(("q", "k", "v", "first"), *out):
-            same(f"{name}, mode {mode}, {t}", a, b)
+            assert torch.equal(a, b), f"{name}, mode {mode}"
 
 
 @pytest.mark.parametrize("dtype", TYPES)
