@@ -166,11 +166,18 @@ def test_few_long_rows(tokens):
     w, o = torch.zeros(dim, 2 * dim, dtype=BF16, device="cuda"), torch.zeros(1, tokens, dim, dtype=BF16, device="cuda")
 
     def us(rows):
-        begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-        for i in range(50):
-            if i == 10:
-                begin.record()
+        def call():
             dsa.mtp_preprocess_rows(e, h, ge, gh, w, o, 0, rows)
+
+        call()
+        torch.cuda.synchronize()
+        graph, (begin, end) = torch.cuda.CUDAGraph(), (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        with torch.cuda.graph(graph):  # (launched one by one they may wait for the host)
+            for _ in range(40):
+                call()
+        graph.replay()
+        begin.record()
+        graph.replay()
         end.record()
         torch.cuda.synchronize()
         return begin.elapsed_time(end)
