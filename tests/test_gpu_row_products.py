@@ -155,6 +155,21 @@ def test_order_of_long_sums(tokens, n, k, dtype):
     assert torch.equal(o[0], in_order(x[0], w, 8 if dtype == BF16 else 4))
 
 
+@pytest.mark.parametrize("dim,rows", [(128, 128), (1024, 5), (4096, 2400)])
+def test_gains_off_their_boundary(dim, rows):
+    """Gains at any address: the general form of the loads gives the same bits."""
+    from tilert_b200.models.deepseek_v3_2 import ops as dsa
+
+    e, h, w = rnd(0, 1, 3, dim, dtype=BF16), rnd(1, 1, 3, dim, dtype=BF16), rnd(2, dim, 2 * dim, dtype=BF16)
+    g, outs = (rnd(3, dim + 4), rnd(4, dim + 4)), []
+    for at_e, at_h in ((0, 0), (1, 0), (0, 3), (2, 1)):
+        ge, gh = (torch.empty(dim + 4, device="cuda")[at: at + dim].copy_(v[:dim]) for v, at in zip(g, (at_e, at_h)))
+        o = torch.zeros(1, 3, dim, dtype=BF16, device="cuda")
+        dsa.mtp_preprocess_rows(e, h, ge, gh, w, o, 0, rows)
+        outs.append(o)
+    assert all(torch.equal(outs[0], o) for o in outs[1:]) and bool(outs[0].any())
+
+
 @pytest.mark.parametrize("tokens", [1, 4])
 def test_few_long_rows(tokens):
     """A rank's row share of an input product, fewer rows than the GPU has warps: no walk of a warp over four rows, which takes as

@@ -1047,7 +1047,8 @@ template <typename X, typename W>
 int launch_gemv_long(TbContext* ctx, const GemvBf16Params& p, cudaStream_t st) {
   // A row per warp while all SMs have a warp for each, else four.  One / two / four tokens, us: 512 rows of 14336 30 / 32 / 36
   // (four rows per warp: 40 / 42 / 46), 2368 rows 32 / 34 / 40 (41 / 42 / 46), 3072 rows 58 / 59 / 64 (42 / 43 / 48); 2368 rows
-  // of 7168 15 / 17 / 21 (19 / 21 / 25), 3000 rows 24 / 26 / 30 (21 / 23 / 27).
+  // of 7168 15 / 17 / 21 (19 / 21 / 25), 3000 rows 24 / 26 / 30 (21 / 23 / 27).  (Both sides before gains came in 16-byte loads,
+  // which take about 1 off each.)
   const bool one = p.n <= ctx->num_sms * (kGemvBf16Threads / 32);
   if (p.n_tokens == 1) return one ? launch_gemv_long<1, 1, X, W>(ctx, p, st) : launch_gemv_long<1, 4, X, W>(ctx, p, st);
   if (p.n_tokens == 2) return one ? launch_gemv_long<2, 1, X, W>(ctx, p, st) : launch_gemv_long<2, 4, X, W>(ctx, p, st);
@@ -1074,7 +1075,7 @@ int launch_gemv_bf16(TbContext* ctx, GemvBf16Params& p, cudaStream_t st) {
     rc = p.n_tokens == 1 ? launch_gemv_short<1>(p, st) : (p.n_tokens == 2 ? launch_gemv_short<2>(p, st) : launch_gemv_short<4>(p, st));
   } else {
     auto a16 = [](const void* q, long long ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 8 == 0; };
-    p.aligned = a16(p.x, p.x_stride) && (p.x2 == nullptr || (a16(p.x2, p.x2_stride) && p.k1 % 8 == 0));
+    p.aligned = a16(p.x, p.x_stride) && a16(p.gamma, 0) && a16(p.gamma2, 0) && (p.x2 == nullptr || (a16(p.x2, p.x2_stride) && p.k1 % 8 == 0));
     const bool half = p.gamma == nullptr || p.round_norm_bf16;  // the staged activations are bf16 values
     TB_REQUIRE(half || !p.w_is_f32);                            // (f32 weights are the router's, which rounds its input)
     if (p.w_is_f32)
