@@ -366,6 +366,16 @@ int tilert_sample_op(TbContext* ctx, const float* logits, long long logits_strid
                      unsigned long long step_value, int* token_out, float* token_logprob_out, float* topn_logprob_out,
                      int* topn_index_out, void* stream);
 
+/* What ends a step of a driver: the next token as a 64-bit number, and the position moved on.
+ *   config_dev NULL: token_out [tokens] = index of the row's largest value, the lowest of equal ones (a value that is no
+ *   number is larger than all); the other sampling arguments are not used.  Otherwise as tilert_sample_op with `sampled`
+ *   its token output, and token_out (may be NULL) the same once more.
+ *   pos (may be NULL): *pos += advance. */
+int tilert_next_token_op(TbContext* ctx, const float* logits, long long logits_stride, int tokens, int vocab,
+                         const float* config_dev, unsigned long long seed, unsigned long long* step_dev, int* sampled,
+                         float* token_logprob_out, float* topn_logprob_out, int* topn_index_out, long long* token_out, int* pos,
+                         int advance, void* stream);
+
 /* ---- latent caches from an external prefill, FP8 wire format -------------------------------- */
 
 /* The decode side of prefill / decode disaggregation: tilert/pd_vllm/profiles/mla_nsa.py:16-41 (layout),

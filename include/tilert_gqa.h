@@ -198,6 +198,11 @@ int tilert_gqa_sample_op(TgContext* ctx, const float* logits, long long logits_s
                          const float* config_dev, unsigned long long seed, unsigned long long* step_dev,
                          unsigned long long step_value, int* token_out, float* token_logprob_out, float* topn_logprob_out,
                          int* topn_index_out, void* stream);
+/* tilert_next_token_op of tilert_b200.h (same kernels, same arguments). */
+int tilert_gqa_next_token_op(TgContext* ctx, const float* logits, long long logits_stride, int tokens, int vocab,
+                             const float* config_dev, unsigned long long seed, unsigned long long* step_dev, int* sampled,
+                             float* token_logprob_out, float* topn_logprob_out, int* topn_index_out, long long* token_out, int* pos,
+                             int advance, void* stream);
 
 #ifdef __cplusplus
 }

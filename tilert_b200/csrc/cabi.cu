@@ -1552,30 +1552,52 @@ extern "C" int tilert_flash_sparse_mla_vproj_op(TbContext* ctx, const void* q, c
 }
 
 // ------------------------------------------------------------------------------ sampling
+namespace {
+
+int next_token(TbContext* ctx, SampleParams p, int tokens, void* stream) {
+  TB_NOT_CHAINABLE(ctx);
+  TB_REQUIRE(ctx != nullptr && p.logits != nullptr && tokens >= 1 && p.vocab >= 1 && p.stride >= p.vocab);
+  TB_REQUIRE(static_cast<long long>(tokens) * kRowCtas < (1ll << 31));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (p.config == nullptr) {
+    TB_REQUIRE(p.token_out != nullptr);
+    const GreedyParams q{p.logits, p.stride, p.vocab, p.token_out, p.pos, p.advance};
+    TB_CUDA(launch(greedy_kernel, dim3(tokens * kRowCtas), dim3(kGreedyThreads), 0, st, q));
+  } else {
+    TB_REQUIRE(p.token != nullptr && (p.topn_logprob == nullptr) == (p.topn_index == nullptr));
+    static bool attr_set[64] = {};
+    if (!attr_set[ctx->device & 63]) {
+      TB_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeldBytes));
+      attr_set[ctx->device & 63] = true;
+    }
+    const size_t part = sizeof(float) * static_cast<size_t>(row_part_len(p.vocab));
+    p.held = part <= kHeldBytes;
+    TB_CUDA(launch(sample_kernel, dim3(tokens * kRowCtas), dim3(kSampleThreads), p.held ? part : 0, st, p));
+  }
+  ++g_launches;
+  TB_CUDA(cudaGetLastError());
+  return TB_OK;
+}
+
+}  // namespace
+
 extern "C" int tilert_sample_op(TbContext* ctx, const float* logits, long long logits_stride, int tokens, int vocab,
                                 const float* config_dev, unsigned long long seed, unsigned long long* step_dev,
                                 unsigned long long step_value, int* token_out, float* token_logprob_out,
                                 float* topn_logprob_out, int* topn_index_out, void* stream) {
-  TB_NOT_CHAINABLE(ctx);
-  TB_REQUIRE(ctx != nullptr && logits != nullptr && config_dev != nullptr && token_out != nullptr);
-  TB_REQUIRE(tokens >= 1 && vocab >= 1 && logits_stride >= vocab);
-  TB_REQUIRE((topn_logprob_out == nullptr) == (topn_index_out == nullptr));
-  SampleParams p{};
-  p.logits = logits;
-  p.stride = logits_stride;
-  p.vocab = vocab;
-  p.config = config_dev;
-  p.seed = seed;
-  p.step = step_dev;
-  p.step_value = step_value;
-  p.token = token_out;
-  p.token_logprob = token_logprob_out;
-  p.topn_logprob = topn_logprob_out;
-  p.topn_index = topn_index_out;
-  TB_CUDA(launch(sample_kernel, dim3(tokens), dim3(kTopkThreads), 0, static_cast<cudaStream_t>(stream), p));
-  ++g_launches;
-  TB_CUDA(cudaGetLastError());
-  return TB_OK;
+  TB_REQUIRE(config_dev != nullptr);
+  return next_token(ctx, SampleParams{logits, logits_stride, vocab, config_dev, seed, step_dev, step_value, false, token_out,
+                                      token_logprob_out, topn_logprob_out, topn_index_out, nullptr, nullptr, 0},
+                    tokens, stream);
+}
+
+extern "C" int tilert_next_token_op(TbContext* ctx, const float* logits, long long logits_stride, int tokens, int vocab,
+                                    const float* config_dev, unsigned long long seed, unsigned long long* step_dev, int* sampled,
+                                    float* token_logprob_out, float* topn_logprob_out, int* topn_index_out, long long* token_out,
+                                    int* pos, int advance, void* stream) {
+  return next_token(ctx, SampleParams{logits, logits_stride, vocab, config_dev, seed, step_dev, 0, false, sampled, token_logprob_out,
+                                      topn_logprob_out, topn_index_out, token_out, pos, advance},
+                    tokens, stream);
 }
 
 // ------------------------------------------------------------------ cache injection (FP8 wire format)

@@ -17,6 +17,7 @@
 #include <cuda.h>
 
 #include "act.cuh"
+#include "cluster.cuh"
 #include "tcgen05.cuh"
 
 namespace tb {
@@ -416,20 +417,6 @@ struct PairTiles {
   int stages, stage_bytes;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
-// shared::cluster address of a CTA's copy of a variable
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -507,7 +494,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
   volatile int* abort = &s_abort;
   auto give_up = [&] {  // a wait that ran out ends both CTAs' roles
     *abort = 1;
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(&s_abort, rank ^ 1u)), "r"(1) : "memory");
+    cluster_store(cluster_addr(&s_abort, rank ^ 1u), 1u);
   };
   TileWalk walk{s_rows, s_tiles, groups, ft, q.bn, 2 * kFeats};
   const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;

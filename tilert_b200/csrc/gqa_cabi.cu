@@ -870,14 +870,40 @@ extern "C" int tilert_gqa_vec_value_op(TgContext* ctx, const float* part, int he
 }
 
 // ------------------------------------------------------------------------------- sampling
+namespace {
+
+int next_token(TgContext* ctx, SampleParams p, int tokens, void* stream) {
+  TB_REQUIRE(ctx != nullptr && p.logits != nullptr && tokens >= 1 && p.vocab >= 1 && p.stride >= p.vocab);
+  TB_REQUIRE(static_cast<long long>(tokens) * kRowCtas < (1ll << 31));
+  if (p.config == nullptr) {
+    TB_REQUIRE(p.token_out != nullptr);
+    return go(greedy_kernel, dim3(tokens * kRowCtas), dim3(kGreedyThreads), 0, stream,
+              GreedyParams{p.logits, p.stride, p.vocab, p.token_out, p.pos, p.advance});
+  }
+  TB_REQUIRE(p.token != nullptr && (p.topn_logprob == nullptr) == (p.topn_index == nullptr));
+  const size_t part = sizeof(float) * static_cast<size_t>(row_part_len(p.vocab));
+  p.held = part <= kHeldBytes;
+  TB_CUDA(allow_smem(reinterpret_cast<const void*>(sample_kernel)));  // (its static part is most of what needs no permission)
+  return go(sample_kernel, dim3(tokens * kRowCtas), dim3(kSampleThreads), p.held ? part : 0, stream, p);
+}
+
+}  // namespace
+
 extern "C" int tilert_gqa_sample_op(TgContext* ctx, const float* logits, long long logits_stride, int tokens, int vocab,
                                     const float* config_dev, unsigned long long seed, unsigned long long* step_dev,
                                     unsigned long long step_value, int* token_out, float* token_logprob_out, float* topn_logprob_out,
                                     int* topn_index_out, void* stream) {
-  TB_REQUIRE(ctx != nullptr && logits != nullptr && config_dev != nullptr && token_out != nullptr);
-  TB_REQUIRE(tokens >= 1 && vocab >= 1 && logits_stride >= vocab);
-  TB_REQUIRE((topn_logprob_out == nullptr) == (topn_index_out == nullptr));
-  const SampleParams p{logits, logits_stride, vocab, config_dev, seed, step_dev, step_value, token_out, token_logprob_out,
-                       topn_logprob_out, topn_index_out};
-  return go(sample_kernel, dim3(tokens), dim3(kTopkThreads), 0, stream, p);
+  TB_REQUIRE(config_dev != nullptr);
+  return next_token(ctx, SampleParams{logits, logits_stride, vocab, config_dev, seed, step_dev, step_value, false, token_out,
+                                      token_logprob_out, topn_logprob_out, topn_index_out, nullptr, nullptr, 0},
+                    tokens, stream);
+}
+
+extern "C" int tilert_gqa_next_token_op(TgContext* ctx, const float* logits, long long logits_stride, int tokens, int vocab,
+                                        const float* config_dev, unsigned long long seed, unsigned long long* step_dev, int* sampled,
+                                        float* token_logprob_out, float* topn_logprob_out, int* topn_index_out, long long* token_out,
+                                        int* pos, int advance, void* stream) {
+  return next_token(ctx, SampleParams{logits, logits_stride, vocab, config_dev, seed, step_dev, 0, false, sampled, token_logprob_out,
+                                      topn_logprob_out, topn_index_out, token_out, pos, advance},
+                    tokens, stream);
 }

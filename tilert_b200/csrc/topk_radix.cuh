@@ -1,5 +1,5 @@
 // Radix selection of the k largest values of one row by one CTA, on the order-preserving unsigned image of
-// f32: exact, equal values by lower index first.  Shared by the indexer's selection and the token sampler.
+// f32: exact, equal values by lower index first.  The token sampler uses the same image of a value.
 #pragma once
 
 #include "common.cuh"
@@ -18,8 +18,8 @@ constexpr int kTopkThreads = 1024;
 constexpr int kTopkItems = 8;  // consecutive elements per thread in the ordered compaction
 
 // Four counting passes over the row and one that collects; bound by the instructions of the passes on one SM.  With a pass of
-// its own for the number of eligible entries and an element at a time the sampler took 53.2 us for 32768 values and 166 for
-// 129280; counted with the first digit and in fours 46.4 and 138.
+// its own for the number of eligible entries and an element at a time a selection of 1024 and what a sampler does behind it took
+// 53.2 us for 32768 values and 166 for 129280; counted with the first digit and in fours 46.4 and 138.
 //
 // One CTA per row.  Selects the k largest logits among [0, n) (entries equal to -inf are skipped),
 // ties by lower index, and writes their indices in ascending order; unused slots get -1.

@@ -300,3 +300,14 @@ def sample(logits, config, token_out, *, seed=0, step=None, step_value=0, token_
     rows = logits.numel() // logits.shape[-1]
     _call("sample", logits, _p(logits), logits.shape[-1], rows, logits.shape[-1], _p(config), seed & ((1 << 63) - 1), _p(step), step_value,
           _p(token_out), _p(token_logprob), _p(topn_logprobs), _p(topn_indices))
+
+
+def next_token(logits, token_out, *, pos=None, advance: int = 0, config=None, seed: int = 0, step=None, sampled=None, token_logprob=None,
+               topn_logprobs=None, topn_indices=None) -> None:
+    """What ends a step: ``token_out`` int64 = the arg-max of ``logits`` [rows, vocab], or with ``config`` a sampled token as
+    ``sample`` leaves it; ``pos`` += ``advance``."""
+    _need("logits", logits, F32)
+    _need("token_out", token_out, I64)
+    rows = logits.numel() // logits.shape[-1]
+    _call("next_token", logits, _p(logits), logits.shape[-1], rows, logits.shape[-1], _p(config), seed & ((1 << 63) - 1), _p(step), _p(sampled),
+          _p(token_logprob), _p(topn_logprobs), _p(topn_indices), _p(token_out), _p(pos), advance)

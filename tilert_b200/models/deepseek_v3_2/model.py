@@ -122,20 +122,21 @@ class DsaModel(SequenceDriver):
             # every rank holds vocab / world rows of the head: exchange (value, index) pairs over peer memory
             ops.argmax_exchange(self.logits, self.rank * self.logits.shape[-1], self.token_out, comm=self.comm)
         else:
-            self._choose(self.logits.view(1, -1))
+            self._choose(self.logits.view(1, -1), 1)
         if self.temp_vars is not None:
             from .temp_var_indices import Idx
 
             self.temp_vars[Idx.TOKEN_OUT].view(-1)[:1].copy_(self.token_out)
             self.temp_vars[Idx.TOKEN_ID].view(-1)[:1].copy_(self.token)
-        self.cur_pos += 1
+        if self.world > 1:
+            self.cur_pos += 1
 
     def _graph_key(self, pos: int) -> int:
         """Indexer scan length: next multiple of 256 above the position, so graphs are reused."""
         return min(self.cache_len, (pos // 256 + 1) * 256)
 
-    def _sample_op(self):
-        return ops.sample
+    def _next_token_op(self):
+        return ops.next_token
 
     def _may_capture(self) -> bool:
         return self.use_graph and not (self.sampling and self.world > 1)  # the gather is a library collective: not captured

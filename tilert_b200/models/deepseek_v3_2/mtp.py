@@ -125,7 +125,7 @@ class MtpDsaModel:
         if self.world > 1:
             ops.argmax_exchange(logits, self.rank * logits.shape[-1], out, comm=self.comm)
         else:
-            out.copy_(torch.argmax(logits.view(out.numel(), -1), dim=-1))
+            ops.next_token(logits.view(out.numel(), -1), out)
 
     # -- the passes --
     def _main_pass(self, tokens: torch.Tensor, n_keys: int) -> torch.Tensor:

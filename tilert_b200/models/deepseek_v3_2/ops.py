@@ -611,3 +611,15 @@ def sample(logits, config, token_out, *, seed=0, step=None, step_value=0, token_
                                          step_value, _p(token_out), _p(token_logprob), _p(topn_logprobs),
                                          _p(topn_indices), _stream()))
 
+
+def next_token(logits, token_out, *, pos=None, advance=0, config=None, seed=0, step=None, sampled=None, token_logprob=None,
+               topn_logprobs=None, topn_indices=None):
+    """What ends a step: ``token_out`` int64 = the arg-max of ``logits`` [rows, vocab], or with ``config`` a sampled token as
+    ``sample`` leaves it; ``pos`` += ``advance``."""
+    _need(logits, F32, "logits")
+    _need(token_out, torch.int64, "token_out")
+    rows = logits.numel() // logits.shape[-1]
+    seed &= (1 << 63) - 1
+    _tb.check(_tb.lib().tilert_next_token_op(_ctx(logits), _p(logits), logits.shape[-1], rows, logits.shape[-1], _p(config), seed, _p(step),
+                                             _p(sampled), _p(token_logprob), _p(topn_logprobs), _p(topn_indices), _p(token_out), _p(pos),
+                                             advance, _stream()))

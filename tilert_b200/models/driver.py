@@ -52,8 +52,9 @@ class SequenceDriver:
         """Steps at positions with the same key have the same launches."""
         raise NotImplementedError
 
-    def _sample_op(self):
-        raise NotImplementedError
+    def _next_token_op(self):
+        """The operator that ends a step on the device; None: torch's arg-max."""
+        return None
 
     # -- reference driver controls (end2end.py:551-577) --
     def reset_sequence(self) -> None:
@@ -86,14 +87,16 @@ class SequenceDriver:
             self.sampling_seed = seed
             self._graphs.clear()
 
-    def _choose(self, logits: torch.Tensor) -> None:
-        """The next token of ``logits`` [1, vocab] into ``token_out``."""
-        if self.sampling:
-            self._sample_op()(logits, self.sampling_config, self.sampled, seed=self.sampling_seed, step=self.sample_step,
-                              token_logprob=self.token_logprob, topn_logprobs=self.topn_logprobs, topn_indices=self.topn_indices)
-            self.token_out.copy_(self.sampled)
-        else:
+    def _choose(self, logits: torch.Tensor, advance: int = 0) -> None:
+        """The next token of ``logits`` [1, vocab] into ``token_out``, and the device position moved on."""
+        op = self._next_token_op()
+        if op is None:
             self.token_out.copy_(torch.argmax(logits.view(-1)))
+            self.cur_pos += advance
+            return
+        sampling = dict(config=self.sampling_config, seed=self.sampling_seed, step=self.sample_step, sampled=self.sampled,
+                        token_logprob=self.token_logprob, topn_logprobs=self.topn_logprobs, topn_indices=self.topn_indices)
+        op(logits, self.token_out, pos=self.cur_pos, advance=advance, **(sampling if self.sampling else {}))
 
     # -- the step --
     def _may_capture(self) -> bool:
@@ -174,7 +177,7 @@ class PortionDriver(SequenceDriver):
 
     def _prefill_portion(self, tokens: list[int], want: list[int], last: bool) -> torch.Tensor:
         """One portion; f32 logits [len(want), vocab] of the wanted places; with ``last`` also those of the last token
-        in ``self.logits``.  Advances the position."""
+        in ``self.logits``.  The position stays."""
         raise NotImplementedError
 
     def _upload(self, values: list[int], dtype: torch.dtype) -> torch.Tensor:
@@ -197,6 +200,11 @@ class PortionDriver(SequenceDriver):
         for lo in range(0, len(tokens), self.portion):
             part = tokens[lo: lo + self.portion]
             here = [w - lo for w in (want if want is not None else []) if lo <= w < lo + len(part)]
-            outs.append(self._prefill_portion(part, here, lo + len(part) == len(tokens)))
-        self._choose(self.logits.view(1, -1))
+            last = lo + len(part) == len(tokens)
+            outs.append(self._prefill_portion(part, here, last))
+            self._pos += len(part)
+            if last:
+                self._choose(self.logits.view(1, -1), len(part))
+            else:
+                self.cur_pos += len(part)
         return self.logits.view(1, -1).clone() if want is None else torch.cat(outs)

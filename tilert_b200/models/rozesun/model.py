@@ -78,11 +78,10 @@ class RozesunModel(PortionDriver):
             st.add = add
             layer.decode(st, nr, self.cur_pos, length)
         st.dense(self.embed, self.logits, a.vocab_size, a.dim, a.eps, gain2=self.final_norm)
-        self._choose(self.logits.view(1, -1))
-        self.cur_pos += 1
+        self._choose(self.logits.view(1, -1), 1)
 
-    def _sample_op(self):
-        return ops.sample
+    def _next_token_op(self):
+        return ops.next_token
 
     # -- prompts --
     def _prefill_portion(self, tokens: list[int], want: list[int], last: bool) -> torch.Tensor:
@@ -104,6 +103,4 @@ class RozesunModel(PortionDriver):
             ops.gemm(xn, self.embed, out, len(want), a.vocab_size, a.dim)
         if last:
             ops.vec_dense(x[n - 1], self.embed, self.logits, a.vocab_size, a.dim, gain2=self.final_norm, eps=a.eps)
-        self.cur_pos += n
-        self._pos += n
         return out
