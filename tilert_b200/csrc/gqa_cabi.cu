@@ -378,9 +378,9 @@ int head_blocks(int heads, int kv_heads) {
   return kv_heads * ((group + kAttnHeads - 1) / kAttnHeads);
 }
 
-template <int DV16>
+template <int D16, int DV16>
 int launch_prefill_attn(const AttnPrefillParams& p, dim3 grid, void* stream) {
-  return go(attn_prefill_kernel<DV16>, grid, dim3(kFaThreads), attn_prefill_smem(p.s.dimp, p.s.vdimp), stream, p);
+  return go(attn_prefill_kernel<D16, DV16>, grid, dim3(kFaThreads), attn_prefill_smem(p.s.dimp, p.s.vdimp), stream, p);
 }
 
 bool prefill_attn_fits(int dimp, int vdimp) { return vdimp <= 256 && attn_prefill_smem(dimp, vdimp) <= kMaxSmem; }
@@ -388,9 +388,12 @@ bool prefill_attn_fits(int dimp, int vdimp) { return vdimp <= 256 && attn_prefil
 int run_prefill_attn(const AttnPrefillParams& p, void* stream) {
   const int group = p.s.heads / p.s.kv_heads, hpb = group < kFaMaxHeads ? group : kFaMaxHeads, tpb = kFaRows / hpb;
   const dim3 grid((p.rows + tpb - 1) / tpb, p.s.kv_heads * ((group + hpb - 1) / hpb));
-  if (p.s.vdimp <= 64) return launch_prefill_attn<4>(p, grid, stream);
-  if (p.s.vdimp <= 128) return launch_prefill_attn<8>(p, grid, stream);
-  return launch_prefill_attn<16>(p, grid, stream);
+  if (p.s.dimp == 128 && p.s.vdimp == 128) return launch_prefill_attn<8, 8>(p, grid, stream);
+  if (p.s.dimp == 192 && p.s.vdimp == 128) return launch_prefill_attn<12, 8>(p, grid, stream);
+  if (p.s.dimp == 64 && p.s.vdimp == 64) return launch_prefill_attn<4, 4>(p, grid, stream);
+  if (p.s.vdimp <= 64) return launch_prefill_attn<0, 4>(p, grid, stream);
+  if (p.s.vdimp <= 128) return launch_prefill_attn<0, 8>(p, grid, stream);
+  return launch_prefill_attn<0, 16>(p, grid, stream);
 }
 
 }  // namespace

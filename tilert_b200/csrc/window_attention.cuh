@@ -435,6 +435,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnRowsP
 // 64 rows per CTA = (tokens x query heads of one key/value head), so the heads of a group share the key tiles.
 // 64 keys per tile; the next keys are requested (cp.async) before a tile's scores, the next values after its product;
 // four warps of 16 rows, three CTAs per SM at 128-wide heads; online softmax in registers.
+// Bound by instructions (half of the issue slots, 1780 of them for 16 rows x 64 keys of 128, went into the addresses of the
+// copies when each was divided out) and by shared memory's reads for the products: mma.sync reaches 550 TFLOP/s here from
+// registers, 460 with a matrix load per two products.  B200, back to back, before -> now: 32 heads of 128 over 8, 2048 tokens
+// that see 2048 keys 449 -> 270 us (254 TFLOP/s); 173 tokens from the start, 16 heads 14.3 -> 9.7; 64 tokens behind 4000, 24 heads
+// 207 -> 111; heads of 80 / 72 (general addresses) 37.6 -> 30.1.  The sums keep their order, so the bits do not change.
 constexpr int kFaRows = 64, kFaKeys = 64, kFaThreads = 128;
 constexpr int kFaMaxHeads = 16;  // query heads of a group per CTA
 
@@ -468,8 +473,48 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// DV16: value tiles of 16 columns the accumulator has room for (vdimp <= 16 * DV16)
-template <int DV16>
+// What a thread loads of a tile's rows: one piece of eight columns of every `step`-th row, so that inside the loop over the
+// tiles an address is an addition.  Pieces `ch1` and up come from the second source.
+struct FaRows {
+  const __nv_bfloat16* src;  // this thread's columns
+  long long ld;
+  int col, row, step;        // of the tile in shared memory; row 64: no share
+
+  __device__ FaRows(int tid, int ch, int ch1, const __nv_bfloat16* src1, long long ld1, const __nv_bfloat16* src2, long long ld2) {
+    int per_row = 1;  // threads on a row: a power of two, at least one a piece
+    while (per_row < ch && per_row < kFaThreads) per_row *= 2;
+    const int c = tid & (per_row - 1);
+    src = c < ch1 ? src1 + c * 8 : src2 + (c - ch1) * 8;
+    ld = c < ch1 ? ld1 : ld2;
+    col = c * 8;
+    step = kFaThreads / per_row;
+    row = c < ch ? tid / per_row : kFaKeys;
+  }
+  // the tile of keys k0 .., key k0 in ring row slot0; keys from hi on are zeros
+  __device__ __forceinline__ void load(__nv_bfloat16* dst, int pitch, int k0, int hi, int slot0, int ring) const {
+    __nv_bfloat16* d = dst + row * pitch + col;
+    if (k0 + kFaKeys <= hi && slot0 + kFaKeys <= ring) {
+      const __nv_bfloat16* g = src + (slot0 + row) * ld;
+      for (int r = row; r < kFaKeys; r += step) {
+        cp_async16(d, g, true);
+        d += step * pitch;
+        g += step * ld;
+      }
+    } else {
+      for (int r = row; r < kFaKeys; r += step) {
+        const bool ok = k0 + r < hi;
+        const long long slot = ok ? slot0 + r - (slot0 + r >= ring ? ring : 0) : 0;
+        cp_async16(d, src + slot * ld, ok);
+        d += step * pitch;
+      }
+    }
+    cp_async_commit();
+  }
+};
+
+// DV16: value tiles of 16 columns the accumulator has room for (vdimp <= 16 * DV16).  D16: dimp = 16 * D16 and vdimp =
+// 16 * DV16, so that the addresses inside a tile are constants; 0: any sizes.
+template <int D16, int DV16>
 __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_kernel(const AttnPrefillParams a) {
   extern __shared__ __align__(16) __nv_bfloat16 fsm[];
   pdl_launch_dependents();
@@ -484,7 +529,8 @@ __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_ke
   const int t0 = (gridDim.x - 1 - blockIdx.x) * tpb;  // the longest ranges first
   const int nt = min(tpb, a.rows - t0);
   const int pos0 = *a.pos;
-  const int qp = s.dimp + 8, vpitch = s.vdimp + 8;
+  const int dimp = D16 > 0 ? D16 * 16 : s.dimp, vdimp = D16 > 0 ? DV16 * 16 : s.vdimp;
+  const int qp = dimp + 8, vpitch = vdimp + 8;
   __nv_bfloat16* qs = fsm;
   __nv_bfloat16* ks = qs + kFaRows * qp;
   __nv_bfloat16* vs = ks + 2 * kFaKeys * qp;
@@ -492,32 +538,20 @@ __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_ke
   const __nv_bfloat16* vc = a.v_cache + g * a.v_head;
   const int lo = s.window > 0 ? max(0, pos0 + t0 - s.window + 1) : 0, hi = pos0 + t0 + nt;  // keys any row sees
 
-  const int dch = s.dimp / 8;
+  const int dch = dimp / 8;
   for (int i = tid; i < kFaRows * dch; i += kFaThreads) {
     const int r = i / dch, c = i - r * dch;
     const int tt = r / hpb, h = r - tt * hpb;
     const bool ok = tt < nt && h < nh;
     const long long row = ok ? static_cast<long long>(t0 + tt) * s.heads + h0 + h : 0;
-    cp_async16(qs + r * qp + c * 8, a.q + row * s.dimp + c * 8, ok);
+    cp_async16(qs + r * qp + c * 8, a.q + row * dimp + c * 8, ok);
   }
-  // rows k0 .. of the keys or values: ch1 pieces of eight from src1, the others from src2
-  auto load_rows = [&](__nv_bfloat16* dst, int pitch, const __nv_bfloat16* src1, long long ld1, int ch1, const __nv_bfloat16* src2,
-                       long long ld2, int ch, int k0) {
-    const int slot0 = k0 % s.ring;
-    for (int i = tid; i < kFaKeys * ch; i += kFaThreads) {
-      const int r = i / ch, c = i - r * ch;
-      const bool ok = k0 + r < hi;
-      const long long slot = ok ? slot0 + r - (slot0 + r >= s.ring ? s.ring : 0) : 0;
-      cp_async16(dst + r * pitch + c * 8, c < ch1 ? src1 + slot * ld1 + c * 8 : src2 + slot * ld2 + (c - ch1) * 8, ok);
-    }
-    cp_async_commit();
-  };
-  auto load_keys = [&](int buf, int k0) {
-    load_rows(ks + buf * kFaKeys * qp, qp, kc, a.k_ld, a.dim1 / 8, a.k2, a.k2_ld, s.dimp / 8, k0);
-  };
-  auto load_values = [&](int k0) { load_rows(vs, vpitch, vc, a.v_ld, s.vdimp / 8, vc, a.v_ld, s.vdimp / 8, k0); };
-  load_keys(0, lo);
-  load_values(lo);
+  const FaRows key_rows(tid, dch, a.dim1 / 8, kc, a.k_ld, a.k2, a.k2_ld), value_rows(tid, vdimp / 8, vdimp / 8, vc, a.v_ld, vc, a.v_ld);
+  auto load_keys = [&](int buf, int k0, int slot0) { key_rows.load(ks + buf * kFaKeys * qp, qp, k0, hi, slot0, s.ring); };
+  auto load_values = [&](int k0, int slot0) { value_rows.load(vs, vpitch, k0, hi, slot0, s.ring); };
+  int slot = lo % s.ring;  // of the first key of the newest key tile
+  load_keys(0, lo, slot);
+  load_values(lo, slot);
 
   float o[DV16 * 2][4];
 #pragma unroll
@@ -539,14 +573,18 @@ __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_ke
     const bool more = tile + 1 < n_tiles;
     cp_async_wait<1>();  // all but the newest group: this tile's keys (its values are the newest)
     __syncthreads();
-    if (more) load_keys(buf ^ 1, k0 + kFaKeys);
+    if (more) {
+      slot = (slot + kFaKeys) % s.ring;
+      load_keys(buf ^ 1, k0 + kFaKeys, slot);
+    }
     const __nv_bfloat16* kt = ks + buf * kFaKeys * qp;
     float sacc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) sacc[i][j] = 0.f;
-    for (int kk = 0; kk < s.dimp / 16; ++kk) {
+#pragma unroll(D16 > 0 ? 4 : 1)
+    for (int kk = 0; kk < dimp / 16; ++kk) {
       uint32_t qa[4];
       ldmatrix_x4(qa, qs + (warp * 16 + (lane & 15)) * qp + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
@@ -591,6 +629,7 @@ __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_ke
       m[i] = mn;
       l[i] *= corr[i];
     }
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f))  // (times one changes nothing)
 #pragma unroll
     for (int i = 0; i < DV16 * 2; ++i) {
       o[i][0] *= corr[0];
@@ -619,7 +658,7 @@ __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_ke
     __syncthreads();
 #pragma unroll
     for (int vb = 0; vb < DV16; ++vb) {
-      if (vb * 16 < s.vdimp) {
+      if (vb * 16 < vdimp) {
 #pragma unroll
         for (int nb = 0; nb < 4; ++nb) {
           uint32_t bv[4];  // keys 0-7 / 8-15 of columns 0-7, then of columns 8-15
@@ -631,7 +670,7 @@ __global__ void __launch_bounds__(kFaThreads, DV16 <= 8 ? 3 : 1) attn_prefill_ke
       }
     }
     __syncthreads();
-    if (more) load_values(k0 + kFaKeys);
+    if (more) load_values(k0 + kFaKeys, slot);
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
