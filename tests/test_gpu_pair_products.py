@@ -100,3 +100,10 @@ def test_forms_have_the_same_bits(ops, gated, out_type):
         assert torch.equal(product(rows), whole[:rows]), rows
     for counts in ([37, 0, 60], [40] * 13, [64] * 4, [100, 200, 130], [300, 256, 1]):  # 64 features, 128, pairs of 96, 192, 224 rows
         assert torch.equal(product(sum(counts), len(counts), counts), whole[: sum(counts)]), counts
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("counts", [[260, 0, 513, 33, 256, 100], [80, 70, 129, 64, 200, 5], [288, 287, 289, 1]])
+@pytest.mark.parametrize("n,k", [(300, 200), (640, 72)])
+def test_short_last_tiles_of_groups(ops, n, k, counts, gated):
+    check(ops, n, k, gated, BF16, counts)

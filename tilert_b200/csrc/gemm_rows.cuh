@@ -44,12 +44,14 @@ struct GemmRowsParams {
 };
 
 // Enumeration of (group, feature tile, token tile); token tiles vary fastest, so that CTAs running together share a
-// weight tile.  `rows0` / `tiles0` are exclusive prefix sums over the groups in shared memory.
+// weight tile, or, with `tokens_outer`, feature tiles do.  `rows0` / `tiles0` are exclusive prefix sums over the groups in shared
+// memory.
 struct TileWalk {
   const int* rows0;
   const int* tiles0;
   int n_groups, ft, bn;
   int bf = 128;          // features of a tile
+  bool tokens_outer = false;
   int group = 0;
 
   struct Tile {
@@ -63,7 +65,14 @@ struct TileWalk {
     while (i >= tiles0[group + 1]) ++group;
     const int local = i - tiles0[group], r0 = rows0[group], r1 = rows0[group + 1];
     const int tt = (r1 - r0 + bn - 1) / bn;
-    const int f = local / tt, t = local - f * tt;
+    int f, t;
+    if (tokens_outer) {
+      t = local / ft;
+      f = local - t * ft;
+    } else {
+      f = local / tt;
+      t = local - f * tt;
+    }
     return {group, f * bf, r0 + t * bn, min(r0 + (t + 1) * bn, r1)};
   }
 };
@@ -409,7 +418,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // 2048 rows, K 4096, gated 11264 features: 250 us (1.51 PFLOP/s), on single SMs in tiles of 128 rows 332; 4096 features, K
 // 11264: 133 us (1.41), 149 in tiles of 256; 1357 rows, gated 18432 features, K 7168: 507 (639); 7168 features, K 8192: 126
 // (152).
+//
+// A group whose count is on the device multiplies its last token tile with as many rows as that has, in steps of 32, and up to half
+// a tile loads only those.  Its feature tiles come in turns of one token tile: with token tiles fastest, of which a group has
+// one or two, every other pair would get short tiles only.  256 rows each (+- 16) of 64 experts: gated, 1536 features, K 4096 427 us
+// (965 TFLOP/s), with whole tiles 463; 4096 features, K 1536 214 (234); 341 rows of 48, spread by a factor of three, gated, 2048 x 7168
+// 864 (935); 75 to 310 rows 1 to 10 % faster.  Without groups short tiles gave nothing (0.97 to 1.01): one pair of 74 has them.
 constexpr int kPairMaxStages = 8;
+constexpr int kPairBox = 16;  // token rows of a copy for a short tile
 
 struct PairTiles {
   int bn;                // token rows of a tile: a multiple of 32, at most 256
@@ -450,7 +466,8 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 
 template <bool GATED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
-    gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const GemmRowsParams p, const PairTiles q) {
+    gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap shortmap,
+                     const GemmRowsParams p, const PairTiles q) {
   constexpr int kWBytes = 128 * kTcK * 2, kFeats = GATED ? 64 : 128;  // of a CTA
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[kPairMaxStages], empty[kPairMaxStages], acc_full[2], acc_empty[2], drain;
@@ -496,9 +513,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     *abort = 1;
     cluster_store(cluster_addr(&s_abort, rank ^ 1u), 1u);
   };
-  TileWalk walk{s_rows, s_tiles, groups, ft, q.bn, 2 * kFeats};
+  TileWalk walk{s_rows, s_tiles, groups, ft, q.bn, 2 * kFeats, p.counts != nullptr};
   const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
-  const int half = q.bn / 2;  // token rows of a CTA
+  auto tokens_of = [&](const TileWalk::Tile& t) { return p.counts != nullptr ? min(q.bn, (t.row1 - t.row0 + 31) & ~31) : q.bn; };
 
   if (warp == 0) {
     uint32_t it = 0, s = 0, ph = 0;
@@ -506,6 +523,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     for (int i = first; ok && i < n_tiles; i += stride) {
       const TileWalk::Tile t = walk.at_warp(i);
       const int f0 = t.feature0 + static_cast<int>(rank) * kFeats;
+      const int bn = tokens_of(t), half = bn / 2;  // token rows of a CTA
+      const bool few = 2 * bn <= q.bn;             // so few that copies of them alone are worth their number
+      const int loaded = few ? half : q.bn / 2;
       const int x0 = t.row0 + static_cast<int>(rank) * half;
       for (int kb = 0; kb < n_kb; ++kb, ++it) {
         if (!mbar_wait_warp(&empty[s], ph ^ 1u, abort)) {
@@ -516,7 +536,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         uint8_t* st = ring + s * q.stage_bytes;
         if (elect_one()) {
           const uint32_t bar = cluster_addr(&full[s], 0);
-          if (rank == 0) mbar_expect_tx(&full[s], 2 * q.stage_bytes);
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * q.blocks * (kWBytes + loaded * kTcK * 2));
           for (int k0 = kb * q.blocks * kTcK, b = 0; b < q.blocks; ++b, k0 += kTcK, st += block_bytes) {
             if (GATED) {
 #pragma unroll
@@ -524,7 +544,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             } else {
               tma_load_2d_pair(st, &wmap, k0, t.group * p.n + f0, bar);
             }
-            tma_load_2d_pair(st + kWBytes, &xmap, k0, x0, bar);
+            if (!few)
+              tma_load_2d_pair(st + kWBytes, &xmap, k0, x0, bar);
+            else
+              for (int r = 0; r < half; r += kPairBox) tma_load_2d_pair(st + kWBytes + r * kTcK * 2, &shortmap, k0, x0 + r, bar);
           }
         }
         if (++s == stages) s = 0, ph ^= 1u;
@@ -543,10 +566,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     for (uint32_t j = from; j < it; ++j) mbar_wait(&empty[j % stages], (j / stages) & 1u, abort);
   } else if (warp == 1) {
     if (rank == 0) {
-      const uint32_t idesc = umma_idesc_bf16(256, q.bn);
       uint32_t s = 0, ph = 0, n_done = 0;
       bool ok = true, seen = false;
       for (int i = first; ok && i < n_tiles; i += stride, ++n_done) {
+        const uint32_t idesc = umma_idesc_bf16(256, tokens_of(walk.at_warp(i)));
         const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
         if (!mbar_wait_warp(&acc_empty[buf], aph ^ 1u, abort)) {
           set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
@@ -602,7 +625,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
       const bool f_ok = f < p.n;
       const float bias = p.bias != nullptr && f_ok ? p.bias[f] : 0.f;
       const uint32_t acc = tmem + buf * 256 + lane_off;
-      const int c0 = part * half;  // (columns in multiples of sixteen)
+      const int half = tokens_of(t) / 2, c0 = part * half;  // (columns in multiples of sixteen)
       for (int c = c0; c < c0 + half && t.row0 + c < t.row1; c += 16) {
         uint32_t r[16];
         tmem_ld16(acc + c, r);

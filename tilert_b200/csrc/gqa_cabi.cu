@@ -123,12 +123,13 @@ int launch_pair(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int b
   const int blocks = bn <= 160 ? 2 : 1;
   PairTiles q{bn, blocks, 0, blocks * (128 * kTcK * 2 + bn / 2 * kTcK * 2)};
   q.stages = 196608 / q.stage_bytes < kPairMaxStages ? 196608 / q.stage_bytes : kPairMaxStages;
-  CUtensorMap wmap, xmap;
+  CUtensorMap wmap, xmap, shortmap;
   int rc = GATED ? make_gated_map(&wmap, p.w, p.n_groups > 0 ? p.n_groups : 1, p.n, p.k, p.ldw) : make_map(&wmap, p.w, w_rows, p.k, p.ldw, 128);
   const long long x_rows = p.n_groups > 0 && p.counts == nullptr ? static_cast<long long>(p.n_groups) * p.rows : p.rows;
   if (rc == TB_OK) rc = make_map(&xmap, p.x, x_rows, p.k, p.ldx, bn / 2);
+  if (rc == TB_OK) rc = make_map(&shortmap, p.x, x_rows, p.k, p.ldx, kPairBox);
   if (rc != TB_OK) return rc;
-  return go(gemm_pair_kernel<GATED>, dim3(ctx->num_sms / 2 * 2), dim3(kTcThreads), static_cast<size_t>(q.stages) * q.stage_bytes + 1024, stream, wmap, xmap, p, q);
+  return go(gemm_pair_kernel<GATED>, dim3(ctx->num_sms / 2 * 2), dim3(kTcThreads), static_cast<size_t>(q.stages) * q.stage_bytes + 1024, stream, wmap, xmap, shortmap, p, q);
 }
 
 template <int BM, bool GATED>
