@@ -182,6 +182,129 @@ int tilert_gqa_expanded_attn_op(TgContext* ctx, const void* q, const void* kv, c
                                 int rot, int vdim, int rank, const int* pos, int window, int ring, float scale,
                                 const float* sink, const float* gate, long long ldg, int per_head, void* out, long long ldo,
                                 void* stream);
+/* ---- whole layers of a portion of tokens ---- */
+
+/* A layer's sizes, weights and work buffers, filled in once; the calls below launch its operators one after the other.  Rows
+ * of weights and activations have strides of pad8(length) elements, prepared queries and cache rows are padded as above.
+ * Fields are one to a line: the Python binding reads them from here. */
+
+/* x += norm1(attention(x)), x += norm2(experts(x)): grouped-query attention, routed experts beside a shared one, RMS norms. */
+typedef struct TgRoutedLayer {
+  int dim;
+  int f32;
+  float eps;
+  int portion;            /* rows that the buffers hold */
+  int heads;
+  int kv_heads;
+  int head_dim;
+  int vdim;
+  int window;
+  int ring;
+  int v_mode;
+  float scale;
+  int experts;            /* 0: no feed-forward */
+  int top;
+  int ff;
+  int shared_ff;          /* 0: no shared expert */
+  float limit;
+  float shared_limit;
+  float alpha;
+  const void* w_qkv;      /* [(heads + kv_heads) * head_dim + kv_heads * vdim] rows */
+  const float* q_gain;
+  const float* k_gain;
+  const float* lambda;
+  const void* w_o;
+  const float* norm1;
+  const void* w_router;
+  const float* router_bias;
+  const void* w_gate_up;  /* [experts][2][ff] rows */
+  const void* w_down;     /* [experts][dim] rows */
+  const void* w_shared_gate_up;
+  const void* w_shared_down;
+  const float* norm2;
+  void* k_cache;
+  void* v_cache;
+  float* v_first;         /* [portion, kv_heads * vdim] (v_mode not 0) */
+  float* qkv;             /* work buffers of `portion` rows, or portion * top */
+  void* q;
+  void* att;
+  float* y;
+  float* logits;
+  int* ids;
+  int* rank;
+  int* slot_row;
+  float* slot_w;
+  int* counts;
+  void* xs;
+  void* hid;
+  void* ye;
+  void* shared_hid;
+  void* shared_y;
+} TgRoutedLayer;
+/* x [portion, pad8(dim)] f32 and xh, the same as activations, are advanced by a layer. */
+int tilert_gqa_routed_layer_op(TgContext* ctx, const TgRoutedLayer* layer, int rows, const int* pos, float* x, void* xh,
+                               void* stream);
+
+/* x += n1b(attention(n1(x))), x += n2b(ff(n2(x))): attention over a latent cache, dense gated feed-forward, layer norms. */
+typedef struct TgLatentLayer {
+  int dim;
+  int f32;
+  float eps;
+  int heads;
+  int head_dim;
+  int rot;
+  int vdim;
+  int q_rank;
+  int kv_rank;
+  int window;
+  int ring;
+  float scale;
+  int gate_rows;          /* heads, or heads * vdim */
+  int ff;                 /* 0: no feed-forward */
+  float limit;
+  float alpha;
+  const float* rope;
+  int positions;
+  int rope_dims;
+  int interleaved;
+  const void* w_z;        /* rows: query latent, latent, key part, gate, each filled with zero rows to a multiple of eight */
+  const float* q_gain;
+  const float* c_gain;
+  const void* w_uq;       /* [heads][pad8(head_dim) + pad8(rot)] rows */
+  const void* w_uk_t;     /* [heads][kv_rank] rows */
+  const void* w_kv;       /* heads * pad16(head_dim), then heads * pad16(vdim) rows; NULL: the absorbed form only */
+  const void* w_uv;       /* [heads][vdim] rows */
+  const float* sink;
+  const void* w_o;
+  const void* w_gate_up;  /* [2][ff] rows */
+  const void* w_down;
+  const float* norm1_gain;
+  const float* norm1_bias;
+  const float* norm1b_gain;
+  const float* norm1b_bias;
+  const float* norm2_gain;
+  const float* norm2_bias;
+  void* cache;
+  float* z;               /* work buffers for the rows of a call */
+  void* cq;
+  float* q;
+  void* att;
+  float* y;
+  void* hid;
+  void* qe;               /* expanded form: [rows, heads, pad16(head_dim) + pad16(rot)], [cached, rows of w_kv] */
+  void* kv;
+  void* qn;               /* absorbed form: [heads, rows, ..] of pad8(head_dim), a cache row, parts, pad8(kv_rank), pad8(vdim) */
+  float* lat;
+  float* part;
+  void* c;
+  float* o;
+} TgLatentLayer;
+/* What the layer before left is settled first: x += norm(y) (+ add) where there is a y_gain, then n1.  The layer leaves its own last
+ * output in layer->y in the same way, for norm n2b, or n1b without a feed-forward.  cached: rows of the cache in use for the expanded
+ * form of the attention, 0 for the absorbed one on n_splits parts of the keys. */
+int tilert_gqa_latent_layer_op(TgContext* ctx, const TgLatentLayer* layer, int rows, int cached, int n_splits, const int* pos, float* x,
+                               void* xh, const float* y, const float* y_gain, const float* y_bias, const float* add, void* stream);
+
 /* One token: lat[h] = [w[h] q[h] | rotated part] with w [heads][rank][ldw] the transposed key expansion, and the cache
  * row of *pos from the latent c and the key part kr. */
 int tilert_gqa_vec_absorb_op(TgContext* ctx, const float* q, int heads, int dim, int rank, int rot, const void* w, long long ldw,

@@ -48,6 +48,14 @@ def parse_header(path: Path = HEADER) -> dict[str, tuple[object, list[object]]]:
     return protos
 
 
+def parse_struct(name: str, path: Path) -> type[ctypes.Structure]:
+    """The ctypes twin of ``typedef struct name { ... } name;`` in the header (one field per declaration)."""
+    text = re.sub(r"/\*.*?\*/", " ", path.read_text(), flags=re.S)
+    body = re.search(r"typedef struct " + name + r"\s*\{(.*?)\}\s*" + name + r"\s*;", text, flags=re.S).group(1)
+    fields = [(d.replace("*", " ").split()[-1], _ctype(d)) for d in body.split(";") if d.strip()]
+    return type(name, (ctypes.Structure,), {"_fields_": fields})
+
+
 def bind(lib_path: Path, header: Path = HEADER, exported_globally: bool = True) -> ctypes.CDLL:
     lib = ctypes.CDLL(str(lib_path), mode=ctypes.RTLD_GLOBAL if exported_globally else ctypes.RTLD_LOCAL)
     for name, (restype, argtypes) in parse_header(header).items():

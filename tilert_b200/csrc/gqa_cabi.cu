@@ -911,3 +911,6 @@ extern "C" int tilert_gqa_next_token_op(TgContext* ctx, const float* logits, lon
                                       topn_logprob_out, topn_index_out, token_out, pos, advance},
                     tokens, stream);
 }
+
+// ------------------------------------------------------------------------------- whole layers
+#include "portion_layers.h"

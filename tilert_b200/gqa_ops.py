@@ -11,6 +11,7 @@ from dataclasses import dataclass
 import torch
 
 import tilert_b200 as _tb
+from tilert_b200 import _cabi
 
 _TYPE = "ralasun"  # the backend that carries these operators
 BF16, F32, I32, I64 = torch.bfloat16, torch.float32, torch.int32, torch.int64
@@ -143,6 +144,26 @@ def gemm(x, w, out, rows: int, n: int, k: int, *, gated: tuple[float, float] | N
         raise ValueError(f"gemm: output type {out.dtype} does not fit input type {x.dtype}")
     _call("gemm", x, _p(x), x.stride(-2), rows, _p(w), w.stride(-2), n, k, int(gated is not None), limit, alpha, n_groups, _p(counts),
           _p(bias), _p(out), out.stride(-2), int(out.dtype == F32), f32)
+
+
+# -- whole layers of a portion: a structure that a layer fills in once, and one call a layer --
+_HEADER = _cabi.header_path("tilert_gqa.h")
+RoutedLayer = _cabi.parse_struct("TgRoutedLayer", _HEADER)
+LatentLayer = _cabi.parse_struct("TgLatentLayer", _HEADER)
+
+
+def structure(kind: type[ctypes.Structure], **fields) -> ctypes.Structure:
+    """A structure with tensors as their addresses (None: null)."""
+    return kind(**{n: v.data_ptr() if isinstance(v, torch.Tensor) else v for n, v in fields.items() if v is not None})
+
+
+def routed_layer(layer, rows: int, pos, x, xh) -> None:
+    _call("routed_layer", x, ctypes.addressof(layer), rows, _p(pos), _p(x), _p(xh))
+
+
+def latent_layer(layer, rows: int, cached: int, n_splits: int, pos, x, xh, y, norm, add) -> None:
+    gain, bias = (None, None) if norm is None else (_p(norm.gain), _p(norm.bias))
+    _call("latent_layer", x, ctypes.addressof(layer), rows, cached, n_splits, _p(pos), _p(x), _p(xh), _p(y), gain, bias, _p(add))
 
 
 def qkv_rows(qkv, q_gain, k_gain, eps: float, v_mode: int, lam, v_first, rows: int, mix, cache, pos, q) -> None:

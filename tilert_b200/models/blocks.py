@@ -3,7 +3,6 @@ of a one-token step and of a portion of tokens."""
 
 from __future__ import annotations
 
-import math
 from dataclasses import dataclass
 
 import torch
@@ -43,6 +42,7 @@ class Scratch:
     def __init__(self, device):
         self.device = torch.device(device)
         self._bufs: dict = {}
+        self._room: dict = {}
 
     def get(self, name: str, *shape: int, dtype=F32) -> torch.Tensor:
         key = (name, shape, dtype)
@@ -50,13 +50,13 @@ class Scratch:
             self._bufs[key] = torch.zeros(*shape, dtype=dtype, device=self.device)
         return self._bufs[key]
 
-    def flat(self, name: str, *shape: int, dtype=F32) -> torch.Tensor:
-        """A contiguous buffer of this shape in memory that grows as needed (never inside a graph: it may move); the
-        contents are whatever was left there, but finite."""
-        n, key = math.prod(shape), (name, dtype)
-        if key not in self._bufs or self._bufs[key].numel() < n:
-            self._bufs[key] = torch.zeros(n, dtype=dtype, device=self.device)
-        return self._bufs[key][:n].view(*shape)
+    def room(self, name: str, n: int, dtype=F32) -> int:
+        """Address of ``n`` elements in memory that grows as needed (never inside a graph: it may move); the contents are
+        whatever was left there, but finite.  Ask again for every call: another layer may have made it grow."""
+        key = (name, dtype)
+        if key not in self._room or self._room[key].numel() < n:
+            self._room[key] = torch.zeros(n, dtype=dtype, device=self.device)
+        return self._room[key].data_ptr()
 
 
 @dataclass
@@ -104,26 +104,17 @@ class Stream:
 
 class RowStream:
     """The residual rows of a portion, f32 ``x`` and ``xh``, what the next sublayer reads.  As in a one-token step a
-    sublayer's output waits: the launch that adds it also norms the next sublayer's input."""
+    sublayer's output waits: the launch that adds it also norms the next sublayer's input.  Layers do that natively."""
 
     def __init__(self, x: torch.Tensor, xh: torch.Tensor, rows: int, dim: int, eps: float):
         self.x, self.xh, self.rows, self.dim, self.eps = x, xh, rows, dim, eps
         self.pending: Pending | None = None
         self.add: torch.Tensor | None = None  # a constant vector, added behind the pending output
 
-    def _advance(self, xh, norm2) -> None:
-        p = self.pending
-        ops.residual_norm(self.x, xh, None if p is None else p.norm, self.eps, self.dim, self.rows, y=None if p is None else p.y,
-                          add=self.add, norm2=norm2)
-        self.pending = self.add = None
-
-    def normed(self, norm) -> torch.Tensor:
-        """The norm of the up-to-date rows as activations."""
-        self._advance(self.xh, norm)
-        return self.xh
-
     def settle(self) -> torch.Tensor:
         """The up-to-date rows."""
-        if self.pending is not None or self.add is not None:
-            self._advance(None, None)
+        p = self.pending
+        if p is not None or self.add is not None:
+            ops.residual_norm(self.x, None, None if p is None else p.norm, self.eps, self.dim, self.rows, y=None if p is None else p.y, add=self.add)
+            self.pending = self.add = None
         return self.x

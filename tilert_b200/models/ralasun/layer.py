@@ -86,6 +86,7 @@ class RalasunLayer:
         self.cache = RingKVCache(m.kv_heads, m.dim, m.vdim, m.window, args.max_seq_len, portion, device, dtype)
         self.n_q, self.n_kv = m.heads * m.dim, m.kv_heads * (m.dim + m.vdim)
         self.head_blocks = ops.head_blocks(m.heads, m.kv_heads)
+        self._native = None  # of a portion's call: made when the first prompt comes, with its work buffers
         self.max_splits = max(1, 2 * ops.num_sms(device) // self.head_blocks)  # (two thread blocks per SM)
 
     def _v_first(self, rows: int):
@@ -124,34 +125,26 @@ class RalasunLayer:
     # -- a portion of tokens --
     def prefill(self, x: torch.Tensor, xh: torch.Tensor, rows: int, cur_pos: torch.Tensor) -> None:
         """x [portion, pad8(dim)] f32 residual, xh the same as activations; both are advanced."""
-        m, w, sc, eps, dim, p, t = self.a.mixer, self.w, self.sc, self.args.eps, self.args.dim, self.portion, self.dtype
-        qkv = sc.get("qkv", p, pad(self.n_q + self.n_kv))
-        ops.gemm(xh, w.qkv, qkv, rows, self.n_q + self.n_kv, dim)
-        q = sc.get("q", p, m.heads, pad(m.dim, 16), dtype=t)
-        ops.qkv_rows(qkv, w.q_gain, w.k_gain, eps, self.v_mode, w.lam, self._v_first(p), rows, m, self.cache, cur_pos, q)
-        att = sc.get("att", p, pad(m.heads * m.vdim), dtype=t)
-        ops.attn_rows(q, m, self.cache, cur_pos, rows, att)
-        y = sc.get("y", p, pad(dim))
-        ops.gemm(att, w.o, y, rows, dim, m.heads * m.vdim)
-        ops.residual_norm(x, xh, w.norm1, eps, dim, rows, y=y)
-        f = self.a.mlp
-        if f is None:
-            return
-        logits = sc.get("router", p, pad(f.experts))
-        ops.gemm(xh, w.router, logits, rows, f.experts, dim, bias=w.router_bias)
-        ids, rank, slot_row = (sc.get(n, p, f.top, dtype=I32) for n in ("ids", "rank", "slot_row"))
-        sw, counts = sc.get("slot_w", p, f.top), sc.get("counts", f.experts, dtype=I32)
-        ops.route_rows(logits, rows, f.experts, f.top, ids, sw, rank, counts)
-        xs = sc.get("xs", p * f.top, pad(dim), dtype=t)
-        ops.gather_rows(xh, rows, dim, f.experts, f.top, ids, rank, counts, xs, slot_row)
-        hid = sc.get("hid", p * f.top, pad(f.ff), dtype=t)
-        ops.gemm(xs, w.gate_up, hid, rows * f.top, f.ff, dim, gated=(f.limit, GATE_ALPHA), n_groups=f.experts, counts=counts)
-        ye = sc.get("ye", p * f.top, pad(dim), dtype=t)
-        ops.gemm(hid, w.down, ye, rows * f.top, dim, f.ff, n_groups=f.experts, counts=counts)
-        ysh = None
-        if f.shared_ff:
-            hsh = sc.get("hsh", p, pad(f.shared_ff), dtype=t)
-            ops.gemm(xh, w.shared_gate_up, hsh, rows, f.shared_ff, dim, gated=(f.shared_limit, GATE_ALPHA))
-            ysh = sc.get("ysh", p, pad(dim), dtype=t)
-            ops.gemm(hsh, w.shared_down, ysh, rows, dim, f.shared_ff)
-        ops.residual_norm(x, xh, w.norm2, eps, dim, rows, experts=ye, slot_row=slot_row, slot_w=sw, shared=ysh)
+        if self._native is None:
+            self._native = self._structure()
+        ops.routed_layer(self._native, rows, cur_pos, x, xh)
+
+    def _structure(self):
+        m, f, w, sc, dim, p, t = self.a.mixer, self.a.mlp, self.w, self.sc, self.args.dim, self.portion, self.dtype
+        fields = dict(dim=dim, f32=int(t is F32), eps=self.args.eps, portion=p, heads=m.heads, kv_heads=m.kv_heads, head_dim=m.dim, vdim=m.vdim,
+                      window=self.cache.window, ring=self.cache.ring, v_mode=self.v_mode, scale=m.scale, w_qkv=w.qkv, q_gain=w.q_gain, k_gain=w.k_gain,
+                      w_o=w.o, norm1=w.norm1, k_cache=self.cache.k, v_cache=self.cache.v, v_first=self._v_first(p),
+                      qkv=sc.get("qkv", p, pad(self.n_q + self.n_kv)), q=sc.get("q", p, m.heads, pad(m.dim, 16), dtype=t),
+                      att=sc.get("att", p, pad(m.heads * m.vdim), dtype=t), y=sc.get("y", p, pad(dim)))
+        fields["lambda"] = w.lam
+        if f is not None:
+            fields |= dict(experts=f.experts, top=f.top, ff=f.ff, limit=f.limit, alpha=GATE_ALPHA, w_router=w.router, router_bias=w.router_bias,
+                           w_gate_up=w.gate_up, w_down=w.down, norm2=w.norm2, logits=sc.get("router", p, pad(f.experts)),
+                           slot_w=sc.get("slot_w", p, f.top), counts=sc.get("counts", f.experts, dtype=I32),
+                           xs=sc.get("xs", p * f.top, pad(dim), dtype=t), hid=sc.get("hid", p * f.top, pad(f.ff), dtype=t),
+                           ye=sc.get("ye", p * f.top, pad(dim), dtype=t))
+            fields |= {n: sc.get(n, p, f.top, dtype=I32) for n in ("ids", "rank", "slot_row")}
+            if f.shared_ff:
+                fields |= dict(shared_ff=f.shared_ff, shared_limit=f.shared_limit, w_shared_gate_up=w.shared_gate_up, w_shared_down=w.shared_down,
+                               shared_hid=sc.get("hsh", p, pad(f.shared_ff), dtype=t), shared_y=sc.get("ysh", p, pad(dim), dtype=t))
+        return ops.structure(ops.RoutedLayer, **fields)

@@ -108,6 +108,7 @@ class RozesunLayer:
         self.sms = ops.num_sms(device)
         self.z_len = weights.off_g + m.gate_rows
         self.ldh = pad(m.dim) + pad(m.rot_dim)
+        self._native = None  # of a portion's call: made when the first prompt comes
 
     def _splits(self, tokens: int, keys: int) -> int:
         """Parts of the key range, of ``per`` tiles of 64 keys each: no more than fill the SMs, and no more than pay (a tile
@@ -145,57 +146,47 @@ class RozesunLayer:
     # -- a portion of tokens --
     def prefill(self, st: RowStream, nr: int, cur_pos: torch.Tensor, pos: int) -> None:
         """Pass ``nr``; ``pos``: the position of the first row, as ``cur_pos`` holds it."""
-        m, w, sc, eps, dim, t, n = self.a.mixer, self.w, self.sc, self.args.eps, self.args.dim, self.dtype, st.rows
-        cache = self.caches[nr]
-        h = st.normed(w.norm1)
-        z = sc.flat("z", n, pad(self.z_len))
-        ops.gemm(h, w.z, z, n, self.z_len, dim)
-        cq = sc.get("cq", self.portion, pad(m.q_rank), dtype=t)
-        ops.latent_tokens(z, w.off_c, w.off_r, m.q_rank, w.q_gain, w.c_gain, eps, n, m, self.rope, cache, cur_pos, cq)
-        q = sc.flat("q", n, m.heads * self.ldh)
-        ops.gemm(cq, w.uq, q, n, m.heads * self.ldh, m.q_rank)
-        att = sc.get("att", self.portion, pad(m.heads * m.vdim), dtype=t)
-        length = pos + n
-        cached = min(length, cache.ring)
+        m, w, sc, t, n = self.a.mixer, self.w, self.sc, self.dtype, st.rows
+        cache, hn = self.caches[nr], m.heads * n
+        if self._native is None:
+            self._native = self._structure()
+        s, length = self._native, pos + n
+        s.cache = cache.rows.data_ptr()
+        s.z = sc.room("z", n * pad(self.z_len))
+        s.q = sc.room("q", n * m.heads * self.ldh)
+        cached, n_splits = min(length, cache.ring), 0
         if w.kv is not None and expansion_pays(m, n, min(length, cache.window or length), cached):
-            self._expanded(q, z, n, cache, cur_pos, cached, att)
+            s.qe = sc.room("qe", hn * (pad(m.dim, 16) + pad(m.rot_dim, 16)), t)
+            s.kv = sc.room("kv", cached * w.kv.shape[0], t)
         else:
-            self._absorbed(q, z, n, cache, cur_pos, length, att)
-        y = sc.get("y", self.portion, pad(dim))
-        ops.gemm(att, w.o, y, n, dim, m.heads * m.vdim)
-        st.pending = Pending(y, w.norm1b)
-        f = self.a.mlp
-        if f is None:
-            return
-        hid = sc.get("hid", self.portion, pad(f.ff), dtype=t)
-        ops.gemm(st.normed(w.norm2), w.gate_up, hid, n, f.ff, dim, gated=(f.limit, GATE_ALPHA))
-        ops.gemm(hid, w.down, y, n, dim, f.ff)
-        st.pending = Pending(y, w.norm2b)
+            cached, n_splits = 0, self._splits(n, cache.visible(length, n))
+            s.qn = sc.room("qn", hn * pad(m.dim), t)
+            s.lat = sc.room("lat", hn * cache.rows.shape[1])
+            s.part = sc.room("part", hn * n_splits * (pad(m.kv_rank, 16) + 2))
+            s.c = sc.room("c", hn * pad(m.kv_rank), t)
+            s.o = sc.room("o", hn * pad(m.vdim))
+        p = st.pending
+        ops.latent_layer(s, n, cached, n_splits, cur_pos, st.x, st.xh, None if p is None else p.y, None if p is None else p.norm, st.add)
+        st.add = None
+        st.pending = Pending(self._y(), w.norm1b if self.a.mlp is None else w.norm2b)
 
-    def _expanded(self, q, z, n: int, cache: LatentCache, cur_pos, cached: int, att) -> None:
-        m, w, sc = self.a.mixer, self.w, self.sc
-        wide = pad(m.dim, 16) + pad(m.rot_dim, 16)
-        qe = sc.flat("qe", n, m.heads, wide, dtype=self.dtype)
-        ops.latent_queries(q, n, m, self.rope, cur_pos, qe)
-        kv = sc.flat("kv", cached, w.kv.shape[0], dtype=self.dtype)
-        ops.gemm(cache.rows, w.kv, kv, cached, w.kv.shape[0], m.kv_rank)
-        ops.expanded_attn(qe, kv, cache, n, m, cur_pos, w.sink, z[:, w.off_g:], m.gate_per_head, att)
+    def _y(self) -> torch.Tensor:
+        return self.sc.get("y", self.portion, pad(self.args.dim))
 
-    def _absorbed(self, q, z, n: int, cache: LatentCache, cur_pos, length: int, att) -> None:
-        m, w, sc, t = self.a.mixer, self.w, self.sc, self.dtype
-        rank, hn = m.kv_rank, m.heads * n
-        qn = sc.flat("qn", hn, pad(m.dim), dtype=t)
-        lat = sc.flat("lat", hn, cache.rows.shape[1])
-        ops.latent_queries(q, n, m, self.rope, cur_pos, qn, lat)
-        ops.gemm(qn, w.uk_t, lat, n, rank, m.dim, n_groups=m.heads)
-        n_splits = self._splits(n, cache.visible(length, n))
-        part = sc.flat("part", hn * n_splits * (pad(rank, 16) + 2))
-        ops.latent_attn(lat, cache, n, m, cur_pos, n_splits, part)
-        c = sc.flat("c", hn, pad(rank), dtype=t)
-        ops.latent_merge(part, n, m, n_splits, w.sink, c)
-        o = sc.flat("o", hn, pad(m.vdim))
-        ops.gemm(c, w.uv, o, n, m.vdim, rank, n_groups=m.heads)
-        ops.gate_heads(o, n, m.heads, m.vdim, z[:, w.off_g:], m.gate_per_head, att)
+    def _structure(self):
+        m, f, w, sc, p, t = self.a.mixer, self.a.mlp, self.w, self.sc, self.portion, self.dtype
+        fields = dict(dim=self.args.dim, f32=int(t is F32), eps=self.args.eps, heads=m.heads, head_dim=m.dim, rot=m.rot_dim, vdim=m.vdim, q_rank=m.q_rank,
+                      kv_rank=m.kv_rank, window=self.caches[0].window, ring=self.caches[0].ring, scale=m.scale, gate_rows=m.gate_rows,
+                      rope=self.rope.table, positions=self.rope.table.shape[0], rope_dims=self.rope.table.shape[1], interleaved=int(self.rope.interleaved),
+                      w_z=w.z, q_gain=w.q_gain, c_gain=w.c_gain, w_uq=w.uq, w_uk_t=w.uk_t, w_kv=w.kv, w_uv=w.uv, sink=w.sink, w_o=w.o,
+                      cq=sc.get("cq", p, pad(m.q_rank), dtype=t), att=sc.get("att", p, pad(m.heads * m.vdim), dtype=t), y=self._y())
+        if f is not None:
+            fields |= dict(ff=f.ff, limit=f.limit, alpha=GATE_ALPHA, w_gate_up=w.gate_up, w_down=w.down, hid=sc.get("hid", p, pad(f.ff), dtype=t))
+        for name in ("norm1", "norm1b", "norm2"):
+            norm = getattr(w, name)
+            if norm is not None:
+                fields |= {f"{name}_gain": norm.gain, f"{name}_bias": norm.bias}
+        return ops.structure(ops.LatentLayer, **fields)
 
     def weight_bytes(self) -> int:
         return self.w.weight_bytes() * len(self.caches)
