@@ -95,7 +95,9 @@ class MtpDsaModel:
         self.guess = z(1, dtype=I64)
         self.use_graph = use_graph
         self._graphs: dict[tuple[str, int], torch.cuda.CUDAGraph] = {}
-        self.pos = 0  # host copy of the position
+        # host copies: a chunk of a prompt is launched without waiting for the one before
+        self.pos = 0
+        self._valid = 0
 
     # -- controls with the reference driver's names (end2end.py:551-577, 137-163) --
     def reset_sequence(self) -> None:
@@ -107,6 +109,7 @@ class MtpDsaModel:
 
     def set_prefill_valid_tokens(self, n: int) -> None:
         self.valid.fill_(n)
+        self._valid = int(n)
 
     def set_prefill_mtp_extra_token(self, token: int) -> None:
         self.extra_token.fill_(token)
@@ -214,16 +217,17 @@ class MtpDsaModel:
         ``get_next_draft_tokens``."""
         if not with_mtp:
             raise ValueError("MtpDsaModel only runs the speculative path; use DsaModel for plain decoding")
-        t = torch.as_tensor(draft_tokens).view(-1).to(self.device, I64)
+        t = torch.as_tensor(draft_tokens, dtype=I64).view(-1)
+        if not t.is_cuda:
+            t = t.pin_memory().to(self.device, non_blocking=True)  # (from pageable memory the host would wait for the stream)
         if t.numel() != N_TOKENS:
             raise ValueError(f"draft_tokens must hold {N_TOKENS} tokens")
         if self.pos + 2 * N_TOKENS > self.cache_len:
             raise ValueError("position too close to the end of the caches")
         self.draft.copy_(t)
-        valid = int(self.valid.item())
-        if valid > 0:
+        if self._valid > 0:
             self._run("prefill")
-            self.pos += valid
+            self.pos += self._valid
         else:
             self._run("verify")
             self.pos += self.get_num_accepted()
