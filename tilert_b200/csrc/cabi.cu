@@ -1494,8 +1494,8 @@ int launch_sparse_mla(TbContext* ctx, const void* q, const void* q_pe, const voi
   static bool attr_set = false;
   if (!attr_set) {
     TB_CUDA(cudaFuncSetAttribute(sparse_mla_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlaSmemBytes));
-    TB_CUDA(cudaFuncSetAttribute(sparse_mla_combine_vproj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kMlaCvSmemBytes));
+    TB_CUDA(cudaFuncSetAttribute(sparse_mla_combine_vproj_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, mla_cv_smem(1)));
+    TB_CUDA(cudaFuncSetAttribute(sparse_mla_combine_vproj_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mla_cv_smem(4)));
     attr_set = true;
   }
   MlaParams p{};
@@ -1519,11 +1519,12 @@ int launch_sparse_mla(TbContext* ctx, const void* q, const void* q_pe, const voi
   TB_CUDA(launch(sparse_mla_kernel, dim3(grid), dim3(kMlaThreads), kMlaSmemBytes, st, p));
   ++g_launches;
   TB_CUDA(cudaGetLastError());
-  if (w_v != nullptr)
-    TB_CUDA(launch(sparse_mla_combine_vproj_kernel, dim3(dim3(heads, tokens)), dim3(128), kMlaCvSmemBytes, st, out_acc,
-                   lse_acc, p.n_splits, reinterpret_cast<__nv_bfloat16*>(out), lse, w_v,
-                   reinterpret_cast<__nv_bfloat16*>(o_out), ctx->status));
-  else
+  if (w_v != nullptr) {
+    const int tok = tokens > 2 ? kMlaMergeTokens : 1;  // (two tokens' own CTAs fit the SMs as well)
+    TB_CUDA(launch(tok == 1 ? sparse_mla_combine_vproj_kernel<1> : sparse_mla_combine_vproj_kernel<kMlaMergeTokens>,
+                   dim3(heads, (tokens + tok - 1) / tok), dim3(128, tok), mla_cv_smem(tok), st, out_acc, lse_acc, p.n_splits,
+                   reinterpret_cast<__nv_bfloat16*>(out), lse, w_v, reinterpret_cast<__nv_bfloat16*>(o_out), tokens, ctx->status));
+  } else
     TB_CUDA(launch(sparse_mla_combine_kernel, dim3(dim3(heads, tokens)), dim3(128), 0, st, out_acc, lse_acc, p.n_splits,
                    reinterpret_cast<__nv_bfloat16*>(out), lse));
   ++g_launches;

@@ -5,6 +5,9 @@
 // its 64-row blocks with one bulk async copy (TMA) per row, computes Q.K^T and P.V with bf16
 // tensor-core MMAs in f32, and writes a normalised partial output plus its log-sum-exp.  A
 // second small kernel merges the chunks.  Algorithmic HBM traffic: topk x 1152 bytes per token.
+//
+// A position with fewer keys than topk leaves chunks without a valid row: their CTAs write what such a chunk contributes (zeros,
+// minus infinity) and go, and the merge does not read it.  Four rows behind 12 to 28 positions, 128 heads, 2048 selectable: 25 -> 12 us.
 #pragma once
 
 #include "common.cuh"
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
     // those accesses before the async-proxy writes of the bulk copies issued below
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (tid < kMlaKeys) {
+    if (tid < kMlaKeys && n_valid > 0) {
       __nv_bfloat16* row = sKV + tid * kMlaPitch;
       if (valid) {
         bulk_g2s(row, p.kv + static_cast<long long>(my_idx) * kMlaDV, kMlaDV * 2, bar);
@@ -91,6 +94,17 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
   };
   // the first block's rows are requested before the queries are staged: the two latencies overlap
   int n_valid = p.blocks_per_split > 0 ? issue_gather(0) : 0;
+  if (p.blocks_per_split == 1 && n_valid == 0) {  // uniform over the CTA
+#pragma unroll 4
+    for (int r = 0; r < kMlaHeads; ++r) {
+      const int head = hg * kMlaHeads + r;
+      if (head >= p.heads) break;
+      const long long base = (static_cast<long long>(tok) * p.heads + head) * p.n_splits + split;
+      *reinterpret_cast<float4*>(p.o_acc + base * kMlaDV + tid * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (tid == 0) p.lse_acc[base] = -INFINITY;
+    }
+    return;
+  }
   // stage the 16 query heads: [512 latent | 64 rope]; all of a thread's loads are requested before the
   // first is stored (a load-store loop would pay one memory round trip per iteration)
   constexpr int kQIters = kMlaHeads * 72 / kMlaThreads;  // 9
@@ -114,7 +128,7 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
   }
   __syncthreads();
 
-  uint32_t phase = 0;  // completed phases of `bar` (a block without valid rows issues no copy)
+  uint32_t phase = 0;  // completed phases of `bar`
   float m_run[2] = {-INFINITY, -INFINITY};
   float l_run[2] = {0.f, 0.f};
   float o[16][4];
@@ -124,12 +138,10 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
   for (int blk = 0; blk < p.blocks_per_split; ++blk) {
     // ---- 64 selected rows (block 0 was requested before the loop) ----
     if (blk > 0) n_valid = issue_gather(blk);
-    bool gave_up = false;
-    if (n_valid > 0) {
-      gave_up = !mbar_wait(bar, phase & 1);
-      if (gave_up) set_status(p.status, ST_WAIT_FULL_TIMEOUT);
-      ++phase;
-    }
+    if (n_valid == 0) continue;  // (uniform; nothing is added)
+    const bool gave_up = !mbar_wait(bar, phase & 1);
+    if (gave_up) set_status(p.status, ST_WAIT_FULL_TIMEOUT);
+    ++phase;
     // a wait that ran out ends the loop for the whole CTA: no further copies are requested, and the one wait
     // below gives the copies already in flight the same budget again before the kernel returns
     if (__syncthreads_or(gave_up ? 1 : 0)) {
@@ -258,17 +270,17 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
   }
 }
 
-// Merge the chunks: o = sum_i exp(lse_i - lse) * o_i.   grid = (heads, tokens), block = 128; n_splits <= 64.
-__global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const float* __restrict__ o_acc,
-                                                                 const float* __restrict__ lse_acc, int n_splits,
-                                                                 __nv_bfloat16* __restrict__ out,
-                                                                 float* __restrict__ lse_out) {
-  pdl_launch_dependents();
-  pdl_wait();
-  __shared__ float s_w[64];
-  __shared__ float s_den, s_mx;
-  const int head = blockIdx.x, tok = blockIdx.y, heads = gridDim.x;
-  const long long th = static_cast<long long>(tok) * heads + head;
+constexpr int kMlaMergeTokens = 4;  // of a CTA at most: 128 threads each
+// o = sum_i exp(lse_i - lse) * o_i over the chunks of one (token, head), four columns a thread of 128; n_splits <= 64.  A chunk without
+// keys is marked by a negative weight and not added (what it left is not read beyond the first batch).
+struct MlaMerged {
+  uint2 o;      // bf16
+  float lse;
+};
+template <int kBatch>
+__device__ __forceinline__ MlaMerged mla_merge(const float* __restrict__ o_acc, const float* __restrict__ lse_acc, int n_splits, long long th) {
+  __shared__ float s_weight[kMlaMergeTokens][64], s_den[kMlaMergeTokens], s_mx[kMlaMergeTokens];
+  float* s_w = s_weight[threadIdx.y];
   if (threadIdx.x < 32) {
     // weights of all chunks, computed once by the first warp
     const int lane = threadIdx.x;
@@ -277,18 +289,17 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const float* __
     const float mx = warp_max(fmaxf(l0, l1));
     const float w0 = mx == -INFINITY ? 0.f : expf(l0 - mx), w1 = mx == -INFINITY ? 0.f : expf(l1 - mx);
     const float den = warp_sum(w0 + w1);
-    s_w[lane] = w0;
-    s_w[lane + 32] = w1;
+    s_w[lane] = l0 == -INFINITY ? -1.f : w0;
+    s_w[lane + 32] = l1 == -INFINITY ? -1.f : w1;
     if (lane == 0) {
-      s_den = den;
-      s_mx = mx;
+      s_den[threadIdx.y] = den;
+      s_mx[threadIdx.y] = mx;
     }
   }
-  // partial outputs in batches of 16 independent loads; the first batch is requested before the
+  // partial outputs in batches of independent loads; the first batch is requested before the
   // barrier, so it overlaps the weights' own load and reductions
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   const float* src = o_acc + th * n_splits * kMlaDV + threadIdx.x * 4;
-  constexpr int kBatch = 16;
   float4 v[kBatch];
 #pragma unroll
   for (int j = 0; j < kBatch; ++j)
@@ -300,12 +311,12 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const float* __
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
       const int i = i0 + kBatch + j;
-      nxt[j] = i < n_splits ? __ldcs(reinterpret_cast<const float4*>(src + static_cast<long long>(i) * kMlaDV))
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
+      nxt[j] = i < n_splits && !(s_w[i] < 0.f) ? __ldcs(reinterpret_cast<const float4*>(src + static_cast<long long>(i) * kMlaDV))
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
-      if (i0 + j < n_splits) {
+      if (i0 + j < n_splits && !(s_w[i0 + j] < 0.f)) {
         const float wgt = s_w[i0 + j];
         acc[0] += wgt * v[j].x; acc[1] += wgt * v[j].y; acc[2] += wgt * v[j].z; acc[3] += wgt * v[j].w;
       }
@@ -313,13 +324,22 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const float* __
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) v[j] = nxt[j];
   }
-  const float den = s_den;
+  const float den = s_den[threadIdx.y];
   const float inv = den > 0.f ? 1.f / den : 0.f;
-  uint2 o2;
-  o2.x = pack_bf16x2(acc[0] * inv, acc[1] * inv);
-  o2.y = pack_bf16x2(acc[2] * inv, acc[3] * inv);
-  *reinterpret_cast<uint2*>(out + th * kMlaDV + threadIdx.x * 4) = o2;
-  if (threadIdx.x == 0 && lse_out != nullptr) lse_out[th] = den > 0.f ? s_mx + logf(den) : -INFINITY;
+  return {make_uint2(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv)), den > 0.f ? s_mx[threadIdx.y] + logf(den) : -INFINITY};
+}
+
+// The merge alone.   grid = (heads, tokens), block = 128.
+__global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const float* __restrict__ o_acc,
+                                                                 const float* __restrict__ lse_acc, int n_splits,
+                                                                 __nv_bfloat16* __restrict__ out,
+                                                                 float* __restrict__ lse_out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long th = static_cast<long long>(blockIdx.y) * gridDim.x + blockIdx.x;
+  const MlaMerged m = mla_merge<16>(o_acc, lse_acc, n_splits, th);
+  *reinterpret_cast<uint2*>(out + th * kMlaDV + threadIdx.x * 4) = m.o;
+  if (threadIdx.x == 0 && lse_out != nullptr) lse_out[th] = m.lse;
 }
 
 // Merge of the chunks fused with the value up-projection of the same head: o[h, :] = W_v[h] . o_lat[h] (128 x 512
@@ -327,24 +347,25 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const float* __
 // bulk copies before the wait for the attention launch -- weights depend on nothing -- so they are in shared memory
 // when the merged latent vector is; thread r then owns output row r.  Saves the separate product launch, which is
 // pure latency at this size (8 MB over the GPU, 1 MB per rank of eight).
-// grid = (heads, tokens), block = 128, dynamic smem = kMlaCvSmemBytes; n_splits <= 64; kv_lora 512, v_head_dim 128.
-constexpr int kMlaCvSmemBytes = 4 * TB_WBLK_BYTES + kMlaDV * 4 + 16;
+// grid = (heads, ceil(tokens / TOK)), block = (128, TOK), dynamic smem = mla_cv_smem(TOK); n_splits <= 64; kv_lora 512, v_head_dim
+// 128.  TOK 4: the tokens of a verify step share the head's weights, and the CTAs fit the SMs once: 13 -> 9 us at four rows.
+constexpr int mla_cv_smem(int tok) { return 4 * TB_WBLK_BYTES + tok * kMlaDV * 4 + 16; }
 
-__global__ void __launch_bounds__(128) sparse_mla_combine_vproj_kernel(const float* __restrict__ o_acc,
+template <int TOK>
+__global__ void __launch_bounds__(128 * TOK) sparse_mla_combine_vproj_kernel(const float* __restrict__ o_acc,
                                                                        const float* __restrict__ lse_acc, int n_splits,
                                                                        __nv_bfloat16* __restrict__ o_lat_out,
                                                                        float* __restrict__ lse_out,
                                                                        const uint8_t* __restrict__ w_v,
-                                                                       __nv_bfloat16* __restrict__ o_out, int* status) {
+                                                                       __nv_bfloat16* __restrict__ o_out, int tokens, int* status) {
   extern __shared__ __align__(128) uint8_t cv_smem[];
   uint8_t* sW = cv_smem;                                              // [4 k blocks][16448]
-  float* s_o = reinterpret_cast<float*>(cv_smem + 4 * TB_WBLK_BYTES);  // [512] merged latent vector (bf16 values)
-  uint64_t* bar = reinterpret_cast<uint64_t*>(s_o + kMlaDV);
-  __shared__ float s_w[64];
-  __shared__ float s_den, s_mx;
-  const int head = blockIdx.x, tok = blockIdx.y, heads = gridDim.x;
-  const int tid = threadIdx.x;
-  if (tid == 0) {
+  float* s_os = reinterpret_cast<float*>(cv_smem + 4 * TB_WBLK_BYTES);  // [TOK][512] merged latent vectors (bf16 values)
+  float* s_o = s_os + threadIdx.y * kMlaDV;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(s_os + TOK * kMlaDV);
+  const int head = blockIdx.x, heads = gridDim.x;
+  const int tid = threadIdx.x, row = static_cast<int>(blockIdx.y) * TOK + threadIdx.y, tok = min(row, tokens - 1);
+  if (tid == 0 && threadIdx.y == 0) {
     mbar_init(bar, 1);
     mbar_fence_init();
     mbar_expect_tx(bar, 4 * TB_WBLK_BYTES);
@@ -354,54 +375,10 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_vproj_kernel(const flo
   pdl_launch_dependents();
   pdl_wait();
   const long long th = static_cast<long long>(tok) * heads + head;
-  if (tid < 32) {
-    const int lane = tid;
-    const float l0 = lane < n_splits ? lse_acc[th * n_splits + lane] : -INFINITY;
-    const float l1 = lane + 32 < n_splits ? lse_acc[th * n_splits + lane + 32] : -INFINITY;
-    const float mx = warp_max(fmaxf(l0, l1));
-    const float w0 = mx == -INFINITY ? 0.f : expf(l0 - mx), w1 = mx == -INFINITY ? 0.f : expf(l1 - mx);
-    const float den = warp_sum(w0 + w1);
-    s_w[lane] = w0;
-    s_w[lane + 32] = w1;
-    if (lane == 0) {
-      s_den = den;
-      s_mx = mx;
-    }
-  }
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  const float* src = o_acc + th * n_splits * kMlaDV + tid * 4;
-  constexpr int kBatch = 16;
-  float4 v[kBatch];
-#pragma unroll
-  for (int j = 0; j < kBatch; ++j)
-    v[j] = j < n_splits ? __ldcs(reinterpret_cast<const float4*>(src + static_cast<long long>(j) * kMlaDV))
-                        : make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncthreads();
-  for (int i0 = 0; i0 < n_splits; i0 += kBatch) {
-    float4 nxt[kBatch];
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      const int i = i0 + kBatch + j;
-      nxt[j] = i < n_splits ? __ldcs(reinterpret_cast<const float4*>(src + static_cast<long long>(i) * kMlaDV))
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      if (i0 + j < n_splits) {
-        const float wgt = s_w[i0 + j];
-        acc[0] += wgt * v[j].x; acc[1] += wgt * v[j].y; acc[2] += wgt * v[j].z; acc[3] += wgt * v[j].w;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) v[j] = nxt[j];
-  }
-  const float den = s_den;
-  const float inv = den > 0.f ? 1.f / den : 0.f;
-  uint2 o2;
-  o2.x = pack_bf16x2(acc[0] * inv, acc[1] * inv);
-  o2.y = pack_bf16x2(acc[2] * inv, acc[3] * inv);
-  if (o_lat_out != nullptr) *reinterpret_cast<uint2*>(o_lat_out + th * kMlaDV + tid * 4) = o2;
-  if (tid == 0 && lse_out != nullptr) lse_out[th] = den > 0.f ? s_mx + logf(den) : -INFINITY;
+  const MlaMerged m = mla_merge<TOK == 1 ? 16 : 8>(o_acc, lse_acc, n_splits, th);
+  const uint2 o2 = m.o;
+  if (o_lat_out != nullptr && row < tokens) *reinterpret_cast<uint2*>(o_lat_out + th * kMlaDV + tid * 4) = o2;
+  if (tid == 0 && lse_out != nullptr && row < tokens) lse_out[th] = m.lse;
   // the product sees the same bf16 values the separate launch would read back
   s_o[tid * 4 + 0] = __uint_as_float(o2.x << 16);
   s_o[tid * 4 + 1] = __uint_as_float(o2.x & 0xffff0000u);
@@ -441,7 +418,7 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_vproj_kernel(const flo
     }
     y = fmaf(part, *reinterpret_cast<const float*>(blk + TB_WBLK_DATA + (tid >> 3) * 4), y);
   }
-  o_out[th * 128 + tid] = f2bf(y);
+  if (row < tokens) o_out[th * 128 + tid] = f2bf(y);
 }
 
 }  // namespace tb
