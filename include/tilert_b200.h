@@ -376,6 +376,12 @@ int tilert_next_token_op(TbContext* ctx, const float* logits, long long logits_s
                          float* token_logprob_out, float* topn_logprob_out, int* topn_index_out, long long* token_out, int* pos,
                          int advance, void* stream);
 
+/* What a pass begins with: x [n, dim] = rows `tokens` of table [vocab, dim] bf16 (a negative token counts from the end), freqs_out [n,
+ * freq_len] = rows *pos .. *pos + n - 1 of freqs [positions, freq_len].  A token or position outside of its table is refused on the
+ * device (status 4). */
+int tilert_step_inputs_op(TbContext* ctx, const long long* tokens, int n, const void* table, int vocab, int dim, const int* pos,
+                          const float* freqs, int positions, int freq_len, void* x, float* freqs_out, void* stream);
+
 /* ---- latent caches from an external prefill, FP8 wire format -------------------------------- */
 
 /* The decode side of prefill / decode disaggregation: tilert/pd_vllm/profiles/mla_nsa.py:16-41 (layout),

@@ -20,6 +20,7 @@
 #include "sparse_mla.cuh"
 #include "allreduce_add.cuh"
 #include "sampler.cuh"
+#include "step_inputs.cuh"
 #include "wstream_gemv.cuh"
 #include "wstream_chain.cuh"
 #include "argmax_exchange.cuh"
@@ -1599,6 +1600,19 @@ extern "C" int tilert_next_token_op(TbContext* ctx, const float* logits, long lo
   return next_token(ctx, SampleParams{logits, logits_stride, vocab, config_dev, seed, step_dev, 0, false, sampled, token_logprob_out,
                                       topn_logprob_out, topn_index_out, token_out, pos, advance},
                     tokens, stream);
+}
+
+extern "C" int tilert_step_inputs_op(TbContext* ctx, const long long* tokens, int n, const void* table, int vocab, int dim, const int* pos,
+                                     const float* freqs, int positions, int freq_len, void* x, float* freqs_out, void* stream) {
+  TB_NOT_CHAINABLE(ctx);
+  TB_REQUIRE(ctx != nullptr && tokens != nullptr && table != nullptr && pos != nullptr && freqs != nullptr && x != nullptr && freqs_out != nullptr);
+  TB_REQUIRE(n >= 1 && vocab >= 1 && dim >= 1 && positions >= 1 && freq_len >= 1);
+  const StepInputsParams p{tokens, reinterpret_cast<const __nv_bfloat16*>(table), vocab, dim, pos, freqs, positions, freq_len,
+                           reinterpret_cast<__nv_bfloat16*>(x), freqs_out, ctx->status};
+  TB_CUDA(launch(step_inputs_kernel, dim3(n), dim3(kStepInputThreads), 0, static_cast<cudaStream_t>(stream), p));
+  ++g_launches;
+  TB_CUDA(cudaGetLastError());
+  return TB_OK;
 }
 
 // ------------------------------------------------------------------ cache injection (FP8 wire format)

@@ -57,6 +57,10 @@ class DsaModel(SequenceDriver):
             for li in range(args.n_layers)
         ]
         self.freqs = precompute_freqs(args).to(dev)
+        self.embed = self.embed.contiguous()
+        # what a step begins with: the token's embedding, the rotary row of its position
+        self.x_in = torch.zeros(1, 1, args.dim, dtype=BF16, device=dev)
+        self.fr_in = torch.zeros(1, *self.freqs.shape[1:], dtype=F32, device=dev)
         self._init_sequence(dev, v_l, use_graph)
         self.full_logits: torch.Tensor | None = None  # world > 1 and sampling: every rank's slice, gathered
         self.temp_vars = temp_vars
@@ -104,8 +108,8 @@ class DsaModel(SequenceDriver):
                 layer.inject_cache(c0[:n], c1[:n], c2[:n], start_pos)
 
     def _step_ops(self, n_keys: int) -> None:
-        x = self.embed[self.token].view(1, 1, -1)
-        fr = self.freqs[self.cur_pos.long()]
+        x, fr = self.x_in, self.fr_in
+        ops.step_inputs(self.token, self.embed, self.cur_pos, self.freqs, x, fr)
         for layer in self.layers:
             x = layer.forward(x, self.cur_pos, fr, n_keys)
         ops.rmsnorm_head_proj(x, self.final_norm, self.head, None, self.logits, eps=self.args.eps)

@@ -72,9 +72,11 @@ class MtpDsaModel:
         self.layers = [DecoderLayer(args, main_w[li], dev, self.cache_len, s, world, comm) for li in range(args.n_layers)]
         self.mtp_layer = DecoderLayer(args, mtp_w, dev, self.cache_len, s, world, comm)
         self.freqs = precompute_freqs(args).to(dev)
+        self.embed = self.embed.contiguous()
+        self.x_in = torch.zeros(1, s, args.dim, dtype=BF16, device=dev)
+        self.fr_in = torch.zeros(s, *self.freqs.shape[1:], dtype=F32, device=dev)
         z = lambda *shape, dtype: torch.zeros(*shape, dtype=dtype, device=dev)  # noqa: E731
         self.cur_pos = z(1, dtype=I32)
-        self.rows = torch.arange(s, dtype=I64, device=dev)
         # step inputs
         self.draft = z(s, dtype=I64)
         self.extra_token = z(1, dtype=I64)      # prefill only: the prompt token after the chunk
@@ -131,10 +133,16 @@ class MtpDsaModel:
             ops.next_token(logits.view(out.numel(), -1), out)
 
     # -- the passes --
+    def _inputs(self, tokens: torch.Tensor, pos: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        """The tokens' embeddings [1, S, dim] and the rotary rows of their positions (buffers that the next pass reuses)."""
+        s = tokens.numel()
+        x, fr = self.x_in[:, :s], self.fr_in[:s]
+        ops.step_inputs(tokens, self.embed, pos, self.freqs, x, fr)
+        return x, fr
+
     def _main_pass(self, tokens: torch.Tensor, n_keys: int) -> torch.Tensor:
         s = tokens.numel()
-        x = self.embed[tokens].view(1, s, -1)
-        fr = self.freqs[self.cur_pos.long() + self.rows[:s]]
+        x, fr = self._inputs(tokens, self.cur_pos)
         for layer in self.layers:
             x = layer.forward(x, self.cur_pos, fr, n_keys)
         ops.rmsnorm_head_proj(x, self.final_norm, self.head, None, self.logits[:, :s], eps=self.args.eps)
@@ -143,7 +151,7 @@ class MtpDsaModel:
     def _mtp_pass(self, next_tokens: torch.Tensor, h: torch.Tensor, pos: torch.Tensor, n_keys: int,
                   x_in: torch.Tensor, logits_out: torch.Tensor) -> torch.Tensor:
         s = next_tokens.numel()
-        e = self.embed[next_tokens].view(1, s, -1)
+        e, fr = self._inputs(next_tokens, pos)
         if self.world > 1 and self.args.dim % self.world == 0:
             # every rank streams dim / world rows of eh_proj into its zero-padded buffer; the stand-alone all-reduce
             # assembles the vector on all ranks (adding zeros: the same bits as the unsharded product)
@@ -153,7 +161,6 @@ class MtpDsaModel:
             ops.padded_allreduce_add(part, None, 0, x_in, comm=self.comm)
         else:
             ops.mtp_preprocess(e, h, self.enorm, self.hnorm, self.w_eh, x_in, eps=self.args.eps)
-        fr = self.freqs[pos.long() + self.rows[:s]]
         x = self.mtp_layer.forward(x_in, pos, fr, n_keys)
         ops.rmsnorm_head_proj(x, self.mtp_norm, self.head, None, logits_out, eps=self.args.eps)
         return x

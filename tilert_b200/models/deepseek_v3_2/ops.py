@@ -623,3 +623,18 @@ def next_token(logits, token_out, *, pos=None, advance=0, config=None, seed=0, s
     _tb.check(_tb.lib().tilert_next_token_op(_ctx(logits), _p(logits), logits.shape[-1], rows, logits.shape[-1], _p(config), seed, _p(step),
                                              _p(sampled), _p(token_logprob), _p(topn_logprobs), _p(topn_indices), _p(token_out), _p(pos),
                                              advance, _stream()))
+
+
+def step_inputs(tokens, table, cur_pos, freqs, x, freqs_out):
+    """The embedding rows of ``tokens`` int64 [S] into ``x`` [1, S, dim] and the rotary rows of the positions from
+    ``cur_pos`` on into ``freqs_out`` [S, ...]."""
+    _need(tokens, torch.int64, "tokens")
+    _need(table, BF16, "table")
+    _need(cur_pos, I32, "cur_pos")
+    _need(freqs, F32, "freqs")
+    _need(x, BF16, "x")
+    _need(freqs_out, F32, "freqs_out")
+    if not (table.is_contiguous() and freqs.is_contiguous() and x.is_contiguous() and freqs_out.is_contiguous() and tokens.is_contiguous()):
+        raise ValueError("step_inputs: contiguous tensors are needed")
+    _tb.check(_tb.lib().tilert_step_inputs_op(_ctx(x), _p(tokens), tokens.numel(), _p(table), table.shape[0], table.shape[1], _p(cur_pos),
+                                              _p(freqs), freqs.shape[0], freqs[0].numel(), _p(x), _p(freqs_out), _stream()))
