@@ -50,6 +50,20 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
   return warp_sum(lane < nw ? red[lane] : 0.f);
 }
 
+// Two sums at once, each added up as cta_sum does; `red` holds 64 floats.
+__device__ __forceinline__ float2 cta_sum2(float a, float b, float* red) {
+  const int lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  __syncthreads();
+  if (lane == 0) {
+    red[threadIdx.x >> 5] = a;
+    red[32 + (threadIdx.x >> 5)] = b;
+  }
+  __syncthreads();
+  return make_float2(warp_sum(lane < nw ? red[lane] : 0.f), warp_sum(lane < nw ? red[32 + lane] : 0.f));
+}
+
 // The gated unit with clamped halves: g sigmoid(alpha g) (u + 1), g = min(gate, limit), u = up within +-limit.
 __device__ __forceinline__ float clamped_gate(float gate, float up, float limit, float alpha) {
   const float g = fminf(gate, limit);

@@ -530,6 +530,7 @@ extern "C" int tilert_gqa_vec_attn_op(TgContext* ctx, const float* qkv, const fl
   a.n_splits = n_splits;
   a.part = part;
   a.counter = reinterpret_cast<unsigned*>(counter);
+  a.pairs = aligned16(part);
   a.out = out;
   const dim3 grid(n_splits, head_blocks(heads, kv_heads), 1);
   const size_t smem = attn_rows_smem(a.s.dimp, a.s.vdimp);

@@ -58,10 +58,14 @@ __device__ __forceinline__ float sum_squares(const float* row, int n) {
   float s = 0.f;
   if (n % 4 == 0 && reinterpret_cast<uintptr_t>(row) % 16 == 0) {
     const float4* r4 = reinterpret_cast<const float4*>(row);
-#pragma unroll 4
-    for (int i = threadIdx.x; i < n / 4; i += blockDim.x) {
-      const float4 v = r4[i];
-      s += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+    for (int i0 = threadIdx.x; i0 < n / 4; i0 += 4 * blockDim.x) {  // four loads at once, however few there are
+      float4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * static_cast<int>(blockDim.x) < n / 4) v[j] = r4[i0 + j * blockDim.x];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * static_cast<int>(blockDim.x) < n / 4) s += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
     }
   } else {
     for (int i = threadIdx.x; i < n; i += blockDim.x) s += row[i] * row[i];
@@ -165,6 +169,7 @@ struct AttnRowsParams {
   int n_splits;
   float* part;           // [heads, rows, n_splits, vdimp] and, behind it, [heads, rows, n_splits, 2] (max, sum)
   unsigned* counter;     // [head blocks], zero between launches
+  int pairs;             // `part` lies on a boundary of 16 bytes
   void* out;             // [rows, ldo], element type float (FUSED) or T
   long long ldo;
 };
@@ -202,7 +207,7 @@ __device__ __forceinline__ void prefetch_range(const AttnRowsParams& a, int g) {
 template <typename T, bool FUSED, typename QT = T>
 __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnRowsParams a) {
   extern __shared__ __align__(16) float smem[];
-  __shared__ float red[32];
+  __shared__ float red[64];
   __shared__ float s_m[kAttnHeads], s_l[kAttnHeads], s_corr[kAttnHeads];
   __shared__ int s_last;
   pdl_launch_dependents();
@@ -226,12 +231,26 @@ __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnRowsP
   if (FUSED) {
     const int nq = s.heads * s.dim, nk = s.kv_heads * s.dim;
     const float* row = a.p.qkv;
-    const float sq = sum_squares(row, nq), sk = sum_squares(row + nq, nk);
-    const float rq = rinv_of(cta_sum(sq, red), nq, a.p.eps), rk = rinv_of(cta_sum(sk, red), nk, a.p.eps);
-    for (int i = tid; i < kAttnHeads * s.dimp; i += kAttnThreads) {
-      const int h = i / s.dimp, d = i - h * s.dimp;
-      const int e = (h0 + h) * s.dim + d;
-      qs[i] = h < nh && d < s.dim ? row[e] * rq * a.p.q_gain[e] * a.scale : 0.f;
+    // the heads' values and gains are requested before the statistics need the whole row
+    constexpr int kQ = 4;
+    float qv[kQ], qg[kQ];
+    auto query = [&](int i, float& v, float& g) {
+      const int h = i / s.dimp, d = i - h * s.dimp, e = (h0 + h) * s.dim + d;
+      const bool ok = h < nh && d < s.dim;
+      v = ok ? row[e] : 0.f;
+      g = ok ? a.p.q_gain[e] : 0.f;
+    };
+#pragma unroll
+    for (int j = 0; j < kQ; ++j)
+      if (tid + j * kAttnThreads < kAttnHeads * s.dimp) query(tid + j * kAttnThreads, qv[j], qg[j]);
+    const float2 ss = cta_sum2(sum_squares(row, nq), sum_squares(row + nq, nk), red);
+    const float rq = rinv_of(ss.x, nq, a.p.eps), rk = rinv_of(ss.y, nk, a.p.eps);
+#pragma unroll
+    for (int j = 0; j < kQ; ++j)
+      if (tid + j * kAttnThreads < kAttnHeads * s.dimp) qs[tid + j * kAttnThreads] = qv[j] * rq * qg[j] * a.scale;
+    for (int i = tid + kQ * kAttnThreads; i < kAttnHeads * s.dimp; i += kAttnThreads) {
+      query(i, qv[0], qg[0]);
+      qs[i] = qv[0] * rq * qg[0] * a.scale;
     }
     if (lo < hi && hi == pos + 1) {  // the CTAs whose range holds the current position write (the same) cache row
       const long long slot = pos % s.ring;
@@ -362,17 +381,13 @@ __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnRowsP
   if (v_active) {
 #pragma unroll
     for (int h = 0; h < kAttnHeads; ++h)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) red2[(kl * kAttnHeads + h) * s.vdimp + vp * 8 + j] = acc[h][j];
+      act_st8(red2 + (kl * kAttnHeads + h) * s.vdimp + vp * 8, acc[h]);
   }
   __syncthreads();
   const bool whole = a.n_splits == 1 && !a.parts_only;
   float* ml = a.part + static_cast<long long>(s.heads) * a.rows * a.n_splits * s.vdimp;
   auto part_of = [&](int h) { return (static_cast<long long>(h0 + h) * a.rows + t) * a.n_splits; };
-  for (int i = tid; i < nh * s.vdimp; i += kAttnThreads) {
-    const int h = i / s.vdimp, v = i - h * s.vdimp;
-    float o = 0.f;
-    for (int k = 0; k < key_lanes; ++k) o += red2[(k * kAttnHeads + h) * s.vdimp + v];
+  auto emit = [&](int h, int v, float o) {
     if (!whole) {
       a.part[(part_of(h) + split) * s.vdimp + v] = o;
     } else if (v < s.vdim) {
@@ -381,6 +396,22 @@ __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnRowsP
         reinterpret_cast<float*>(a.out)[dst] = o / s_l[h];
       else
         act_st(reinterpret_cast<T*>(a.out) + dst, o / s_l[h]);
+    }
+  };
+  for (int i = tid; i < nh * s.vdimp / 2; i += kAttnThreads) {
+    const int h = 2 * i / s.vdimp, v = 2 * i - h * s.vdimp;
+    float2 o = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < key_lanes; ++k) {
+      const float2 r = *reinterpret_cast<const float2*>(red2 + (k * kAttnHeads + h) * s.vdimp + v);
+      o.x += r.x;
+      o.y += r.y;
+    }
+    if (!whole && a.pairs) {
+      *reinterpret_cast<float2*>(a.part + (part_of(h) + split) * s.vdimp + v) = o;
+    } else {
+      emit(h, v, o.x);
+      emit(h, v + 1, o.y);
     }
   }
   if (whole) return;
@@ -400,22 +431,61 @@ __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnRowsP
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  // two values of a head a thread: the first parts are requested before their weights are known
+  constexpr int kParts = 16;
+  const bool pairs = a.pairs && s.vdim % 2 == 0;
+  const int mine = 2 * tid, my_h = pairs && mine < nh * s.vdim ? mine / s.vdim : -1, my_v = mine - my_h * s.vdim;
+  float2 got[kParts];
+  auto request = [&](int h, int v, int k0) {
+    const float* src = a.part + part_of(h) * s.vdimp + v;
+#pragma unroll
+    for (int j = 0; j < kParts; ++j)
+      if (k0 + j < a.n_splits) got[j] = __ldcg(reinterpret_cast<const float2*>(src + static_cast<long long>(k0 + j) * s.vdimp));
+  };
+  if (my_h >= 0) request(my_h, my_v, 0);
   // weight of every part, one warp per head: exp(max - overall max), and the overall sum (red2 is free again)
   float* wgt = red2;  // [kAttnHeads][n_splits]
   if (warp < nh) {
     const float* mh = ml + part_of(warp) * 2;
-    float m = -INFINITY, l = 0.f;
-    for (int k = lane; k < a.n_splits; k += 32) m = fmaxf(m, __ldcg(mh + 2 * k));
+    const float m0 = lane < a.n_splits ? __ldcg(mh + 2 * lane) : -INFINITY, l0 = lane < a.n_splits ? __ldcg(mh + 2 * lane + 1) : 0.f;
+    float m = m0, l = 0.f;
+    for (int k = lane + 32; k < a.n_splits; k += 32) m = fmaxf(m, __ldcg(mh + 2 * k));
     m = warp_max(m);
     for (int k = lane; k < a.n_splits; k += 32) {
-      const float c = expf(__ldcg(mh + 2 * k) - m);  // an empty part has max -inf: weight 0
+      const float c = expf((k < 32 ? m0 : __ldcg(mh + 2 * k)) - m);  // an empty part has max -inf: weight 0
       wgt[warp * a.n_splits + k] = c;
-      l += c * __ldcg(mh + 2 * k + 1);
+      l += c * (k < 32 ? l0 : __ldcg(mh + 2 * k + 1));
     }
     l = warp_sum(l);
     if (lane == 0) s_l[warp] = l;
   }
   __syncthreads();
+  if (pairs) {
+    for (int i = mine; i < nh * s.vdim; i += 2 * kAttnThreads) {
+      const int h = i / s.vdim, v = i - h * s.vdim;
+      const float* w = wgt + h * a.n_splits;
+      float2 o = make_float2(0.f, 0.f);
+      for (int k0 = 0; k0 < a.n_splits; k0 += kParts) {
+        if (i != mine || k0 > 0) request(h, v, k0);
+#pragma unroll
+        for (int j = 0; j < kParts; ++j)
+          if (k0 + j < a.n_splits) {
+            o.x += w[k0 + j] * got[j].x;
+            o.y += w[k0 + j] * got[j].y;
+          }
+      }
+      const long long dst = t * a.ldo + (h0 + h) * s.vdim + v;
+      const float ox = o.x / s_l[h], oy = o.y / s_l[h];
+      if (FUSED) {
+        reinterpret_cast<float*>(a.out)[dst] = ox;
+        reinterpret_cast<float*>(a.out)[dst + 1] = oy;
+      } else {
+        act_st(reinterpret_cast<T*>(a.out) + dst, ox);
+        act_st(reinterpret_cast<T*>(a.out) + dst + 1, oy);
+      }
+    }
+    return;
+  }
   for (int i = tid; i < nh * s.vdim; i += kAttnThreads) {
     const int h = i / s.vdim, v = i - h * s.vdim;
     const float* src = a.part + part_of(h) * s.vdimp + v;
