@@ -663,32 +663,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 }
 
 // ------------------------------------------------------------------ f32
-// Tiles of BF features x BT tokens, K by KB through shared memory; a thread has 4 features x RT tokens of one of KG equal
-// parts of every step of K, and the parts' sums are added in order at the end.  The next KB of both operands are in
-// registers while a step is computed, and the reads of a step are 16 bytes along K from rows an odd number of 16-byte units
-// apart (no bank conflicts).  Two shapes: 64 x 64 where such tiles fill the SMs twice, else 32 x 32 with four groups of
-// threads along K: few rows leave a walk along K bound by latency, which larger steps of more warps shorten.
-// 97 rows, 1152 features, K 1024: 19.5 us (64 x 64 tiles without a next step on its way 128); 388 x 704 x 1024: 35.5
-// (136); 200 x 2048 x 1024 on 64 x 64 tiles: 67.0 (150).
+// Tiles of BF features x BT tokens, K by KB through shared memory; a thread has 4 features x 8 tokens (gated: 4 pairs x 4) of one of
+// KG equal parts of every step of K, and the parts' sums are added pairwise at the end, by all threads.  The next KB of both operands
+// are in registers while a step is computed, and the reads of a step are 16 bytes along K from rows an odd number of 16-byte
+// units apart (no bank conflicts).  Two shapes: 64 x 64 where such tiles fill the SMs twice, else 32 x 32 with a warp or two a part
+// of K: few rows leave a walk along K bound by latency.
+// Bound by the reads from shared memory and the instructions around the multiplications: 16 bytes a lane take four cycles of the one
+// load path even where lanes share them, so 4 x 2 outputs a thread, as it was, took 24 of them for 32 multiplications of a warp, 12
+// loads for 128 take 48.  B200, 4 x 2 -> now: 97 rows, 1088 features, K 1024 17.7 -> 14.1 us; 388 rows over 16 experts, gated 704
+// features, K 1024 78.7 -> 59.3, 1024 features, K 704 53.0 -> 40.7; 200 x 2048 x 1024 on 64 x 64 tiles 65.8 -> 50.0; 64 x 4000 x 1600,
+// gated, 78.6 -> 61.8.  (Three stages by cp.async with the weights kept as bf16: as fast, gated 5 % slower for the conversions of
+// every read.  Eight tokens a thread where gated: 70 us in place of 59.)
 template <int BF, int BT, int KB, int KG, bool GATED>
 struct F32Shape {
-  static constexpr int kFt = BF / 4;                     // threads along the features
-  static constexpr int kRt = BF * BT == 1024 ? 2 : 4;    // tokens of a thread
-  static constexpr int kGroup = kFt * (BT / kRt);        // threads of a part of K
+  static constexpr int kRt = GATED ? 4 : 8;              // tokens of a thread
+  static constexpr int kFt = BF / 4, kTt = BT / kRt;     // threads along the features, along the tokens
+  static constexpr int kGroup = kFt * kTt;               // threads of a part of K
   static constexpr int kThreads = kGroup * KG;
   static constexpr int kW = GATED ? 2 : 1;
   static constexpr int kPitch = KB + 4;                  // (KB / 4 + 1) units of 16 bytes
   static constexpr int kWPieces = (BF * KB / 8 + kThreads - 1) / kThreads, kXPieces = (BT * KB / 4 + kThreads - 1) / kThreads;  // loads of a thread
-  static constexpr int kFloats = (kW * BF + BT) * kPitch;
-  static_assert((KB / 4) % 2 == 0 && KB % (4 * KG) == 0 && kThreads <= 512, "odd pitch, whole parts");
-  static_assert((KG - 1) * kW * 4 * kRt * kGroup <= kFloats, "the parts' sums fit the operands' place");
+  static constexpr int kOperands = (kW * BF + BT) * kPitch, kSums = KG / 2 * kW * BF * BT;  // floats, one in the other's place
+  static constexpr size_t kSmemBytes = sizeof(float) * (kOperands > kSums ? kOperands : kSums);
+  static_assert((KB / 4) % 2 == 0 && KB % (4 * KG) == 0 && kThreads == 512 && (KG & (KG - 1)) == 0, "odd pitch, whole parts, pairs of parts");
 };
 
 template <int BF, int BT, int KB, int KG, bool GATED>
-__global__ void __launch_bounds__(F32Shape<BF, BT, KB, KG, GATED>::kThreads) gemm_f32_kernel(const GemmRowsParams p) {
+__global__ void __launch_bounds__(F32Shape<BF, BT, KB, KG, GATED>::kThreads, 1) gemm_f32_kernel(const GemmRowsParams p) {
   using S = F32Shape<BF, BT, KB, KG, GATED>;
   constexpr int kW = S::kW, RT = S::kRt;
-  __shared__ __align__(16) float buf[S::kFloats];
+  extern __shared__ __align__(16) float buf[];
   float(*ws)[BF][S::kPitch] = reinterpret_cast<float(*)[BF][S::kPitch]>(buf);
   float(*xs)[S::kPitch] = reinterpret_cast<float(*)[S::kPitch]>(buf + kW * BF * S::kPitch);
   __shared__ int s_rows[kMaxGroups + 1], s_tiles[kMaxGroups + 1];
@@ -700,53 +704,57 @@ __global__ void __launch_bounds__(F32Shape<BF, BT, KB, KG, GATED>::kThreads) gem
   const int n_tiles = s_tiles[groups];
   TileWalk walk{s_rows, s_tiles, groups, ft, BT, BF};
   const int kg = threadIdx.x / S::kGroup, th = threadIdx.x - kg * S::kGroup;
-  const int tf = th % S::kFt, tt = th / S::kFt;  // features tf + kFt i, tokens tt + (BT / RT) i
+  const int tf = th % S::kFt, tt = th / S::kFt;  // features tf + kFt i, tokens tt + kTt i
   for (int i = blockIdx.x; i < n_tiles; i += gridDim.x) {
     const TileWalk::Tile t = walk.at(i);
+    // this thread's pieces of a step: eight along K of weight rows, four of token rows, the same place along K in all of them
+    constexpr int kWRows = S::kThreads / (KB / 8), kXRows = S::kThreads / (KB / 4);  // rows apart
+    const int wr0 = threadIdx.x / (KB / 8), wk = threadIdx.x % (KB / 8) * 8, xr0 = threadIdx.x / (KB / 4), xk = threadIdx.x % (KB / 4) * 4;
+    const __nv_bfloat16* wp = p.w + (static_cast<long long>(t.group) * kW * p.n + t.feature0 + wr0) * p.ldw + wk;
+    const float* xp = p.x + static_cast<long long>(t.row0 + xr0) * p.ldx + xk;
     uint4 wr[kW][S::kWPieces];
     float4 xr[S::kXPieces];
     auto request = [&](int k0) {
 #pragma unroll
       for (int e = 0; e < S::kWPieces; ++e) {
-        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 8), k = k0 + c % (KB / 8) * 8;
+        const bool ok = k0 + wk < p.k && wr0 + e * kWRows < min(BF, p.n - t.feature0);
 #pragma unroll
-        for (int h = 0; h < kW; ++h) {
-          const long long row = (static_cast<long long>(t.group) * kW + h) * p.n + t.feature0 + r;
-          wr[h][e] = c < BF * KB / 8 && k < p.k && t.feature0 + r < p.n ? __ldg(reinterpret_cast<const uint4*>(p.w + row * p.ldw + k)) : make_uint4(0u, 0u, 0u, 0u);
-        }
+        for (int h = 0; h < kW; ++h)
+          wr[h][e] = ok ? __ldg(reinterpret_cast<const uint4*>(wp + (static_cast<long long>(h) * p.n + e * kWRows) * p.ldw + k0)) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int e = 0; e < S::kXPieces; ++e) {
-        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 4), k = k0 + c % (KB / 4) * 4;
-        xr[e] = c < BT * KB / 4 && k < p.k && t.row0 + r < t.row1 ? *reinterpret_cast<const float4*>(p.x + static_cast<long long>(t.row0 + r) * p.ldx + k)
-                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool ok = k0 + xk < p.k && xr0 + e * kXRows < min(BT, t.row1 - t.row0);
+        xr[e] = ok ? *reinterpret_cast<const float4*>(xp + e * kXRows * p.ldx + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     };
-    auto deposit = [&](int k0) {  // what lies between k and the end of its piece is no operand
+    auto deposit = [&](int k0) {  // (a piece may reach past K)
+      const bool whole = k0 + KB <= p.k;
 #pragma unroll
       for (int e = 0; e < S::kWPieces; ++e) {
-        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 8), k = c % (KB / 8) * 8;
-        if (c >= BF * KB / 8) break;
+        if (wr0 + e * kWRows >= BF) break;
 #pragma unroll
         for (int h = 0; h < kW; ++h) {
           float f[8];
           bf16x8_to_f32(wr[h][e], f);
+          if (!whole) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (k0 + k + j >= p.k) f[j] = 0.f;
-          *reinterpret_cast<float4*>(&ws[h][r][k]) = make_float4(f[0], f[1], f[2], f[3]);
-          *reinterpret_cast<float4*>(&ws[h][r][k + 4]) = make_float4(f[4], f[5], f[6], f[7]);
+            for (int j = 0; j < 8; ++j)
+              if (k0 + wk + j >= p.k) f[j] = 0.f;
+          }
+          act_st8(&ws[h][wr0 + e * kWRows][wk], f);
         }
       }
 #pragma unroll
       for (int e = 0; e < S::kXPieces; ++e) {
-        const int c = threadIdx.x + e * S::kThreads, r = c / (KB / 4), k = c % (KB / 4) * 4;
-        if (c >= BT * KB / 4) break;
+        if (xr0 + e * kXRows >= BT) break;
         float4 v = xr[e];
-        if (k0 + k + 1 >= p.k) v.y = 0.f;
-        if (k0 + k + 2 >= p.k) v.z = 0.f;
-        if (k0 + k + 3 >= p.k) v.w = 0.f;
-        *reinterpret_cast<float4*>(&xs[r][k]) = v;
+        if (!whole) {
+          if (k0 + xk + 1 >= p.k) v.y = 0.f;
+          if (k0 + xk + 2 >= p.k) v.z = 0.f;
+          if (k0 + xk + 3 >= p.k) v.w = 0.f;
+        }
+        *reinterpret_cast<float4*>(&xs[xr0 + e * kXRows][xk]) = v;
       }
     };
     float acc[kW][4][RT];
@@ -762,11 +770,11 @@ __global__ void __launch_bounds__(F32Shape<BF, BT, KB, KG, GATED>::kThreads) gem
       deposit(k0);
       __syncthreads();
       if (k0 + KB < p.k) request(k0 + KB);
-#pragma unroll 4
+#pragma unroll
       for (int c = kg * (KB / KG); c < (kg + 1) * (KB / KG); c += 4) {
         float4 xv[RT];
 #pragma unroll
-        for (int b = 0; b < RT; ++b) xv[b] = *reinterpret_cast<const float4*>(&xs[tt + BT / RT * b][c]);
+        for (int b = 0; b < RT; ++b) xv[b] = *reinterpret_cast<const float4*>(&xs[tt + S::kTt * b][c]);
 #pragma unroll
         for (int h = 0; h < kW; ++h)
 #pragma unroll
@@ -782,37 +790,55 @@ __global__ void __launch_bounds__(F32Shape<BF, BT, KB, KG, GATED>::kThreads) gem
           }
       }
     }
-    if (KG > 1) {
-      __syncthreads();  // the last step has been read
+    // the parts' sums, half of the parts at a time into shared memory and onto the other half's
+    float4* sums = reinterpret_cast<float4*>(buf);
 #pragma unroll
-      for (int h = 0; h < kW; ++h)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < RT; ++b)
-            if (kg > 0) buf[(((kg - 1) * kW + h) * 4 * RT + a * RT + b) * S::kGroup + th] = acc[h][a][b];
-      __syncthreads();
-      if (kg > 0) continue;  // (the next tile's first step waits for the threads that read)
-#pragma unroll
-      for (int g = 0; g < KG - 1; ++g)
+    for (int half = KG / 2; half > 0; half /= 2) {
+      __syncthreads();  // the last step, or the sums of the round before, have been read
+      if (kg >= half && kg < 2 * half) {
 #pragma unroll
         for (int h = 0; h < kW; ++h)
 #pragma unroll
           for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int b = 0; b < RT; ++b) acc[h][a][b] += buf[((g * kW + h) * 4 * RT + a * RT + b) * S::kGroup + th];
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < RT; ++b) {
-        const int f = t.feature0 + tf + S::kFt * a, r = t.row0 + tt + BT / RT * b;
-        if (f < p.n && r < t.row1) {
-          const float v = GATED ? clamped_gate(acc[0][a][b], acc[kW - 1][a][b], p.limit, p.alpha)
-                                : acc[0][a][b] + (p.bias != nullptr ? p.bias[f] : 0.f);
-          reinterpret_cast<float*>(p.out)[static_cast<long long>(r) * p.ldo + f] = v;
-        }
+            for (int b = 0; b < RT; b += 4)
+              sums[((((kg - half) * kW + h) * 4 + a) * (RT / 4) + b / 4) * S::kGroup + th] =
+                  make_float4(acc[h][a][b], acc[h][a][b + 1], acc[h][a][b + 2], acc[h][a][b + 3]);
       }
+      __syncthreads();
+      if (kg < half) {
+#pragma unroll
+        for (int h = 0; h < kW; ++h)
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < RT; b += 4) {
+              const float4 v = sums[(((kg * kW + h) * 4 + a) * (RT / 4) + b / 4) * S::kGroup + th];
+              acc[h][a][b] += v.x;
+              acc[h][a][b + 1] += v.y;
+              acc[h][a][b + 2] += v.z;
+              acc[h][a][b + 3] += v.w;
+            }
+      }
+    }
+    // the first part's threads have them now: out through shared memory, by all
+    __syncthreads();
+    if (kg == 0) {
+#pragma unroll
+      for (int h = 0; h < kW; ++h)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < RT; ++b) buf[(h * BT + tt + S::kTt * b) * BF + tf + S::kFt * a] = acc[h][a][b];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < BF * BT; e += S::kThreads) {
+      const int r = e / BF, f = e - r * BF;
+      if (t.feature0 + f >= p.n || t.row0 + r >= t.row1) continue;
+      const float v = buf[e];
+      reinterpret_cast<float*>(p.out)[static_cast<long long>(t.row0 + r) * p.ldo + t.feature0 + f] =
+          GATED ? clamped_gate(v, buf[(kW - 1) * BF * BT + e], p.limit, p.alpha) : v + (p.bias != nullptr ? p.bias[t.feature0 + f] : 0.f);
+    }
   }
 }
 

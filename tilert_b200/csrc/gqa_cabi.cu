@@ -144,7 +144,8 @@ int launch_tc(TgContext* ctx, const GemmRowsParams& p, long long w_rows, void* s
 
 template <int BF, int BT, int KB, int KG, bool GATED>
 int launch_f32(TgContext* ctx, const GemmRowsParams& p, void* stream) {
-  return go(gemm_f32_kernel<BF, BT, KB, KG, GATED>, dim3(ctx->num_sms * 4), dim3(F32Shape<BF, BT, KB, KG, GATED>::kThreads), 0, stream, p);
+  using S = F32Shape<BF, BT, KB, KG, GATED>;
+  return go(gemm_f32_kernel<BF, BT, KB, KG, GATED>, dim3(ctx->num_sms), dim3(S::kThreads), S::kSmemBytes, stream, p);
 }
 
 template <bool GATED>
@@ -312,8 +313,8 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     // rows per group as the host knows them: an average where the counts are on the device
     const int each = n_groups > 0 && counts != nullptr ? (rows + n_groups - 1) / n_groups : rows;
     const long long large = static_cast<long long>(n_groups > 0 ? n_groups : 1) * ((n + 63) / 64) * ((each + 63) / 64);
-    if (large >= 2 * ctx->num_sms && each >= 48) return gated ? launch_f32<64, 64, 32, 1, true>(ctx, p, stream) : launch_f32<64, 64, 32, 1, false>(ctx, p, stream);
-    return gated ? launch_f32<32, 32, 64, 4, true>(ctx, p, stream) : launch_f32<32, 32, 128, 4, false>(ctx, p, stream);
+    if (large >= 2 * ctx->num_sms && each >= 48) return gated ? launch_f32<64, 64, 64, 2, true>(ctx, p, stream) : launch_f32<64, 64, 64, 4, false>(ctx, p, stream);
+    return gated ? launch_f32<32, 32, 128, 8, true>(ctx, p, stream) : launch_f32<32, 32, 128, 16, false>(ctx, p, stream);
   }
   const long long w_rows = static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n;
   // One SM (128 or 64 features x 64 token rows) or a pair (256 x up to 256) on a tile: what takes the fewest rounds over the
