@@ -153,8 +153,10 @@ LatentLayer = _cabi.parse_struct("TgLatentLayer", _HEADER)
 
 
 def structure(kind: type[ctypes.Structure], **fields) -> ctypes.Structure:
-    """A structure with tensors as their addresses (None: null)."""
-    return kind(**{n: v.data_ptr() if isinstance(v, torch.Tensor) else v for n, v in fields.items() if v is not None})
+    """A structure with tensors as their addresses (None: null); it keeps them alive."""
+    made = kind(**{n: v.data_ptr() if isinstance(v, torch.Tensor) else v for n, v in fields.items() if v is not None})
+    made.tensors = [v for v in fields.values() if isinstance(v, torch.Tensor)]
+    return made
 
 
 def routed_layer(layer, rows: int, pos, x, xh) -> None:
