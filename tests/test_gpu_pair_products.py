@@ -79,6 +79,13 @@ def test_one_weight(ops, rows, n, k, gated, out_type):
 
 
 @pytest.mark.parametrize("out_type", [BF16, F32])
+@pytest.mark.parametrize("rows,n,k", [  # tiles of 64 features: 32 rows (the last two: 64), stages of four blocks of K, the last one short
+    (1, 7, 8), (31, 65, 64), (32, 64, 256), (33, 200, 264), (97, 130, 448), (37, 2048, 1032), (300, 64, 3000), (150, 2048, 200), (173, 3000, 330)])
+def test_small_tiles(ops, rows, n, k, out_type):
+    check(ops, n, k, False, out_type, None, rows)
+
+
+@pytest.mark.parametrize("out_type", [BF16, F32])
 @pytest.mark.parametrize("gated", [False, True])
 def test_forms_have_the_same_bits(ops, gated, out_type):
     """A row's result does not depend on the tile it is in (64 or 128 features on one SM, 256 on a pair with 64 to 256 rows, one or

@@ -1,6 +1,6 @@
 // Products of many token rows with bf16 weights (prefill):  out[t, n] = W[n, :] . x[t, :].
 //
-//   gemm_tc_kernel<BM, GATED>   bf16 rows on the tensor cores, an SM on a tile: few tokens, small groups
+//   gemm_tc_kernel<BM, BN, GATED>   bf16 rows on the tensor cores, an SM on a tile: few tokens, small groups
 //   gemm_pair_kernel<GATED>     the same, a pair of SMs on a tile
 //   gemm_f32_kernel<.., GATED>  f32 rows, f32 arithmetic (the exact mode)
 //
@@ -9,7 +9,7 @@
 // group is device data, so the tiles are enumerated on the device and the grid is the SM count.
 //
 // Tensor-core kernel: persistent, warp-specialised, one CTA per SM.  The 128 or 64 weight rows of a tile are M (so a TMEM
-// lane is an output feature and a store covers consecutive features), 64 token rows are N; K goes by 128.  One thread
+// lane is an output feature and a store covers consecutive features), 64 or 32 token rows are N.  One thread
 // issues the TMA loads (128-byte swizzle) into a ring of stages, one thread issues the tcgen05.mma, eight warps read
 // the accumulators back; two accumulators alternate so that the epilogue of a tile overlaps the products of the next.
 #pragma once
@@ -116,21 +116,22 @@ constexpr int kTcEpiWarps = 8;  // two per quarter of the TMEM lanes, each with 
 constexpr int kTcThreads = 64 + 32 * kTcEpiWarps;  // and a producer warp, an MMA warp
 constexpr int kTcK = 64;
 
-// BM features x 64 token rows.  Few tiles leave most SMs idle and a step along K bound by one SM's loads and by the
-// hand-shakes of a stage: 64 features spread the weights over twice the SMs.  37 rows, 2048 features, K 5632: 16.0 us in tiles
-// of 64 features, 18.3 of 128, 24.0 with stages of 64 along K; 173 x 2048 x 2048 8.5, 9.1, 10.9.
-// A stage is two blocks of 64 along K, since its hand-shakes cost as much as a block's products; one where two would leave two
-// stages.
-template <int BM, bool GATED>
+// BM features x BN token rows.  Few tiles leave most SMs idle, and a tile's time is that of its steps along K.  A step is bound by
+// shared memory: 64 x 64 x 16 is 32 cycles of the tensor core, in which it reads 4 KB, as much as that memory gives, and what the
+// copies write comes on top; and waiting for a stage and releasing it takes 120 to 170 cycles in which no product is issued.
+// So tiles are small where there are few, and a stage is four blocks of 64 along K, two or one where fewer than three stages would
+// fit.  B200, stages of two blocks -> of four -> and tiles of 32 rows: 37 rows, 2048 features, K 5632 16.4 -> 14.1 -> 11.8 us; K 2048
+// 8.3 -> 7.4 -> 6.4; 2048 rows, 64 features, K 4096 12.5 -> 10.3 -> 8.9; 173 x 3072 x 2048, which keeps tiles of 64 rows, 8.7 -> 7.9.
+// Three blocks: 14.4 and 12.9 us at the first of these.
+template <int BM, int BN, bool GATED>
 struct TcShape {
-  static constexpr int kBN = 64;
-  static constexpr int kBlocks = GATED && BM == 128 ? 1 : 2;
+  static constexpr int kBlocks = GATED ? 128 / BM : (BM == 64 ? 4 : 2);
   static constexpr int kWBytes = BM * kTcK * 2;
-  static constexpr int kXBytes = kBN * kTcK * 2;
+  static constexpr int kXBytes = BN * kTcK * 2;
   static constexpr int kBlockBytes = (GATED ? 2 : 1) * kWBytes + kXBytes;
   static constexpr int kStageBytes = kBlocks * kBlockBytes;
   static constexpr int kStages = 196608 / kStageBytes < 8 ? 196608 / kStageBytes : 8;
-  static constexpr int kAccCols = GATED ? 2 * kBN : kBN;
+  static constexpr int kAccCols = GATED ? 2 * BN : BN;
   static constexpr int kTmemCols = 2 * kAccCols;
   static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM allocation size");
   static constexpr size_t kSmemBytes = static_cast<size_t>(kStages) * kStageBytes + 1024;  // + alignment of the ring
@@ -236,11 +237,10 @@ __device__ __forceinline__ void store_eight(const GemmRowsParams& p, StoreForm h
   }
 }
 
-template <int BM, bool GATED>
+template <int BM, int BN, bool GATED>
 __global__ void __launch_bounds__(kTcThreads, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const GemmRowsParams p) {
-  using S = TcShape<BM, GATED>;
-  constexpr int BN = S::kBN;
+  using S = TcShape<BM, BN, GATED>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[S::kStages], empty[S::kStages], acc_full[2], acc_empty[2], drain;
   __shared__ uint32_t s_tmem;
@@ -277,18 +277,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   tile_prefix(p, BN, ft, s_rows, s_tiles);
   const int groups = p.n_groups > 0 ? p.n_groups : 1;
   const int n_tiles = warp_uniform(s_tiles[groups]);
-  const int n_kb = (p.k + kTcK * S::kBlocks - 1) / (kTcK * S::kBlocks);  // (what lies beyond K is zero)
+  const int n_blocks = (p.k + kTcK - 1) / kTcK;  // (what lies beyond K in the last one is zero)
   volatile int* abort = &s_abort;
   TileWalk walk{s_rows, s_tiles, groups, ft, BN, BM};
 
   if (warp == 0) {
-    uint32_t it = 0;
+    uint32_t it = 0, s = 0, ph = 0;
     bool ok = true;
     for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x) {
       const TileWalk::Tile t = walk.at_warp(i);
       const int wrow = t.group * (GATED ? 2 : 1) * p.n + t.feature0;
-      for (int kb = 0; kb < n_kb; ++kb, ++it) {
-        const uint32_t s = it % S::kStages, ph = (it / S::kStages) & 1u;
+      for (int kb = 0; kb < n_blocks; kb += S::kBlocks, ++it) {
         if (!mbar_wait_warp(&empty[s], ph ^ 1u, abort)) {
           set_status(p.status, ST_WAIT_EMPTY_TIMEOUT);
           ok = false;
@@ -296,15 +295,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         uint8_t* st = ring + s * S::kStageBytes;
         if (elect_one()) {
-          mbar_expect_tx(&full[s], S::kStageBytes);
+          const int blocks = min(S::kBlocks, n_blocks - kb);
+          mbar_expect_tx(&full[s], blocks * S::kBlockBytes);
 #pragma unroll
           for (int b = 0; b < S::kBlocks; ++b, st += S::kBlockBytes) {
-            const int k0 = (kb * S::kBlocks + b) * kTcK;
+            if (b >= blocks) break;
+            const int k0 = (kb + b) * kTcK;
             tma_load_2d(st, &wmap, k0, wrow, &full[s]);
             if (GATED) tma_load_2d(st + S::kWBytes, &wmap, k0, wrow + p.n, &full[s]);
             tma_load_2d(st + (GATED ? 2 : 1) * S::kWBytes, &xmap, k0, t.row0, &full[s]);
           }
         }
+        if (++s == S::kStages) s = 0, ph ^= 1u;
       }
     }
     if (!ok) *abort = 1;
@@ -312,7 +314,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     for (uint32_t j = it > S::kStages ? it - S::kStages : 0; j < it; ++j) mbar_wait(&full[j % S::kStages], (j / S::kStages) & 1u);
   } else if (warp == 1) {
     constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
-    uint32_t it = 0, n_done = 0;
+    const uint32_t base0 = smem_u32(ring);
+    uint32_t s = 0, ph = 0, base = base0, n_done = 0;
     bool ok = true, seen = false;
     for (int i = blockIdx.x; ok && i < n_tiles; i += gridDim.x, ++n_done) {
       const uint32_t buf = n_done & 1u, aph = (n_done >> 1) & 1u;
@@ -323,29 +326,33 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       tc_fence_after();
       const uint32_t d = tmem + buf * S::kAccCols;
-      for (int kb = 0; kb < n_kb; ++kb, ++it) {
-        const uint32_t s = it % S::kStages, ph = (it / S::kStages) & 1u;
+      for (int kb = 0; kb < n_blocks; kb += S::kBlocks) {
         if (!mbar_wait_warp(&full[s], ph, abort, seen)) {
           set_status(p.status, ST_WAIT_FULL_TIMEOUT);
           ok = false;
           break;
         }
-        seen = mbar_test(&full[(it + 1) % S::kStages], ((it + 1) / S::kStages) & 1u);  // (known by the time it is asked for)
-        const uint32_t base = smem_u32(ring + s * S::kStageBytes);
+        uint64_t* const done = &empty[s];
+        if (++s == S::kStages) s = 0, ph ^= 1u;
+        seen = mbar_test(&full[s], ph);  // (known by the time it is asked for)
+        const int blocks = n_blocks - kb;
         const uint64_t wd = umma_desc_sw128(base), ud = umma_desc_sw128(base + S::kWBytes);
         const uint64_t xd = umma_desc_sw128(base + (GATED ? 2 : 1) * S::kWBytes);
         if (elect_one()) {
 #pragma unroll
-          for (int b = 0; b < S::kBlocks; ++b)
+          for (int b = 0; b < S::kBlocks; ++b) {
+            if (b >= blocks) break;
 #pragma unroll
             for (int q = 0; q < kTcK / 16; ++q) {  // 32 bytes along K per instruction
               const uint32_t off = (b * S::kBlockBytes + q * 32) >> 4;
               umma_bf16(d, wd + off, xd + off, idesc, (kb | b | q) != 0);
               if (GATED) umma_bf16(d + BN, ud + off, xd + off, idesc, (kb | b | q) != 0);
             }
-          umma_commit(&empty[s]);
-          if (kb == n_kb - 1) umma_commit(&acc_full[buf]);
+          }
+          umma_commit(done);
+          if (blocks <= S::kBlocks) umma_commit(&acc_full[buf]);
         }
+        base = s == 0 ? base0 : base + S::kStageBytes;
       }
     }
     if (!ok) *abort = 1;

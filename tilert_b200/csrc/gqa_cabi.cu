@@ -132,14 +132,14 @@ int launch_pair(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int b
   return go(gemm_pair_kernel<GATED>, dim3(ctx->num_sms / 2 * 2), dim3(kTcThreads), static_cast<size_t>(q.stages) * q.stage_bytes + 1024, stream, wmap, xmap, shortmap, p, q);
 }
 
-template <int BM, bool GATED>
+template <int BM, int BN, bool GATED>
 int launch_tc(TgContext* ctx, const GemmRowsParams& p, long long w_rows, void* stream) {
   CUtensorMap wmap, xmap;
   int rc = make_map(&wmap, p.w, w_rows, p.k, p.ldw, BM);
   const long long x_rows = p.n_groups > 0 && p.counts == nullptr ? static_cast<long long>(p.n_groups) * p.rows : p.rows;
-  if (rc == TB_OK) rc = make_map(&xmap, p.x, x_rows, p.k, p.ldx, TcShape<BM, GATED>::kBN);
+  if (rc == TB_OK) rc = make_map(&xmap, p.x, x_rows, p.k, p.ldx, BN);
   if (rc != TB_OK) return rc;
-  return go(gemm_tc_kernel<BM, GATED>, dim3(ctx->num_sms), dim3(kTcThreads), TcShape<BM, GATED>::kSmemBytes, stream, wmap, xmap, p);
+  return go(gemm_tc_kernel<BM, BN, GATED>, dim3(ctx->num_sms), dim3(kTcThreads), TcShape<BM, BN, GATED>::kSmemBytes, stream, wmap, xmap, p);
 }
 
 template <int BF, int BT, int KB, int KG, bool GATED>
@@ -149,8 +149,9 @@ int launch_f32(TgContext* ctx, const GemmRowsParams& p, void* stream) {
 }
 
 template <bool GATED>
-int launch_single(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int bm, void* stream) {
-  return bm == 64 ? launch_tc<64, GATED>(ctx, p, w_rows, stream) : launch_tc<128, GATED>(ctx, p, w_rows, stream);
+int launch_single(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int bm, int bn, void* stream) {
+  if (bm == 128) return launch_tc<128, 64, GATED>(ctx, p, w_rows, stream);
+  return bn == 32 ? launch_tc<64, 32, GATED>(ctx, p, w_rows, stream) : launch_tc<64, 64, GATED>(ctx, p, w_rows, stream);
 }
 
 QkvShape qkv_shape(int heads, int kv_heads, int dim, int vdim, int ring, int window) {
@@ -317,10 +318,11 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     return gated ? launch_f32<32, 32, 128, 8, true>(ctx, p, stream) : launch_f32<32, 32, 128, 16, false>(ctx, p, stream);
   }
   const long long w_rows = static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n;
-  // One SM (128 or 64 features x 64 token rows) or a pair (256 x up to 256) on a tile: what takes the fewest rounds over the
-  // SMs, a round being the steps along K of a tile.  The microseconds of a step of 64 are measured ones (2048 x 6208 x 4096,
-  // 1357 x 7168 x 18432, gated 1357 x 18432 x 7168 and others at every tile size, 37 and 173 x 2048 x 2048 to 5632 on single
-  // SMs).
+  // One SM (128 features x 64 token rows, 64 x 64 or 64 x 32) or a pair (256 x up to 256) on a tile: what takes the fewest rounds
+  // over the SMs, a round being the steps along K of a tile.  The microseconds of a step of 64 are measured ones (2048 x 6208 x
+  // 4096, 1357 x 7168 x 18432, gated 1357 x 18432 x 7168 and others at every tile size, 37 and 173 x 2048 x 2048 to 5632 on
+  // single SMs).  37 x 2048 x 5632: 11.8 us in tiles of 64 x 32, 14.1, 19.5 of 128 x 64, 19.1 in pairs; 150 x 2048 x 1000: 7.6, 7.2,
+  // 7.9, 8.2; 64 x 16000 x 4096: 33.3, 28.7, 26.3, 27.4.
   const int n_kb = (p.k + kTcK - 1) / kTcK, wide = n_groups > 0 ? n_groups : 1;
   auto tiles = [&](int feats, int bn) { return static_cast<long long>(wide) * ((n + feats - 1) / feats) * ((rows + bn - 1) / bn); };
   auto round_up = [](long long tiles, int units) { return static_cast<double>((tiles + units - 1) / units); };
@@ -329,11 +331,12 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     // which a group may need a second that it does not fill.  Below 64 rows a group it is the weights'
     // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 114 us, in pairs 141; 75 rows
     // 97 in pairs, was 120; 156 rows 303, 256 rows 440; gated, 1000 to 1536 features), in small tiles if the groups that
-    // there can be are few (16 rows over 30 experts 16.0 us, in tiles of 128 features 19.5).
+    // there can be are few (16 rows over 30 experts 16.0 us, in tiles of 128 features 19.5), of 32 rows where those hold a group (97
+    // rows over 4, gated, 700 x 1024 13.9 -> 10.5 us; 16 over 16, gated, 500 x 1500 16.7 -> 14.4).
     const int each = rows / n_groups, bn = (each * 6 / 5 + 31) / 32 * 32;
     if (each < 64) {
       const int bm = static_cast<long long>(rows < n_groups ? rows : n_groups) * ((n + 127) / 128) <= ctx->num_sms ? 64 : 128;
-      return gated ? launch_single<true>(ctx, p, w_rows, bm, stream) : launch_single<false>(ctx, p, w_rows, bm, stream);
+      return gated ? launch_single<true>(ctx, p, w_rows, bm, bn, stream) : launch_single<false>(ctx, p, w_rows, bm, bn, stream);
     }
     return gated ? launch_pair<true>(ctx, p, w_rows, bn < 256 ? bn : 256, stream) : launch_pair<false>(ctx, p, w_rows, bn < 256 ? bn : 256, stream);
   }
@@ -345,9 +348,10 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     if (c < pair) pair = c, bn = 64 + 32 * i;
   }
   if (gated) return launch_pair<true>(ctx, p, w_rows, bn, stream);
-  const double large = round_up(tiles(128, 64), ctx->num_sms) * n_kb * 0.17, small = round_up(tiles(64, 64), ctx->num_sms) * n_kb * 0.145;
-  if (large > pair && small > pair) return launch_pair<false>(ctx, p, w_rows, bn, stream);
-  return launch_single<false>(ctx, p, w_rows, small <= large ? 64 : 128, stream);
+  const double large = round_up(tiles(128, 64), ctx->num_sms) * n_kb * 0.17, mid = round_up(tiles(64, 64), ctx->num_sms) * n_kb * 0.12,
+               small = round_up(tiles(64, 32), ctx->num_sms) * n_kb * 0.096;
+  if (pair < large && pair < mid && pair < small) return launch_pair<false>(ctx, p, w_rows, bn, stream);
+  return launch_single<false>(ctx, p, w_rows, large < mid && large < small ? 128 : 64, small <= mid ? 32 : 64, stream);
 }
 
 // ------------------------------------------------------------------------------- attention of a portion
