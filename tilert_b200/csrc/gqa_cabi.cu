@@ -596,10 +596,9 @@ template <int MT>
 int launch_latent(const LatentAttnParams& p, void* stream) {
   const dim3 grid(p.n_splits, (p.n_rows + 16 * MT - 1) / (16 * MT));
   const size_t smem = latent_attn_smem(MT, p.r.row);
-  if (p.r.rankp <= 128) return go(latent_attn_kernel<MT, 1>, grid, dim3(kLaThreads), smem, stream, p);
-  if (p.r.rankp <= 256) return go(latent_attn_kernel<MT, 2>, grid, dim3(kLaThreads), smem, stream, p);
-  if (p.r.rankp <= 512) return go(latent_attn_kernel<MT, 4>, grid, dim3(kLaThreads), smem, stream, p);
-  return go(latent_attn_kernel<MT, 8>, grid, dim3(kLaThreads), smem, stream, p);
+  if (p.r.rankp <= 256) return go(latent_attn_kernel<MT, 1>, grid, dim3(kLaThreads), smem, stream, p);
+  if (p.r.rankp <= 512) return go(latent_attn_kernel<MT, 2>, grid, dim3(kLaThreads), smem, stream, p);
+  return go(latent_attn_kernel<MT, 4>, grid, dim3(kLaThreads), smem, stream, p);
 }
 
 }  // namespace

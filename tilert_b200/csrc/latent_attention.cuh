@@ -5,6 +5,11 @@
 // CTA, the key range split over CTAs.  Every part leaves its unnormalised sum, its largest score and its sum of
 // exponentials; who reads them merges (latent_merge_kernel, or the staging of the value product of a one-token step).
 // Key tiles are copied two deep by cp.async; a tile is read twice, as keys and (its first rankp columns) as values.
+//
+// Sixteen warps sum the values, eight of them score, each in two chains of products.  Bound by latency at one token and, with 32
+// rows, by mma.sync (1088 a tile of 576 columns) and the barriers between its phases.  Eight warps for both, one chain -> now:
+// 37 tokens x 16 heads, 4037 keys of 512 + 64, seven parts 43.8 -> 42.4 us; 100 x 8, 1000 of 256 + 64 20.2 -> 14.9; one token, 32 heads,
+// 6000 keys 10.0 -> 9.1.  Sixteen warps that score eight keys each read the queries twice as often: 48 us at the first.
 #pragma once
 
 #include "act.cuh"
@@ -14,7 +19,8 @@
 
 namespace tb {
 
-constexpr int kLaThreads = 256, kLaWarps = 8, kLaKeys = 64;
+constexpr int kLaThreads = 512, kLaWarps = 16, kLaKeys = 64;
+constexpr int kLaGroups = 8;  // warps that score
 
 struct LatentAttnParams {
   LatentRow r;
@@ -30,16 +36,16 @@ struct LatentAttnParams {
 
 __host__ __device__ inline size_t latent_attn_smem(int mt, int row) {
   return static_cast<size_t>(16 * mt + 2 * kLaKeys) * (row + 8) * 2 + static_cast<size_t>(16 * mt) * (kLaKeys + 8) * 2 +
-         sizeof(float) * (2 + 1) * kLaWarps * 16 * mt;
+         sizeof(float) * (2 + 1) * kLaGroups * 16 * mt;
 }
 
-// MT: tiles of 16 query rows; NV: blocks of 16 value columns per warp (rankp <= 128 * NV)
+// MT: tiles of 16 query rows; NV: blocks of 16 value columns per warp (rankp <= 256 * NV)
 template <int MT, int NV>
 __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const LatentAttnParams a) {
   extern __shared__ __align__(16) __nv_bfloat16 lsm[];
   constexpr int M = 16 * MT;
-  constexpr int KG = kLaWarps / MT;      // warps side by side over the keys of a tile
-  constexpr int KW = kLaKeys / KG;       // keys per warp: 8 or 16
+  constexpr int KG = kLaGroups / MT;     // warps side by side over the keys of a tile
+  constexpr int KW = kLaKeys / KG;       // keys of each: 8 or 16
   constexpr int PP = kLaKeys + 8;
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -48,7 +54,7 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
   __nv_bfloat16* ks = qs + M * kp;                  // [2][kLaKeys][kp]
   __nv_bfloat16* ps = ks + 2 * kLaKeys * kp;        // [M][PP]
   float* s_mx = reinterpret_cast<float*>(ps + M * PP);  // [2][KG][M]
-  float* s_l = s_mx + 2 * kLaWarps * M;             // [KG][M]
+  float* s_l = s_mx + 2 * KG * M;                   // [KG][M]
   pdl_wait();
   const int pos0 = *a.pos;
   const int r0 = blockIdx.y * M, r1 = min(r0 + M, a.n_rows);
@@ -93,6 +99,7 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
   }
 
   const int mt = warp % MT, kg = warp / MT;          // scores: this warp's rows and keys
+  const bool scores = kg < KG;                       // (half of the warps; all sum values)
   const int srow = mt * 16 + (lane >> 2);            // and + 8
   int qpos[2];
 #pragma unroll
@@ -119,41 +126,44 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
     __syncthreads();  // this tile is here, and the other buffer, ps and s_mx[buf] are free
     if (k0 + kLaKeys < hi) load_keys(buf ^ 1, k0 + kLaKeys);
     const __nv_bfloat16* kt = ks + buf * kLaKeys * kp;
+    float* mxs = s_mx + buf * KG * M;
     float s[KW / 8][4];
+    if (scores) {
+      float s2[KW / 8][4];  // every other sixteen columns: two chains of products
 #pragma unroll
-    for (int i = 0; i < KW / 8; ++i)
+      for (int i = 0; i < KW / 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 2
-    for (int kk = 0; kk < row; kk += 32) {
-      uint32_t qa[2][4];
-      ldmatrix_x4(qa[0], qs + (mt * 16 + (lane & 15)) * kp + kk + (lane >> 4) * 8);
-      ldmatrix_x4(qa[1], qs + (mt * 16 + (lane & 15)) * kp + kk + 16 + (lane >> 4) * 8);
+        for (int j = 0; j < 4; ++j) s[i][j] = s2[i][j] = 0.f;
+#pragma unroll 3
+      for (int kk = 0; kk < row; kk += 32) {
+        uint32_t qa[2][4];
+        ldmatrix_x4(qa[0], qs + (mt * 16 + (lane & 15)) * kp + kk + (lane >> 4) * 8);
+        ldmatrix_x4(qa[1], qs + (mt * 16 + (lane & 15)) * kp + kk + 16 + (lane >> 4) * 8);
 #pragma unroll
-      for (int i = 0; i < KW / 8; ++i) {
-        uint32_t kb[4];  // eight keys, four pieces of eight along the row
-        ldmatrix_x4(kb, kt + (kg * KW + i * 8 + (lane & 7)) * kp + kk + (lane >> 3) * 8);
-        const uint32_t b0[2] = {kb[0], kb[1]}, b1[2] = {kb[2], kb[3]};
-        mma_bf16_16816(s[i], qa[0], b0);
-        mma_bf16_16816(s[i], qa[1], b1);
+        for (int i = 0; i < KW / 8; ++i) {
+          uint32_t kb[4];  // eight keys, four pieces of eight along the row
+          ldmatrix_x4(kb, kt + (kg * KW + i * 8 + (lane & 7)) * kp + kk + (lane >> 3) * 8);
+          const uint32_t b0[2] = {kb[0], kb[1]}, b1[2] = {kb[2], kb[3]};
+          mma_bf16_16816(s[i], qa[0], b0);
+          mma_bf16_16816(s2[i], qa[1], b1);
+        }
       }
-    }
-    float mx[2] = {-INFINITY, -INFINITY};
+      float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-    for (int i = 0; i < KW / 8; ++i)
+      for (int i = 0; i < KW / 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int kpos = k0 + kg * KW + i * 8 + (lane & 3) * 2 + (j & 1), q = j >> 1;
-        const bool ok = kpos < hi && kpos <= qpos[q] && qpos[q] - kpos < win;
-        s[i][j] = ok ? s[i][j] * a.scale : -INFINITY;
-        mx[q] = fmaxf(mx[q], s[i][j]);
+        for (int j = 0; j < 4; ++j) {
+          const int kpos = k0 + kg * KW + i * 8 + (lane & 3) * 2 + (j & 1), q = j >> 1;
+          const bool ok = kpos < hi && kpos <= qpos[q] && qpos[q] - kpos < win;
+          s[i][j] = ok ? (s[i][j] + s2[i][j]) * a.scale : -INFINITY;
+          mx[q] = fmaxf(mx[q], s[i][j]);
+        }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 1));
+        mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 2));
+        if ((lane & 3) == 0) mxs[kg * M + srow + 8 * q] = mx[q];
       }
-    float* mxs = s_mx + buf * kLaWarps * M;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 1));
-      mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 2));
-      if ((lane & 3) == 0) mxs[kg * M + srow + 8 * q] = mx[q];
     }
     __syncthreads();
     float corr[MT][2], msafe[MT][2];
@@ -168,15 +178,17 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
         corr[i][q] = __expf(m_run[i][q] - msafe[i][q]);
         m_run[i][q] = m;
       }
+    if (scores) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const float ms = MT == 1 || mt == 0 ? msafe[0][q] : msafe[MT - 1][q];
-      l_run[q] *= MT == 1 || mt == 0 ? corr[0][q] : corr[MT - 1][q];
+      for (int q = 0; q < 2; ++q) {
+        const float ms = MT == 1 || mt == 0 ? msafe[0][q] : msafe[MT - 1][q];
+        l_run[q] *= MT == 1 || mt == 0 ? corr[0][q] : corr[MT - 1][q];
 #pragma unroll
-      for (int i = 0; i < KW / 8; ++i) {
-        const float e0 = __expf(s[i][2 * q] - ms), e1 = __expf(s[i][2 * q + 1] - ms);
-        l_run[q] += e0 + e1;
-        *reinterpret_cast<uint32_t*>(ps + (srow + 8 * q) * PP + kg * KW + i * 8 + (lane & 3) * 2) = pack_bf16x2(e0, e1);
+        for (int i = 0; i < KW / 8; ++i) {
+          const float e0 = __expf(s[i][2 * q] - ms), e1 = __expf(s[i][2 * q + 1] - ms);
+          l_run[q] += e0 + e1;
+          *reinterpret_cast<uint32_t*>(ps + (srow + 8 * q) * PP + kg * KW + i * 8 + (lane & 3) * 2) = pack_bf16x2(e0, e1);
+        }
       }
     }
 #pragma unroll
@@ -227,7 +239,7 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
   for (int q = 0; q < 2; ++q) {
     l_run[q] += __shfl_xor_sync(0xffffffffu, l_run[q], 1);
     l_run[q] += __shfl_xor_sync(0xffffffffu, l_run[q], 2);
-    if ((lane & 3) == 0) s_l[kg * M + srow + 8 * q] = l_run[q];
+    if (scores && (lane & 3) == 0) s_l[kg * M + srow + 8 * q] = l_run[q];
   }
   __syncthreads();
   // a warp's m_run covers every row; warp 0 writes the rows' maxima and sums
