@@ -320,6 +320,10 @@ __global__ void __launch_bounds__(kGemvBf16Threads, 1) gemv_bf16_kernel(const Ge
 
 // Variant for few rows (router gate, indexer head weights): one CTA per pair of rows, the warps
 // split K, so the dependent load chain is K / (8 warps * 256) iterations instead of K / 256.
+// Latency: a few round trips to L2 and what four tokens move through shared memory.  The activations stay in registers until they
+// are normalised, go to shared memory once, in pieces with their halves apart (scalar stores eight floats apart met in four
+// banks), and are read once for both rows.  Scalar staging, a pass per row -> now: 64 rows of 7168, four tokens 11.5 -> 9.0 us,
+// inside attn_prep_kernel 10.8 -> 7.8; one token 256 rows 5.9 -> 5.2.
 constexpr int kGemvBf16SmallThreads = 256;
 constexpr int kGemvBf16SmallRows = 2;
 
@@ -354,11 +358,8 @@ __device__ __forceinline__ void gemv_bf16_ksplit_body(const GemvBf16Params& p, i
     }
   }
   pdl_wait();
-  float ss[TOK];
-#pragma unroll
-  for (int t = 0; t < TOK; ++t) ss[t] = 0.f;
-  // all of this thread's activation loads first (k <= 8192: at most four per token), then the staging:
-  // a plain loop would pay one memory round trip per iteration
+  // all of this thread's activation loads first (k <= 8192: at most four pieces of eight per token) and, behind them, the gains of
+  // the same elements: a plain loop would pay one memory round trip per iteration
   uint4 xraw[4][TOK];
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
@@ -368,113 +369,116 @@ __device__ __forceinline__ void gemv_bf16_ksplit_body(const GemvBf16Params& p, i
       xraw[it][t] = (i < p.k && t < p.n_tokens) ? *reinterpret_cast<const uint4*>(p.x + t * p.x_stride + i)
                                                 : make_uint4(0, 0, 0, 0);
   }
+  auto piece_of = [&](int it, int t, float (&f)[8]) {
+    const uint32_t wv[4] = {xraw[it][t].x, xraw[it][t].y, xraw[it][t].z, xraw[it][t].w};
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int i = (it * kGemvBf16SmallThreads + threadIdx.x) * 8;
-    if (i < p.k) {
-#pragma unroll
-      for (int t = 0; t < TOK; ++t) {
-        const uint32_t wv[4] = {xraw[it][t].x, xraw[it][t].y, xraw[it][t].z, xraw[it][t].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float a = __uint_as_float(wv[j] << 16), b = __uint_as_float(wv[j] & 0xffff0000u);
-          xs[t * p.k + i + 2 * j] = a;
-          xs[t * p.k + i + 2 * j + 1] = b;
-          ss[t] += a * a + b * b;
-        }
-      }
+    for (int j = 0; j < 4; ++j) {
+      f[2 * j] = __uint_as_float(wv[j] << 16);
+      f[2 * j + 1] = __uint_as_float(wv[j] & 0xffff0000u);
     }
-  }
+  };
+  float rinv[TOK];
+  float4 gm[4][2];
   if (p.gamma != nullptr) {
-    // gains of this thread's elements (k <= 8192: at most 8 groups of 4), requested before the
-    // reduction so their latency hides behind it
-    float4 gm[8];
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int i = (it * kGemvBf16SmallThreads + threadIdx.x) * 4;
-      gm[it] = i < p.k ? __ldg(reinterpret_cast<const float4*>(p.gamma + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int it = 0; it < 4; ++it) {
+      const int i = (it * kGemvBf16SmallThreads + threadIdx.x) * 8;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        gm[it][h] = i < p.k ? __ldg(reinterpret_cast<const float4*>(p.gamma + i) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
-      const float s = warp_sum(ss[t]);
+      float ss = 0.f;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        float f[8];
+        piece_of(it, t, f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ss += f[2 * j] * f[2 * j] + f[2 * j + 1] * f[2 * j + 1];
+      }
+      const float s = warp_sum(ss);
       if (lane == 0) red[t][warp] = s;
     }
     __syncthreads();
-    float rinv[TOK];
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
       float tot = lane < 8 ? red[t][lane] : 0.f;
       tot = warp_sum(tot);
       rinv[t] = rsqrtf(tot / static_cast<float>(p.k) + p.eps);
     }
+  }
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int i = (it * kGemvBf16SmallThreads + threadIdx.x) * 4;
-      if (i < p.k) {
-        const float g4[4] = {gm[it].x, gm[it].y, gm[it].z, gm[it].w};
+  for (int it = 0; it < 4; ++it) {
+    const int piece = it * kGemvBf16SmallThreads + threadIdx.x, i = piece * 8;
+    if (i < p.k) {
 #pragma unroll
-        for (int t = 0; t < TOK; ++t) {
-          float4 xv = *reinterpret_cast<float4*>(&xs[t * p.k + i]);
-          float o[4] = {xv.x * rinv[t] * g4[0], xv.y * rinv[t] * g4[1], xv.z * rinv[t] * g4[2], xv.w * rinv[t] * g4[3]};
-          if (p.round_norm_bf16) {
+      for (int t = 0; t < TOK; ++t) {
+        float f[8];
+        piece_of(it, t, f);
+        if (p.gamma != nullptr) {
+          const float g[8] = {gm[it][0].x, gm[it][0].y, gm[it][0].z, gm[it][0].w, gm[it][1].x, gm[it][1].y, gm[it][1].z, gm[it][1].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] = bf2f(f2bf(o[j]));
+          for (int j = 0; j < 8; ++j) {
+            f[j] = f[j] * rinv[t] * g[j];
+            if (p.round_norm_bf16) f[j] = bf2f(f2bf(f[j]));
           }
-          *reinterpret_cast<float4*>(&xs[t * p.k + i]) = make_float4(o[0], o[1], o[2], o[3]);
           if (p.xnorm_out != nullptr && block == 0 && t < p.n_tokens) {
-            uint2 ob;
-            ob.x = pack_bf16x2(o[0], o[1]);
-            ob.y = pack_bf16x2(o[2], o[3]);
-            *reinterpret_cast<uint2*>(p.xnorm_out + t * p.xnorm_stride + i) = ob;
+            uint2* out = reinterpret_cast<uint2*>(p.xnorm_out + t * p.xnorm_stride + i);
+            out[0] = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+            out[1] = make_uint2(pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
           }
         }
+        GemvX<float>::put(reinterpret_cast<uint8_t*>(xs + t * p.k), p.k, piece, f);
       }
     }
   }
   __syncthreads();
 
+  float acc[kGemvBf16SmallRows][TOK];
 #pragma unroll
-  for (int r = 0; r < kGemvBf16SmallRows; ++r) {
-    const int row = block * kGemvBf16SmallRows + r;
-    float acc[TOK];
+  for (int r = 0; r < kGemvBf16SmallRows; ++r)
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) acc[t] = 0.f;
-    if (row < p.n) {
+    for (int t = 0; t < TOK; ++t) acc[r][t] = 0.f;
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int k0 = warp * kslice + lane * 8 + it * 256;
-        if (k0 < (warp + 1) * kslice) {
-          float wf[8];
-          if (p.w_is_f32) {
-            const uint4 w0 = wpre[r][it][0], w1 = wpre[r][it][1];
-            wf[0] = __uint_as_float(w0.x); wf[1] = __uint_as_float(w0.y); wf[2] = __uint_as_float(w0.z);
-            wf[3] = __uint_as_float(w0.w); wf[4] = __uint_as_float(w1.x); wf[5] = __uint_as_float(w1.y);
-            wf[6] = __uint_as_float(w1.z); wf[7] = __uint_as_float(w1.w);
-          } else {
-            const uint4 wv = wpre[r][it][0];
-            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+  for (int it = 0; it < 4; ++it) {
+    const int k0 = warp * kslice + lane * 8 + it * 256;
+    if (k0 < (warp + 1) * kslice) {
+      float wf[kGemvBf16SmallRows][8];  // (rows past the end: zeros)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              wf[2 * j] = __uint_as_float(ww[j] << 16);
-              wf[2 * j + 1] = __uint_as_float(ww[j] & 0xffff0000u);
-            }
-          }
+      for (int r = 0; r < kGemvBf16SmallRows; ++r) {
+        const uint4 w0 = wpre[r][it][0], w1 = wpre[r][it][1];
+        if (p.w_is_f32) {
+          wf[r][0] = __uint_as_float(w0.x); wf[r][1] = __uint_as_float(w0.y); wf[r][2] = __uint_as_float(w0.z);
+          wf[r][3] = __uint_as_float(w0.w); wf[r][4] = __uint_as_float(w1.x); wf[r][5] = __uint_as_float(w1.y);
+          wf[r][6] = __uint_as_float(w1.z); wf[r][7] = __uint_as_float(w1.w);
+        } else {
+          const uint32_t ww[4] = {w0.x, w0.y, w0.z, w0.w};
 #pragma unroll
-          for (int t = 0; t < TOK; ++t) {
-            const float4 xa = *reinterpret_cast<const float4*>(&xs[t * p.k + k0]);
-            const float4 xb = *reinterpret_cast<const float4*>(&xs[t * p.k + k0 + 4]);
-            acc[t] += wf[0] * xa.x + wf[1] * xa.y + wf[2] * xa.z + wf[3] * xa.w + wf[4] * xb.x + wf[5] * xb.y +
-                      wf[6] * xb.z + wf[7] * xb.w;
+          for (int j = 0; j < 4; ++j) {
+            wf[r][2 * j] = __uint_as_float(ww[j] << 16);
+            wf[r][2 * j + 1] = __uint_as_float(ww[j] & 0xffff0000u);
           }
         }
       }
-    }
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      const float s = warp_sum(acc[t]);
-      if (lane == 0) part[r][t][warp] = s;
+      for (int t = 0; t < TOK; ++t) {
+        float x[8];
+        GemvX<float>::get(reinterpret_cast<const uint8_t*>(xs + t * p.k), p.k, k0 / 8, x);
+#pragma unroll
+        for (int r = 0; r < kGemvBf16SmallRows; ++r)
+          acc[r][t] += wf[r][0] * x[0] + wf[r][1] * x[1] + wf[r][2] * x[2] + wf[r][3] * x[3] + wf[r][4] * x[4] + wf[r][5] * x[5] +
+                       wf[r][6] * x[6] + wf[r][7] * x[7];
+      }
     }
   }
+#pragma unroll
+  for (int r = 0; r < kGemvBf16SmallRows; ++r)
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+      const float s = warp_sum(acc[r][t]);
+      if (lane == 0) part[r][t][warp] = s;
+    }
   __syncthreads();
   if (threadIdx.x < kGemvBf16SmallRows * TOK) {
     const int r = threadIdx.x / TOK, t = threadIdx.x % TOK;
