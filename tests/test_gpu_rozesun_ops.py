@@ -334,3 +334,23 @@ def test_bad_sizes_are_refused(ops):
     with pytest.raises(tb.TilertError):
         ops.vec_gated(torch.zeros(8, device="cuda"), torch.zeros(2, 4, 8, dtype=BF16, device="cuda"), torch.zeros(4, device="cuda"), 4, 8, 1.0, ALPHA,
                       y=torch.zeros(8, device="cuda"))
+
+
+@pytest.mark.parametrize("heads,tokens", [(4, 1), (1, 20), (16, 37)])
+def test_scores_are_summed_along_the_row(ops, heads, tokens):
+    """One chain of products a score, sixteen columns after the other, whatever else the kernel's shape: 2^30 + 1 - 2^30 is 0 in
+    f32, and would be 1 with every other block of columns summed apart.  Exact."""
+    from tilert_b200.kv_cache import LatentCache
+
+    mix = mixer(WIDE, heads, 16, 16, 16, 16, 96, scale=1.0)
+    cache = LatentCache(mix.kv_rank, mix.rot_dim, None, 200, tokens, "cuda", BF16)
+    n, rankp = heads * tokens, ops.pad(mix.kv_rank, 16)
+    lat = torch.zeros(n, cache.rows.shape[1], device="cuda")
+    lat[:, 0] = lat[:, 32] = 2.0 ** 15
+    lat[:, 16] = 1.0
+    cache.rows.zero_()
+    cache.rows[:, 0], cache.rows[:, 16], cache.rows[:, 32] = 2.0 ** 15, 1.0, -(2.0 ** 15)
+    pos, part = torch.tensor([100], dtype=I32, device="cuda"), torch.zeros(n * (rankp + 2), device="cuda")
+    ops.latent_attn(lat, cache, tokens, mix, pos, 1, part)
+    largest, total = part[n * rankp:].view(heads, tokens, 2).unbind(-1)
+    assert bool((largest == 0).all()) and torch.equal(total, torch.arange(101.0, 101.0 + tokens, device="cuda").expand(heads, tokens))

@@ -6,10 +6,11 @@
 // exponentials; who reads them merges (latent_merge_kernel, or the staging of the value product of a one-token step).
 // Key tiles are copied two deep by cp.async; a tile is read twice, as keys and (its first rankp columns) as values.
 //
-// Sixteen warps sum the values, eight of them score, each in two chains of products.  Bound by latency at one token and, with 32
-// rows, by mma.sync (1088 a tile of 576 columns) and the barriers between its phases.  Eight warps for both, one chain -> now:
-// 37 tokens x 16 heads, 4037 keys of 512 + 64, seven parts 43.8 -> 42.4 us; 100 x 8, 1000 of 256 + 64 20.2 -> 14.9; one token, 32 heads,
-// 6000 keys 10.0 -> 9.1.  Sixteen warps that score eight keys each read the queries twice as often: 48 us at the first.
+// Sixteen warps sum the values, eight of them score, each score in one chain of products along the row (a sum in another order moves
+// the bf16 probabilities, and through four layers the outputs by 0.3 %).  Bound by latency at one token and, with 32 rows, by
+// mma.sync (1088 a tile of 576 columns) and the barriers between its phases.  Eight warps for both -> now: 37 tokens x 16 heads,
+// 4037 keys of 512 + 64, seven parts 43.7 -> 42.5 us; 100 x 8, 1000 of 256 + 64 19.3 -> 14.9; one token, 32 heads, 6000 keys 10.0 -> 9.2.
+// Sixteen warps that score eight keys each read the queries twice as often: 48 us at the first.
 #pragma once
 
 #include "act.cuh"
@@ -129,24 +130,24 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
     float* mxs = s_mx + buf * KG * M;
     float s[KW / 8][4];
     if (scores) {
-      float s2[KW / 8][4];  // every other sixteen columns: two chains of products
 #pragma unroll
       for (int i = 0; i < KW / 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = s2[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
 #pragma unroll 3
       for (int kk = 0; kk < row; kk += 32) {
-        uint32_t qa[2][4];
+        uint32_t qa[2][4], kb[KW / 8][4];  // eight keys each, four pieces of eight along the row
         ldmatrix_x4(qa[0], qs + (mt * 16 + (lane & 15)) * kp + kk + (lane >> 4) * 8);
         ldmatrix_x4(qa[1], qs + (mt * 16 + (lane & 15)) * kp + kk + 16 + (lane >> 4) * 8);
 #pragma unroll
-        for (int i = 0; i < KW / 8; ++i) {
-          uint32_t kb[4];  // eight keys, four pieces of eight along the row
-          ldmatrix_x4(kb, kt + (kg * KW + i * 8 + (lane & 7)) * kp + kk + (lane >> 3) * 8);
-          const uint32_t b0[2] = {kb[0], kb[1]}, b1[2] = {kb[2], kb[3]};
-          mma_bf16_16816(s[i], qa[0], b0);
-          mma_bf16_16816(s2[i], qa[1], b1);
-        }
+        for (int i = 0; i < KW / 8; ++i) ldmatrix_x4(kb[i], kt + (kg * KW + i * 8 + (lane & 7)) * kp + kk + (lane >> 3) * 8);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < KW / 8; ++i) {
+            const uint32_t b[2] = {kb[i][2 * h], kb[i][2 * h + 1]};
+            mma_bf16_16816(s[i], qa[h], b);
+          }
       }
       float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kLaThreads, 1) latent_attn_kernel(const Latent
         for (int j = 0; j < 4; ++j) {
           const int kpos = k0 + kg * KW + i * 8 + (lane & 3) * 2 + (j & 1), q = j >> 1;
           const bool ok = kpos < hi && kpos <= qpos[q] && qpos[q] - kpos < win;
-          s[i][j] = ok ? (s[i][j] + s2[i][j]) * a.scale : -INFINITY;
+          s[i][j] = ok ? s[i][j] * a.scale : -INFINITY;
           mx[q] = fmaxf(mx[q], s[i][j]);
         }
 #pragma unroll
