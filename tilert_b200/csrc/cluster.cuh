@@ -10,9 +10,20 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// All threads of the cluster; what they wrote before is visible behind it.
+// The barrier of all threads of the cluster in two halves; what they wrote ahead of the first is visible behind the second.  Another
+// CTA's shared memory may be touched only once that CTA is known to run: a kernel passes the barrier before its first such access,
+// the halves at its start and right ahead of that access, so that the wait costs nothing.  (Whole warps, converged.)
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 // shared::cluster address of a CTA's copy of a variable
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {

@@ -108,10 +108,11 @@ struct GreedyParams {
 };
 
 // The index of a row's largest value, the lowest of equal ones; a value that is no number counts as the largest of all.
-// Latency: four loads a thread at 32768 values on eight SMs.  A reduction on one SM, a copy of its result and a kernel that
-// advances the position took 11.6 us there and 29.3 at 129280 values, this launch 2.3 and 4.2.
+// Latency: two 16-byte loads a thread at 32768 values on eight SMs.  A reduction on one SM, a copy of its result and a kernel that
+// advances the position took 11.6 us there and 29.3 at 129280 values, this launch 2.2 and 4.0.
 __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kGreedyThreads) greedy_kernel(const GreedyParams p) {
   __shared__ unsigned long long s_warp[kGreedyThreads / 32], s_cta[kRowCtas];
+  cluster_arrive();
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, rank = static_cast<int>(cluster_rank()), tok = blockIdx.x / kRowCtas;
@@ -126,6 +127,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kGreedyThread
   const uint32_t first = __reduce_min_sync(0xffffffffu, key == best ? static_cast<uint32_t>(index) : 0x7fffffffu);
   if (lane == 0) s_warp[tid >> 5] = pair_of(best, static_cast<int>(first));
   __syncthreads();
+  cluster_wait();  // the first CTA runs
   if (tid == 0) {
     unsigned long long top = s_warp[0];
     for (int w = 1; w < kGreedyThreads / 32; ++w) top = max(top, s_warp[w]);
@@ -144,7 +146,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kGreedyThread
 // A row over a cluster of eight CTAs, its parts in shared memory (read again from L2 where they do not fit): the maximum, the
 // two sums and the counts of each digit meet over distributed shared memory, and the first CTA finds the digits, sorts the
 // candidates and picks.  Eleven bits a digit: with eight, nearly all of a vocabulary's logits count into the same few words.
-// Bound by the instructions of the passes, some ten cluster barriers and the sort: 16.6 us for 32768 values, 23.3 for 129280; the
+// Bound by the instructions of the passes, some ten cluster barriers and the sort: 15.8 us for 32768 values, 22.4 for 129280; the
 // same steps on one CTA a token took 47.5 and 138.
 __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kSampleThreads) sample_kernel(const SampleParams p) {
   extern __shared__ float s_part[];
@@ -155,6 +157,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kSampleThread
   __shared__ uint32_t s_digit[4];  // prefix, values equal to it that are wanted, as many as there are, whether all values are wanted
   __shared__ int s_mine, s_total, s_base, s_pick, s_keep;
   __shared__ float s_warp_tot[32];
+  cluster_arrive();
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -179,6 +182,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kSampleThread
   if (lane == 0) red[warp] = m;
   __syncthreads();
   m = warp_max(red[lane]);
+  cluster_wait();  // all CTAs run
   if (tid < kRowCtas) cluster_store(cluster_addr(&s_max[rank], tid), __float_as_uint(m));
   cluster_sync_all();
   m = s_max[0];
