@@ -804,7 +804,7 @@ extern "C" int tilert_expert_select_up_gate_silu_op(TbContext* ctx, const void* 
                                                     int* idx_out, int* slot_ids, float* slot_w, void* stream) {
   TB_REQUIRE(ctx != nullptr && hidden != nullptr && scores != nullptr && w_packed != nullptr);
   TB_REQUIRE(hidden_out != nullptr && probs_out != nullptr && idx_out != nullptr && tokens >= 1 && tokens <= 4);
-  TB_REQUIRE(n_experts <= 256 && top_k <= 31 && (n_groups == 1 || (32 % n_groups == 0 && n_experts % 32 == 0)));
+  TB_REQUIRE(n_experts <= 256 && top_k <= 31 && top_k <= n_experts && (n_groups == 1 || (32 % n_groups == 0 && n_experts % 32 == 0)));
   TB_REQUIRE((2 * inter) % TB_TILE_ROWS == 0 && dim % TB_KBLOCK == 0);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (slot_ids == nullptr) slot_ids = reinterpret_cast<int*>(ctx->small);

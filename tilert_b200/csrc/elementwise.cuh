@@ -205,8 +205,10 @@ __global__ void rotate128_kernel(const __nv_bfloat16* __restrict__ in, __nv_bflo
 // One warp per token; n_experts <= 256 (8 per lane).
 //   scores [tokens, n_experts] f32  ->  probs [tokens, top_k] f32, ids [tokens, top_k] i32,
 //   slot_ids [tokens, top_k + 1] i32 = (shared-expert id, ids...), slot_w [tokens, top_k + 1] = (1, probs...)
-// Routing of one token by one warp.  On return lane k (< top_k) holds the k-th selected expert in
-// `my_id` and its renormalised, scaled weight in `my_w`.
+// Routing of one token by one warp.  On return lane k (< top_k <= n_experts) holds the k-th selected expert in
+// `my_id` and its renormalised, scaled weight in `my_w`.  Weights are read at the ids, so they are distinct experts whatever the
+// scores are: a score that is no number counts as the largest, and where fewer than top_k are above minus infinity the lowest
+// of the others follow.
 __device__ __forceinline__ void expert_select_warp(const float* __restrict__ scores, const float* __restrict__ bias,
                                                    int n_experts, int n_groups, int n_limited, int top_k,
                                                    float route_scale, int& my_id, float& my_w) {
@@ -220,6 +222,7 @@ __device__ __forceinline__ void expert_select_warp(const float* __restrict__ sco
       const float s = 1.0f / (1.0f + expf(-__ldcg(scores + e)));
       orig[j] = s;
       sel[j] = bias != nullptr ? s + bias[e] : s;
+      if (sel[j] != sel[j]) sel[j] = INFINITY;
     } else {
       orig[j] = 0.f;
       sel[j] = -INFINITY;
@@ -263,7 +266,8 @@ __device__ __forceinline__ void expert_select_warp(const float* __restrict__ sco
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int e = lane * per_lane + j;
-      if (j < per_lane && e < n_experts && (sel[j] > best)) { best = sel[j]; best_e = e; }
+      // (a taken expert is marked by no number, which is neither above nor equal)
+      if (j < per_lane && e < n_experts && (sel[j] > best || (sel[j] == best && best_e == 0x7fffffff))) { best = sel[j]; best_e = e; }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -274,7 +278,7 @@ __device__ __forceinline__ void expert_select_warp(const float* __restrict__ sco
     float w = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      if (lane * per_lane + j == best_e) { w = orig[j]; sel[j] = -INFINITY; }
+      if (lane * per_lane + j == best_e) { w = orig[j]; sel[j] = __int_as_float(0x7fc00000); }
     }
     w = __shfl_sync(0xffffffffu, w, best_e / per_lane);
     wsum += w;
