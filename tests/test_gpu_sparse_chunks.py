@@ -78,3 +78,43 @@ def test_chunks_without_keys(ops, tokens, split, kind, pos):
         ops.flash_sparse_mla(args[0][:, t: t + 1].contiguous(), args[1][:, t: t + 1].contiguous(), args[2], args[3], args[4][:, t: t + 1].contiguous(), cur1,
                              lat1, softmax_scale=scale, split_size=split, out_acc=a1, lse_acc=l1, w_v=w_v, o_out=one)
         assert torch.equal(one[0, 0], o2[0, t])
+
+
+@pytest.mark.parametrize("tokens", [1, 4])
+@pytest.mark.parametrize("split", [64, 128])
+@pytest.mark.parametrize("kind", ["nan_row", "nan_alone", "nan_query", "inf_alone", "inf_row"])
+def test_what_is_no_number_is_not_lost(ops, tokens, split, kind):
+    """A cache row or a query with a NaN, or with an infinity that makes scores +inf (the result is no number) or -inf (no weight, but
+    its values are infinite), among other keys and alone in its chunk.  NaN where the plain f64 result has it, close elsewhere."""
+    heads, topk, rows, pos, scale = 40, 1280, 700, 600, 0.05  # (ten or twenty chunks: the merge's first batch and the next)
+    gen = torch.Generator().manual_seed(tokens)
+    q, qp, kv, pe = (torch.randn(*s, generator=gen).to(BF16) for s in ((1, tokens, heads, 512), (1, tokens, heads, 64), (1, rows, 512), (1, rows, 64)))
+    bad = 3
+    if kind == "nan_query":
+        q[0, 0, 1, 7] = float("nan")
+    elif kind.startswith("nan"):
+        kv[0, bad, 9] = float("nan")
+    else:
+        kv[0, bad, 9] = float("inf")
+    sel = torch.full((tokens, topk), -1, dtype=I32)
+    sel[:, :200] = torch.arange(10, 210, dtype=I32)
+    sel[:, 1279 if kind.endswith("alone") else 70] = bad
+    acc = torch.zeros(tokens, heads, topk // split, 512, device="cuda")
+    lse_acc, lse = torch.zeros(tokens, heads, topk // split, device="cuda"), torch.zeros(tokens, heads, device="cuda")
+    out, lat = (torch.zeros(1, tokens, heads, 512, dtype=BF16, device="cuda") for _ in range(2))
+    args = (q.cuda(), qp.cuda(), kv.cuda(), pe.cuda(), sel.view(1, tokens, topk).cuda(), torch.tensor([pos], dtype=I32, device="cuda"))
+    ops.flash_sparse_mla(*args, out, softmax_scale=scale, split_size=split, out_acc=acc, lse=lse, lse_acc=lse_acc)
+    w_v, o2 = torch.zeros(heads, 4, 16448, dtype=torch.uint8, device="cuda"), torch.zeros(1, tokens, heads, 128, dtype=BF16, device="cuda")
+    ops.flash_sparse_mla(*args, lat, softmax_scale=scale, split_size=split, out_acc=acc, lse_acc=lse_acc, w_v=w_v, o_out=o2)
+    for t in range(tokens):
+        ok = [int(i) for i in sel[t] if i >= 0]
+        k, p = kv[0, ok].to(F64), pe[0, ok].to(F64)
+        z = (q[0, t].to(F64) @ k.T + qp[0, t].to(F64) @ p.T) * scale
+        want, norm = torch.softmax(z, -1) @ k, torch.logsumexp(z, -1)
+        for got in (out, lat):
+            a = got[0, t].cpu().to(F64)
+            assert torch.equal(a.isnan(), want.isnan())
+            assert float((a - want).nan_to_num(0.0).abs().max()) <= 2.0 ** -7 * float(kv[kv.isfinite()].abs().max())
+        fine = norm.isfinite()
+        assert float((lse[t].cpu().to(F64) - norm)[fine].abs().max()) < 0.02 if bool(fine.any()) else True
+        assert bool(lse[t].cpu()[~fine].isnan().all()) and bool(want.isnan().any()) == (kind != "nan_query" or t == 0)

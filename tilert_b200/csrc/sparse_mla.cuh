@@ -7,7 +7,7 @@
 // second small kernel merges the chunks.  Algorithmic HBM traffic: topk x 1152 bytes per token.
 //
 // A position with fewer keys than topk leaves chunks without a valid row: their CTAs write what such a chunk contributes (zeros,
-// minus infinity) and go, and the merge does not read it.  Four rows behind 12 to 28 positions, 128 heads, 2048 selectable: 25 -> 12 us.
+// minus infinity) and go; the merge adds none of it, and behind its first batch of chunks does not read it.  Four rows behind 12 to 28 positions, 128 heads, 2048 selectable: 25 -> 12 us.
 #pragma once
 
 #include "common.cuh"
@@ -24,6 +24,10 @@ constexpr int kMlaPPitch = 72;   // bf16 elements per P row
 constexpr int kMlaThreads = 128;
 constexpr int kMlaSmemBytes =
     (kMlaHeads + kMlaKeys) * kMlaPitch * 2 + kMlaHeads * kMlaPPitch * 2 + 2 * 4 * kMlaHeads * 4 + kMlaKeys * 4 + 16;
+
+// Log-sum-exp of a chunk: minus infinity says that it holds no key, this that no key of it has a weight (all scores are minus
+// infinity), so that what such keys' values may be -- infinities, no numbers -- still reaches the sum.
+constexpr float kMlaNoWeight = -3.402823466e38f;
 
 struct MlaParams {
   const __nv_bfloat16* q_lat;   // [tokens, heads, 512]
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int r = j >> 1;
-        pv[j] = (m_new[r] == -INFINITY) ? 0.f : exp2f(s[n][j] - m_new[r]);
+        pv[j] = m_new[r] == -INFINITY && s[n][j] == s[n][j] ? 0.f : exp2f(s[n][j] - m_new[r]);  // (no number stays none)
         pv[j] = bf2f(f2bf(pv[j]));  // the sum uses the same rounded probabilities as P.V
         bsum[r] += pv[j];
       }
@@ -259,20 +263,21 @@ __global__ void __launch_bounds__(kMlaThreads) sparse_mla_kernel(const MlaParams
   for (int r = 0; r < 2; ++r) {
     const int head = hg * kMlaHeads + g + 8 * r;
     if (head >= p.heads) continue;
-    const float inv = l_run[r] > 0.f ? 1.f / l_run[r] : 0.f;
+    const float inv = l_run[r] == 0.f ? 0.f : 1.f / l_run[r];
     const long long base = (static_cast<long long>(tok) * p.heads + head) * p.n_splits + split;
     float* dst = p.o_acc + base * kMlaDV + warp * 128;
 #pragma unroll
     for (int n = 0; n < 16; ++n)
       *reinterpret_cast<float2*>(dst + n * 8 + 2 * qd) = make_float2(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
     if (warp == 0 && qd == 0)
-      p.lse_acc[base] = l_run[r] > 0.f ? m_run[r] * 0.6931471805599453f + logf(l_run[r]) : -INFINITY;
+      p.lse_acc[base] = l_run[r] == 0.f ? (phase > 0 ? kMlaNoWeight : -INFINITY) : m_run[r] * 0.6931471805599453f + logf(l_run[r]);
   }
 }
 
 constexpr int kMlaMergeTokens = 4;  // of a CTA at most: 128 threads each
 // o = sum_i exp(lse_i - lse) * o_i over the chunks of one (token, head), four columns a thread of 128; n_splits <= 64.  A chunk without
-// keys is marked by a negative weight and not added (what it left is not read beyond the first batch).
+// keys is marked by a negative weight and not added (what it left is not read beyond the first batch).  One whose sum is no number has no
+// number as its weight.
 struct MlaMerged {
   uint2 o;      // bf16
   float lse;
@@ -286,8 +291,8 @@ __device__ __forceinline__ MlaMerged mla_merge(const float* __restrict__ o_acc, 
     const int lane = threadIdx.x;
     const float l0 = lane < n_splits ? lse_acc[th * n_splits + lane] : -INFINITY;
     const float l1 = lane + 32 < n_splits ? lse_acc[th * n_splits + lane + 32] : -INFINITY;
-    const float mx = warp_max(fmaxf(l0, l1));
-    const float w0 = mx == -INFINITY ? 0.f : expf(l0 - mx), w1 = mx == -INFINITY ? 0.f : expf(l1 - mx);
+    const float top = warp_max(fmaxf(l0, l1)), mx = top <= kMlaNoWeight ? 0.f : top;
+    const float w0 = l0 <= kMlaNoWeight ? 0.f : expf(l0 - mx), w1 = l1 <= kMlaNoWeight ? 0.f : expf(l1 - mx);
     const float den = warp_sum(w0 + w1);
     s_w[lane] = l0 == -INFINITY ? -1.f : w0;
     s_w[lane + 32] = l1 == -INFINITY ? -1.f : w1;
@@ -325,8 +330,8 @@ __device__ __forceinline__ MlaMerged mla_merge(const float* __restrict__ o_acc, 
     for (int j = 0; j < kBatch; ++j) v[j] = nxt[j];
   }
   const float den = s_den[threadIdx.y];
-  const float inv = den > 0.f ? 1.f / den : 0.f;
-  return {make_uint2(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv)), den > 0.f ? s_mx[threadIdx.y] + logf(den) : -INFINITY};
+  const float inv = den == 0.f ? 0.f : 1.f / den;
+  return {make_uint2(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv)), den == 0.f ? -INFINITY : s_mx[threadIdx.y] + logf(den)};
 }
 
 // The merge alone.   grid = (heads, tokens), block = 128.
