@@ -378,7 +378,7 @@ int tilert_next_token_op(TbContext* ctx, const float* logits, long long logits_s
 
 /* What a pass begins with: x [n, dim] = rows `tokens` of table [vocab, dim] bf16 (a negative token counts from the end), freqs_out [n,
  * freq_len] = rows *pos .. *pos + n - 1 of freqs [positions, freq_len].  A token or position outside of its table is refused on the
- * device (status 4). */
+ * device: status 4, and both of its rows are filled with no numbers. */
 int tilert_step_inputs_op(TbContext* ctx, const long long* tokens, int n, const void* table, int vocab, int dim, const int* pos,
                           const float* freqs, int positions, int freq_len, void* x, float* freqs_out, void* stream);
 

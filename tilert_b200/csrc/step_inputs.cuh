@@ -21,7 +21,8 @@ struct StepInputsParams {
   int* status;
 };
 
-// grid = tokens.  A token or position outside of its table is refused: status 4, nothing is stored.
+// grid = tokens.  A token or position outside of its table is refused: status 4, and rows that are no number, so that nothing computed
+// from them passes for a result.
 __global__ void __launch_bounds__(kStepInputThreads) step_inputs_kernel(const StepInputsParams p) {
   pdl_launch_dependents();
   pdl_wait();
@@ -29,12 +30,15 @@ __global__ void __launch_bounds__(kStepInputThreads) step_inputs_kernel(const St
   long long tok = p.tokens[t];
   if (tok < 0) tok += p.vocab;
   const long long pos = static_cast<long long>(*p.pos) + t;
+  __nv_bfloat16* dst = p.x + static_cast<long long>(t) * p.dim;
   if (tok < 0 || tok >= p.vocab || pos < 0 || pos >= p.positions) {  // uniform over the CTA
     if (tid == 0) set_status(p.status, ST_BAD_ARGUMENT);
+    const float none = __int_as_float(0x7fc00000);
+    for (int i = tid; i < p.freq_len; i += kStepInputThreads) p.fr[t * p.freq_len + i] = none;
+    for (int i = tid; i < p.dim; i += kStepInputThreads) dst[i] = f2bf(none);
     return;
   }
   const __nv_bfloat16* src = p.table + tok * p.dim;
-  __nv_bfloat16* dst = p.x + static_cast<long long>(t) * p.dim;
   for (int i = tid; i < p.freq_len; i += kStepInputThreads) p.fr[t * p.freq_len + i] = p.freqs[pos * p.freq_len + i];
   if (p.dim % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.table) | reinterpret_cast<uintptr_t>(p.x)) & 15) == 0) {
 #pragma unroll 2

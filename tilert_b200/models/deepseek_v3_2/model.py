@@ -107,6 +107,15 @@ class DsaModel(SequenceDriver):
                 n = c0.shape[0] if end_pos is None else end_pos - start_pos
                 layer.inject_cache(c0[:n], c1[:n], c2[:n], start_pos)
 
+    def forward(self, token: int | torch.Tensor, pos: int) -> None:
+        """``SequenceDriver.forward``; a token outside of the vocabulary is refused, or, where only the device knows it, leaves NaN
+        logits and device status 4."""
+        if not isinstance(token, torch.Tensor):
+            ops.check_tokens([token], self.embed.shape[0])
+        elif not token.is_cuda:
+            ops.check_tokens(token.view(-1)[:1].tolist(), self.embed.shape[0])
+        super().forward(token, pos)
+
     def _step_ops(self, n_keys: int) -> None:
         x, fr = self.x_in, self.fr_in
         ops.step_inputs(self.token, self.embed, self.cur_pos, self.freqs, x, fr)

@@ -99,7 +99,7 @@ class MtpDsaModel:
         self._graphs: dict[tuple[str, int], torch.cuda.CUDAGraph] = {}
         # host copies: a chunk of a prompt is launched without waiting for the one before
         self.pos = 0
-        self._valid = 0
+        self._valid, self._extra = 0, 0
 
     # -- controls with the reference driver's names (end2end.py:551-577, 137-163) --
     def reset_sequence(self) -> None:
@@ -115,6 +115,7 @@ class MtpDsaModel:
 
     def set_prefill_mtp_extra_token(self, token: int) -> None:
         self.extra_token.fill_(token)
+        self._extra = token
 
     def get_num_accepted(self) -> int:
         return int(self.n_accepted.item())
@@ -221,16 +222,22 @@ class MtpDsaModel:
         """One speculative step for ``draft_tokens`` [4] at the current position (or one prefill chunk
         when ``set_prefill_valid_tokens`` was given a non-zero count), as ``ShowHandsDSALayer.forward``
         (end2end.py:551-558).  Results: ``get_num_accepted`` / ``get_predicted_tokens`` /
-        ``get_next_draft_tokens``."""
+        ``get_next_draft_tokens``.  A token outside of the vocabulary is refused, or, where only the device knows it, leaves
+        NaN logits in its row and device status 4."""
         if not with_mtp:
             raise ValueError("MtpDsaModel only runs the speculative path; use DsaModel for plain decoding")
         t = torch.as_tensor(draft_tokens, dtype=I64).view(-1)
+        if self._valid > 0 and not isinstance(self._extra, torch.Tensor):
+            ops.check_tokens([self._extra], self.embed.shape[0])
         if not t.is_cuda:
+            ops.check_tokens(t.tolist(), self.embed.shape[0])
             t = t.pin_memory().to(self.device, non_blocking=True)  # (from pageable memory the host would wait for the stream)
         if t.numel() != N_TOKENS:
             raise ValueError(f"draft_tokens must hold {N_TOKENS} tokens")
         if self.pos + 2 * N_TOKENS > self.cache_len:
             raise ValueError("position too close to the end of the caches")
+        if self.pos + N_TOKENS > self.freqs.shape[0]:
+            raise ValueError("position past the end of the rotary table")
         self.draft.copy_(t)
         if self._valid > 0:
             self._run("prefill")

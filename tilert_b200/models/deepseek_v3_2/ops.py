@@ -625,9 +625,16 @@ def next_token(logits, token_out, *, pos=None, advance=0, config=None, seed=0, s
                                              advance, _stream()))
 
 
+def check_tokens(tokens, vocab):
+    """Refuse token ids of the host outside of the vocabulary (negative ones count from the end)."""
+    for t in tokens:
+        if not -vocab <= t < vocab:
+            raise ValueError(f"token {t} is outside of the vocabulary of {vocab}")
+
+
 def step_inputs(tokens, table, cur_pos, freqs, x, freqs_out):
     """The embedding rows of ``tokens`` int64 [S] into ``x`` [1, S, dim] and the rotary rows of the positions from
-    ``cur_pos`` on into ``freqs_out`` [S, ...]."""
+    ``cur_pos`` on into ``freqs_out`` [S, ...].  What lies outside of a table becomes NaN, and device status 4."""
     _need(tokens, torch.int64, "tokens")
     _need(table, BF16, "table")
     _need(cur_pos, I32, "cur_pos")
