@@ -76,6 +76,10 @@ int tilert_gqa_gather_norm_op(TgContext* ctx, const float* x, long long ldx, con
 int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, int rows, const void* w, long long ldw, int n, int k,
                        int gated, float limit, float alpha, int n_groups, const int* counts, const float* bias, void* out,
                        long long ldo, int out_f32, int f32, void* stream);
+/* How such a product of bf16 rows is cut on a GPU of `sms` SMs: tile[3] = SMs on a tile (1 or 2), its features (of a gated product,
+ * pairs of a gate and an up row on two SMs, each of the two on one), its token rows.  counted: the groups' counts are on the device.
+ * Host code, no context. */
+int tilert_gqa_gemm_tile(int rows, int n, int k, int gated, int n_groups, int counted, int sms, int* tile);
 
 /* ---- attention of a portion of tokens ---- */
 

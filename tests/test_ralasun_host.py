@@ -9,7 +9,7 @@ import torch
 
 from oracle import ralasun as R
 from ralasun_models import CONFIGS, case, row_errors
-from tilert_b200 import _cabi, build, synthetic
+from tilert_b200 import _cabi, build, gqa_ops, synthetic
 from tilert_b200.kv_cache import RingKVCache
 from tilert_b200.models import registry
 from tilert_b200.models.driver import SequenceDriver
@@ -209,3 +209,15 @@ def test_trace_runner_refuses_a_type_the_family_does_not_run_in(tmp_path, monkey
     monkeypatch.setattr("sys.stdin", io.StringIO(""))
     assert trace_run.main(["--model", str(tmp_path), "--dtype", "float32", "--out", str(tmp_path)]) == 3
     assert "float32" in capsys.readouterr().err
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_small_groups_get_small_tiles(gated):
+    """Where the counts of the groups are on the device: tiles of 32 rows as long as those hold an average group and a fifth, also
+    with fewer rows than groups, if such tiles do not outnumber the SMs."""
+    tile = lambda rows, groups, n=1000: gqa_ops.gemm_tile(rows, n, 1024, gated=gated, n_groups=groups, counted=True)  # noqa: E731
+    for rows, groups in ((1, 1), (1, 30), (2, 3), (16, 30), (12, 64), (16, 16), (18, 1000)):
+        assert tile(rows, groups) == (1, 64, 32), (rows, groups)
+    assert tile(26 * 4, 4) == (1, 64, 32) and tile(28 * 4, 4) == (1, 64, 64) and tile(63 * 4, 4) == (1, 64, 64)
+    assert tile(16, 30, 1409) == (1, 128, 64)  # 16 groups of twelve tiles: more than the SMs
+    assert tile(64 * 4, 4) == (2, 128 if gated else 256, 96) and tile(300 * 4, 4)[2] == 256

@@ -154,6 +154,47 @@ int launch_single(TgContext* ctx, const GemmRowsParams& p, long long w_rows, int
   return bn == 32 ? launch_tc<64, 32, GATED>(ctx, p, w_rows, stream) : launch_tc<64, 64, GATED>(ctx, p, w_rows, stream);
 }
 
+// The tile of a product of bf16 rows: one SM (128 features x 64 token rows, 64 x 64 or 64 x 32) or a pair (256 x up to 256; gated
+// 128 pairs) on it, what takes the fewest rounds over the SMs, a round being the steps along K of a tile.  The microseconds of a
+// step of 64 are measured ones (2048 x 6208 x 4096, 1357 x 7168 x 18432, gated 1357 x 18432 x 7168 and others at every tile size,
+// 37 and 173 x 2048 x 2048 to 5632 on single SMs).  37 x 2048 x 5632: 11.8 us in tiles of 64 x 32, 14.1, 19.5 of 128 x 64, 19.1 in
+// pairs; 150 x 2048 x 1000: 7.6, 7.2, 7.9, 8.2; 64 x 16000 x 4096: 33.3, 28.7, 26.3, 27.4.
+struct RowTile {
+  bool pair;
+  int features, tokens;
+};
+RowTile row_tile(int rows, int n, int k, bool gated, int n_groups, bool counted, int sms) {
+  const int n_kb = (k + kTcK - 1) / kTcK, wide = n_groups > 0 ? n_groups : 1;
+  auto tiles = [&](int feats, int bn) { return static_cast<long long>(wide) * ((n + feats - 1) / feats) * ((rows + bn - 1) / bn); };
+  auto round_up = [](long long tiles, int units) { return static_cast<double>((tiles + units - 1) / units); };
+  if (n_groups > 0 && counted) {
+    // The counts are on the device: a tile that holds an average group and a fifth, or, above 213 rows a group, the largest, of
+    // which a group may need a second that it does not fill.  Below 64 rows a group it is the weights'
+    // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 114 us, in pairs 141; 75 rows
+    // 97 in pairs, was 120; 156 rows 303, 256 rows 440; gated, 1000 to 1536 features), in small tiles if the groups that
+    // there can be are few (16 rows over 30 experts 16.0 us, in tiles of 128 features 19.5), of 32 rows where those hold a group (97
+    // rows over 4, gated, 700 x 1024 13.9 -> 10.5 us; 16 over 16, gated, 500 x 1500 16.7 -> 14.4), as they do where there are
+    // fewer rows than groups.
+    const int each = rows > n_groups ? rows / n_groups : 1, bn = (each * 6 / 5 + 31) / 32 * 32;
+    if (each >= 64) return {true, gated ? 128 : 256, bn < 256 ? bn : 256};
+    const bool few = static_cast<long long>(rows < n_groups ? rows : n_groups) * ((n + 127) / 128) <= sms;
+    return few ? RowTile{false, 64, bn == 32 ? 32 : 64} : RowTile{false, 128, 64};
+  }
+  constexpr double kStep[] = {0.17, 0.19, 0.22, 0.295, 0.30, 0.335, 0.37};  // pairs: 64, 96, .. 256 rows
+  double pair = 1e30;
+  int bn = 0;
+  for (int i = 0; i < 7; ++i) {
+    const double c = round_up(tiles(gated ? 128 : 256, 64 + 32 * i), sms / 2) * n_kb * kStep[i] + 0.4;
+    if (c < pair) pair = c, bn = 64 + 32 * i;
+  }
+  if (gated) return {true, 128, bn};
+  const double large = round_up(tiles(128, 64), sms) * n_kb * 0.17, mid = round_up(tiles(64, 64), sms) * n_kb * 0.12,
+               small = round_up(tiles(64, 32), sms) * n_kb * 0.096;
+  if (pair < large && pair < mid && pair < small) return {true, 256, bn};
+  if (large < mid && large < small) return {false, 128, 64};
+  return {false, 64, small <= mid ? 32 : 64};
+}
+
 QkvShape qkv_shape(int heads, int kv_heads, int dim, int vdim, int ring, int window) {
   return {heads, kv_heads, dim, vdim, pad_to(dim, 16), pad_to(vdim, 16), ring, window};
 }
@@ -284,6 +325,15 @@ extern "C" int tilert_gqa_gather_norm_op(TgContext* ctx, const float* x, long lo
 }
 
 // ------------------------------------------------------------------------------- products
+extern "C" int tilert_gqa_gemm_tile(int rows, int n, int k, int gated, int n_groups, int counted, int sms, int* tile) {
+  TB_REQUIRE(rows >= 1 && n >= 1 && k >= 1 && n_groups >= 0 && n_groups <= kMaxGroups && sms >= 2 && tile != nullptr);
+  const RowTile t = row_tile(rows, n, k, gated != 0, n_groups, counted != 0, sms);
+  tile[0] = t.pair ? 2 : 1;
+  tile[1] = t.features;
+  tile[2] = t.tokens;
+  return TB_OK;
+}
+
 extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, int rows, const void* w, long long ldw, int n, int k,
                                   int gated, float limit, float alpha, int n_groups, const int* counts, const float* bias, void* out,
                                   long long ldo, int out_f32, int f32, void* stream) {
@@ -318,40 +368,9 @@ extern "C" int tilert_gqa_gemm_op(TgContext* ctx, const void* x, long long ldx, 
     return gated ? launch_f32<32, 32, 128, 8, true>(ctx, p, stream) : launch_f32<32, 32, 128, 16, false>(ctx, p, stream);
   }
   const long long w_rows = static_cast<long long>(n_groups > 0 ? n_groups : 1) * per * n;
-  // One SM (128 features x 64 token rows, 64 x 64 or 64 x 32) or a pair (256 x up to 256) on a tile: what takes the fewest rounds
-  // over the SMs, a round being the steps along K of a tile.  The microseconds of a step of 64 are measured ones (2048 x 6208 x
-  // 4096, 1357 x 7168 x 18432, gated 1357 x 18432 x 7168 and others at every tile size, 37 and 173 x 2048 x 2048 to 5632 on
-  // single SMs).  37 x 2048 x 5632: 11.8 us in tiles of 64 x 32, 14.1, 19.5 of 128 x 64, 19.1 in pairs; 150 x 2048 x 1000: 7.6, 7.2,
-  // 7.9, 8.2; 64 x 16000 x 4096: 33.3, 28.7, 26.3, 27.4.
-  const int n_kb = (p.k + kTcK - 1) / kTcK, wide = n_groups > 0 ? n_groups : 1;
-  auto tiles = [&](int feats, int bn) { return static_cast<long long>(wide) * ((n + feats - 1) / feats) * ((rows + bn - 1) / bn); };
-  auto round_up = [](long long tiles, int units) { return static_cast<double>((tiles + units - 1) / units); };
-  if (n_groups > 0 && counts != nullptr) {
-    // The counts are on the device: a tile that holds an average group and a fifth, or, above 213 rows a group, the largest, of
-    // which a group may need a second that it does not fill.  Below 64 rows a group it is the weights'
-    // stream that costs, and single SMs keep more of it on its way (16 rows each of 64 experts: 114 us, in pairs 141; 75 rows
-    // 97 in pairs, was 120; 156 rows 303, 256 rows 440; gated, 1000 to 1536 features), in small tiles if the groups that
-    // there can be are few (16 rows over 30 experts 16.0 us, in tiles of 128 features 19.5), of 32 rows where those hold a group (97
-    // rows over 4, gated, 700 x 1024 13.9 -> 10.5 us; 16 over 16, gated, 500 x 1500 16.7 -> 14.4).
-    const int each = rows / n_groups, bn = (each * 6 / 5 + 31) / 32 * 32;
-    if (each < 64) {
-      const int bm = static_cast<long long>(rows < n_groups ? rows : n_groups) * ((n + 127) / 128) <= ctx->num_sms ? 64 : 128;
-      return gated ? launch_single<true>(ctx, p, w_rows, bm, bn, stream) : launch_single<false>(ctx, p, w_rows, bm, bn, stream);
-    }
-    return gated ? launch_pair<true>(ctx, p, w_rows, bn < 256 ? bn : 256, stream) : launch_pair<false>(ctx, p, w_rows, bn < 256 ? bn : 256, stream);
-  }
-  constexpr double kStep[] = {0.17, 0.19, 0.22, 0.295, 0.30, 0.335, 0.37};  // pairs: 64, 96, .. 256 rows
-  double pair = 1e30;
-  int bn = 0;
-  for (int i = 0; i < 7; ++i) {
-    const double c = round_up(tiles(gated ? 128 : 256, 64 + 32 * i), ctx->num_sms / 2) * n_kb * kStep[i] + 0.4;
-    if (c < pair) pair = c, bn = 64 + 32 * i;
-  }
-  if (gated) return launch_pair<true>(ctx, p, w_rows, bn, stream);
-  const double large = round_up(tiles(128, 64), ctx->num_sms) * n_kb * 0.17, mid = round_up(tiles(64, 64), ctx->num_sms) * n_kb * 0.12,
-               small = round_up(tiles(64, 32), ctx->num_sms) * n_kb * 0.096;
-  if (pair < large && pair < mid && pair < small) return launch_pair<false>(ctx, p, w_rows, bn, stream);
-  return launch_single<false>(ctx, p, w_rows, large < mid && large < small ? 128 : 64, small <= mid ? 32 : 64, stream);
+  const RowTile t = row_tile(rows, n, k, gated, n_groups, counts != nullptr, ctx->num_sms);
+  if (t.pair) return gated ? launch_pair<true>(ctx, p, w_rows, t.tokens, stream) : launch_pair<false>(ctx, p, w_rows, t.tokens, stream);
+  return gated ? launch_single<true>(ctx, p, w_rows, t.features, t.tokens, stream) : launch_single<false>(ctx, p, w_rows, t.features, t.tokens, stream);
 }
 
 // ------------------------------------------------------------------------------- attention of a portion

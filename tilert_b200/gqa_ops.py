@@ -146,6 +146,13 @@ def gemm(x, w, out, rows: int, n: int, k: int, *, gated: tuple[float, float] | N
           _p(bias), _p(out), out.stride(-2), int(out.dtype == F32), f32)
 
 
+def gemm_tile(rows: int, n: int, k: int, *, gated: bool = False, n_groups: int = 0, counted: bool = False, sms: int = 148) -> tuple[int, int, int]:
+    """(SMs, features, token rows) of a tile of ``gemm`` on bf16 rows; needs no GPU."""
+    tile = (ctypes.c_int * 3)()
+    _tb.check(_tb.lib(_TYPE).tilert_gqa_gemm_tile(rows, n, k, int(gated), n_groups, int(counted), sms, ctypes.addressof(tile)), _TYPE)
+    return tuple(tile)
+
+
 # -- whole layers of a portion: a structure that a layer fills in once, and one call a layer --
 _HEADER = _cabi.header_path("tilert_gqa.h")
 RoutedLayer = _cabi.parse_struct("TgRoutedLayer", _HEADER)
