@@ -254,6 +254,7 @@ typedef struct TgLatentLayer {
   int dim;
   int f32;
   float eps;
+  int portion;            /* rows that cq, att, y and hid hold */
   int heads;
   int head_dim;
   int rot;
@@ -289,13 +290,16 @@ typedef struct TgLatentLayer {
   const float* norm2_gain;
   const float* norm2_bias;
   void* cache;
-  float* z;               /* work buffers for the rows of a call */
   void* cq;
-  float* q;
   void* att;
   float* y;
   void* hid;
-  void* qe;               /* expanded form: [rows, heads, pad16(head_dim) + pad16(rot)], [cached, rows of w_kv] */
+  int work_rows;          /* what the buffers behind hold: rows of a call, cache rows of kv, parts of the keys in part */
+  int work_cached;
+  int work_splits;
+  float* z;
+  float* q;
+  void* qe;               /* expanded form: [rows, heads, pad16(head_dim) + pad16(rot)], [cached, rows of w_kv]; else NULL */
   void* kv;
   void* qn;               /* absorbed form: [heads, rows, ..] of pad8(head_dim), a cache row, parts, pad8(kv_rank), pad8(vdim) */
   float* lat;
@@ -305,7 +309,8 @@ typedef struct TgLatentLayer {
 } TgLatentLayer;
 /* What the layer before left is settled first: x += norm(y) (+ add) where there is a y_gain, then n1.  The layer leaves its own last
  * output in layer->y in the same way, for norm n2b, or n1b without a feed-forward.  cached: rows of the cache in use for the expanded
- * form of the attention, 0 for the absorbed one on n_splits parts of the keys. */
+ * form of the attention, 0 for the absorbed one on n_splits parts of the keys.  More than the buffers hold, or a form without its
+ * buffers, is refused. */
 int tilert_gqa_latent_layer_op(TgContext* ctx, const TgLatentLayer* layer, int rows, int cached, int n_splits, const int* pos, float* x,
                                void* xh, const float* y, const float* y_gain, const float* y_bias, const float* add, void* stream);
 

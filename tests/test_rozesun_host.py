@@ -1,11 +1,13 @@
 """Host side of the Rozesun design, without a GPU: the restatement's own consistency, configuration, weights, registry,
 cache sizes and the choice of the attention's form."""
 
+import ctypes
 import json
 
 import pytest
 import torch
 
+import tilert_b200
 from oracle import rozesun as R
 from ralasun_models import row_errors
 from rozesun_models import CONFIGS, case
@@ -141,3 +143,51 @@ def test_rotation_table():
     t = gqa_ops.rotation_table(300.0, 6, 50, "cpu")
     a = torch.tensor([49 * 300.0 ** (-2 * i / 6) for i in range(3)], dtype=F64)
     assert t.shape == (50, 6) and torch.allclose(t[49].double(), torch.cat([torch.cos(a), torch.sin(a)]), atol=1e-7)
+
+
+def _latent(**fields):
+    """A native layer whose buffers are host memory: nothing that is refused looks at them."""
+    rows = torch.zeros(64, 64)
+    sizes = dict(dim=64, f32=0, eps=1e-6, portion=8, heads=2, head_dim=16, rot=8, vdim=16, q_rank=16, kv_rank=16, ring=32, scale=1.0, gate_rows=2, ff=0)
+    s = gqa_ops.structure(gqa_ops.LatentLayer, **(sizes | dict(w_kv=rows.to(torch.bfloat16), cache=rows.to(torch.bfloat16), cq=rows.to(torch.bfloat16),
+                                                               att=rows.to(torch.bfloat16), y=rows, z=rows, q=rows)))
+    for name in ("qe", "kv", "qn", "lat", "part", "c", "o"):
+        setattr(s, name, rows.data_ptr())
+    s.work_rows, s.work_cached, s.work_splits = 6, 24, 3
+    for name, value in fields.items():
+        setattr(s, name, value)
+    return s, rows
+
+
+@pytest.mark.parametrize("rows,cached,splits,fields", [
+    (9, 24, 0, {}), (7, 24, 0, {}), (6, 25, 0, {}), (6, 33, 0, {"work_cached": 40}), (6, 24, 0, {"kv": None}), (6, 24, 0, {"qe": None}), (6, 24, 0, {"f32": 1}),
+    (6, 24, 0, {"w_kv": None}), (7, 0, 3, {}), (6, 0, 4, {}), (6, 0, 0, {}), (6, 0, 3, {"part": None}), (6, 0, 3, {"lat": None}), (6, 0, 3, {"c": None}),
+    (6, 0, 3, {"cache": None}), (6, 0, 3, {"ff": 8}), (0, 24, 0, {})])
+def test_native_layer_refuses_more_than_its_buffers_hold(rows, cached, splits, fields):
+    """By the C entry, ahead of anything that needs a GPU (the context is an address that nothing reads)."""
+    lib = tilert_b200.load_backend("ralasun")
+    s, buf = _latent(**fields)
+    p = buf.data_ptr()
+    assert lib.tilert_gqa_latent_layer_op(p, ctypes.addressof(s), rows, cached, splits, p, p, p, None, None, None, None, None) == -2
+    assert lib.tilert_gqa_routed_layer_op(p, ctypes.addressof(gqa_ops.RoutedLayer(portion=8)), 9, p, p, p, None) == -2
+
+
+def test_native_layer_takes_tensors_of_the_declared_types():
+    f32, half, ints = torch.zeros(8, 64), torch.zeros(8, 64, dtype=torch.bfloat16), torch.zeros(8, dtype=torch.int32)
+    for f, t in ((0, half), (1, f32)):
+        s = gqa_ops.structure(gqa_ops.RoutedLayer, dim=64, f32=f, portion=8, w_qkv=half, q_gain=f32, q=t, ids=ints, w_o=None)
+        assert s.w_qkv == half.data_ptr() and s.q == t.data_ptr() and s.w_o is None
+    for name, t in (("w_qkv", f32), ("q_gain", half), ("q", f32), ("ids", f32), ("q", half.T), ("dim", f32), ("q", 5)):
+        with pytest.raises(ValueError, match=name):
+            gqa_ops.structure(gqa_ops.RoutedLayer, **{"f32": 0, name: t})
+    pos, x = torch.zeros(1, dtype=torch.int32), torch.zeros(8, 64)
+    routed, (latent, _) = gqa_ops.RoutedLayer(dim=64, portion=8), _latent()
+    norm = gqa_ops.Norm(torch.ones(64), centered=True)
+    for bad in ((pos.long(), x, half), (pos, half, half), (pos, x, x), (pos, x[:4], half), (pos, x, half[:, :56]), (pos, x[:, ::2], half)):
+        with pytest.raises(ValueError):
+            gqa_ops.routed_layer(routed, 6, *bad)
+        with pytest.raises(ValueError):
+            gqa_ops.latent_layer(latent, 6, 24, 0, *bad, x, norm, None)
+    for y, n, add in ((half, norm, None), (x, gqa_ops.Norm(torch.ones(64)), None), (None, norm, None), (x, norm, half)):
+        with pytest.raises(ValueError):
+            gqa_ops.latent_layer(latent, 6, 24, 0, pos, x, half, y, n, add)

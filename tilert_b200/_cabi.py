@@ -49,11 +49,14 @@ def parse_header(path: Path = HEADER) -> dict[str, tuple[object, list[object]]]:
 
 
 def parse_struct(name: str, path: Path) -> type[ctypes.Structure]:
-    """The ctypes twin of ``typedef struct name { ... } name;`` in the header (one field per declaration)."""
+    """The ctypes twin of ``typedef struct name { ... } name;`` in the header (one field per declaration); ``pointees`` are the
+    types that its pointers are declared with."""
     text = re.sub(r"/\*.*?\*/", " ", path.read_text(), flags=re.S)
     body = re.search(r"typedef struct " + name + r"\s*\{(.*?)\}\s*" + name + r"\s*;", text, flags=re.S).group(1)
-    fields = [(d.replace("*", " ").split()[-1], _ctype(d)) for d in body.split(";") if d.strip()]
-    return type(name, (ctypes.Structure,), {"_fields_": fields})
+    decls = [" ".join(d.split()) for d in body.split(";") if d.strip()]
+    named = [(d.replace("*", " ").split()[-1], d) for d in decls]
+    return type(name, (ctypes.Structure,), {"_fields_": [(n, _ctype(d)) for n, d in named],
+                                            "pointees": {n: d.split("*")[0].strip() for n, d in named if "*" in d}})
 
 
 def bind(lib_path: Path, header: Path = HEADER, exported_globally: bool = True) -> ctypes.CDLL:

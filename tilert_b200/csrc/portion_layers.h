@@ -51,8 +51,13 @@ extern "C" int tilert_gqa_routed_layer_op(TgContext* ctx, const TgRoutedLayer* l
 extern "C" int tilert_gqa_latent_layer_op(TgContext* ctx, const TgLatentLayer* layer, int rows, int cached, int n_splits, const int* pos, float* x,
                                           void* xh, const float* y, const float* y_gain, const float* y_bias, const float* add, void* stream) {
   TB_REQUIRE(ctx != nullptr && layer != nullptr && rows >= 1 && x != nullptr && xh != nullptr && cached >= 0);
-  TB_REQUIRE(cached == 0 || (layer->w_kv != nullptr && !layer->f32));
   const TgLatentLayer& l = *layer;
+  TB_REQUIRE(rows <= l.portion && rows <= l.work_rows && l.cache != nullptr && l.z != nullptr && l.cq != nullptr && l.q != nullptr && l.att != nullptr &&
+             l.y != nullptr && (l.ff == 0 || l.hid != nullptr));
+  if (cached > 0)
+    TB_REQUIRE(!l.f32 && l.w_kv != nullptr && l.qe != nullptr && l.kv != nullptr && cached <= l.work_cached && cached <= l.ring);
+  else
+    TB_REQUIRE(l.qn != nullptr && l.lat != nullptr && l.part != nullptr && l.c != nullptr && l.o != nullptr && n_splits >= 1 && n_splits <= l.work_splits);
   const int dimp = pad_to(l.dim, 8), n_att = l.heads * l.vdim, rankp = pad_to(l.kv_rank, 8);
   const int off_c = pad_to(l.q_rank, 8), off_r = off_c + rankp, off_g = off_r + pad_to(l.rot, 8), z_len = off_g + l.gate_rows, ldz = pad_to(z_len, 8);
   const int ldh = pad_to(l.head_dim, 8) + pad_to(l.rot, 8), per_head = l.gate_rows == l.heads;

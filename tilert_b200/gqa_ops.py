@@ -160,17 +160,47 @@ LatentLayer = _cabi.parse_struct("TgLatentLayer", _HEADER)
 
 
 def structure(kind: type[ctypes.Structure], **fields) -> ctypes.Structure:
-    """A structure with tensors as their addresses (None: null); it keeps them alive."""
+    """A structure with tensors as their addresses (None: null); it keeps them alive.  They have the types that the header declares: bf16
+    where it has ``const void*`` (weights), activations where it has ``void*``."""
+    act = F32 if fields["f32"] else BF16
+    types = {"float": F32, "int": I32, "const void": BF16, "void": act}
+    for n, v in fields.items():
+        want = kind.pointees.get(n)
+        if v is None or want is None and not isinstance(v, torch.Tensor):
+            continue
+        if want is None or not isinstance(v, torch.Tensor):
+            raise ValueError(f"{n}: {'a tensor' if want else 'no tensor'} is wanted")
+        want = types.get(want) or types[want.removeprefix("const ")]
+        if v.dtype != want or not v.is_contiguous():
+            raise ValueError(f"{n} must be a contiguous {want} tensor, got {v.dtype} strides {tuple(v.stride())}")
     made = kind(**{n: v.data_ptr() if isinstance(v, torch.Tensor) else v for n, v in fields.items() if v is not None})
     made.tensors = [v for v in fields.values() if isinstance(v, torch.Tensor)]
     return made
 
 
+def _rows_of_layer(layer, rows: int, pos, x, xh) -> None:
+    """What a native layer takes for granted of its caller's tensors."""
+    _need("x", x, F32)
+    _need("pos", pos, I32)
+    if xh.dtype != (F32 if layer.f32 else BF16):
+        raise ValueError(f"xh must hold the layer's activations, got {xh.dtype}")
+    for name, t in (("x", x), ("xh", xh)):
+        if t.dim() != 2 or t.shape[0] < rows or t.shape[1] != pad(layer.dim) or not t.is_contiguous():
+            raise ValueError(f"{name} must be [{rows} or more, {pad(layer.dim)}], got {tuple(t.shape)} strides {tuple(t.stride())}")
+
+
 def routed_layer(layer, rows: int, pos, x, xh) -> None:
+    _rows_of_layer(layer, rows, pos, x, xh)
     _call("routed_layer", x, ctypes.addressof(layer), rows, _p(pos), _p(x), _p(xh))
 
 
 def latent_layer(layer, rows: int, cached: int, n_splits: int, pos, x, xh, y, norm, add) -> None:
+    _rows_of_layer(layer, rows, pos, x, xh)
+    if norm is not None:
+        _need("y", y, F32)
+        if not norm.centered:
+            raise ValueError("the norms of a latent layer are layer norms")
+    _need("add", add, F32, optional=True)
     gain, bias = (None, None) if norm is None else (_p(norm.gain), _p(norm.bias))
     _call("latent_layer", x, ctypes.addressof(layer), rows, cached, n_splits, _p(pos), _p(x), _p(xh), _p(y), gain, bias, _p(add))
 

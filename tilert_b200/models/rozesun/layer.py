@@ -152,8 +152,10 @@ class RozesunLayer:
             self._native = self._structure()
         s, length = self._native, pos + n
         s.cache = cache.rows.data_ptr()
+        s.work_rows = n
         s.z = sc.room("z", n * pad(self.z_len))
         s.q = sc.room("q", n * m.heads * self.ldh)
+        s.qe = s.kv = s.qn = s.lat = s.part = s.c = s.o = None  # (of the form that is taken, below)
         cached, n_splits = min(length, cache.ring), 0
         if w.kv is not None and expansion_pays(m, n, min(length, cache.window or length), cached):
             s.qe = sc.room("qe", hn * (pad(m.dim, 16) + pad(m.rot_dim, 16)), t)
@@ -165,6 +167,7 @@ class RozesunLayer:
             s.part = sc.room("part", hn * n_splits * (pad(m.kv_rank, 16) + 2))
             s.c = sc.room("c", hn * pad(m.kv_rank), t)
             s.o = sc.room("o", hn * pad(m.vdim))
+        s.work_cached, s.work_splits = cached, n_splits
         p = st.pending
         ops.latent_layer(s, n, cached, n_splits, cur_pos, st.x, st.xh, None if p is None else p.y, None if p is None else p.norm, st.add)
         st.add = None
@@ -175,7 +178,7 @@ class RozesunLayer:
 
     def _structure(self):
         m, f, w, sc, p, t = self.a.mixer, self.a.mlp, self.w, self.sc, self.portion, self.dtype
-        fields = dict(dim=self.args.dim, f32=int(t is F32), eps=self.args.eps, heads=m.heads, head_dim=m.dim, rot=m.rot_dim, vdim=m.vdim, q_rank=m.q_rank,
+        fields = dict(dim=self.args.dim, f32=int(t is F32), eps=self.args.eps, portion=p, heads=m.heads, head_dim=m.dim, rot=m.rot_dim, vdim=m.vdim, q_rank=m.q_rank,
                       kv_rank=m.kv_rank, window=self.caches[0].window, ring=self.caches[0].ring, scale=m.scale, gate_rows=m.gate_rows,
                       rope=self.rope.table, positions=self.rope.table.shape[0], rope_dims=self.rope.table.shape[1], interleaved=int(self.rope.interleaved),
                       w_z=w.z, q_gain=w.q_gain, c_gain=w.c_gain, w_uq=w.uq, w_uk_t=w.uk_t, w_kv=w.kv, w_uv=w.uv, sink=w.sink, w_o=w.o,
