@@ -155,6 +155,21 @@ def test_shared_driver_positions_prefill_and_generation():
         m.forward(1, 50)
 
 
+def test_shared_driver_without_an_operator_does_not_sample():
+    class Moving(Counting):
+        def _step_ops(self, key):
+            self.logits.zero_()
+            self.logits[0, 0, 6] = 1.0
+            self._choose(self.logits.view(1, -1), 1)
+
+    m = Moving()
+    m.forward(2, 0)
+    assert int(m.token_out) == 6 and int(m.cur_pos) == 1
+    m.set_sampling(temperature=0.7)
+    with pytest.raises(NotImplementedError):
+        m.forward(2, 1)
+
+
 def test_shared_generator_loop():
     class Gen(SequenceGenerator):
         def __init__(self, m):

@@ -53,7 +53,7 @@ class SequenceDriver:
         raise NotImplementedError
 
     def _next_token_op(self):
-        """The operator that ends a step on the device; None: torch's arg-max."""
+        """The operator that ends a step on the device; None: torch's arg-max, for a driver that does not sample."""
         return None
 
     # -- reference driver controls (end2end.py:551-577) --
@@ -91,6 +91,8 @@ class SequenceDriver:
         """The next token of ``logits`` [1, vocab] into ``token_out``, and the device position moved on."""
         op = self._next_token_op()
         if op is None:
+            if self.sampling:
+                raise NotImplementedError("this driver has no operator that samples")
             self.token_out.copy_(torch.argmax(logits.view(-1)))
             self.cur_pos += advance
             return
