@@ -66,3 +66,30 @@ def test_rows_of_one_value(ops, fill):
     top, ids = torch.zeros(1, 256, device="cuda"), torch.zeros(1, 256, dtype=torch.int32, device="cuda")
     ops.sample(logits, torch.tensor([0.0, 1.0, 0.0, 0.0], device="cuda"), tok, topn_logprobs=top, topn_indices=ids)
     assert ids[0].tolist() == list(range(256)) and int(tok) == 0
+
+
+@pytest.mark.parametrize("vocab", [3, 1025, 33333, 262144, 262177, 300000])
+def test_sampled_token_by_the_restated_rule(ops, vocab):
+    """Rows kept in shared memory (up to 262144 values) and read again from memory (beyond) against the f64 restatement: the token that
+    the same uniform number falls to, the 256 largest, their log-probabilities.  The sums have f32 exponentials of differences up to
+    20 (an error of 2^-20 each, relative) in eight parts: bounds of 1e-4 and 2e-4, as for one part in test_gpu_ops.py."""
+    from oracle import ops as oo
+
+    gen = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(2, vocab, generator=gen) * 2.5
+    logits[1, vocab // 2:] = logits[1, vocab // 2:].round()  # ties, across the CTAs' parts
+    tok, lp = torch.zeros(2, dtype=torch.int64, device="cuda"), torch.zeros(2, device="cuda")
+    one, top, ids = torch.zeros(2, dtype=torch.int32, device="cuda"), torch.zeros(2, 256, device="cuda"), torch.zeros(2, 256, dtype=torch.int32, device="cuda")
+    for cfg, seed in (((0.0, 1.0, 0.0, 0.0), 1), ((1.0, 1.0, 50.0, 0.0), 2), ((0.7, 0.9, 0.0, 1.0), 3), ((1.3, 0.5, 40.0, 1.0), 4), ((1.0, 1.0, 0.0, 0.0), 5)):
+        step = torch.tensor([11, 0], device="cuda")
+        ops.next_token(logits.cuda(), tok, config=torch.tensor(cfg, device="cuda"), seed=seed, step=step, sampled=one, token_logprob=lp, topn_logprobs=top,
+                       topn_indices=ids)
+        assert step.tolist() == [12, 0] and one.tolist() == tok.tolist()
+        for t in range(2):
+            order, bounds, logp = oo.sample_intervals(logits[t], cfg[0], cfg[1], int(cfg[2]), cfg[3] != 0)
+            all_ids = torch.argsort(-logits[t].double(), stable=True)[:1024]
+            got, u, n = int(tok[t]), oo.sample_uniform(seed, 11, t), min(256, vocab)
+            j = int((order == got).nonzero()[0])
+            assert j == 0 if cfg[0] == 0.0 else (float(bounds[j - 1]) if j else 0.0) - 1e-4 <= u < float(bounds[j]) + 1e-4
+            assert ids[t, :n].tolist() == all_ids[:n].tolist() and bool((ids[t, n:] == -1).all())
+            assert float((top[t, :n].cpu().double() - logp[:n]).abs().max()) < 2e-4 and abs(float(lp[t]) - float(logp[(all_ids == got).nonzero()[0]])) < 2e-4

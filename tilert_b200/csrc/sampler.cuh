@@ -145,7 +145,9 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kGreedyThread
 // ------------------------------------------------------------------ sampling
 // A row over a cluster of eight CTAs, its parts in shared memory (read again from L2 where they do not fit): the maximum, the
 // two sums and the counts of each digit meet over distributed shared memory, and the first CTA finds the digits, sorts the
-// candidates and picks.  Eleven bits a digit: with eight, nearly all of a vocabulary's logits count into the same few words.
+// candidates and picks.  The sums are those of the parts, added in the parts' order: log-probabilities and the ends of a nucleus have
+// last bits of their own, the order of the candidates has none.  Eleven bits a digit: with eight, nearly all of a vocabulary's logits
+// count into the same few words.
 // Bound by the instructions of the passes, some ten cluster barriers and the sort: 15.8 us for 32768 values, 22.4 for 129280; the
 // same steps on one CTA a token took 47.5 and 138.
 __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kSampleThreads) sample_kernel(const SampleParams p) {

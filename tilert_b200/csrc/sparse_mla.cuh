@@ -7,7 +7,8 @@
 // second small kernel merges the chunks.  Algorithmic HBM traffic: topk x 1152 bytes per token.
 //
 // A position with fewer keys than topk leaves chunks without a valid row: their CTAs write what such a chunk contributes (zeros,
-// minus infinity) and go; the merge adds none of it, and behind its first batch of chunks does not read it.  Four rows behind 12 to 28 positions, 128 heads, 2048 selectable: 25 -> 12 us.
+// minus infinity) and go; the merge adds none of it, and behind its first batch of chunks does not read it.  Four rows behind
+// 12 to 28 positions, 128 heads, 2048 selectable: 25 -> 12 us.
 #pragma once
 
 #include "common.cuh"
