@@ -114,3 +114,13 @@ def test_forms_have_the_same_bits(ops, gated, out_type):
 @pytest.mark.parametrize("n,k", [(300, 200), (640, 72)])
 def test_short_last_tiles_of_groups(ops, n, k, counts, gated):
     check(ops, n, k, gated, BF16, counts)
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("n,k", [(7, 8), (130, 264)])
+@pytest.mark.parametrize("counts", [[0] * 20 + [33] + [0] * 19, [1, 0, 1] * 7, [0, 64] + [0] * 70])
+def test_fewer_rows_than_groups(ops, n, k, counts, gated):
+    """Tiles of 32 rows, of which a group may need two."""
+    rows = sum(counts)
+    assert ops.gemm_tile(rows, n, k, gated=gated, n_groups=len(counts), counted=True)[1:] == (64, 32)
+    check(ops, n, k, gated, BF16, counts)
