@@ -12,7 +12,7 @@ from ralasun_models import CONFIGS, case, row_errors
 from tilert_b200 import _cabi, build, gqa_ops, synthetic
 from tilert_b200.kv_cache import RingKVCache
 from tilert_b200.models import registry
-from tilert_b200.models.driver import SequenceDriver
+from tilert_b200.models.driver import PortionDriver, SequenceDriver
 from tilert_b200.models.generator import SequenceGenerator
 from tilert_b200.models.ralasun.layer import LayerWeights
 from tilert_b200.models.ralasun.model_args import RalasunArgs
@@ -168,6 +168,31 @@ def test_shared_driver_without_an_operator_does_not_sample():
     m.set_sampling(temperature=0.7)
     with pytest.raises(NotImplementedError):
         m.forward(2, 1)
+
+
+def test_portions_choose_once_a_prompt():
+    """At the end of a prompt, an empty one too, and the position moves by its tokens."""
+    class Portions(PortionDriver):
+        position_limit, portion, max_window = Counting.position_limit, 4, 8
+
+        def __init__(self):
+            self._init_sequence("cpu", 8, use_graph=False)
+            self.limit, self.chosen = 50, 0
+
+        def _prefill_portion(self, tokens, want, last):
+            self.logits.zero_()
+            self.logits[0, 0, tokens[-1]] = 1.0
+            return torch.zeros(len(want), 8)
+
+        def _choose(self, logits, advance=0):
+            self.chosen += 1
+            super()._choose(logits, advance)
+
+    m = Portions()
+    m.prefill([1, 2, 3, 4, 5, 6])
+    assert (m.chosen, int(m.token_out), int(m.cur_pos), m._pos) == (1, 6, 6, 6)
+    m.logits[0, 0, 3] = 2.0
+    assert m.prefill([]).shape == (1, 8) and (m.chosen, int(m.token_out), int(m.cur_pos), m._pos) == (2, 3, 6, 6)
 
 
 def test_shared_generator_loop():

@@ -209,4 +209,6 @@ class PortionDriver(SequenceDriver):
                 self._choose(self.logits.view(1, -1), len(part))
             else:
                 self.cur_pos += len(part)
+        if not tokens:  # (the next token of the logits that there are, as at any prompt's end)
+            self._choose(self.logits.view(1, -1))
         return self.logits.view(1, -1).clone() if want is None else torch.cat(outs)
