@@ -1,5 +1,5 @@
 // Radix selection of the k largest values of one row by one CTA, on the order-preserving unsigned image of
-// f32: exact, equal values by lower index first.  The token sampler uses the same image of a value.
+// f32: exact, equal values by lower index first.  The token sampler and the routing use the same image of a value.
 #pragma once
 
 #include "common.cuh"
